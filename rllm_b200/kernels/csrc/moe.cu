@@ -253,9 +253,12 @@ moe_sort_kernel(const int* ids, int P, int E, int bm, int* offsets,
   for (int e = threadIdx.x; e <= E; e += blockDim.x) offsets[e] = start[e];
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     const int n = tstart[e + 1] - tstart[e];
+    // tiles of 128 (moe_tcgen05.cu) may be any multiple of 16 pairs up to that: an expert's tiles get equal shares, so
+    // that none is left with a few pairs behind a whole pass over the weights
+    const int rows = bm == 128 && n > 0 ? ((cnt[e] + n - 1) / n + 15) / 16 * 16 : bm;
     for (int i = 0; i < n; ++i) {
       tile_expert[tstart[e] + i] = e;
-      tile_row0[tstart[e] + i] = start[e] + i * bm;
+      tile_row0[tstart[e] + i] = start[e] + i * rows;
     }
   }
   for (int p = threadIdx.x; p < P; p += blockDim.x) {
@@ -267,7 +270,7 @@ moe_sort_kernel(const int* ids, int P, int E, int bm, int* offsets,
 RLLM_EXPORT int rllm_moe_sort(const int* ids, int P, int E, int bm, int* offsets, int* sorted, int* tile_expert,
                               int* tile_row0, int* meta, cudaStream_t stream) {
   if (P <= 0) return 0;
-  if (E <= 0 || E > 2048 || (bm != 16 && bm != 64)) return RLLM_E_BADARG;
+  if (E <= 0 || E > 2048 || (bm != 16 && bm != 64 && bm != 128)) return RLLM_E_BADARG;
   const size_t smem = (size_t)(4 * E + 2) * sizeof(int);
   rllm_launch_pdl(moe_sort_kernel, dim3(1), dim3(1024), (size_t)(smem), stream, ids, P, E, bm, offsets, sorted, tile_expert, tile_row0, meta);
   RLLM_LAUNCH_CHECK();

@@ -986,6 +986,19 @@ def latent_attention_mma(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor
 # routed experts (moe.cu)
 # ---------------------------------------------------------------------------
 MOE_SMALL_PAIRS = 64      # up to this many (token, expert) pairs a step the expert products use row tiles of 16
+MOE_TCGEN05_FROM = 65     # from this many pairs on they run on the tcgen05 kernels (tiles of up to 128 pairs); below,
+                          # one 16-row tile an expert streams the weights as fast (64 pairs over 32 experts of
+                          # 2048 x 1024: 81 us; 68 pairs: 121 us in tiles of 64, 75 us on tcgen05)
+
+
+def moe_tcgen05_takes(pairs: int, h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor) -> bool:
+    """Whether the experts' products of this many (token, expert) pairs run on the tcgen05 kernels: bfloat16, sizes
+    and pointers that TMA takes.  RLLM_TILE_GEMM=simt and RLLM_GEMM=library|no_tcgen05 keep them off."""
+    import os
+    return (pairs >= MOE_TCGEN05_FROM and h.dtype is torch.bfloat16 and h.shape[1] % 8 == 0 and w_down.shape[2] % 8 == 0
+            and (h.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16 == 0
+            and not os.environ.get("RLLM_TILE_GEMM", "").startswith("s")
+            and os.environ.get("RLLM_GEMM") not in ("library", "no_tcgen05"))
 
 
 def moe_route(h: torch.Tensor, w_router: torch.Tensor, top: int):
@@ -1034,7 +1047,10 @@ def moe_experts(h: torch.Tensor, ids: torch.Tensor, w_gate_up: torch.Tensor, w_d
     assert w_gate_up.dtype is h.dtype and w_down.dtype is h.dtype and ids.dtype is torch.int32
     _contig(h, "h"); _contig(w_gate_up, "w_gate_up"); _contig(w_down, "w_down"); _contig(ids, "ids")
     P = T * top
-    bm = 16 if P <= MOE_SMALL_PAIRS else 64
+    y = torch.empty((P, F), dtype=h.dtype, device=h.device)
+    out = torch.empty((P, H), dtype=h.dtype, device=h.device)
+    tcgen05 = moe_tcgen05_takes(P, h, w_gate_up, w_down)
+    bm = 128 if tcgen05 else (16 if P <= MOE_SMALL_PAIRS else 64)
     max_tiles = min(P, -(-P // bm) + E)
     meta = torch.empty(1 + (E + 1) + P + 2 * max_tiles, dtype=torch.int32, device=h.device)
     m_tiles, offsets, sorted_pairs = meta[0:1], meta[1:E + 2], meta[E + 2:E + 2 + P]
@@ -1042,8 +1058,14 @@ def moe_experts(h: torch.Tensor, ids: torch.Tensor, w_gate_up: torch.Tensor, w_d
     tile_row0 = meta[E + 2 + P + max_tiles:]
     _check(lib.rllm_moe_sort(_ptr(ids), c_int(P), c_int(E), c_int(bm), _ptr(offsets), _ptr(sorted_pairs),
                              _ptr(tile_expert), _ptr(tile_row0), _ptr(m_tiles), _stream()), "moe_sort")
-    y = torch.empty((P, F), dtype=h.dtype, device=h.device)
-    out = torch.empty((P, H), dtype=h.dtype, device=h.device)
+    if tcgen05:
+        lib = build.load_library("moe_tcgen05")
+        _check(lib.rllm_moe_experts_tcgen05(
+            _ptr(h), _ptr(w_gate_up), _ptr(w_down), _ptr(y), _ptr(out), _ptr(offsets), _ptr(sorted_pairs),
+            _ptr(tile_expert), _ptr(tile_row0), _ptr(m_tiles), c_int(max_tiles), c_int(P), c_int(E), c_int(H), c_int(F),
+            c_int(top), c_float(limit), c_float(alpha), c_float(up_shift), _ptr(gemm_error_word(h.device)), _stream()),
+            "moe_experts_tcgen05")
+        return out
     _check(lib.rllm_moe_experts(_ptr(h), _ptr(w_gate_up), _ptr(w_down), _ptr(y), _ptr(out), _ptr(offsets),
                                 _ptr(sorted_pairs), _ptr(tile_expert), _ptr(tile_row0), _ptr(m_tiles),
                                 c_int(max_tiles), c_int(bm), c_int(H), c_int(F), c_int(top), c_float(limit),
