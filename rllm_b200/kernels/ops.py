@@ -426,33 +426,24 @@ def _sample_asserts(logits, temperature, top_k, top_p, min_p, seeds, gen_index, 
     assert seeds.dtype is torch.int64 and gen_index.dtype is torch.int64 and out.dtype is torch.int32
 
 
-_sample_scratch = {}
-
-
 def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor, top_p: torch.Tensor,
            min_p: torch.Tensor, seeds: torch.Tensor, gen_index: torch.Tensor, out: torch.Tensor,
            with_select: bool = True) -> None:
     """out[r] = the next token of row r: argmax for greedy rows, else a draw after temperature, top-k,
-    top-p and min-p.  Every row is worked on by several CTAs, in a chain of small kernels.
-    ``with_select=False`` leaves the top-k / top-p kernels out (the caller knows that no row uses them)."""
+    top-p and min-p.  A cluster of CTAs works on every row.
+    ``with_select=False`` leaves top-k and top-p out (the caller knows that no row uses them)."""
     lib = build.load_library("sampling")
     R, V = logits.shape
     _sample_asserts(logits, temperature, top_k, top_p, min_p, seeds, gen_index, out)
-    lib.rllm_sample_scratch_bytes.restype = c_longlong
-    need = int(lib.rllm_sample_scratch_bytes(c_int(R), c_int(V)))
-    scratch = _sample_scratch.get(logits.device)
-    if scratch is None or scratch.numel() < need:
-        scratch = torch.empty(max(need, 1 << 20), dtype=torch.uint8, device=logits.device)
-        _sample_scratch[logits.device] = scratch
     _check(lib.rllm_sample(_ptr(logits), c_int(R), c_int(V), c_int(logits.stride(0)), _ptr(temperature),
                            _ptr(top_k), _ptr(top_p), _ptr(min_p), _ptr(seeds), _ptr(gen_index), _ptr(out),
-                           _ptr(scratch), c_int(1 if with_select else 0), _stream()), "sample")
+                           c_int(1 if with_select else 0), _stream()), "sample")
 
 
 def sample_one_cta(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor, top_p: torch.Tensor,
                    min_p: torch.Tensor, seeds: torch.Tensor, gen_index: torch.Tensor, out: torch.Tensor) -> None:
     """The same sampling with one CTA a row in one kernel (slow for large vocabularies; kept as the
-    simple form that the chain of kernels is checked against)."""
+    simple form that the clusters are checked against)."""
     lib = build.load_library("sampling")
     R, V = logits.shape
     _sample_asserts(logits, temperature, top_k, top_p, min_p, seeds, gen_index, out)
