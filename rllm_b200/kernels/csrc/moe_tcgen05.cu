@@ -123,25 +123,26 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      unsigned it = 0, ti = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++ti) {
-        const MoeTile t = moe_tile(tile_expert, tile_row0, offsets, tile % m_tiles, m_tiles);
-        // instruction descriptor: float32 accumulate, bfloat16 A and B, both K-major, M = 128, N = the tile's pairs
-        const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((t.rows + 15) >> 4) << 18) | ((128u >> 4) << 24);
-        const unsigned buf = ti & 1, use = ti >> 1;
-        ok = mbar_wait(&acc_empty[buf], (use & 1) ^ 1, err);
+    // The whole warp walks the loop and one lane issues: with uniform control flow around them ... 
+    unsigned it = 0, ti = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++ti) {
+      const MoeTile t = moe_tile(tile_expert, tile_row0, offsets, tile % m_tiles, m_tiles);
+      // instruction descriptor: float32 accumulate, bfloat16 A and B, both K-major, M = 128, N = the tile's pairs
+      const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((t.rows + 15) >> 4) << 18) | ((128u >> 4) << 24);
+      const unsigned buf = ti & 1, use = ti >> 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], (use & 1) ^ 1, err));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const unsigned acc = tmem_base + buf * 256;
+      for (int kb = 0; kb < num_kb; ++kb, ++it) {
+        const int s = it % MT_STAGES;
+        ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (it / MT_STAGES) & 1, err));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const unsigned acc = tmem_base + buf * 256;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % MT_STAGES;
-          ok = mbar_wait(&full[s], (it / MT_STAGES) & 1, err);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          unsigned char* sa = base + s * MT_STAGE;
-          const unsigned long long d0 = umma_desc(sa), d1 = umma_desc(sa + MT_PANEL), db = umma_desc(sa + 2 * MT_PANEL);
+        unsigned char* sa = base + s * MT_STAGE;
+        const unsigned long long d0 = umma_desc(sa), d1 = umma_desc(sa + MT_PANEL), db = umma_desc(sa + 2 * MT_PANEL);
+        if (umma_elect()) {
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             umma_bf16(acc, d0 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
@@ -149,10 +150,11 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
           }
           umma_commit(&empty[s]);
         }
-        if (ok) umma_commit(&acc_full[buf]);
+        __syncwarp();
       }
+      if (ok && umma_elect()) umma_commit(&acc_full[buf]);
+      __syncwarp();
     }
-    __syncwarp();
   } else if (warp < 6) {
     const int quarter = warp & 3;
     unsigned ti = 0;

@@ -62,8 +62,13 @@ __device__ __forceinline__ unsigned long long umma_desc(const void* tile) {
 __device__ __forceinline__ void umma_bf16(unsigned tmem_d, unsigned long long da, unsigned long long db,
                                           unsigned idesc, unsigned accumulate) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+#ifdef UM_MASK
                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
                ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+#else
+               "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+               ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
+#endif
                : "memory");
 }
 // The same with the A operand in tensor memory: row i of A in lane i, two bfloat16 of K a 32-bit column
@@ -74,6 +79,12 @@ __device__ __forceinline__ void umma_bf16_tmem_a(unsigned tmem_d, unsigned ta, u
                "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
                ::"r"(tmem_d), "r"(ta), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
                : "memory");
+}
+// one lane of the (whole) warp, always the same
+__device__ __forceinline__ bool umma_elect() {
+  unsigned one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
 }
 __device__ __forceinline__ void umma_commit(void* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tg_smem(bar)) : "memory");

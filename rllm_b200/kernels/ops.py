@@ -973,6 +973,41 @@ def latent_attention_mma(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor
            "latent_attention_mma")
 
 
+# (token, head) rows of prompt portions from which they run on the tcgen05 kernel.  Its CTA walks all keys of 128 rows (2.9 us
+# a tile of 64 keys of 576 values, however few rows there are), while the mma.sync kernel cuts the keys too where there are
+# few rows: 640 rows x 4,096 keys 190 against 115 us, 1,600 rows 189 against 238, 2,048 x 128 17 against 17.
+LATENT_TCGEN05_MIN_ROWS = 1024
+
+
+def latent_attention_tcgen05_takes(dtype: torch.dtype, dk: int, dv: int, rows: int, cache: torch.Tensor) -> bool:
+    """Whether prompt portions with this many (token, head) rows run on the tcgen05 kernel.
+    RLLM_LATENT_ATTENTION=mma keeps them on the mma.sync kernel (simt: on the CUDA cores)."""
+    import os
+    return (dtype is torch.bfloat16 and dk % 8 == 0 and dk <= 576 and dv % 8 == 0 and dv <= min(dk, 512)
+            and rows >= LATENT_TCGEN05_MIN_ROWS and cache.data_ptr() % 16 == 0
+            and os.environ.get("RLLM_LATENT_ATTENTION") not in ("simt", "mma"))
+
+
+def latent_attention_tcgen05(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor,
+                             q_start: torch.Tensor, seq_lens: torch.Tensor, seq_begin: int, seq_end: int, num_tokens: int,
+                             heads: int, dk: int, dv: int, window: int, scale: float, sink: Optional[torch.Tensor],
+                             err: torch.Tensor) -> None:
+    """The attention of ``latent_attention_simt`` on the tcgen05 tensor cores, for the prompt portions (``num_tokens``
+    tokens) of sequences seq_begin .. seq_end-1 of the step; q and out hold all of the step's tokens."""
+    lib = build.load_library("latent_attention_tcgen05")
+    T = q.shape[0]
+    assert q.shape == (T, heads * dk) and out.shape == (T, heads * dv) and cache.shape[3] == dk
+    assert q.dtype is torch.bfloat16 and cache.dtype is torch.bfloat16 and out.dtype is torch.bfloat16
+    _contig(q, "q"); _contig(out, "out"); _contig(cache, "cache"); _contig(block_table, "block_table")
+    if sink is not None:
+        assert sink.dtype is torch.float32 and sink.numel() == heads
+    _check(lib.rllm_latent_attention_tcgen05(
+        _ptr(q), c_int(T), _ptr(out), _ptr(cache), _ptr(block_table), c_int(block_table.shape[1]), _ptr(q_start),
+        _ptr(seq_lens), c_int(seq_begin), c_int(seq_end), c_int(num_tokens), c_int(heads), c_int(dk), c_int(dv),
+        c_int(cache.shape[2]), c_int(cache.shape[0]), c_int(window), c_float(scale), _ptr(sink), _ptr(err), _stream()),
+        "latent_attention_tcgen05")
+
+
 # ---------------------------------------------------------------------------
 # routed experts (moe.cu)
 # ---------------------------------------------------------------------------

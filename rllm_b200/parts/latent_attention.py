@@ -154,13 +154,22 @@ class LatentAttention(Mixer):
             ops.latent_q_rot(q, qt, ctx.positions, inv_freq, H, self.nope, self.rot, self.rot_dims, self.kv_rank,
                              magnitude=self.magnitude)
         o = torch.empty((T, H * self.kv_rank), dtype=x.dtype, device=x.device)
-        if ops.latent_attention_mma_takes(x.dtype, dk, self.kv_rank):
+        window = int(self.window or 0)
+        nd = ctx.num_decode
+        if T > nd and ops.latent_attention_tcgen05_takes(x.dtype, dk, self.kv_rank, (T - nd) * H, cache.k):
+            ops.latent_attention_tcgen05(qt, o, cache.k, table, ctx.q_start, ctx.seq_lens, nd, ctx.num_seqs, T - nd, H, dk,
+                                         self.kv_rank, window, self.scale, self.sink, ctx.err)
+            if nd:
+                ops.latent_attention_mma(qt[:nd], o[:nd], cache.k, table, ctx.q_start, ctx.seq_lens, nd, 1, H, dk,
+                                         self.kv_rank, window, self.scale, self.sink, ctx.err,
+                                         max_seq_len=max(ctx.seq_lens_host[:nd]))
+        elif ops.latent_attention_mma_takes(x.dtype, dk, self.kv_rank):
             ops.latent_attention_mma(qt, o, cache.k, table, ctx.q_start, ctx.seq_lens, ctx.num_seqs, ctx.max_q_len, H,
-                                     dk, self.kv_rank, int(self.window or 0), self.scale, self.sink, ctx.err,
+                                     dk, self.kv_rank, window, self.scale, self.sink, ctx.err,
                                      max_seq_len=ctx.max_seq_len)
         else:
             ops.latent_attention_simt(qt, o, cache.k, table, ctx.positions, ctx.token_seq, H, dk, self.kv_rank,
-                                      int(self.window or 0), self.scale, self.sink, ctx.err)
+                                      window, self.scale, self.sink, ctx.err)
         ov = torch.empty((T, H * self.vdim), dtype=x.dtype, device=x.device)
         ops.head_gemm(o.view(T, H, self.kv_rank), self.w_uv, ov.view(T, H, self.vdim), b_kn=False)
         if self.gate:

@@ -1,0 +1,80 @@
+"""Attention of prompt portions over latent rows on the tcgen05 kernel against float64: rows of one to nine panels (with
+one set of value panels and two, with values in one part and two), heads that do and do not divide a tile of 128 rows,
+every page size, windows whose old pages are gone, sinks, several sequences of which the first are another kernel's, and
+cache rows that no token has written (NaN)."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("lens,news,first,heads,dk,dv,page,window,sink", [
+    ([83, 41, 190], [50, 7, 190], 0, 16, 576, 512, 16, 0, True), ([129, 64, 65], [1, 64, 65], 1, 16, 576, 512, 16, 0, False),
+    ([700], [65], 0, 16, 576, 512, 16, 100, True), ([300], [120], 0, 8, 288, 256, 16, 0, True),
+    ([83, 41], [50, 19], 0, 3, 56, 48, 16, 0, True), ([129, 64], [129, 64], 0, 5, 144, 128, 8, 33, False),
+    ([90], [90], 0, 1, 40, 40, 16, 1, False), ([150, 260], [140, 33], 0, 2, 304, 264, 16, 0, False),
+    ([150], [150], 0, 20, 96, 64, 32, 0, True), ([500], [70], 0, 7, 512, 512, 64, 0, False),
+    ([257], [200], 0, 16, 448, 392, 4, 77, True), ([64], [64], 0, 128, 384, 320, 16, 0, True), ([33], [33], 0, 200, 64, 64, 128, 0, False)])
+def test_latent_attention_on_tcgen05(lens, news, first, heads, dk, dv, page, window, sink):
+    from rllm_b200.kernels import ops
+    g = torch.Generator(device="cuda")
+    g.manual_seed(dk + heads)
+    randn = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    S, T = len(lens), sum(news)
+    pages = sum(-(-n // page) for n in lens)
+    order = torch.randperm(pages + 2, generator=g, device="cuda").tolist()
+    cache = torch.full((pages + 2, 1, page, dk), float("nan"), dtype=torch.bfloat16, device="cuda")
+    table = torch.full((S, max(-(-n // page) for n in lens)), -1, dtype=torch.int32)
+    rows = []
+    for s, n in enumerate(lens):
+        r = randn(n, dk).bfloat16()
+        rows.append(r.double())
+        for b in range(-(-n // page)):
+            if window and (b + 1) * page <= n - news[s] - window + 1:
+                continue                                       # given back: no query of this step sees it
+            table[s, b] = order.pop()
+            m = min(page, n - b * page)
+            cache[table[s, b], 0, :m] = r[b * page: b * page + m]
+    q = randn(T, heads * dk).bfloat16()
+    sk = randn(heads) + 1.0 if sink else None
+    starts = [0]
+    for m in news:
+        starts.append(starts[-1] + m)
+    out = torch.full((T, heads * dv), 7.0, dtype=torch.bfloat16, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ops.latent_attention_tcgen05(q, out, cache, table.cuda(), torch.tensor(starts, dtype=torch.int32, device="cuda"),
+                                 torch.tensor(lens, dtype=torch.int32, device="cuda"), first, S, T - starts[first], heads, dk,
+                                 dv, window, dk ** -0.5, sk, err)
+    assert int(err.item()) == 0
+    assert bool((out[: starts[first]] == 7.0).all())
+    for s in range(first, S):
+        n, m = lens[s], news[s]
+        pos, key = torch.arange(n - m, n, device="cuda")[:, None], torch.arange(n, device="cuda")
+        hidden = (key > pos) | ((key <= pos - window) if window else (key < 0))
+        for h in range(heads):
+            sc = q[starts[s]: starts[s + 1], h * dk: (h + 1) * dk].double() @ rows[s].t() * dk ** -0.5
+            sc = sc.masked_fill(hidden, -math.inf)
+            if sink:
+                sc = torch.cat([sc, sk[h].double().expand(m, 1)], 1)
+            p = torch.softmax(sc, 1)[:, :n]
+            want = p @ rows[s][:, :dv]
+            got = out[starts[s]: starts[s + 1], h * dv: (h + 1) * dv].double()
+            # weights and the result are each rounded once to bfloat16, by at most 2^-8 of themselves (a significand of 8
+            # bits): together 2^-7 of the sum of the terms' sizes, beside which the float32 sums and exponentials are small
+            bound = 2.0 ** -7 * (p @ rows[s][:, :dv].abs()) + 1e-5
+            assert bool(((got - want).abs() <= bound).all()), (s, h, float(((got - want).abs() / bound).max()))
+
+
+def test_which_prompt_portions_take_the_tcgen05_latent_attention(monkeypatch):
+    from rllm_b200.kernels import ops
+    c = torch.zeros(2, 1, 16, 576, dtype=torch.bfloat16, device="cuda")
+    assert ops.latent_attention_tcgen05_takes(torch.bfloat16, 576, 512, 1024, c)
+    assert not ops.latent_attention_tcgen05_takes(torch.bfloat16, 576, 512, 1023, c)
+    assert not ops.latent_attention_tcgen05_takes(torch.float32, 576, 512, 4096, c)
+    assert not ops.latent_attention_tcgen05_takes(torch.bfloat16, 584, 512, 4096, c)
+    assert not ops.latent_attention_tcgen05_takes(torch.bfloat16, 300, 260, 4096, c)
+    assert not ops.latent_attention_tcgen05_takes(torch.bfloat16, 576, 512, 4096, c.view(-1)[4:])
+    monkeypatch.setenv("RLLM_LATENT_ATTENTION", "mma")
+    assert not ops.latent_attention_tcgen05_takes(torch.bfloat16, 576, 512, 4096, c)

@@ -38,8 +38,8 @@ def test_experts_on_tcgen05(T, H, F, E, top, one, limit, alpha, shift):
     got = ops.moe_experts(h, ids, wgu, wd, limit, alpha, shift)
     want = by_expert(h, ids, wgu, wd, limit, alpha, shift)
     ops.check_gemm_errors(h.device)
-    # a result is rounded once, by at most 2^-9 of itself; an activation that falls to the other of two neighbours
-    # moves one of F terms by 2^-8 of it
+    # a result is rounded once, by at most 2^-8 of itself (about 2^-9 in the mean); an activation that falls to the other
+    # of two neighbours moves one of F terms by 2^-7 of it
     assert float((got.double() - want).norm() / want.norm()) <= 2.0 ** -8
     assert float((got.double() - want).abs().max()) <= 2.0 ** -8 * (float(want.abs().max()) + float(wd.abs().max()) * 8)
 
