@@ -45,11 +45,13 @@ template <int BN> constexpr int tg_smem_bytes() { return tg_stages<BN>() * tg_st
 // Persistent: CTA b takes the output tiles b, b + gridDim.x, ... (rows of tiles first, so that CTAs
 // running side by side share a weight tile in L2).  Two accumulators in TMEM: the epilogue of a
 // tile runs while the tensor cores work on the next.
-template <int BN, int EPI>
+// HEADS: tiles_m x tiles_n tiles of every one of several products; A, W and out of product h lie h head strides further
+// (the maps' third coordinate; c_head).
+template <int BN, int EPI, bool HEADS>
 __global__ void __launch_bounds__(TG_THREADS)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                     void* __restrict__ out, int ldo, int M, int N, int K, int up_offset, int tiles_m,
-                    int num_tiles, int* __restrict__ err, GateAct ga) {
+                    int num_tiles, int* __restrict__ err, GateAct ga, int tiles_n, long long c_head) {
   constexpr int STAGES = tg_stages<BN>();
   constexpr int NOUT = (EPI == TG_EPI_SILU) ? BN / 2 : BN;     // output columns of a tile
   extern __shared__ unsigned char tg_raw[];
@@ -85,7 +87,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       unsigned it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const int m0 = (tile % tiles_m) * TG_BM, n0 = (tile / tiles_m) * NOUT;
+        const int m0 = (tile % tiles_m) * TG_BM, tn = tile / tiles_m, n0 = (HEADS ? tn % tiles_n : tn) * NOUT;
+        const int head = HEADS ? tn / tiles_n : 0;
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % STAGES;
           const unsigned phase = (it / STAGES) & 1;
@@ -94,6 +97,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           unsigned char* sa = stage_mem + s * tg_stage_bytes<BN>();
           unsigned char* sb = sa + TG_BM * TG_BK * 2;
           mbar_expect_tx(&full[s], (unsigned)tg_stage_bytes<BN>());
+          if (HEADS) {
+            tma_load_3d(sa, &map_a, kb * TG_BK, m0, head, &full[s]);
+            tma_load_3d(sb, &map_w, kb * TG_BK, n0, head, &full[s]);
+            continue;
+          }
           tma_load_2d(sa, &map_a, kb * TG_BK, m0, &full[s]);
           if (EPI == TG_EPI_SILU) {
             tma_load_2d(sb, &map_w, kb * TG_BK, n0, &full[s]);
@@ -141,7 +149,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     unsigned ti = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++ti) {
-      const int m0 = (tile % tiles_m) * TG_BM, n0 = (tile / tiles_m) * NOUT;
+      const int m0 = (tile % tiles_m) * TG_BM, tn = tile / tiles_m, n0 = (HEADS ? tn % tiles_n : tn) * NOUT;
+      const size_t at = HEADS ? (size_t)(tn / tiles_n) * c_head : 0;
       const unsigned buf = ti & 1, use = ti >> 1;
       const int m = m0 + quarter * 32 + lane;
       ok = mbar_wait(&acc_full[buf], use & 1, err);
@@ -169,7 +178,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (m < M) {
           const int n = n0 + c0;
           if (EPI == TG_EPI_F32) {
-            float* o = (float*)out + (size_t)m * ldo + n;
+            float* o = (float*)out + at + (size_t)m * ldo + n;
             if (n + 32 <= N && (((uintptr_t)o) & 15) == 0) {
 #pragma unroll
               for (int j = 0; j < 32; j += 4)
@@ -179,7 +188,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
               for (int j = 0; j < 32; ++j) if (n + j < N) o[j] = __uint_as_float(r[j]);
             }
           } else {
-            bf16* o = (bf16*)out + (size_t)m * ldo + n;
+            bf16* o = (bf16*)out + at + (size_t)m * ldo + n;
             if (n + 32 <= N && (((uintptr_t)o) & 15) == 0) {
 #pragma unroll
               for (int j = 0; j < 32; j += 8) {
@@ -212,6 +221,29 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
+// maps' boxes: TG_BM rows of A, NOUT rows of W
+template <int BN, int EPI, bool HEADS>
+static int tg_run(const CUtensorMap& ma, const CUtensorMap& mw, void* out, int ldo, int M, int N, int K, int up_offset,
+                  int heads, long long c_head, int* err, cudaStream_t stream, GateAct ga) {
+  constexpr int NOUT = (EPI == TG_EPI_SILU) ? BN / 2 : BN;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, EPI, HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         tg_smem_bytes<BN>());
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  const int tiles_m = (M + TG_BM - 1) / TG_BM, tiles_n = (N + NOUT - 1) / NOUT;
+  const long long num_tiles = (long long)tiles_m * tiles_n * heads;
+  if (num_tiles > (1ll << 30)) return RLLM_E_UNSUPPORTED;
+  const int num_sms = tg_num_sms();
+  const int grid = (int)(num_tiles < num_sms ? num_tiles : num_sms);
+  gemm_tcgen05_kernel<BN, EPI, HEADS><<<grid, TG_THREADS, tg_smem_bytes<BN>(), stream>>>(
+      ma, mw, out, ldo, M, N, K, up_offset, tiles_m, (int)num_tiles, err, ga, tiles_n, c_head);
+  RLLM_LAUNCH_CHECK();
+  return 0;
+}
+
 template <int BN, int EPI>
 static int tg_launch(const void* a, int lda, const void* w, int ldw, int w_rows, void* out, int ldo, int M, int N,
                      int K, int up_offset, int* err, cudaStream_t stream,
@@ -222,22 +254,26 @@ static int tg_launch(const void* a, int lda, const void* w, int ldw, int w_rows,
   if (rc) return rc;
   rc = tg_make_map(&mw, w, w_rows, K, ldw, NOUT);
   if (rc) return rc;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         tg_smem_bytes<BN>());
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
+  return tg_run<BN, EPI, false>(ma, mw, out, ldo, M, N, K, up_offset, 1, 0, err, stream, ga);
+}
+
+// Tile width 256, 192 or 128 for N columns of `rows` tiles of rows: the one with the least estimated time = rounds of the
+// persistent CTAs x width x a factor for what a narrower tile costs (A is read again more often, the epilogue overlaps
+// less).
+static int tg_width(long long rows, int N) {
+  int bn = N > 192 ? 256 : (N > 128 ? 192 : 128);
+  if (N > 128) {
+    const long long sms = tg_num_sms();
+    double best = 1e30;
+    const int widths[3] = {256, 192, 128};
+    const double factor[3] = {1.0, 1.05, 1.3};
+    for (int i = 0; i < 3; ++i) {
+      const long long tiles = rows * ((N + widths[i] - 1) / widths[i]);
+      const double cost = (double)((tiles + sms - 1) / sms) * widths[i] * factor[i];
+      if (cost < best * 0.999) { best = cost; bn = widths[i]; }
+    }
   }
-  const int tiles_m = (M + TG_BM - 1) / TG_BM;
-  const long long num_tiles = (long long)tiles_m * ((N + NOUT - 1) / NOUT);
-  if (num_tiles > (1ll << 30)) return RLLM_E_UNSUPPORTED;
-  const int num_sms = tg_num_sms();
-  const int grid = (int)(num_tiles < num_sms ? num_tiles : num_sms);
-  gemm_tcgen05_kernel<BN, EPI><<<grid, TG_THREADS, tg_smem_bytes<BN>(), stream>>>(ma, mw, out, ldo, M, N, K, up_offset,
-                                                                                  tiles_m, (int)num_tiles, err, ga);
-  RLLM_LAUNCH_CHECK();
-  return 0;
+  return bn;
 }
 
 // epilogue 0: out bfloat16 [M, N]; 1: out float32 [M, N]; 2: W = [gate rows (N); up rows (N)] stacked,
@@ -250,20 +286,7 @@ RLLM_EXPORT int rllm_gemm_tcgen05(const void* a, int lda, const void* w, int ldw
   if (K <= 0 || lda < K || ldw < K || ldo < N || !err) return RLLM_E_BADARG;
   // TMA: 16-byte aligned bases and row strides
   if (K % 8 || lda % 8 || ldw % 8 || (((uintptr_t)a | (uintptr_t)w) & 15)) return RLLM_E_UNSUPPORTED;
-  // Tile width 256, 192 or 128: the one with the least estimated time = rounds of the persistent CTAs x
-  // width x a factor for what a narrower tile costs (A is read again more often, the epilogue overlaps less).
-  int bn = N > 192 ? 256 : (N > 128 ? 192 : 128);
-  if (N > 128) {
-    const long long tm = (M + TG_BM - 1) / TG_BM, sms = tg_num_sms();
-    double best = 1e30;
-    const int widths[3] = {256, 192, 128};
-    const double factor[3] = {1.0, 1.05, 1.3};
-    for (int i = 0; i < 3; ++i) {
-      const long long tiles = tm * ((N + widths[i] - 1) / widths[i]);
-      const double cost = (double)((tiles + sms - 1) / sms) * widths[i] * factor[i];
-      if (cost < best * 0.999) { best = cost; bn = widths[i]; }
-    }
-  }
+  const int bn = tg_width((M + TG_BM - 1) / TG_BM, N);
 #define TG_BY_WIDTH(EPI_)                                                                                      \
   if (bn == 256) return tg_launch<256, EPI_>(a, lda, w, ldw, N, out, ldo, M, N, K, 0, err, stream);            \
   if (bn == 192) return tg_launch<192, EPI_>(a, lda, w, ldw, N, out, ldo, M, N, K, 0, err, stream);            \
@@ -276,4 +299,27 @@ RLLM_EXPORT int rllm_gemm_tcgen05(const void* a, int lda, const void* w, int ldw
                                          GateAct{limit, slope, shift});
   }
   return RLLM_E_BADARG;
+}
+
+template <int BN>
+static int tg_launch_heads(const void* a, long long lda, long long a_head, const void* w, long long ldw, long long w_head,
+                           void* out, int ldo, long long c_head, int M, int N, int K, int heads, int* err, cudaStream_t stream) {
+  CUtensorMap ma, mw;
+  int rc = tg_make_map3(&ma, a, M, K, lda, heads, a_head, TG_BM);
+  if (!rc) rc = tg_make_map3(&mw, w, N, K, ldw, heads, w_head, BN);
+  if (rc) return rc;
+  return tg_run<BN, TG_EPI_BF16, true>(ma, mw, out, ldo, M, N, K, 0, heads, c_head, err, stream, GateAct{INFINITY, 1.f, 0.f});
+}
+
+// Several products at once, bfloat16: out[h] [M, N] = A[h] [M, K] . W[h] [N, K]^T, all strides in elements.
+RLLM_EXPORT int rllm_head_gemm_tcgen05(const void* a, long long lda, long long a_head, const void* w, long long ldw,
+                                       long long w_head, void* out, int ldo, long long c_head, int M, int N, int K, int heads,
+                                       int* err, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || heads <= 0) return 0;
+  if (K <= 0 || !err) return RLLM_E_BADARG;
+  if (K % 8 || lda % 8 || a_head % 8 || ldw % 8 || w_head % 8 || (((uintptr_t)a | (uintptr_t)w) & 15)) return RLLM_E_UNSUPPORTED;
+  const int bn = tg_width((long long)((M + TG_BM - 1) / TG_BM) * heads, N);
+  if (bn == 256) return tg_launch_heads<256>(a, lda, a_head, w, ldw, w_head, out, ldo, c_head, M, N, K, heads, err, stream);
+  if (bn == 192) return tg_launch_heads<192>(a, lda, a_head, w, ldw, w_head, out, ldo, c_head, M, N, K, heads, err, stream);
+  return tg_launch_heads<128>(a, lda, a_head, w, ldw, w_head, out, ldo, c_head, M, N, K, heads, err, stream);
 }

@@ -111,43 +111,41 @@ RLLM_EXPORT int rllm_latent_prep(const void* a, int a_stride, int q_rank, int kv
 // ---------------------------------------------------------------------------
 // the queries' rotated part: q[t, h, dim : dim+rot] rotated -> qt[t, h, kv_rank : kv_rank+rot]
 // ---------------------------------------------------------------------------
+// A block a token; a thread one pair of some heads, whose angle it makes once (a thread a pair and head, with 64-bit index
+// divisions: 17 us at 2,048 tokens x 16 heads x 64; now at most the 10 us that issuing it takes).
 template <typename T>
 __global__ void latent_q_rot_kernel(const T* q, T* qt, const int* positions,
                                     const double* inv_freq, float mag, int heads, int dim, int rot,
-                                    int rot_dims, int kv_rank, long long total) {
+                                    int rot_dims, int kv_rank) {
   pdl_wait();
   pdl_launch();
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= total) return;
-  const int half = rot / 2;
-  const int i = (int)(idx % half);
-  const long long th = idx / half;
-  const int h = (int)(th % heads);
-  const long long t = th / heads;
-  const T* src = q + ((size_t)t * heads + h) * (dim + rot) + dim;
-  T* dst = qt + ((size_t)t * heads + h) * (kv_rank + rot) + kv_rank;
-  const float u = to_f32(src[2 * i]), v = to_f32(src[2 * i + 1]);
-  if (2 * i + 1 < rot_dims) {
-    float c, sn;
-    rot_cos_sin<T>(positions[t], inv_freq[i], &c, &sn);
-    c *= mag; sn *= mag;
-    dst[2 * i] = from_f32<T>(u * c - v * sn);
-    dst[2 * i + 1] = from_f32<T>(v * c + u * sn);
-  } else {
-    dst[2 * i] = from_f32<T>(u);
-    dst[2 * i + 1] = from_f32<T>(v);
+  const int half = rot / 2, t = blockIdx.x;
+  const int per = max(1, (int)blockDim.x / half);              // heads side by side
+  for (int w = threadIdx.x; w < per * half; w += blockDim.x) {
+    const int i = w % half;
+    const bool turns = 2 * i + 1 < rot_dims;
+    float c = 1.f, sn = 0.f;
+    if (turns) {
+      rot_cos_sin<T>(positions[t], inv_freq[i], &c, &sn);
+      c *= mag; sn *= mag;
+    }
+    for (int h = w / half; h < heads; h += per) {
+      const T* src = q + ((size_t)t * heads + h) * (dim + rot) + dim;
+      T* dst = qt + ((size_t)t * heads + h) * (kv_rank + rot) + kv_rank;
+      const float u = to_f32(src[2 * i]), v = to_f32(src[2 * i + 1]);
+      dst[2 * i] = turns ? from_f32<T>(u * c - v * sn) : from_f32<T>(u);
+      dst[2 * i + 1] = turns ? from_f32<T>(v * c + u * sn) : from_f32<T>(v);
+    }
   }
 }
 
 RLLM_EXPORT int rllm_latent_q_rot(const void* q, void* qt, const int* positions, const double* inv_freq, float mag, int T,
                                   int heads, int dim, int rot, int rot_dims, int kv_rank, int dtype,
                                   cudaStream_t stream) {
-  const long long total = (long long)T * heads * (rot / 2);
-  if (total <= 0) return 0;
+  if (T <= 0 || heads <= 0 || rot < 2) return 0;
   if (rot & 1 || rot_dims > rot || (rot_dims & 1)) return RLLM_E_BADARG;
-  const unsigned blocks = (unsigned)((total + 255) / 256);
-  RLLM_DISPATCH_DTYPE(dtype, TT, (rllm_launch_pdl(latent_q_rot_kernel<TT>, dim3(blocks), dim3(256), (size_t)(0), stream, 
-      (const TT*)q, (TT*)qt, positions, inv_freq, mag, heads, dim, rot, rot_dims, kv_rank, total)));
+  RLLM_DISPATCH_DTYPE(dtype, TT, (rllm_launch_pdl(latent_q_rot_kernel<TT>, dim3(T), dim3(256), (size_t)(0), stream,
+      (const TT*)q, (TT*)qt, positions, inv_freq, mag, heads, dim, rot, rot_dims, kv_rank)));
   RLLM_LAUNCH_CHECK();
   return 0;
 }

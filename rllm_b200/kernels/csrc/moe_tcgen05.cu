@@ -123,7 +123,7 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
     __syncwarp();
   } else if (warp == 1) {
-    // The whole warp walks the loop and one lane issues: with uniform control flow around them ... 
+    // the whole warp walks the loop, one lane issues (154 -> 151 us against a lane that walks alone)
     unsigned it = 0, ti = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++ti) {

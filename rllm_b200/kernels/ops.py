@@ -892,6 +892,21 @@ def latent_q_rot(q: torch.Tensor, qt: torch.Tensor, positions: torch.Tensor, inv
                                  c_int(dtype_code(q.dtype)), _stream()), "latent_q_rot")
 
 
+# results from which the products per head run on the tcgen05 kernel.  16 heads: 2,048 rows x 512 of 128 61 -> 21 us,
+# 2,048 x 128 of 512 29 -> 16, 1,024 x 128 of 512 (2^21 results) 21 -> 16; at half of that both take what a launch takes.
+HEAD_GEMM_TCGEN05_FROM = 1 << 21
+
+
+def head_gemm_tcgen05_takes(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor) -> bool:
+    """Whether the tcgen05 kernel takes ``head_gemm``'s operands ([heads, N, K] weights): what TMA can address.
+    RLLM_TILE_GEMM=simt and RLLM_GEMM=library|no_tcgen05 keep it off."""
+    import os
+    return (a.dtype is torch.bfloat16 and a.shape[2] % 8 == 0 and a.stride(0) % 8 == 0 and a.stride(1) % 8 == 0
+            and (a.data_ptr() | b.data_ptr()) % 16 == 0 and c.stride(0) < 2 ** 31
+            and not os.environ.get("RLLM_TILE_GEMM", "").startswith("s")
+            and os.environ.get("RLLM_GEMM") not in ("library", "no_tcgen05"))
+
+
 def head_gemm(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, b_kn: bool) -> None:
     """c[m, h, :] = a[m, h, :] . b[h] for every head h.  a [M, heads, K], c [M, heads, N]: views with unit
     stride in the last dim; b [heads, K, N] (``b_kn``) or [heads, N, K], contiguous."""
@@ -901,6 +916,13 @@ def head_gemm(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, b_kn: bool) -> 
     assert c.shape[:2] == (M, heads) and a.stride(2) == 1 and c.stride(2) == 1 and a.dtype is b.dtype is c.dtype
     assert b.shape == ((heads, K, N) if b_kn else (heads, N, K))
     _contig(b, "b")
+    if M * heads * N >= HEAD_GEMM_TCGEN05_FROM and not b_kn and head_gemm_tcgen05_takes(a, b, c):
+        lib = build.load_library("gemm_tcgen05")
+        _check(lib.rllm_head_gemm_tcgen05(
+            _ptr(a), c_longlong(a.stride(0)), c_longlong(a.stride(1)), _ptr(b), c_longlong(b.stride(1)),
+            c_longlong(b.stride(0)), _ptr(c), c_int(c.stride(0)), c_longlong(c.stride(1)), c_int(M), c_int(N), c_int(K),
+            c_int(heads), _ptr(gemm_error_word(a.device)), _stream()), "head_gemm_tcgen05")
+        return
     _check(lib.rllm_head_gemm(_ptr(a), c_longlong(a.stride(0)), c_longlong(a.stride(1)), _ptr(b),
                               c_longlong(b.stride(1)), c_longlong(b.stride(0)), c_int(1 if b_kn else 0), _ptr(c),
                               c_longlong(c.stride(0)), c_longlong(c.stride(1)), c_int(M), c_int(N), c_int(K),
