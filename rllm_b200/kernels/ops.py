@@ -5,6 +5,7 @@ a missing compiler or a size that a kernel refuses raises an error.
 from __future__ import annotations
 
 import ctypes
+import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from typing import Optional
 
@@ -36,7 +37,9 @@ def _ptr(t: Optional[torch.Tensor]) -> c_void_p:
 
 
 def _stream() -> c_void_p:
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current device's current stream.  Its handle alone: ``torch.cuda.current_stream()`` makes an object of it, which
+    took 3.2 us a launch against 0.2 (a decoded token's feed-forward issues in 38 us, two launches)."""
+    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 LAUNCHES = [0]      # entry-point calls so far (each launches at least one kernel)
@@ -134,12 +137,13 @@ def rope_kv_write(qkv: torch.Tensor, positions: torch.Tensor, token_seq: torch.T
 
 
 PLAIN_GATE = (float("inf"), 1.0, 0.0)
+_PLAIN_GATE_ARGS = tuple(c_float(v) for v in PLAIN_GATE)
 
 
 def _gate_args(gate):
     """(limit, slope, shift) of a gated product: g' sigmoid(slope g') (u' + shift), g' = min(g, limit), u' = u kept
     within +-limit; ``PLAIN_GATE`` is silu(g) u."""
-    return tuple(c_float(float(v)) for v in gate)
+    return _PLAIN_GATE_ARGS if gate is PLAIN_GATE else tuple(c_float(float(v)) for v in gate)
 
 
 def silu_mul(gate_up: torch.Tensor, out: torch.Tensor, gate=PLAIN_GATE) -> None:
@@ -273,7 +277,6 @@ def small_m_rows(num_rows: int, dtype: torch.dtype, weights=()) -> bool:
     9 to 16 rows: if every one of ``weights`` has few enough rows for the kernels' one-wave form (16 rows a
     CTA, seven CTAs an SM); measured at batch 16, context 4096, four layers: Llama-1B shapes 16 % faster
     than the library path, 3B shapes equal, 8B shapes (whose gate_up has too many rows) 6 % slower."""
-    import os
     if dtype is not torch.bfloat16 or num_rows <= 0 or os.environ.get("RLLM_GEMM") == "library":
         return False
     if num_rows > int(os.environ.get("RLLM_FUSED_M_MAX", FUSED_M_MAX)):
@@ -290,7 +293,6 @@ def small_m_rows(num_rows: int, dtype: torch.dtype, weights=()) -> bool:
 
 
 def small_m_takes(x: torch.Tensor, w: torch.Tensor) -> bool:
-    import os
     return (x.dtype is torch.bfloat16 and 0 < x.shape[0] <= SMALL_M_MAX and x.shape[1] % 8 == 0
             and x.stride(0) % 8 == 0 and w.stride(0) % 8 == 0 and os.environ.get("RLLM_GEMM") != "library")
 
@@ -347,7 +349,6 @@ def tcgen05_takes(x: torch.Tensor, w: torch.Tensor, silu: bool = False) -> bool:
     """Whether the tcgen05 kernel should compute x . w^T.  ``silu``: w is [gate; up] stacked and the
     output has half of w's rows.  With the environment variable RLLM_GEMM=tcgen05 every shape it can
     take goes to it (used by tests, so that tiny models run through it)."""
-    import os
     mode = os.environ.get("RLLM_GEMM", "")
     if mode in ("library", "no_tcgen05"):
         return False
@@ -365,14 +366,13 @@ def gemm_bf16(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype) -> Optio
     takes the shape (the caller then uses the library's matrix product).  Few rows:
     the weight-streaming kernel; more: the tcgen05 kernel."""
     if small_m_takes(x, w):
-        import os
         if w.shape[0] > 65536 and (x.shape[0] > 8 or os.environ.get("RLLM_HEAD") == "library"):
             return None                 # very tall weights (the vocabulary) at 9 to 16 rows: the library's kernel is ahead
-        out = torch.empty((x.shape[0], w.shape[0]), dtype=out_dtype, device=x.device)
+        out = x.new_empty((x.shape[0], w.shape[0]), dtype=out_dtype)
         gemm_small_m(x, w, out)
         return out
     if tcgen05_takes(x, w):
-        out = torch.empty((x.shape[0], w.shape[0]), dtype=out_dtype, device=x.device)
+        out = x.new_empty((x.shape[0], w.shape[0]), dtype=out_dtype)
         gemm_tcgen05(x, w, out)
         return out
     return None
@@ -639,14 +639,12 @@ def mma_attention_takes(nq: int, nkv: int, d: int) -> bool:
 def use_mma_attention(dtype: torch.dtype, nq: int, nkv: int, d: int) -> bool:
     """bfloat16 with a head size the tensor-core attention kernels take; other
     cases (float32, other head sizes) go to the CUDA-core kernel."""
-    import os
     return dtype is torch.bfloat16 and mma_attention_takes(nq, nkv, d) and os.environ.get("RLLM_ATTENTION") != "simt"
 
 
 def use_tcgen05_attention(dtype: torch.dtype, nq: int, nkv: int, d: int, page_size: int) -> bool:
     """Prompt portions go to the tcgen05 attention kernel when it takes the sizes;
     RLLM_ATTENTION=mma (or simt) keeps them on the older kernels."""
-    import os
     return (dtype is torch.bfloat16 and attention_prefill_tcgen05_supported(nq, nkv, d, page_size)
             and os.environ.get("RLLM_ATTENTION") not in ("simt", "mma"))
 
@@ -900,7 +898,6 @@ HEAD_GEMM_TCGEN05_FROM = 1 << 21
 def head_gemm_tcgen05_takes(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor) -> bool:
     """Whether the tcgen05 kernel takes ``head_gemm``'s operands ([heads, N, K] weights): what TMA can address.
     RLLM_TILE_GEMM=simt and RLLM_GEMM=library|no_tcgen05 keep it off."""
-    import os
     return (a.dtype is torch.bfloat16 and a.shape[2] % 8 == 0 and a.stride(0) % 8 == 0 and a.stride(1) % 8 == 0
             and (a.data_ptr() | b.data_ptr()) % 16 == 0 and c.stride(0) < 2 ** 31
             and not os.environ.get("RLLM_TILE_GEMM", "").startswith("s")
@@ -957,7 +954,6 @@ LATENT_SPLIT_KEYS = 128          # keys a split (a multiple of 64, at absolute p
 
 def latent_attention_mma_takes(dtype: torch.dtype, dk: int, dv: int) -> bool:
     """Whether the tensor-core kernel computes this attention (RLLM_LATENT_ATTENTION=simt keeps it on the CUDA cores)."""
-    import os
     return (dtype is torch.bfloat16 and dk % 8 == 0 and dv <= min(dk, 512)
             and os.environ.get("RLLM_LATENT_ATTENTION") != "simt")
 
@@ -1004,7 +1000,6 @@ LATENT_TCGEN05_MIN_ROWS = 1024
 def latent_attention_tcgen05_takes(dtype: torch.dtype, dk: int, dv: int, rows: int, cache: torch.Tensor) -> bool:
     """Whether prompt portions with this many (token, head) rows run on the tcgen05 kernel.
     RLLM_LATENT_ATTENTION=mma keeps them on the mma.sync kernel (simt: on the CUDA cores)."""
-    import os
     return (dtype is torch.bfloat16 and dk % 8 == 0 and dk <= 576 and dv % 8 == 0 and dv <= min(dk, 512)
             and rows >= LATENT_TCGEN05_MIN_ROWS and cache.data_ptr() % 16 == 0
             and os.environ.get("RLLM_LATENT_ATTENTION") not in ("simt", "mma"))
@@ -1042,7 +1037,6 @@ MOE_TCGEN05_FROM = 65     # from this many pairs on they run on the tcgen05 kern
 def moe_tcgen05_takes(pairs: int, h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor) -> bool:
     """Whether the experts' products of this many (token, expert) pairs run on the tcgen05 kernels: bfloat16, sizes
     and pointers that TMA takes.  RLLM_TILE_GEMM=simt and RLLM_GEMM=library|no_tcgen05 keep them off."""
-    import os
     return (pairs >= MOE_TCGEN05_FROM and h.dtype is torch.bfloat16 and h.shape[1] % 8 == 0 and w_down.shape[2] % 8 == 0
             and (h.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16 == 0
             and not os.environ.get("RLLM_TILE_GEMM", "").startswith("s")
@@ -1667,7 +1661,6 @@ def channel_delta_scan(c: torch.Tensor, step: torch.Tensor, b: torch.Tensor, dt_
     float32 [heads]; state float32 [slots, heads, d, dv].  q and k are made unit vectors (``unit_eps`` under the
     root), q is multiplied by d^(-1/2).  Returns o float32 [T, heads dv].  Portions of bfloat16 activations take the
     tensor-core form, sixteen tokens at a time (d up to 128); the result differs by rounding only."""
-    import os
     lib = build.load_library("channel_delta")
     T = c.shape[0]
     assert c.shape[1] == 2 * kv * d + heads * dv and c.stride(1) == 1
@@ -1795,7 +1788,6 @@ def linear_state_scan(a: torch.Tensor, state: torch.Tensor, q_start: torch.Tenso
     ``LINEAR_STATE_CHUNKED_FROM`` tokens on (the first ``num_decode`` sequences, of one token each, aside) go in chunks
     of 64 side by side on the tensor cores (heads up to 128 x 128); the result differs by rounding only.  ``tables`` keeps
     the rotation tables of a step for its other calls."""
-    import os
     lib = build.load_library("linear_state")
     heads, d, dv = state.shape[1:]
     T = a.shape[0]
@@ -1888,14 +1880,12 @@ def talking_prep(qkv: torch.Tensor, positions: torch.Tensor, token_seq: torch.Te
 
 def shared_key_tcgen05_takes(dtype: torch.dtype, nq: int, nkv: int, dkp: int, dvp: int, page_size: int) -> bool:
     """Prompt portions go to the tcgen05 kernel when it takes the sizes (RLLM_ATTENTION=mma or simt keeps them off it)."""
-    import os
     return (dtype is torch.bfloat16 and dkp % 64 == 0 and dkp <= 512 and dvp in (64, 128) and page_size in (16, 32, 64)
             and nq // nkv <= 128 and os.environ.get("RLLM_ATTENTION") not in ("simt", "mma"))
 
 
 def shared_key_mma_takes(dtype: torch.dtype, nq: int, dkp: int, dvt: int) -> bool:
     """bfloat16 sizes that the mma.sync kernel takes (RLLM_ATTENTION=simt keeps them on the CUDA cores)."""
-    import os
     if dtype is not torch.bfloat16 or os.environ.get("RLLM_ATTENTION") == "simt":
         return False
     lib = build.load_library("shared_key_attention")

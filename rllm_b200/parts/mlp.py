@@ -43,7 +43,9 @@ class GatedMLP(FeedForward):
         self.gate = (float(p["limit"]) if p.get("limit") is not None else float("inf"),
                      float(p["slope"]) if p.get("slope") is not None else 1.0,
                      float(p["up_shift"]) if p.get("up_shift") is not None else 0.0)
-        if self.gate != ops.PLAIN_GATE and self.activation != "silu":
+        if self.gate == ops.PLAIN_GATE:
+            self.gate = ops.PLAIN_GATE
+        elif self.activation != "silu":
             raise ValueError("limit, slope and up_shift go with the activation 'silu'")
         if not self.gate[0] > 0:
             raise ValueError("limit must be positive")
@@ -72,7 +74,7 @@ class GatedMLP(FeedForward):
         return self.activation == "silu" and fused_residual_takes(num_rows, dtype, self.w_gate_up, self.w_down)
 
     def forward(self, x, residual=None):
-        act = torch.empty((x.shape[0], self.inter), dtype=x.dtype, device=x.device)
+        act = (x.x if isinstance(x, ScaledRows) else x).new_empty((x.shape[0], self.inter))
         if self.activation != "silu":
             ops.act_mul(linear(x, self.w_gate_up), act, self.activation)
         elif isinstance(x, ScaledRows):

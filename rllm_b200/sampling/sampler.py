@@ -132,12 +132,12 @@ class Sampler:
         s = host[: 4 * R].view(np.int64).reshape(2, R)
         f = host[4 * R: 7 * R].view(np.float32).reshape(3, R)
         k = host[7 * R: 8 * R]
-        for r, row in enumerate(rows):
-            p = row.params
-            f[0, r], f[1, r], f[2, r] = p.temperature, p.top_p, p.min_p
-            k[r] = p.top_k
-            s[0, r] = np.int64(np.uint64(row.seed & 0xFFFFFFFFFFFFFFFF).astype(np.int64))
-            s[1, r] = row.gen_index
+        params = [row.params for row in rows]
+        f[0], f[1], f[2] = [p.temperature for p in params], [p.top_p for p in params], [p.min_p for p in params]
+        for r, p in enumerate(params):
+            k[r] = p.top_k                        # one by one: a number beyond 32 bits is refused
+        s.view(np.uint64)[0] = [row.seed & 0xFFFFFFFFFFFFFFFF for row in rows]
+        s[1] = [row.gen_index for row in rows]
         with torch.cuda.device(self.device):
             dev[: 8 * R].copy_(self._pinned[self._slot][0][: 8 * R], non_blocking=True)
             copied.record()
