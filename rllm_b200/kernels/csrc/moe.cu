@@ -436,11 +436,51 @@ __global__ void weighted_slot_sum_kernel(const T* y, const float* c, T* out,
   out[idx] = from_f32<T>(v);
 }
 
+// the same eight values a thread (bfloat16, H a multiple of 8, 16-byte aligned): 2,048 x top 4 x 2,048, 42 MB, 22.7 us with
+// single values, 7.7 (5.5 TB/s)
+__global__ void __launch_bounds__(256)
+weighted_slot_sum8_kernel(const bf16* y, const float* c, bf16* out, int slots, int H8, unsigned total, const bf16* extra,
+                          const float* extra_gate) {
+  pdl_wait();
+  pdl_launch();
+  const unsigned idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= total) return;
+  const unsigned t = idx / H8, i = (idx - t * H8) * 8;
+  const size_t H = (size_t)H8 * 8;
+  float v[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = 0.f;
+#pragma unroll 4
+  for (int k = 0; k < slots; ++k) {
+    float a[8];
+    load8(y + ((size_t)t * slots + k) * H + i, a);
+    const float w = c[(size_t)t * slots + k];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = fmaf(w, a[j], v[j]);
+  }
+  if (extra) {
+    float a[8];
+    load8(extra + t * H + i, a);
+    const float w = extra_gate ? 1.0f / (1.0f + expf(-extra_gate[t])) : 1.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = fmaf(w, a[j], v[j]);
+  }
+  store8(out + t * H + i, v);
+}
+
 RLLM_EXPORT int rllm_weighted_slot_sum(const void* y, const float* c, void* out, int T, int slots, int H,
                                        const void* extra, const float* extra_gate, int dtype, cudaStream_t stream) {
   const long long total = (long long)T * H;
   if (total <= 0) return 0;
   if (slots <= 0) return RLLM_E_BADARG;
+  if (dtype == RLLM_DT_BF16 && H % 8 == 0 && total / 8 < (1ll << 31) &&
+      (((uintptr_t)y | (uintptr_t)out | (uintptr_t)extra) & 15) == 0) {
+    const unsigned n = (unsigned)(total / 8);
+    rllm_launch_pdl(weighted_slot_sum8_kernel, dim3((n + 255) / 256), dim3(256), (size_t)0, stream, (const bf16*)y, c,
+                    (bf16*)out, slots, H / 8, n, (const bf16*)extra, extra_gate);
+    RLLM_LAUNCH_CHECK();
+    return 0;
+  }
   const unsigned blocks = (unsigned)((total + 255) / 256);
   RLLM_DISPATCH_DTYPE(dtype, TT, (rllm_launch_pdl(weighted_slot_sum_kernel<TT>, dim3(blocks), dim3(256), (size_t)(0), stream, 
       (const TT*)y, c, (TT*)out, slots, H, total, (const TT*)extra, extra_gate)));

@@ -1,0 +1,111 @@
+"""The kernels that take eight (the convolution: four) values an access, at the sizes and alignments where they begin and
+end, against float64 and against the forms with single values, which rows that start elsewhere still take."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def gen(seed):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    return lambda *s: torch.randn(*s, generator=g, device="cuda")
+
+
+def close(got, want, size):
+    # one rounding to bfloat16 (at most 2^-8 of the result) and a few of float32
+    return bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * size + 1e-7).all())
+
+
+@pytest.mark.parametrize("T,H,pad,wd", [(5, 8, 0, "float32"), (3, 2048, 8, "float32"), (2, 8192, 16, "bfloat16"), (2, 8200, 8, "float32"),
+                                        (4, 264, 3, "float32"), (1, 1000, 8, "bfloat16")])
+def test_gated_rmsnorm_rows(T, H, pad, wd):
+    from rllm_b200.kernels import ops
+    r = gen(H + pad)
+    x, w = r(T, H) * 3, (1 + 0.1 * r(H)).to(getattr(torch, wd))
+    g = r(T, H + pad).bfloat16()[:, pad:]
+    got = ops.gated_rmsnorm(x, g, w, 1e-5, torch.bfloat16)
+    want = x.double() * torch.rsqrt(x.double().square().mean(1, keepdim=True) + 1e-5) * w.double() * torch.sigmoid(g.double())
+    assert close(got, want, 4.0)
+
+
+@pytest.mark.parametrize("T,E,groups,pad", [(3, 4096, 2, 8), (5, 64, 4, 0), (2, 8192, 1, 8), (2, 16400, 2, 8), (3, 96, 3, 5), (2, 20, 5, 4)])
+def test_silu_gated_group_rmsnorm_rows(T, E, groups, pad):
+    from rllm_b200.kernels import ops
+    r = gen(E + pad)
+    y, w = r(T, E) * 2, 1 + 0.1 * r(E)
+    z = r(T, E + pad).bfloat16()[:, pad:]
+    got = ops.silu_gated_group_rmsnorm(y, z, w, 1e-5, groups, torch.bfloat16)
+    v = (y.double() * torch.nn.functional.silu(z.double())).view(T, groups, -1)
+    want = (v * torch.rsqrt(v.square().mean(-1, keepdim=True) + 1e-5)).view(T, E) * w.double()
+    assert close(got, want, 8.0)
+
+
+@pytest.mark.parametrize("T,K,H", [(1, 1, 8), (7, 4, 2048), (33, 5, 264), (9, 2, 100)])
+@pytest.mark.parametrize("extra", ["none", "row", "gated"])
+def test_weighted_sum_of_slots(T, K, H, extra):
+    from rllm_b200.kernels import ops
+    r = gen(T + H)
+    y, c, e, g = r(T * K, H).bfloat16(), r(T, K), r(T, H).bfloat16(), r(T)
+    out = torch.empty(T, H, dtype=torch.bfloat16, device="cuda")
+    ops.weighted_slot_sum(y, c, out, extra=None if extra == "none" else e, extra_gate=g if extra == "gated" else None)
+    want = torch.einsum("tk,tkh->th", c.double(), y.double().view(T, K, H))
+    if extra != "none":
+        want = want + e.double() * (torch.sigmoid(g.double())[:, None] if extra == "gated" else 1.0)
+    assert close(out, want, 4.0 * K)
+
+
+@pytest.mark.parametrize("P,E", [(1, 1), (31, 3), (33, 40), (2048, 5), (8192, 32), (5000, 2048)])
+@pytest.mark.parametrize("bm", [16, 64, 128])
+def test_pairs_sorted_by_expert(P, E, bm):
+    """Every pair once, within its expert's range, and tiles that cover the ranges."""
+    from rllm_b200.kernels import build
+    from rllm_b200.kernels.ops import _check, _ptr, _stream, c_int
+    r = torch.Generator(device="cuda")
+    r.manual_seed(P)
+    ids = torch.randint(0, E, (P,), generator=r, device="cuda", dtype=torch.int32)
+    most = min(P, -(-P // bm) + E)
+    off, pairs, te, tr, n = (torch.full((k,), -1, dtype=torch.int32, device="cuda") for k in (E + 1, P, most, most, 1))
+    _check(build.load_library("moe").rllm_moe_sort(_ptr(ids), c_int(P), c_int(E), c_int(bm), _ptr(off), _ptr(pairs), _ptr(te),
+                                                   _ptr(tr), _ptr(n), _stream()), "moe_sort")
+    count = torch.bincount(ids.long(), minlength=E)
+    assert off.tolist() == [0] + count.cumsum(0).tolist()
+    assert sorted(pairs.tolist()) == list(range(P)) and bool((ids[pairs.long()].diff() >= 0).all())
+    at, off, te, tr = 0, off.tolist(), te.tolist(), tr.tolist()
+    for e in range(E):
+        rows, covered = [], off[e]
+        while at < int(n) and te[at] == e:
+            rows.append(tr[at])
+            at += 1
+        for i, r0 in enumerate(rows):
+            end = rows[i + 1] if i + 1 < len(rows) else off[e + 1]
+            assert r0 == covered and 0 < end - r0 <= bm
+            covered = end
+        assert covered == off[e + 1]
+    assert at == int(n)
+
+
+@pytest.mark.parametrize("lens", [[1], [8], [2, 1, 1, 30, 3], [9, 17], [64], [1, 7, 8, 1]])
+@pytest.mark.parametrize("E,pad,bias", [(4, 0, True), (512, 4, True), (516, 8, False), (1028, 2, True)])
+def test_convolution_of_prompt_portions(lens, E, pad, bias):
+    """Runs of eight tokens within a sequence, across sequences and behind the last; tails that go on from before; the same
+    numbers as a token at a time."""
+    from rllm_b200.kernels import ops
+    r = gen(E + sum(lens))
+    T, S = sum(lens), len(lens)
+    x = r(T, E + pad).bfloat16()[:, pad:]
+    w, b = r(E, 4) * 0.4, r(E) * 0.1 if bias else None
+    tail = r(S + 1, 3, E)
+    starts = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+    seq = torch.repeat_interleave(torch.arange(S, dtype=torch.int32), torch.tensor(lens)).cuda()
+    slots = torch.arange(S, 0, -1, dtype=torch.int32, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    new, at = tail.clone(), 0
+    got = ops.causal_conv(x, w, b, new, starts, seq, slots, S, True, err)
+    for s, n in enumerate(lens):
+        past = torch.cat([tail[slots[s].long()].double(), x[at: at + n].double()])
+        acc = sum(w[:, k].double() * past[k: k + n] for k in range(4)) + (b.double() if bias else 0.0)
+        assert close(got[at: at + n], torch.nn.functional.silu(acc), 4.0)
+        assert torch.equal(new[slots[s].long()], past[n:].float())
+        at += n
+    assert int(err) == 0 and torch.equal(new[0], tail[0])
