@@ -43,8 +43,7 @@ RLLM_EXPORT int rllm_lightning_scan(const void* q, const void* k, const void* v,
   if (dtype == RLLM_DT_BF16 && max_chunks > 0 && !lightning_mma_disabled() && stride % 2 == 0) {
     // long portions of bfloat16 activations: the chunk passes on the tensor cores, where the head's sizes are built
     auto chain = [&]() {
-      rllm_launch_pdl(lightning_chain_kernel<false>, dim3(heads, num_seqs, (d * dv + 255) / 256), dim3(256), (size_t)0, stream,
-                      decay, LtSteps{}, state, work, q_start, slots, num_slots, max_chunks, heads, d, dv);
+      lightning_chain<false>(decay, LtSteps{}, state, work, q_start, slots, num_slots, num_seqs, max_chunks, heads, d, dv, stream);
     };
     bool done = false;
 #define LTC_GO(D_, DV_)                                                                                          \

@@ -24,6 +24,8 @@ __device__ __forceinline__ float lt_step(const LtSteps& p, int t, int h, int hea
   return v > 20.f ? v : log1pf(expf(v));
 }
 
+template <int V> struct __align__(4 * V) LtVec { float v[V]; };
+
 #define LT_TOKENS 8
 #define LT_CHUNK 64
 #define LT_TILE 8            // a thread's tile of S is LT_TILE x LT_TILE
@@ -232,14 +234,16 @@ lightning_kernel(const T* q, const T* k, const T* v, int stride, const float* de
 
 // work[s * max_chunks + c] holds chunk c's end state from a zero start; afterwards it holds chunk c's start
 // state, and the slot holds the sequence's state after its last token.
-template <bool STEPS>
+// V: how many neighbouring values of a state a thread chains (4 where d dv allows it: 16-byte accesses, eight chunks of them
+// on their way; 2,048 tokens of 64 heads of 128 x 64, 134 MB through L2 and memory: 35 us with single values, 19).
+template <bool STEPS, int V>
 __global__ void __launch_bounds__(256)
 lightning_chain_kernel(const float* decay, LtSteps steps, float* state, float* work, const int* q_start, const int* slots,
                        int num_slots, int max_chunks, int heads, int d, int dv) {
   pdl_wait();
   pdl_launch();
   const int h = blockIdx.x, s = blockIdx.y;
-  const int e = blockIdx.z * blockDim.x + threadIdx.x;
+  const int e = (blockIdx.z * blockDim.x + threadIdx.x) * V;
   if (e >= d * dv) return;
   const int slot = slots[s];
   if (slot < 0 || slot >= num_slots) return;
@@ -249,28 +253,45 @@ lightning_chain_kernel(const float* decay, LtSteps steps, float* state, float* w
   const float full = STEPS ? 0.f : powf(lam, (float)LT_CHUNK);
   const float rate = STEPS ? expf(steps.a_log[h]) : 0.f;
   float* sp = state + ((size_t)slot * heads + h) * d * dv + e;
-  float cur = *sp;
+  typedef LtVec<V> Vec;
+  Vec cur = *(const Vec*)sp;
   const int chunks = (len + LT_CHUNK - 1) / LT_CHUNK;
   float* w0 = work + ((size_t)s * max_chunks * heads + h) * d * dv + e;
   const size_t step = (size_t)heads * d * dv;
   // eight chunks' end states are fetched before the chain runs over them (the loads do not depend on it)
   for (int c0 = 0; c0 < chunks; c0 += 8) {
-    float z[8], sum[8];
+    Vec z[8];
+    float sum[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u)
       sum[u] = (STEPS && c0 + u < chunks) ? steps.chunk_dt[((size_t)s * max_chunks + c0 + u) * heads + h] : 0.f;
 #pragma unroll
-    for (int u = 0; u < 8; ++u) z[u] = (c0 + u < chunks) ? w0[(size_t)(c0 + u) * step] : 0.f;
+    for (int u = 0; u < 8; ++u) if (c0 + u < chunks) z[u] = *(const Vec*)(w0 + (size_t)(c0 + u) * step);
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       if (c0 + u < chunks) {
-        w0[(size_t)(c0 + u) * step] = cur;
+        *(Vec*)(w0 + (size_t)(c0 + u) * step) = cur;
         const int n = min(LT_CHUNK, len - (c0 + u) * LT_CHUNK);
-        cur = fmaf(STEPS ? expf(-rate * sum[u]) : (n == LT_CHUNK ? full : powf(lam, (float)n)), cur, z[u]);
+        const float f = STEPS ? expf(-rate * sum[u]) : (n == LT_CHUNK ? full : powf(lam, (float)n));
+#pragma unroll
+        for (int i = 0; i < V; ++i) cur.v[i] = fmaf(f, cur.v[i], z[u].v[i]);
       }
     }
   }
-  *sp = cur;
+  *(Vec*)sp = cur;
+}
+
+// the chain between the two chunk passes, whichever form they have
+template <bool STEPS>
+static void lightning_chain(const float* decay, LtSteps steps, float* state, float* work, const int* q_start, const int* slots,
+                            int num_slots, int num_seqs, int max_chunks, int heads, int d, int dv, cudaStream_t stream) {
+  const int n = d * dv;
+  if (n % 4 == 0 && (((uintptr_t)state | (uintptr_t)work) & 15) == 0)
+    rllm_launch_pdl(lightning_chain_kernel<STEPS, 4>, dim3(heads, num_seqs, (n / 4 + 255) / 256), dim3(256), (size_t)0, stream,
+                    decay, steps, state, work, q_start, slots, num_slots, max_chunks, heads, d, dv);
+  else
+    rllm_launch_pdl(lightning_chain_kernel<STEPS, 1>, dim3(heads, num_seqs, (n + 255) / 256), dim3(256), (size_t)0, stream,
+                    decay, steps, state, work, q_start, slots, num_slots, max_chunks, heads, d, dv);
 }
 
 template <typename T, int NS, bool STEPS>
@@ -292,8 +313,7 @@ static int lightning_launch(const T* q, const T* k, const T* v, int stride, cons
     const dim3 grid(heads, num_seqs * max_chunks, gz);
     rllm_launch_pdl(lightning_kernel<T, NS, 1, STEPS>, grid, dim3(threads), (size_t)0, stream, q, k, v, stride, decay, steps,
                     state, work, q_start, slots, num_slots, max_chunks, out, heads, d, dv, err);
-    rllm_launch_pdl(lightning_chain_kernel<STEPS>, dim3(heads, num_seqs, (d * dv + 255) / 256), dim3(256), (size_t)0, stream,
-                    decay, steps, state, work, q_start, slots, num_slots, max_chunks, heads, d, dv);
+    lightning_chain<STEPS>(decay, steps, state, work, q_start, slots, num_slots, num_seqs, max_chunks, heads, d, dv, stream);
     rllm_launch_pdl(lightning_kernel<T, NS, 2, STEPS>, grid, dim3(threads), (size_t)0, stream, q, k, v, stride, decay, steps,
                     state, work, q_start, slots, num_slots, max_chunks, out, heads, d, dv, err);
   }

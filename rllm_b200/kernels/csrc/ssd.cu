@@ -40,8 +40,7 @@ RLLM_EXPORT int rllm_ssd_scan(const void* xbc, int stride, int dtype, const floa
     const bf16* x = (const bf16*)xbc;
     const bf16 *B = x + (size_t)heads * P, *C = B + (size_t)groups * N;
     auto chain = [&]() {
-      rllm_launch_pdl(lightning_chain_kernel<true>, dim3(heads, num_seqs, (N * P + 255) / 256), dim3(256), (size_t)0, stream,
-                      (const float*)nullptr, steps, state, work, q_start, slots, num_slots, max_chunks, heads, N, P);
+      lightning_chain<true>(nullptr, steps, state, work, q_start, slots, num_slots, num_seqs, max_chunks, heads, N, P, stream);
     };
 #define SSD_GO(D_, DV_)                                                                                            \
   ltc_launch<D_, DV_, true>(C, B, x, stride, nullptr, steps, work, q_start, num_seqs, max_chunks, out, heads, N, P, \
