@@ -1,8 +1,9 @@
 // Paged causal attention on CUDA cores, for float32 and bfloat16 caches: the
 // kernel of the true 32-bit path, and the fallback of the bfloat16 path for
 // shapes its tensor-core kernels refuse.  One warp per (query token, query
-// head); it serves prompt portions and single decoded tokens alike, since a
-// token's keys are read from the cache through the block table either way.
+// head), or a block of eight where there are few of them; it serves prompt
+// portions and single decoded tokens alike, since a token's keys are read from
+// the cache through the block table either way.
 //
 // Contract (the reference's intended one, crates/rllm-kernels/src/cuda/
 // paged_attention.cu:88-179 for the math; its prefill kernel ignores earlier
@@ -23,9 +24,17 @@
 //   slopes      float32 [nq]: slopes[h] * (p - j) is taken off the score of key j (after scaling and cap):
 //               a bias that grows with the distance between query and key.
 //
-// Keys are walked in groups of 32 aligned to absolute positions, so the
-// arithmetic of a row does not depend on how the sequence was cut into steps,
-// on the batch around it, or on which pages hold it.
+// Keys are walked in groups of 32 aligned to absolute positions; four groups
+// (128 keys at absolute positions) make a partial result from an empty start,
+// and a row's partial results are added up in order.  So the arithmetic of a
+// row does not depend on how the sequence was cut into steps, on the batch
+// around it, on which pages hold it, or on how many warps share it.
+//
+// What bounds it is latency: a lane's key and the 32 values of a group are loads
+// that wait for nothing but the block table, so eight keys' worth of them are
+// kept on their way.  Four sequences of 100 to 3,000 keys, one token each, 32
+// heads of 64 in float32: 1,225 us with a warp a row and a load at a time, 616 with
+// loads ahead, 92 with eight warps a row; 6,400 rows of up to 300 keys 264 -> 183.
 #include "common.cuh"
 #include <math.h>
 
@@ -48,10 +57,12 @@ template <> struct Vec8<bf16> {
   }
 };
 
-// d: the size of a query and key head; dv: of a value and output head (they may differ).  VEC: d is a
-// multiple of 8 and keys are fetched eight at a time; otherwise one by one.
-template <typename T, bool VEC>
-__global__ void __launch_bounds__(32 * ATT_WARPS)
+#define ATT_PART 128         // keys of a partial result
+
+// d: the size of a query and key head; dv: of a value and output head (they may differ), up to 32 RD.  VEC: d is a
+// multiple of 8 and keys are fetched eight at a time; otherwise one by one.  WPR warps share a row.
+template <typename T, bool VEC, int RD, int WPR>
+__global__ void __launch_bounds__(32 * (WPR == 1 ? ATT_WARPS : WPR))
 attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out,
                       const T* __restrict__ kcache, const T* __restrict__ vcache,
                       const int* __restrict__ block_table, int max_blocks,
@@ -60,9 +71,11 @@ attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out
                       int keep_first, int chunk, float softcap, const float* __restrict__ sinks,
                       const T* __restrict__ gate, int gate_stride, int gate_mode,
                       const float* __restrict__ slopes, int shared_keys, int v_ld, int* __restrict__ err) {
-  extern __shared__ float qs[];  // [ATT_WARPS][d]
+  constexpr int U = WPR == 1 ? 16 / RD : 8;          // keys whose values are on their way together
+  constexpr int UK = WPR == 1 && RD > 2 ? 4 : 8;     // and pieces of a key (many rows: warps hide it, registers cost warps)
+  extern __shared__ float qs[];  // WPR 1: [ATT_WARPS][d]; else [d] and the warps' partial results [WPR][32 RD + 2]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long gw = (long long)blockIdx.x * ATT_WARPS + warp;
+  const long long gw = WPR == 1 ? (long long)blockIdx.x * ATT_WARPS + warp : (long long)blockIdx.x;
   if (gw >= (long long)T_tokens * nq) return;
   const int t = (int)(gw / nq), h = (int)(gw - (long long)t * nq);
   const int kvh = h / (nq / nkv);
@@ -79,87 +92,135 @@ attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out
   const int kept_start = (chunk > 0) ? min(qpos / chunk * chunk, kept_end) : 0;
   const float inv_cap = softcap > 0.f ? 1.0f / softcap : 0.f;
   const float slope = slopes ? slopes[h] : 0.f;
-  float* myq = qs + warp * d;
+  float* myq = WPR == 1 ? qs + warp * d : qs;
   const T* qrow = q + (size_t)t * q_stride + (size_t)h * d;
-  for (int i = lane; i < d; i += 32) myq[i] = to_f32(qrow[i]);
-  __syncwarp();
-
-  float m = -INFINITY, l = 0.f;
-  float acc[ATT_MAX_D / 32];
-#pragma unroll
-  for (int r = 0; r < ATT_MAX_D / 32; ++r) acc[r] = 0.f;
+  if (WPR == 1) {
+    for (int i = lane; i < d; i += 32) myq[i] = to_f32(qrow[i]);
+    __syncwarp();
+  } else {
+    for (int i = threadIdx.x; i < d; i += 32 * WPR) myq[i] = to_f32(qrow[i]);
+    __syncthreads();
+  }
   const int* bt = block_table + (size_t)s * max_blocks;
 
-  for (int range = 0; range < 2; ++range) {
-  const int lo = range == 0 ? kept_start : kstart, hi = range == 0 ? kept_end : kend;
-  for (int j0 = (lo / 32) * 32; j0 < hi; j0 += 32) {
-    const int j = j0 + lane;
-    const bool valid = (j >= lo) && (j < hi);
-    float score = -INFINITY;
-    int page = -1;
-    if (valid) {
-      page = bt[j / page_size];
-      if (page < 0 || page >= num_pages) {
-        atomicOr(err, 4);
-        page = -1;
-      } else {
-        const T* kp = kcache + (((size_t)page * pg_heads + pg_h) * page_size + (j % page_size)) * d;
-        float dot = 0.f;
-        if (VEC) {
-          for (int i = 0; i < d; i += 8) {
-            float kv[8];
-            Vec8<T>::load(kp + i, kv);
+  // the row's parts, the kept range's and then the recent range's
+  const int kept_first = kept_start / ATT_PART, kept_parts = kept_end > kept_start ? (kept_end - 1) / ATT_PART - kept_first + 1 : 0;
+  const int first = kstart / ATT_PART, parts = kept_parts + (kend - 1) / ATT_PART - first + 1;
+  float m_row = -INFINITY, l_row = 0.f, row[RD];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) dot = fmaf(myq[i + u], kv[u], dot);
+  for (int r = 0; r < RD; ++r) row[r] = 0.f;
+  for (int p0 = 0; p0 < parts; p0 += WPR) {
+    const int part = p0 + (WPR == 1 ? 0 : warp);
+    float m = -INFINITY, l = 0.f, acc[RD];
+#pragma unroll
+    for (int r = 0; r < RD; ++r) acc[r] = 0.f;
+    if (part < parts) {
+      const bool kept = part < kept_parts;
+      const int base = (kept ? kept_first + part : first + part - kept_parts) * ATT_PART;
+      const int lo = max(kept ? kept_start : kstart, base), hi = min(kept ? kept_end : kend, base + ATT_PART);
+      for (int j0 = (lo / 32) * 32; j0 < hi; j0 += 32) {
+        const int j = j0 + lane;
+        const bool valid = (j >= lo) && (j < hi);
+        float score = -INFINITY;
+        int page = -1;
+        if (valid) {
+          page = bt[j / page_size];
+          if (page < 0 || page >= num_pages) {
+            atomicOr(err, 4);
+            page = -1;
+          } else {
+            const T* kp = kcache + (((size_t)page * pg_heads + pg_h) * page_size + (j % page_size)) * d;
+            float dot = 0.f;
+            if (VEC) {
+#pragma unroll UK
+              for (int i = 0; i < d; i += 8) {
+                float kv[8];
+                Vec8<T>::load(kp + i, kv);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) dot = fmaf(myq[i + u], kv[u], dot);
+              }
+            } else {
+#pragma unroll UK
+              for (int i = 0; i < d; ++i) dot = fmaf(myq[i], to_f32(kp[i]), dot);
+            }
+            score = dot * scale;
+            if (softcap > 0.f) score = softcap * tanhf(score * inv_cap);
+            if (slopes) score -= slope * (float)(qpos - j);
           }
-        } else {
-          for (int i = 0; i < d; ++i) dot = fmaf(myq[i], to_f32(kp[i]), dot);
         }
-        score = dot * scale;
-        if (softcap > 0.f) score = softcap * tanhf(score * inv_cap);
-        if (slopes) score -= slope * (float)(qpos - j);
+        const float cmax = warp_max(score);
+        const float m_new = fmaxf(m, cmax);
+        if (m_new == -INFINITY) continue;  // nothing visible in this group (warp-uniform)
+        const float p = (score == -INFINITY) ? 0.f : expf(score - m_new);
+        const float corr = (m == -INFINITY) ? 0.f : expf(m - m_new);
+        l = l * corr + warp_sum(p);
+#pragma unroll
+        for (int r = 0; r < RD; ++r) acc[r] *= corr;
+        m = m_new;
+        const int jn = min(32, hi - j0);
+        for (int j8 = max(0, lo - j0) & ~(U - 1); j8 < jn; j8 += U) {
+          float pj[U], v[U][RD];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            pj[u] = __shfl_sync(0xffffffffu, p, j8 + u);
+            const int pg = __shfl_sync(0xffffffffu, page, j8 + u);
+            const T* vp = vcache + (((size_t)max(pg, 0) * pg_heads + pg_h) * page_size + ((j0 + j8 + u) % page_size)) * v_row + v_off;
+#pragma unroll
+            for (int r = 0; r < RD; ++r) v[u][r] = (pg >= 0 && lane + 32 * r < dv) ? to_f32(vp[lane + 32 * r]) : 0.f;
+          }
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int r = 0; r < RD; ++r) acc[r] = fmaf(pj[u], v[u][r], acc[r]);       // a key that is not there: 0 * 0
+        }
       }
     }
-    const float cmax = warp_max(score);
-    const float m_new = fmaxf(m, cmax);
-    if (m_new == -INFINITY) continue;  // nothing visible in this group (warp-uniform)
-    const float p = (score == -INFINITY) ? 0.f : expf(score - m_new);
-    const float corr = (m == -INFINITY) ? 0.f : expf(m - m_new);
-    l = l * corr + warp_sum(p);
+    // the partial results in order
+    auto add = [&](float pm, float pl, const float (&pa)[RD]) {
+      if (pm == -INFINITY) return;
+      const float m_new = fmaxf(m_row, pm);
+      const float old = (m_row == -INFINITY) ? 0.f : expf(m_row - m_new), now = expf(pm - m_new);
+      l_row = l_row * old + pl * now;
 #pragma unroll
-    for (int r = 0; r < ATT_MAX_D / 32; ++r) acc[r] *= corr;
-    m = m_new;
-    const int jn = min(32, hi - j0);
-    for (int jj = max(0, lo - j0); jj < jn; ++jj) {
-      const float pj = __shfl_sync(0xffffffffu, p, jj);
-      const int pg = __shfl_sync(0xffffffffu, page, jj);
-      if (pg < 0) continue;
-      const T* vp = vcache + (((size_t)pg * pg_heads + pg_h) * page_size + ((j0 + jj) % page_size)) * v_row + v_off;
+      for (int r = 0; r < RD; ++r) row[r] = row[r] * old + pa[r] * now;
+      m_row = m_new;
+    };
+    if (WPR == 1) {
+      add(m, l, acc);
+    } else {
+      float* mine = qs + d + warp * (32 * RD + 2);
 #pragma unroll
-      for (int r = 0; r < ATT_MAX_D / 32; ++r) {
-        const int i = lane + 32 * r;
-        if (i < dv) acc[r] = fmaf(pj, to_f32(vp[i]), acc[r]);
-      }
+      for (int r = 0; r < RD; ++r) mine[lane + 32 * r] = acc[r];
+      if (lane == 0) { mine[32 * RD] = m; mine[32 * RD + 1] = l; }
+      __syncthreads();
+      if (warp == 0)
+        for (int w = 0; w < WPR && p0 + w < parts; ++w) {
+          const float* theirs = qs + d + w * (32 * RD + 2);
+#pragma unroll
+          for (int r = 0; r < RD; ++r) acc[r] = theirs[lane + 32 * r];
+          add(theirs[32 * RD], theirs[32 * RD + 1], acc);
+        }
+      __syncthreads();
     }
   }
-  }
+  if (WPR != 1 && warp != 0) return;
   if (sinks) {                                   // one more term of the denominator
     const float sk = sinks[h];
-    const float m_new = fmaxf(m, sk);
-    const float corr = (m == -INFINITY) ? 0.f : expf(m - m_new);
-    l = l * corr + expf(sk - m_new);
+    const float m_new = fmaxf(m_row, sk);
+    const float corr = (m_row == -INFINITY) ? 0.f : expf(m_row - m_new);
+    l_row = l_row * corr + expf(sk - m_new);
 #pragma unroll
-    for (int r = 0; r < ATT_MAX_D / 32; ++r) acc[r] *= corr;
+    for (int r = 0; r < RD; ++r) row[r] *= corr;
   }
   T* orow = out + ((size_t)t * nq + h) * dv;
-  float inv = (l > 0.f) ? 1.0f / l : 0.f;
+  float inv = (l_row > 0.f) ? 1.0f / l_row : 0.f;
   const T* grow = gate_mode ? gate + (size_t)t * gate_stride : nullptr;
   if (gate_mode == 1) inv *= 1.0f / (1.0f + expf(-to_f32(grow[h])));
 #pragma unroll
-  for (int r = 0; r < ATT_MAX_D / 32; ++r) {
+  for (int r = 0; r < RD; ++r) {
     const int i = lane + 32 * r;
     if (i < dv) {
-      float v = acc[r] * inv;
+      float v = row[r] * inv;
       if (gate_mode == 2) v *= 1.0f / (1.0f + expf(-to_f32(grow[(size_t)h * dv + i])));
       orow[i] = from_f32<T>(v);
     }
@@ -182,16 +243,28 @@ RLLM_EXPORT int rllm_attention_simt_kv(const void* q, int q_stride, void* out, c
     return RLLM_E_BADARG;
   if (dv > ATT_MAX_D || d > 2816) return RLLM_E_UNSUPPORTED;
   const bool vec = d % 8 == 0 && q_stride % 8 == 0 && (((uintptr_t)q | (uintptr_t)kcache) & 31) == 0;
-  const long long warps = (long long)T * nq;
-  const unsigned blocks = (unsigned)((warps + ATT_WARPS - 1) / ATT_WARPS);
-  const size_t smem = (size_t)ATT_WARPS * d * sizeof(float);
-#define ATT_GO(VEC_)                                                                                        \
+  const long long rows = (long long)T * nq;
+  // Eight warps a row where rows are few and long (the block table's width bounds the keys): 792 rows x 1,033 keys 426 us
+  // with one warp, 227 with eight, 3,200 x 1,000 447 and 327, 32 x 101 27 and 24; but 2,048 rows x 64 keys 24 and 38,
+  // 6,400 x 300 184 and 294.
+  const long long keys = (long long)max_blocks * page_size;
+  const bool share = (rows <= 4096 && keys >= 512) || (rows <= 512 && keys >= 96);
+  const unsigned blocks = (unsigned)(share ? rows : (rows + ATT_WARPS - 1) / ATT_WARPS);
+  const int rd = dv <= 64 ? 2 : (dv <= 128 ? 4 : 8);
+  const size_t smem = (share ? (size_t)d + 8 * (32 * rd + 2) : (size_t)ATT_WARPS * d) * sizeof(float);
+#define ATT_ONE(VEC_, RD_, WPR_)                                                                            \
   RLLM_DISPATCH_DTYPE(dtype, T_,                                                                            \
-    (attention_simt_kernel<T_, VEC_><<<blocks, 32 * ATT_WARPS, smem, stream>>>(                             \
+    (attention_simt_kernel<T_, VEC_, RD_, WPR_><<<blocks, 32 * (WPR_ == 1 ? ATT_WARPS : WPR_), smem, stream>>>(  \
         (const T_*)q, q_stride, (T_*)out, (const T_*)kcache, (const T_*)vcache, block_table,                \
         max_blocks, positions, token_seq, T, nq, nkv, d, dv, page_size, num_pages, window, scale, keep_first,  \
         chunk, softcap, sinks, (const T_*)gate, gate_stride, gate_mode, slopes, shared_keys, v_ld, err)))
+#define ATT_GO(VEC_)                                                                                        \
+  do {                                                                                                      \
+    if (share) { if (rd == 2) ATT_ONE(VEC_, 2, 8); else if (rd == 4) ATT_ONE(VEC_, 4, 8); else ATT_ONE(VEC_, 8, 8); }  \
+    else { if (rd == 2) ATT_ONE(VEC_, 2, 1); else if (rd == 4) ATT_ONE(VEC_, 4, 1); else ATT_ONE(VEC_, 8, 1); }        \
+  } while (0)
   if (vec) ATT_GO(true); else ATT_GO(false);
+#undef ATT_ONE
 #undef ATT_GO
   RLLM_LAUNCH_CHECK();
   return 0;
