@@ -122,8 +122,9 @@ causal_conv_run_kernel(const T* x, int stride, const TW* w, const TW* bias, floa
 
 // Four taps, bfloat16 rows in steps of four channels on 8-byte boundaries (prompt portions): a thread takes four channels and
 // CV_RUN tokens.  Where a run lies in one sequence, which is nearly always, all its inputs are asked for at once; a token at
-// a time behind the last one's arithmetic, one channel a thread, 2,048 x 4,608 took 37 us, 29 so, 20 with the short silu
-// (38 MB; 6 us at the copy rate).  The same sums in the same order.
+// a time behind the last one's arithmetic, one channel a thread, 2,048 x 4,608 took 37 us, 29 so (38 MB; 6 us at the copy rate;
+// the exponential and the division of silu bound it).  The same sums in the same order and the same silu as
+// causal_conv_run_kernel: a decoded token has the same bits whether or not another sequence of the step brings a prompt.
 template <typename TW>
 __global__ void __launch_bounds__(128)
 causal_conv4_kernel(const bf16* x, int stride, const TW* w, const TW* bias, float* tail, const int* q_start,
@@ -151,7 +152,7 @@ causal_conv4_kernel(const bf16* x, int stride, const TW* w, const TW* bias, floa
       float acc = b[i];
 #pragma unroll
       for (int k = 0; k < 4; ++k) acc = fmaf(wv[i][k], win[k][i], acc);
-      o[i] = fast_silu(acc);
+      o[i] = ss_silu(acc);
     }
     uint2 raw;
     *(__nv_bfloat162*)&raw.x = __floats2bfloat162_rn(o[0], o[1]);

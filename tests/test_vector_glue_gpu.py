@@ -88,8 +88,7 @@ def test_pairs_sorted_by_expert(P, E, bm):
 @pytest.mark.parametrize("lens", [[1], [8], [2, 1, 1, 30, 3], [9, 17], [64], [1, 7, 8, 1]])
 @pytest.mark.parametrize("E,pad,bias", [(4, 0, True), (512, 4, True), (516, 8, False), (1028, 2, True)])
 def test_convolution_of_prompt_portions(lens, E, pad, bias):
-    """Runs of eight tokens within a sequence, across sequences and behind the last; tails that go on from before; the same
-    numbers as a token at a time."""
+    """Runs of eight tokens within a sequence, across sequences and behind the last; tails that go on from before."""
     from rllm_b200.kernels import ops
     r = gen(E + sum(lens))
     T, S = sum(lens), len(lens)
@@ -109,3 +108,32 @@ def test_convolution_of_prompt_portions(lens, E, pad, bias):
         assert torch.equal(new[slots[s].long()], past[n:].float())
         at += n
     assert int(err) == 0 and torch.equal(new[0], tail[0])
+
+
+def conv_of(x, w, b, tail, lens, any_long):
+    from rllm_b200.kernels import ops
+    S = len(lens)
+    starts = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device="cuda")
+    seq = torch.repeat_interleave(torch.arange(S, dtype=torch.int32), torch.tensor(lens)).cuda()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = ops.causal_conv(x, w, b, tail, starts, seq, torch.arange(S, dtype=torch.int32, device="cuda"), S, any_long, err)
+    assert int(err) == 0
+    return out
+
+
+@pytest.mark.parametrize("E", [512, 4608])
+def test_a_decoded_token_of_the_convolution_does_not_depend_on_its_batch(E):
+    """The same bits in a step of decoded tokens and beside a prompt portion, and the portion the same bits whether its
+    rows are read four channels at a time or one; sums of -100 to 100, where an exponential is least good."""
+    r = gen(E)
+    x, w, b = (r(45, E) * 20).bfloat16(), r(E, 4), r(E) * 0.1
+    alone, mixed, single = (r(6, 3, E) for _ in range(3))
+    mixed.copy_(alone)
+    single.copy_(alone)
+    decoded = conv_of(x[:5], w, b, alone, [1] * 5, False)
+    both = conv_of(x, w, b, mixed, [1] * 5 + [40], True)
+    assert torch.equal(decoded, both[:5]) and torch.equal(alone[:5], mixed[:5])
+    odd = torch.zeros(45, E + 1, dtype=torch.bfloat16, device="cuda")[:, 1:]
+    odd.copy_(x)                                           # rows on 2-byte boundaries: one channel a thread
+    assert torch.equal(conv_of(odd, w, b, single, [1] * 5 + [40], True), both) and torch.equal(single, mixed)
+    assert float(both.float().min()) < -0.2 and float(both.float().max()) > 50
