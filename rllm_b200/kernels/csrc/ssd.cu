@@ -98,13 +98,15 @@ silu_gated_group_rmsnorm_kernel(const float* y, const T* z, int z_stride, const 
 }
 
 // The same for bfloat16 gates and results where rows and groups start on 16 bytes: eight values an access, all of a
-// thread's loads on their way before the sum.  2,048 x 4,096 in two groups: 44.6 us with single values, 24.8 so, 17.9
-// with the gate's short sigmoid (67 MB; 10 us at the copy rate).
+// thread's loads on their way before the sum.  The sum runs over shared memory in the order of the form above, so that a
+// row has the same bits wherever it starts.  2,048 x 4,096 in two groups, 67 MB: 44.6 us with single values, 10 at the copy
+// rate; the gates' exponentials and divisions bound it.
 #define SGN_KEEP 4
 __global__ void __launch_bounds__(256)
 silu_gated_group_rmsnorm8_kernel(const float* y, const bf16* z, int z_stride, const float* w, bf16* out, int E, int size,
                                  float eps) {
   __shared__ float red[32];
+  extern __shared__ __align__(16) float sgn_x[];        // [size]
   pdl_wait();
   pdl_launch();
   const size_t base = (size_t)blockIdx.x * E + (size_t)blockIdx.y * size;
@@ -122,16 +124,19 @@ silu_gated_group_rmsnorm8_kernel(const float* y, const bf16* z, int z_stride, co
     }
   }
 #pragma unroll
-  for (int u = 0; u < SGN_KEEP; ++u)
-    if ((threadIdx.x + u * blockDim.x) * 8 < size) {
+  for (int u = 0; u < SGN_KEEP; ++u) {
+    const int i = (threadIdx.x + u * blockDim.x) * 8;
+    if (i < size) {
       float zv[8];
       unpack8(gate[u], zv);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        v[u][j] *= fast_silu(zv[j]);
-        ss = fmaf(v[u][j], v[u][j], ss);
-      }
+      for (int j = 0; j < 8; ++j) v[u][j] *= lt_silu(zv[j]);
+      *(float4*)(sgn_x + i) = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
+      *(float4*)(sgn_x + i + 4) = make_float4(v[u][4], v[u][5], v[u][6], v[u][7]);
     }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < size; i += blockDim.x) ss = fmaf(sgn_x[i], sgn_x[i], ss);
   ss = block_sum(ss, red);
   const float r = 1.0f / sqrtf(ss / (float)size + eps);
 #pragma unroll
@@ -157,7 +162,7 @@ RLLM_EXPORT int rllm_silu_gated_group_rmsnorm(const float* y, const void* z, int
   threads = threads < 32 ? 32 : (threads > 256 ? 256 : threads);
   if (dtype == RLLM_DT_BF16 && size % 8 == 0 && size <= 256 * 8 * SGN_KEEP && z_stride % 8 == 0 &&
       (((uintptr_t)y | (uintptr_t)z | (uintptr_t)w | (uintptr_t)out) & 15) == 0) {
-    rllm_launch_pdl(silu_gated_group_rmsnorm8_kernel, dim3(T, groups), dim3(threads), (size_t)0, stream, y, (const bf16*)z,
+    rllm_launch_pdl(silu_gated_group_rmsnorm8_kernel, dim3(T, groups), dim3(threads), (size_t)size * 4, stream, y, (const bf16*)z,
                     z_stride, w, (bf16*)out, E, size, eps);
     RLLM_LAUNCH_CHECK();
     return 0;

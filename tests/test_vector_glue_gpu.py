@@ -137,3 +137,30 @@ def test_a_decoded_token_of_the_convolution_does_not_depend_on_its_batch(E):
     odd.copy_(x)                                           # rows on 2-byte boundaries: one channel a thread
     assert torch.equal(conv_of(odd, w, b, single, [1] * 5 + [40], True), both) and torch.equal(single, mixed)
     assert float(both.float().min()) < -0.2 and float(both.float().max()) > 50
+
+
+def shifted(t):
+    """The same rows one element further, where they no longer start on 16 bytes."""
+    wide = torch.zeros(t.shape[0], t.shape[1] + 1, dtype=t.dtype, device="cuda")
+    wide[:, 1:] = t
+    return wide[:, 1:]
+
+
+# gates at which an exponential or a reciprocal of fewer bits shows: e^-x large, near the largest float32, and past it
+EDGES = (-5.0, -20.0, -60.0, -86.0, -88.0, -100.0, 20.0, 100.0)
+
+
+@pytest.mark.parametrize("T,E,groups", [(3, 4096, 2), (7, 64, 4), (2, 8192, 1), (3, 360, 3), (33, 2048, 1)])
+def test_group_rmsnorm_has_the_bits_of_its_single_value_form(T, E, groups):
+    from rllm_b200.kernels import ops
+    r = gen(E)
+    y, z, w = r(T, E) * 2, (r(T, E) * 8).bfloat16(), 1 + 0.1 * r(E)
+    for i, v in enumerate(EDGES):
+        z[:, i::11] = v
+    y[-1] *= 1e33                                          # a row whose small gates carry it
+    z[-1] = -88.0
+    got = ops.silu_gated_group_rmsnorm(y, z, w, 1e-5, groups, torch.bfloat16)
+    assert torch.equal(got, ops.silu_gated_group_rmsnorm(y, shifted(z), w, 1e-5, groups, torch.bfloat16))
+    v = (y.double() * torch.nn.functional.silu(z.double())).view(T, groups, -1)
+    want = (v * torch.rsqrt(v.square().mean(-1, keepdim=True) + 1e-5)).view(T, E) * w.double()
+    assert close(got, want, 8.0)
