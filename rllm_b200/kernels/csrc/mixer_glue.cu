@@ -320,13 +320,15 @@ RLLM_EXPORT int rllm_rms_mean2(const void* a, const void* b, const void* wa, con
 }
 
 // The same for bfloat16 rows of up to 8,192 values that start on 16 bytes: eight values an access, all of a thread's loads
-// on their way before the sum, nothing read twice.  2,048 x 2,048: 19.4 us with single values in two passes, 12.8
-// so, 10.1 with the gate's short sigmoid (33 MB; 5 us at the copy rate).
+// on their way before the sum, nothing read twice.  The sum runs over shared memory in the order of the form below (256
+// threads), so that a row has the same bits wherever it starts.  2,048 x 2,048, 33 MB: 19.4 us with single values in two
+// passes, 5 at the copy rate; the gates' exponentials and divisions bound it.
 #define GRN_KEEP 4
 template <typename TW>
 __global__ void __launch_bounds__(256)
 gated_rmsnorm8_kernel(const float* x, const bf16* g, int g_stride, const TW* w, bf16* out, int H, float eps) {
   __shared__ float red[32];
+  extern __shared__ __align__(16) float grn_x[];        // [H]
   pdl_wait();
   pdl_launch();
   const size_t base = (size_t)blockIdx.x * H;
@@ -343,11 +345,15 @@ gated_rmsnorm8_kernel(const float* x, const bf16* g, int g_stride, const TW* w, 
     }
   }
 #pragma unroll
-  for (int u = 0; u < GRN_KEEP; ++u)
-    if ((threadIdx.x + u * blockDim.x) * 8 < H) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) ss = fmaf(v[u][j], v[u][j], ss);
+  for (int u = 0; u < GRN_KEEP; ++u) {
+    const int i = (threadIdx.x + u * blockDim.x) * 8;
+    if (i < H) {
+      *(float4*)(grn_x + i) = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
+      *(float4*)(grn_x + i + 4) = make_float4(v[u][4], v[u][5], v[u][6], v[u][7]);
     }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < H; i += blockDim.x) ss = fmaf(grn_x[i], grn_x[i], ss);
   ss = block_sum(ss, red);
   const float r = 1.0f / sqrtf(ss / (float)H + eps);
 #pragma unroll
@@ -358,7 +364,7 @@ gated_rmsnorm8_kernel(const float* x, const bf16* g, int g_stride, const TW* w, 
       load8(w + i, wv);
       unpack8(gate[u], gv);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[u][j] = v[u][j] * r * wv[j] * fast_sigmoid(gv[j]);
+      for (int j = 0; j < 8; ++j) v[u][j] = v[u][j] * r * wv[j] * (1.0f / (1.0f + expf(-gv[j])));
       store8(out + base + i, v[u]);
     }
   }
@@ -389,8 +395,7 @@ RLLM_EXPORT int rllm_gated_rmsnorm(const float* x, const void* g, int g_stride, 
   if (H <= 0) return RLLM_E_BADARG;
   if (dtype == RLLM_DT_BF16 && H % 8 == 0 && H <= 256 * 8 * GRN_KEEP && g_stride % 8 == 0 &&
       (((uintptr_t)x | (uintptr_t)g | (uintptr_t)w | (uintptr_t)out) & 15) == 0) {
-    const int threads = min(256, (H / 8 + 31) / 32 * 32);
-    RLLM_DISPATCH_DTYPE(w_dtype, TW, (rllm_launch_pdl(gated_rmsnorm8_kernel<TW>, dim3(T), dim3(threads), (size_t)0, stream,
+    RLLM_DISPATCH_DTYPE(w_dtype, TW, (rllm_launch_pdl(gated_rmsnorm8_kernel<TW>, dim3(T), dim3(256), (size_t)H * 4, stream,
                                                       x, (const bf16*)g, g_stride, (const TW*)w, (bf16*)out, H, eps)));
     RLLM_LAUNCH_CHECK();
     return 0;

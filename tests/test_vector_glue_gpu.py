@@ -164,3 +164,16 @@ def test_group_rmsnorm_has_the_bits_of_its_single_value_form(T, E, groups):
     v = (y.double() * torch.nn.functional.silu(z.double())).view(T, groups, -1)
     want = (v * torch.rsqrt(v.square().mean(-1, keepdim=True) + 1e-5)).view(T, E) * w.double()
     assert close(got, want, 8.0)
+
+
+@pytest.mark.parametrize("T,H,wd", [(5, 8, "float32"), (3, 2048, "float32"), (2, 8192, "bfloat16"), (4, 264, "float32"), (33, 1000, "bfloat16")])
+def test_gated_rmsnorm_has_the_bits_of_its_single_value_form(T, H, wd):
+    from rllm_b200.kernels import ops
+    r = gen(H)
+    x, g, w = r(T, H) * 3, (r(T, H) * 8).bfloat16(), (1 + 0.1 * r(H)).to(getattr(torch, wd))
+    for i, v in enumerate(EDGES):
+        g[:, i::11] = v
+    got = ops.gated_rmsnorm(x, g, w, 1e-5, torch.bfloat16)
+    assert torch.equal(got, ops.gated_rmsnorm(x, shifted(g), w, 1e-5, torch.bfloat16))
+    want = x.double() * torch.rsqrt(x.double().square().mean(1, keepdim=True) + 1e-5) * w.double() * torch.sigmoid(g.double())
+    assert close(got, want, 4.0)
