@@ -75,12 +75,6 @@ __device__ __forceinline__ float block_sum(float v, float* smem32) {
   return t;
 }
 
-// 1 / (1 + e^-x) and x times it with the special-function unit's exponential and reciprocal (about 2^-21 of the result),
-// for results that are rounded to bfloat16; expf and a division take four times the instructions, which bounds the kernels
-// that do little else
-__device__ __forceinline__ float fast_sigmoid(float x) { return __fdividef(1.0f, 1.0f + __expf(-x)); }
-__device__ __forceinline__ float fast_silu(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
-
 // The gate of a gated feed-forward: g' sigmoid(slope g') (u' + shift) with g' = min(g, limit) and u' = u kept within
 // +-limit.  {infinity, 1, 0}: silu(g) u.
 struct GateAct { float limit, slope, shift; };

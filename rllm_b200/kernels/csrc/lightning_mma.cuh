@@ -139,8 +139,8 @@ __device__ __forceinline__ void ltc_stage_rows(bf16 (*dst)[W + 8], const bf16* s
 
 // The same in two halves for rows of 16-byte aligned, whole heads: what a thread stages of an array, eight values a load,
 // all of them on their way before any is used (array after array, each staged before the next was asked for, left a
-// block four trips to L2 one after the other.  2,048 tokens, 16 heads of 128 x 128: end states 23 -> 18 us, outputs 79 -> 41;
-// 64 heads of 128 x 64: 39 -> 32 and 125 -> 71).
+// block four trips to L2 one after the other.  2,048 tokens, 64 heads of 128 x 64, nothing activated: end states 39 -> 32 us,
+// outputs 125 -> 71).  The same activation as the walk's and that of fewer values a load: the same bits.
 template <int W> struct LtcRows {
   static constexpr int N = LTC_CHUNK * W / (LTC_THREADS * 8);
   uint4 raw[N];
@@ -162,7 +162,7 @@ template <int W> struct LtcRows {
         float v[8];
         unpack8(raw[u], v);
 #pragma unroll
-        for (int x = 0; x < 8; ++x) v[x] = fast_silu(v[x]);
+        for (int x = 0; x < 8; ++x) v[x] = lt_silu(v[x]);
         store8(&dst[j][c], v);
       }
     }
@@ -208,7 +208,7 @@ lightning_mma_pass1_kernel(const bf16* k, const bf16* v, int stride, int wide, c
       unpack8(rk.raw[u], o);
 #pragma unroll
       for (int x = 0; x < 8; ++x) {
-        const float kw = (STEPS ? o[x] : __bfloat162float(__float2bfloat16_rn(fast_silu(o[x])))) * w;   // the rounded key, weighted
+        const float kw = (STEPS ? o[x] : __bfloat162float(__float2bfloat16_rn(lt_silu(o[x])))) * w;   // the rounded key, weighted
         hi[x] = __bfloat162float(__float2bfloat16_rn(kw));
         lo[x] = kw - hi[x];
       }

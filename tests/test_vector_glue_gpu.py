@@ -177,3 +177,27 @@ def test_gated_rmsnorm_has_the_bits_of_its_single_value_form(T, H, wd):
     assert torch.equal(got, ops.gated_rmsnorm(x, shifted(g), w, 1e-5, torch.bfloat16))
     want = x.double() * torch.rsqrt(x.double().square().mean(1, keepdim=True) + 1e-5) * w.double() * torch.sigmoid(g.double())
     assert close(got, want, 4.0)
+
+
+@pytest.mark.parametrize("heads,d,dv", [(3, 32, 64), (2, 64, 128), (2, 128, 128)])
+def test_chunk_passes_have_the_same_bits_wherever_rows_start(heads, d, dv):
+    """Rows on 16-byte boundaries (eight values a load), on 8-byte boundaries and on 4-byte boundaries."""
+    from rllm_b200.kernels import ops
+    r = gen(d + dv)
+    T, cols = 1000, heads * (2 * d + dv)
+    a = (r(T, cols) * 12).bfloat16()
+    for i, v in enumerate(EDGES):
+        a[:, i::13] = v
+    outs = []
+    for pad in (0, 4, 2):
+        wide = torch.zeros(T, cols + pad, dtype=torch.bfloat16, device="cuda")
+        wide[:, pad:] = a
+        q, k, v = wide[:, pad: pad + heads * d], wide[:, pad + heads * d: pad + 2 * heads * d], wide[:, pad + 2 * heads * d:]
+        state, err = r(1, heads, d, dv) * 0 + 0.5, torch.zeros(1, dtype=torch.int32, device="cuda")
+        decay = torch.linspace(0.9, 0.99, heads, device="cuda")
+        o = ops.lightning_scan(q, k, v, decay, state, torch.tensor([0, T], dtype=torch.int32, device="cuda"),
+                               torch.zeros(1, dtype=torch.int32, device="cuda"), 1, err, max_q_len=T)
+        assert int(err) == 0
+        outs.append((o, state))
+    for o, state in outs[1:]:
+        assert torch.equal(o, outs[0][0]) and torch.equal(state, outs[0][1])
