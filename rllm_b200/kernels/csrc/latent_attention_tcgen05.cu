@@ -118,12 +118,13 @@ latent_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, bf16* out, cons
         page[i] = it < ntiles && j < kend ? bt[j / page_size] : -2;
       }
     };
-    int at[2];                                    // the rows' places in the cache; -1: zeros
+    int at[2];                                    // the rows' places in the cache; -1: zeros (also for rows that the window
+                                                  // hides from all of this CTA's queries: 0 times infinity is no 0)
     auto find = [&](int it) {
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int j = (tile_lo + it) * LT_BN + lane + 32 * i;
-        at[i] = page[i] >= 0 && page[i] < num_pages ? page[i] * page_size + j % page_size : -1;
+        at[i] = page[i] >= 0 && page[i] < num_pages && j >= kmin ? page[i] * page_size + j % page_size : -1;
         if (at[i] < 0 && page[i] != -2 && j >= kmin) atomicOr(err, 4);   // a visible key without a page
       }
     };

@@ -78,3 +78,32 @@ def test_which_prompt_portions_take_the_tcgen05_latent_attention(monkeypatch):
     assert not ops.latent_attention_tcgen05_takes(torch.bfloat16, 576, 512, 4096, c.view(-1)[4:])
     monkeypatch.setenv("RLLM_LATENT_ATTENTION", "mma")
     assert not ops.latent_attention_tcgen05_takes(torch.bfloat16, 576, 512, 4096, c)
+
+
+@pytest.mark.parametrize("heads,dk,dv,window", [(16, 576, 512, 100), (8, 288, 256, 40), (128, 144, 128, 1)])
+def test_rows_that_the_window_hides_do_not_reach_the_output(heads, dk, dv, window):
+    """Rows behind every query's window that still have their page hold infinities and NaN."""
+    from rllm_b200.kernels import ops
+    g = torch.Generator(device="cuda")
+    g.manual_seed(dk)
+    n, m, page = 300, 24, 16
+    first = n - m - window + 1                             # the oldest key that the oldest query sees
+    rows = torch.randn(n, dk, generator=g, device="cuda").bfloat16()
+    cache = torch.zeros(-(-n // page), 1, page, dk, dtype=torch.bfloat16, device="cuda")
+    cache.view(-1, dk)[:n] = rows
+    cache.view(-1, dk)[:first] = math.inf
+    cache.view(-1, dk)[:first:3] = math.nan
+    table = torch.arange(cache.shape[0], dtype=torch.int32, device="cuda")[None].contiguous()
+    q = torch.randn(m, heads * dk, generator=g, device="cuda").bfloat16()
+    out, err = torch.empty(m, heads * dv, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    ops.latent_attention_tcgen05(q, out, cache, table, torch.tensor([0, m], dtype=torch.int32, device="cuda"),
+                                 torch.tensor([n], dtype=torch.int32, device="cuda"), 0, 1, m, heads, dk, dv, window, dk ** -0.5,
+                                 None, err)
+    assert int(err) == 0
+    pos, key = torch.arange(n - m, n, device="cuda")[:, None], torch.arange(n, device="cuda")
+    hidden = (key > pos) | (key <= pos - window)
+    sc = torch.einsum("mhd,kd->hmk", q.view(m, heads, dk).double(), rows.double()) * dk ** -0.5
+    p = torch.softmax(sc.masked_fill(hidden, -math.inf), 2)
+    want, size = p @ rows[:, :dv].double(), p @ rows[:, :dv].double().abs()
+    got = out.view(m, heads, dv).transpose(0, 1).double()
+    assert bool(((got - want).abs() <= 2.0 ** -7 * size + 1e-5).all())       # the bound of the test above
