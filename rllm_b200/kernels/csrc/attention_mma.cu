@@ -903,12 +903,8 @@ static int launch_prefill(const bf16* q, int q_stride, bf16* out, const bf16* kc
   const int bq = BM / g;
   const int tiles = (num_tokens + bq - 1) / bq + (seq_end - seq_begin);
   const size_t smem = prefill_smem<D>();
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_prefill_kernel<D, OPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SmemLimit limit;
+  if (const int e = limit.allow(attention_prefill_kernel<D, OPT>, smem)) return e;
   if ((long long)tiles * nkv > 0x7fffffffLL) return RLLM_E_UNSUPPORTED;
   dim3 grid(tiles * nkv);
   attention_prefill_kernel<D, OPT><<<grid, NTHREADS, smem, stream>>>(q, q_stride, out, kc, vc, bt, max_blocks, q_start,
@@ -989,13 +985,8 @@ static int launch_decode_small(int warps, bf16* qkv, int q_stride, bf16* out, bf
                              cudaStream_t stream, int small_below, AttnOpts opt) {
   if (SMALL) max_chunks *= CHUNK / CHUNK_SMALL;      // the grid and the workspace's stride: room for the smaller chunks
   const size_t smem = (size_t)warps * dec_warp_smem<D, STAGES, TBN>();
-  static size_t configured = 0;
-  if (smem > configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_decode_kernel<D, STAGES, TBN, SMALL, OPT>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    configured = smem;
-  }
+  static SmemLimit limit;
+  if (const int e = limit.allow(attention_decode_kernel<D, STAGES, TBN, SMALL, OPT>, smem)) return e;
   float* ws_o = ws;
   float* ws_ml = ws + (size_t)num_seqs * nq * max_chunks * D;
   const unsigned per_seq = (unsigned)((max_chunks + warps - 1) / warps);

@@ -525,12 +525,8 @@ static int at_launch(const void* q, int q_stride, int num_q_rows, void* out, con
     rc = at_encode(&mv, 2, vcache, dims, strides, box);
     if (rc) return rc;
   }
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attention_tcgen05_kernel<D, OPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, at_smem_bytes<D>());
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SmemLimit limit;
+  if (const int e = limit.allow(attention_tcgen05_kernel<D, OPT>, at_smem_bytes<D>())) return e;
   const int bq = AT_BM / g;
   const long long tiles = (num_tokens + bq - 1) / bq + (seq_end - seq_begin);
   if (tiles * nkv > 0x7fffffffLL) return RLLM_E_UNSUPPORTED;

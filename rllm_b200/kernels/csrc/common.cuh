@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include "smem_limit.h"
 
 #define RLLM_DT_F32 0
 #define RLLM_DT_BF16 1

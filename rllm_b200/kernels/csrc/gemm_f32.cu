@@ -112,13 +112,8 @@ template <int BM, int BN, int TM, int TN, int BK, int STAGES, bool VEC>
 static int gf_launch(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K,
                      cudaStream_t stream) {
   typedef GemmF32<BM, BN, TM, TN, BK, STAGES> S;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_f32_kernel<BM, BN, TM, TN, BK, STAGES, VEC>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SmemLimit limit;
+  if (const int e = limit.allow(gemm_f32_kernel<BM, BN, TM, TN, BK, STAGES, VEC>, S::SMEM)) return e;
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   if (grid.y > 65535) return RLLM_E_UNSUPPORTED;
   gemm_f32_kernel<BM, BN, TM, TN, BK, STAGES, VEC><<<grid, S::THREADS, S::SMEM, stream>>>(A, lda, W, ldw, C, ldc, M, N, K);

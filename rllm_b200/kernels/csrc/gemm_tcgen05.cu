@@ -226,13 +226,8 @@ template <int BN, int EPI, bool HEADS>
 static int tg_run(const CUtensorMap& ma, const CUtensorMap& mw, void* out, int ldo, int M, int N, int K, int up_offset,
                   int heads, long long c_head, int* err, cudaStream_t stream, GateAct ga) {
   constexpr int NOUT = (EPI == TG_EPI_SILU) ? BN / 2 : BN;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, EPI, HEADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         tg_smem_bytes<BN>());
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SmemLimit limit;
+  if (const int e = limit.allow(gemm_tcgen05_kernel<BN, EPI, HEADS>, tg_smem_bytes<BN>())) return e;
   const int tiles_m = (M + TG_BM - 1) / TG_BM, tiles_n = (N + NOUT - 1) / NOUT;
   const long long num_tiles = (long long)tiles_m * tiles_n * heads;
   if (num_tiles > (1ll << 30)) return RLLM_E_UNSUPPORTED;

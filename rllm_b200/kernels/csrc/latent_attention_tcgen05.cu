@@ -397,12 +397,8 @@ RLLM_EXPORT int rllm_latent_attention_tcgen05(const void* q, int num_q_rows, voi
   if (rc) return rc;
   const int panels = (dk + 63) / 64, parts = (dv + 64 * LT_VP - 1) / (64 * LT_VP);
   const int sets = lt_smem(panels, 2) <= LT_SMEM_MAX ? 2 : 1, smem = lt_smem(panels, sets);
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(latent_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LT_SMEM_MAX);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SmemLimit limit;
+  if (const int e = limit.allow(latent_tcgen05_kernel, LT_SMEM_MAX)) return e;
   const long long tiles = (((long long)num_tokens * heads + LT_BM - 1) / LT_BM + (seq_end - seq_begin)) * parts;
   if (tiles > 0x7fffffffLL) return RLLM_E_UNSUPPORTED;
   latent_tcgen05_kernel<<<dim3((unsigned)tiles), LT_THREADS, smem, stream>>>(

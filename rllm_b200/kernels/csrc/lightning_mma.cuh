@@ -467,12 +467,9 @@ static bool ltc_launch(const bf16* q, const bf16* k, const bf16* v, int stride, 
                        int dv, cudaStream_t stream, Chain chain) {
   const dim3 grid(heads, num_seqs * max_chunks);
   const size_t s1 = sizeof(LtcSmem1<D, DV>), s2 = sizeof(LtcSmem2<D, DV / LtcSplit<D, DV>::N>);
-  static bool allowed = false;
-  if (!allowed) {
-    cudaFuncSetAttribute(lightning_mma_pass1_kernel<D, DV, STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1);
-    cudaFuncSetAttribute(lightning_mma_pass2_kernel<D, DV, STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2);
-    allowed = true;
-  }
+  static SmemLimit limit1, limit2;                  // (refused: the launch then says so)
+  limit1.allow(lightning_mma_pass1_kernel<D, DV, STEPS>, s1);
+  limit2.allow(lightning_mma_pass2_kernel<D, DV, STEPS>, s2);
   // rows that start on 8-byte boundaries are fetched four values a load, on 16-byte boundaries (whole heads) eight
   const int wide8 = stride % 8 == 0 && d % 8 == 0 && dv % 8 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) == 0;
   const int wide = wide8 ? 2 : (stride % 4 == 0 && d % 4 == 0 && dv % 4 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 7) == 0);

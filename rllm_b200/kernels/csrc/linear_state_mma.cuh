@@ -613,14 +613,9 @@ static int lsm_launch(const bf16* a, LsArgs p, const float2* table, float* state
                       const int* slots, int num_slots, int num_seqs, int chunk0, int max_chunks, bf16* out, int* err,
                       cudaStream_t stream) {
   const size_t s1 = sizeof(LsmSmem1<D, DV, GATE>), s2 = sizeof(LsmSmem2<D, DV, GATE>);
-  static bool allowed = false;
-  if (!allowed) {
-    cudaError_t e = cudaFuncSetAttribute(ls_mma_pass1_kernel<D, DV, GATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(ls_mma_pass2_kernel<D, DV, GATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s2);
-    if (e != cudaSuccess) return (int)e;
-    allowed = true;
-  }
+  static SmemLimit limit1, limit2;
+  if (const int e = limit1.allow(ls_mma_pass1_kernel<D, DV, GATE>, s1)) return e;
+  if (const int e = limit2.allow(ls_mma_pass2_kernel<D, DV, GATE>, s2)) return e;
   // rows that start on 8-byte boundaries are fetched four values a load (the rotated pairs' partners too)
   const int wide = p.stride % 4 == 0 && p.d % 4 == 0 && p.dv % 4 == 0 && p.rd % 8 == 0 && (((uintptr_t)a) & 7) == 0 &&
                    (((uintptr_t)p.lower | (uintptr_t)p.f_bias) & 15) == 0;

@@ -244,12 +244,8 @@ template <bool GATE>
 static int moe_tcgen05_launch(const CUtensorMap& mw, const CUtensorMap& mb, const void* h, void* out, const int* offsets,
                               const int* sorted, const int* tile_expert, const int* tile_row0, const int* meta,
                               int max_tiles, int K, int n_out, int top, GateAct ga, int* err, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(moe_tcgen05_kernel<GATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, MT_SMEM);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SmemLimit limit;
+  if (const int e = limit.allow(moe_tcgen05_kernel<GATE>, MT_SMEM)) return e;
   const int tiles_f = (n_out + (GATE ? 127 : 255)) / (GATE ? 128 : 256);
   const long long tiles = (long long)max_tiles * tiles_f;
   if (tiles > (1ll << 30)) return RLLM_E_UNSUPPORTED;

@@ -619,12 +619,8 @@ static int sample_cluster_launch(const float* logits, int R, int V, int ld, cons
   while (cs > 1 && (cs / 2) * 2048 >= V) cs /= 2;
   const long long range = (long long)((((V + cs - 1) / cs) + 3) & ~3) * 4;
   const int staged = range <= SC_STAGED_MAX ? 1 : 0;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(sample_cluster_kernel<THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SC_STAGED_MAX + SC_SELECT_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SmemLimit limit;
+  if (const int e = limit.allow(sample_cluster_kernel<THREADS>, SC_STAGED_MAX + SC_SELECT_BYTES)) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cs, R); cfg.blockDim = dim3(THREADS);
   cfg.dynamicSmemBytes = (staged ? (size_t)range : 0) + (select ? SC_BINS * 12 + SC_BINS * 8 / cs : 0); cfg.stream = stream;

@@ -389,13 +389,8 @@ static int sk_launch(const void* q, int num_q_rows, void* out, const void* kcach
     if (rc) return rc;
   }
   const int smem = sk_smem<DV, BIG>(panels);
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(shared_key_tcgen05_kernel<DV, BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         sk_smem<DV, BIG>(BIG ? 8 : 4));
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
+  static SmemLimit limit;
+  if (const int e = limit.allow(shared_key_tcgen05_kernel<DV, BIG>, sk_smem<DV, BIG>(BIG ? 8 : 4))) return e;
   const int bq = SK_BM / g;
   const long long tiles = (num_tokens + bq - 1) / bq + (seq_end - seq_begin);
   if (tiles * nkv > 0x7fffffffLL) return RLLM_E_UNSUPPORTED;
