@@ -896,9 +896,13 @@ HEAD_GEMM_TCGEN05_FROM = 1 << 21
 
 
 def head_gemm_tcgen05_takes(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor) -> bool:
-    """Whether the tcgen05 kernel takes ``head_gemm``'s operands ([heads, N, K] weights): what TMA can address.
-    RLLM_TILE_GEMM=simt and RLLM_GEMM=library|no_tcgen05 keep it off."""
-    return (a.dtype is torch.bfloat16 and a.shape[2] % 8 == 0 and a.stride(0) % 8 == 0 and a.stride(1) % 8 == 0
+    """Whether the tcgen05 kernel takes ``head_gemm``'s operands ([heads, N, K] weights): what TMA can address (no rows
+    that are one another or overlap, strides below 2^40 bytes), 2^30 tiles at most.  RLLM_TILE_GEMM=simt and
+    RLLM_GEMM=library|no_tcgen05 keep it off."""
+    M, heads, K = a.shape
+    return (a.dtype is torch.bfloat16 and K % 8 == 0 and a.stride(0) % 8 == 0 and a.stride(1) % 8 == 0
+            and K <= a.stride(0) < 2 ** 39 and K <= a.stride(1) < 2 ** 39 and b.stride(0) < 2 ** 39
+            and -(-M // 128) * heads * -(-c.shape[2] // 128) <= 2 ** 30
             and (a.data_ptr() | b.data_ptr()) % 16 == 0 and c.stride(0) < 2 ** 31
             and not os.environ.get("RLLM_TILE_GEMM", "").startswith("s")
             and os.environ.get("RLLM_GEMM") not in ("library", "no_tcgen05"))

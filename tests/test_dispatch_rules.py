@@ -1,0 +1,17 @@
+"""Which kernel a call takes, as far as sizes and strides decide it: no GPU."""
+import torch
+
+from rllm_b200.kernels import ops
+
+BF16 = torch.bfloat16
+
+
+def test_products_per_head_whose_rows_tma_cannot_address_keep_the_general_kernel():
+    a, b = torch.empty(2048, 16, 128, dtype=BF16, device="meta"), torch.empty(16, 512, 128, dtype=BF16, device="meta")
+    c = torch.empty(2048, 16, 512, dtype=BF16, device="meta")
+    takes = lambda x: ops.head_gemm_tcgen05_takes(x, b, c)  # noqa: E731
+    assert takes(a) and takes(a.new_empty(16, 2048, 128).transpose(0, 1))
+    assert not takes(a[:1].expand(2048, 16, 128)) and not takes(a[:, :1].expand(2048, 16, 128))
+    flat = torch.empty(2048 * 64 + 16 * 8 + 128, dtype=BF16, device="meta")
+    assert not takes(flat.as_strided((2048, 16, 128), (64, 128, 1))) and not takes(flat.as_strided((2048, 16, 128), (128, 8, 1)))
+    assert not takes(torch.empty(1, dtype=BF16, device="meta").as_strided((2048, 16, 128), (2 ** 39, 128, 1)))

@@ -50,3 +50,22 @@ def test_rotation_of_the_queries_part(dtype, T, heads, dim, rot, turns, kv):
     tol = 2.0 ** -8 if dtype is torch.bfloat16 else 4e-6
     assert bool(((qt[:, :, kv:].double() - want).abs() <= tol * want.abs() + 1e-5).all())
     assert bool((qt[:, :, :kv] == 7.0).all())
+
+
+@pytest.mark.parametrize("form", ["one row for all", "one head for all", "rows that overlap"])
+def test_products_of_rows_that_share_memory(form):
+    from rllm_b200.kernels import ops
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    M, heads, K, N = 2048, 16, 128, 128
+    if form == "rows that overlap":
+        a = torch.randn(M * 64 + heads * 8192 * 2, generator=g, device="cuda").bfloat16().as_strided((M, heads, K), (64, 8192, 1))
+    else:
+        a = torch.randn(M, heads, K, generator=g, device="cuda").bfloat16()
+        a = a[:1].expand(M, heads, K) if form == "one row for all" else a[:, :1].expand(M, heads, K)
+    b, c = torch.randn(heads, N, K, generator=g, device="cuda").bfloat16(), torch.empty(M, heads, N, device="cuda").bfloat16()
+    ops.head_gemm(a, b, c, b_kn=False)
+    ops.check_gemm_errors(a.device)
+    want = torch.einsum("mhk,hnk->mhn", a.double(), b.double())
+    size = torch.einsum("mhk,hnk->mhn", a.double().abs(), b.double().abs())
+    assert bool(((c.double() - want).abs() <= 2.0 ** -8 * want.abs() + K * 2.0 ** -23 * size).all())
