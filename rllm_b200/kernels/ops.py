@@ -1040,8 +1040,12 @@ MOE_TCGEN05_FROM = 65     # from this many pairs on they run on the tcgen05 kern
 
 def moe_tcgen05_takes(pairs: int, h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor) -> bool:
     """Whether the experts' products of this many (token, expert) pairs run on the tcgen05 kernels: bfloat16, sizes
-    and pointers that TMA takes.  RLLM_TILE_GEMM=simt and RLLM_GEMM=library|no_tcgen05 keep them off."""
-    return (pairs >= MOE_TCGEN05_FROM and h.dtype is torch.bfloat16 and h.shape[1] % 8 == 0 and w_down.shape[2] % 8 == 0
+    and pointers that TMA takes, 2^30 weight rows and tiles at most.  RLLM_TILE_GEMM=simt and
+    RLLM_GEMM=library|no_tcgen05 keep them off."""
+    E, H, F = w_down.shape
+    most = 1 << 30
+    tiles = min(pairs, -(-pairs // 128) + E) * max(-(-F // 128), -(-H // 256))
+    return (E * 2 * F <= most and E * H <= most and tiles <= most and pairs >= MOE_TCGEN05_FROM and h.dtype is torch.bfloat16 and h.shape[1] % 8 == 0 and w_down.shape[2] % 8 == 0
             and (h.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16 == 0
             and not os.environ.get("RLLM_TILE_GEMM", "").startswith("s")
             and os.environ.get("RLLM_GEMM") not in ("library", "no_tcgen05"))

@@ -1,4 +1,5 @@
 """Which kernel a call takes, as far as sizes and strides decide it: no GPU."""
+import pytest
 import torch
 
 from rllm_b200.kernels import ops
@@ -15,3 +16,13 @@ def test_products_per_head_whose_rows_tma_cannot_address_keep_the_general_kernel
     flat = torch.empty(2048 * 64 + 16 * 8 + 128, dtype=BF16, device="meta")
     assert not takes(flat.as_strided((2048, 16, 128), (64, 128, 1))) and not takes(flat.as_strided((2048, 16, 128), (128, 8, 1)))
     assert not takes(torch.empty(1, dtype=BF16, device="meta").as_strided((2048, 16, 128), (2 ** 39, 128, 1)))
+
+
+@pytest.mark.parametrize("E,H,F,pairs,takes", [
+    (32, 2048, 1024, 65, True), (32, 2048, 1024, 64, False), (1 << 20, 8, 512, 4096, True),
+    (1 << 20, 8, 520, 4096, False), (1 << 20, 1024, 8, 4096, True), (1 << 20, 1032, 8, 4096, False),
+    (1, 8, 1 << 15, 1 << 28, True), (1, 8, 1 << 15, 1 << 30, False)])
+def test_experts_beyond_the_tensor_maps_keep_the_kernels_that_took_them(E, H, F, pairs, takes):
+    h = torch.empty(4, H, dtype=BF16, device="meta")
+    wgu, wd = torch.empty(E, 2 * F, H, dtype=BF16, device="meta"), torch.empty(E, H, F, dtype=BF16, device="meta")
+    assert ops.moe_tcgen05_takes(pairs, h, wgu, wd) is takes
