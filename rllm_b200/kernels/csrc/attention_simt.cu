@@ -58,6 +58,7 @@ template <> struct Vec8<bf16> {
 };
 
 #define ATT_PART 128         // keys of a partial result
+#define ATT_RESULT(RD) (32 * (RD) + 3)   // its floats: weighted values, largest score, sum of weights, whether NaN was passed over
 
 // d: the size of a query and key head; dv: of a value and output head (they may differ), up to 32 RD.  VEC: d is a
 // multiple of 8 and keys are fetched eight at a time; otherwise one by one.  WPR warps share a row.
@@ -73,7 +74,7 @@ attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out
                       const float* __restrict__ slopes, int shared_keys, int v_ld, int* __restrict__ err) {
   constexpr int U = WPR == 1 ? 16 / RD : 8;          // keys whose values are on their way together
   constexpr int UK = WPR == 1 && RD > 2 ? 4 : 8;     // and pieces of a key (many rows: warps hide it, registers cost warps)
-  extern __shared__ float qs[];  // WPR 1: [ATT_WARPS][d]; else [d] and the warps' partial results [WPR][32 RD + 2]
+  extern __shared__ float qs[];  // WPR 1: [ATT_WARPS][d]; else [d] and the warps' partial results [WPR][ATT_RESULT(RD)]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long gw = WPR == 1 ? (long long)blockIdx.x * ATT_WARPS + warp : (long long)blockIdx.x;
   if (gw >= (long long)T_tokens * nq) return;
@@ -112,6 +113,7 @@ attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out
   for (int p0 = 0; p0 < parts; p0 += WPR) {
     const int part = p0 + (WPR == 1 ? 0 : warp);
     float m = -INFINITY, l = 0.f, acc[RD];
+    bool lost = false;               // a group whose scores are all NaN stood before the part's first score
 #pragma unroll
     for (int r = 0; r < RD; ++r) acc[r] = 0.f;
     if (part < parts) {
@@ -150,7 +152,10 @@ attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out
         }
         const float cmax = warp_max(score);
         const float m_new = fmaxf(m, cmax);
-        if (m_new == -INFINITY) continue;  // nothing visible in this group (warp-uniform)
+        if (m_new == -INFINITY) {          // nothing visible in this group (warp-uniform), or nothing but NaN
+          lost |= __any_sync(0xffffffffu, score != score);
+          continue;
+        }
         const float p = (score == -INFINITY) ? 0.f : expf(score - m_new);
         const float corr = (m == -INFINITY) ? 0.f : expf(m - m_new);
         l = l * corr + warp_sum(p);
@@ -176,7 +181,12 @@ attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out
       }
     }
     // the partial results in order
-    auto add = [&](float pm, float pl, const float (&pa)[RD]) {
+    auto add = [&](float pm, float pl, const float (&pa)[RD], bool nan) {
+      if (nan && m_row != -INFINITY) {            // as where the part's groups follow the row's others: the row is NaN
+        l_row = NAN;
+#pragma unroll
+        for (int r = 0; r < RD; ++r) row[r] = NAN;
+      }
       if (pm == -INFINITY) return;
       const float m_new = fmaxf(m_row, pm);
       const float old = (m_row == -INFINITY) ? 0.f : expf(m_row - m_new), now = expf(pm - m_new);
@@ -186,19 +196,19 @@ attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out
       m_row = m_new;
     };
     if (WPR == 1) {
-      add(m, l, acc);
+      add(m, l, acc, lost);
     } else {
-      float* mine = qs + d + warp * (32 * RD + 2);
+      float* mine = qs + d + warp * ATT_RESULT(RD);
 #pragma unroll
       for (int r = 0; r < RD; ++r) mine[lane + 32 * r] = acc[r];
-      if (lane == 0) { mine[32 * RD] = m; mine[32 * RD + 1] = l; }
+      if (lane == 0) { mine[32 * RD] = m; mine[32 * RD + 1] = l; mine[32 * RD + 2] = lost ? 1.f : 0.f; }
       __syncthreads();
       if (warp == 0)
         for (int w = 0; w < WPR && p0 + w < parts; ++w) {
-          const float* theirs = qs + d + w * (32 * RD + 2);
+          const float* theirs = qs + d + w * ATT_RESULT(RD);
 #pragma unroll
           for (int r = 0; r < RD; ++r) acc[r] = theirs[lane + 32 * r];
-          add(theirs[32 * RD], theirs[32 * RD + 1], acc);
+          add(theirs[32 * RD], theirs[32 * RD + 1], acc, theirs[32 * RD + 2] != 0.f);
         }
       __syncthreads();
     }
@@ -251,7 +261,7 @@ RLLM_EXPORT int rllm_attention_simt_kv(const void* q, int q_stride, void* out, c
   const bool share = (rows <= 4096 && keys >= 512) || (rows <= 512 && keys >= 96);
   const unsigned blocks = (unsigned)(share ? rows : (rows + ATT_WARPS - 1) / ATT_WARPS);
   const int rd = dv <= 64 ? 2 : (dv <= 128 ? 4 : 8);
-  const size_t smem = (share ? (size_t)d + 8 * (32 * rd + 2) : (size_t)ATT_WARPS * d) * sizeof(float);
+  const size_t smem = (share ? (size_t)d + 8 * ATT_RESULT(rd) : (size_t)ATT_WARPS * d) * sizeof(float);
 #define ATT_ONE(VEC_, RD_, WPR_)                                                                            \
   RLLM_DISPATCH_DTYPE(dtype, T_,                                                                            \
     (attention_simt_kernel<T_, VEC_, RD_, WPR_><<<blocks, 32 * (WPR_ == 1 ? ATT_WARPS : WPR_), smem, stream>>>(  \

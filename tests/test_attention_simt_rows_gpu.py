@@ -51,3 +51,26 @@ def test_a_row_alone_and_among_many(d, dv, opts):
         want, size = w @ vals[:, h // 4], w @ vals[:, h // 4].abs()
         # a score is a sum of d float32 products (some d 2^-24 of its size), which its weight takes over; then as many sums
         assert bool(((many[:, h * dv: (h + 1) * dv].double() - want).abs() <= 3e-5 * size + 1e-7).all())
+
+
+@pytest.mark.parametrize("d", [64, 40])
+@pytest.mark.parametrize("bad,seen", [((256, 257), 257), ((128, 256), 300), ((384, 400), 400), ((130, 131), 200)])
+def test_a_key_that_is_not_a_number_shows_in_the_result(d, bad, seen):
+    """NaN scores that fill a part of 128 keys, or all of a part that the row sees, behind a part of numbers."""
+    from rllm_b200.kernels import ops
+    g = torch.Generator(device="cuda")
+    g.manual_seed(d + seen)
+    page, nq = 16, 4
+    pages = 64
+    k, v = (torch.randn(pages, 1, page, d, generator=g, device="cuda") for _ in range(2))
+    k.view(-1, d)[bad[0]: bad[1]] = math.nan
+    table = torch.arange(pages, dtype=torch.int32, device="cuda")[None].contiguous()
+    for rows in (1, 1100):                                  # eight warps a row (the table is wide), and one
+        q = torch.randn(rows, nq * d, generator=g, device="cuda")
+        out, err = torch.zeros(rows, nq * d, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        pos = torch.full((rows,), seen - 1, dtype=torch.int32, device="cuda")
+        ops.attention_simt_kv(q, nq * d, out, k, v, table, pos, torch.zeros_like(pos), nq, 1, 0, d ** -0.5, err)
+        assert int(err) == 0 and bool(torch.isnan(out).all())
+        pos.fill_(bad[0] - 1)                               # and does not where the key lies ahead
+        ops.attention_simt_kv(q, nq * d, out, k, v, table, pos, torch.zeros_like(pos), nq, 1, 0, d ** -0.5, err)
+        assert bool(torch.isfinite(out).all())
