@@ -564,6 +564,19 @@ BIKOVIK_SIZES = {
 }
 
 
+# entry points of ``ops`` whose launches the step tables of ``--design`` time one by one
+STEP_KERNELS = (
+    "latent_attention_mma", "latent_attention_tcgen05", "attention_prefill_tcgen05", "attention_prefill_bf16",
+    "attention_decode_bf16", "moe_experts", "moe_route", "head_gemm", "mingru_scan", "gated_postnorm_add",
+    "depth_average", "rmsnorm", "silu_mul", "latent_prep", "latent_q_rot", "rope_kv_write", "gemm_small_m",
+    "moe_choose", "gemm_small_m_residual", "gemm_small_m_rstd", "gemm_tcgen05", "embedding", "lightning_scan",
+    "selective_scan", "causal_conv", "streams_read", "streams_write", "head_norm_kv_write", "attention_simt_kv",
+    "rms_mean2", "gated_rmsnorm", "act_mul", "moe_choose_sigmoid", "weighted_slot_sum", "layernorm", "add_rows",
+    "add_row_bias", "mlstm_scan", "head_gated_rmsnorm", "act", "sigmoid_gate", "postnorm_add", "ssd_scan",
+    "silu_gated_group_rmsnorm", "channel_delta_scan", "channel_delta_step", "activation_rows", "linear_state_scan",
+    "talking_prep", "dyt", "shared_key_attention_tcgen05", "shared_key_attention_mma", "softcap_rows")
+
+
 def compare_designs(args):
     """Prefill and decode throughput of Fasulix at sizes that resemble a real model's layers (random weights)
     beside the Llama of equal size, through the same step function; and, from one eager prefill step and one
@@ -596,8 +609,8 @@ def compare_designs(args):
             first = ctx - Tn // S
             vis = sum(p + 1 - lo(p) + min(keep if window else 0, lo(p)) for p in range(first, ctx)) * S
             return vis, S * (ctx - lo(first) + min(keep if window else 0, lo(first)))
-        if name == "latent_attention_mma":
-            q, heads, dk, dv, window = a[0], a[8], a[9], a[10], a[11]
+        if name in ("latent_attention_mma", "latent_attention_tcgen05"):
+            q, (heads, dk, dv, window) = a[0], a[8:12] if name == "latent_attention_mma" else a[9:13]
             vis = sum(min(p + 1, window or p + 1) for p in range(ctx - Tn // S, ctx)) * S
             keys = S * min(ctx, (window or ctx) + Tn // S)
             return 2.0 * (dk + dv) * heads * vis, 2.0 * (keys * dk + q.numel() + a[1].numel())
@@ -705,16 +718,7 @@ def compare_designs(args):
 
     def kernel_table(runner, entries, shape):
         """One eager step with CUDA events around every entry point of ``ops`` (L2 flushed before the step)."""
-        names = [n for n in dir(ops) if callable(getattr(ops, n)) and n in (
-            "latent_attention_mma", "attention_prefill_tcgen05", "attention_prefill_bf16", "attention_decode_bf16",
-            "moe_experts", "moe_route", "head_gemm", "mingru_scan", "gated_postnorm_add", "depth_average", "rmsnorm",
-            "silu_mul", "latent_prep", "latent_q_rot", "rope_kv_write", "gemm_small_m", "moe_choose", "gemm_small_m_residual",
-            "gemm_small_m_rstd", "gemm_tcgen05", "embedding", "lightning_scan", "selective_scan", "causal_conv",
-            "streams_read", "streams_write", "head_norm_kv_write", "attention_simt_kv", "rms_mean2", "gated_rmsnorm",
-            "act_mul", "moe_choose_sigmoid", "weighted_slot_sum", "layernorm", "add_rows", "add_row_bias", "mlstm_scan",
-            "head_gated_rmsnorm", "act", "sigmoid_gate", "postnorm_add", "ssd_scan", "silu_gated_group_rmsnorm",
-            "channel_delta_scan", "channel_delta_step", "activation_rows", "linear_state_scan", "talking_prep", "dyt",
-            "shared_key_attention_tcgen05", "shared_key_attention_mma", "softcap_rows")]
+        names = [n for n in dir(ops) if callable(getattr(ops, n)) and n in STEP_KERNELS]
         saved, log = {}, []
 
         def wrap(name, fn):
