@@ -69,3 +69,21 @@ def test_products_of_rows_that_share_memory(form):
     want = torch.einsum("mhk,hnk->mhn", a.double(), b.double())
     size = torch.einsum("mhk,hnk->mhn", a.double().abs(), b.double().abs())
     assert bool(((c.double() - want).abs() <= 2.0 ** -8 * want.abs() + K * 2.0 ** -23 * size).all())
+
+
+@pytest.mark.parametrize("T,heads,rot,turns", [(255, 16, 64, 64), (256, 16, 64, 48), (256, 31, 32, 32), (256, 33, 32, 32), (300, 3, 600, 598)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_rotation_has_the_same_bits_a_token_at_a_time(dtype, T, heads, rot, turns):
+    """Around the size from which a block takes a token: a token alone is rotated a thread a pair."""
+    from rllm_b200.kernels import ops
+    g = torch.Generator(device="cuda")
+    g.manual_seed(T + heads)
+    q = torch.randn(T, heads * (8 + rot), generator=g, device="cuda").to(dtype)
+    pos = torch.randint(0, 9000, (T,), generator=g, device="cuda", dtype=torch.int32)
+    f = torch.rand(turns // 2, generator=g, device="cuda", dtype=torch.float64)
+    many, one = (torch.full((T, heads * (16 + rot)), 7.0, device="cuda", dtype=dtype) for _ in range(2))
+    ops.latent_q_rot(q, many, pos, f, heads, 8, rot, turns, 16, magnitude=0.75)
+    for t in range(0, T, 5):
+        ops.latent_q_rot(q[t: t + 1], one[t: t + 1], pos[t: t + 1], f, heads, 8, rot, turns, 16, magnitude=0.75)
+        assert torch.equal(one[t], many[t])
+    assert bool((many.view(T, heads, -1)[:, :, :16] == 7.0).all())
