@@ -436,8 +436,9 @@ __global__ void weighted_slot_sum_kernel(const T* y, const float* c, T* out,
   out[idx] = from_f32<T>(v);
 }
 
-// the same eight values a thread (bfloat16, H a multiple of 8, 16-byte aligned): 2,048 x top 4 x 2,048, 42 MB, 22.7 us with
-// single values, 7.7 (5.5 TB/s)
+// the same eight values a thread (bfloat16, H a multiple of 8, 16-byte aligned, 2^17 results or more): 2,048 x top 4 x 2,048,
+// 42 MB, 22.7 us with single values, 7.7 (5.5 TB/s); 33 x 4,096 2.4 and 2.0; fewer results leave SMs without work: 33 x 2,880
+// 2.1 and 2.2, 1 x 2,048 1.5 and 1.8
 __global__ void __launch_bounds__(256)
 weighted_slot_sum8_kernel(const bf16* y, const float* c, bf16* out, int slots, int H8, unsigned total, const bf16* extra,
                           const float* extra_gate) {
@@ -473,7 +474,7 @@ RLLM_EXPORT int rllm_weighted_slot_sum(const void* y, const float* c, void* out,
   const long long total = (long long)T * H;
   if (total <= 0) return 0;
   if (slots <= 0) return RLLM_E_BADARG;
-  if (dtype == RLLM_DT_BF16 && H % 8 == 0 && total / 8 < (1ll << 31) &&
+  if (dtype == RLLM_DT_BF16 && H % 8 == 0 && total >= (1ll << 17) && total / 8 < (1ll << 31) &&
       (((uintptr_t)y | (uintptr_t)out | (uintptr_t)extra) & 15) == 0) {
     const unsigned n = (unsigned)(total / 8);
     rllm_launch_pdl(weighted_slot_sum8_kernel, dim3((n + 255) / 256), dim3(256), (size_t)0, stream, (const bf16*)y, c,

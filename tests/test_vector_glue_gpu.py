@@ -201,3 +201,22 @@ def test_chunk_passes_have_the_same_bits_wherever_rows_start(heads, d, dv):
         outs.append((o, state))
     for o, state in outs[1:]:
         assert torch.equal(o, outs[0][0]) and torch.equal(state, outs[0][1])
+
+
+@pytest.mark.parametrize("T,K,H", [(64, 4, 2048), (63, 4, 2048), (497, 3, 264), (2048, 1, 64)])
+@pytest.mark.parametrize("extra", ["none", "row", "gated"])
+def test_weighted_sum_of_slots_has_the_same_bits_a_row_at_a_time(T, K, H, extra):
+    """Around 2^17 results, from which eight values a thread are taken: a row alone takes single values."""
+    from rllm_b200.kernels import ops
+    r = gen(T + H)
+    y, c, e, g = r(T * K, H).bfloat16(), r(T, K), r(T, H).bfloat16(), r(T)
+    many, one = (torch.empty(T, H, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    opts = lambda a, b: dict(extra=None if extra == "none" else e[a:b], extra_gate=g[a:b] if extra == "gated" else None)  # noqa: E731
+    ops.weighted_slot_sum(y, c, many, **opts(0, T))
+    for t in range(T):
+        ops.weighted_slot_sum(y[t * K: (t + 1) * K], c[t: t + 1], one[t: t + 1], **opts(t, t + 1))
+    assert torch.equal(one, many)
+    want = torch.einsum("tk,tkh->th", c.double(), y.double().view(T, K, H))
+    if extra != "none":
+        want = want + e.double() * (torch.sigmoid(g.double())[:, None] if extra == "gated" else 1.0)
+    assert close(many, want, 4.0 * K)
