@@ -321,8 +321,9 @@ RLLM_EXPORT int rllm_rms_mean2(const void* a, const void* b, const void* wa, con
 
 // The same for bfloat16 rows of up to 8,192 values that start on 16 bytes: eight values an access, all of a thread's loads
 // on their way before the sum, nothing read twice.  The sum runs over shared memory in the order of the form below (256
-// threads), so that a row has the same bits wherever it starts.  2,048 x 2,048, 33 MB: 19.4 us with single values in two
-// passes, 5 at the copy rate; the gates' exponentials and divisions bound it.
+// threads), so that a row has the same bits wherever it starts.  Single values / eight an access, in a graph: 33 x 2,048 6.1 /
+// 2.8 us, 2,048 x 2,048 13.1 / 13.2, 2,048 x 4,096 27 / 21, 2,048 x 8,192 81 / 37, 300 x 1,024 3.8 / 3.1; short rows leave most
+// of the 256 threads without a value: 2,048 x 1,024 8.1 / 10.8, 2,048 x 512 5.5 / 9.8, 8 x 512 2.4 / 2.5: they take single values.
 #define GRN_KEEP 4
 template <typename TW>
 __global__ void __launch_bounds__(256)
@@ -393,7 +394,7 @@ RLLM_EXPORT int rllm_gated_rmsnorm(const float* x, const void* g, int g_stride, 
                                    int dtype, int T, int H, float eps, cudaStream_t stream) {
   if (T <= 0) return 0;
   if (H <= 0) return RLLM_E_BADARG;
-  if (dtype == RLLM_DT_BF16 && H % 8 == 0 && H <= 256 * 8 * GRN_KEEP && g_stride % 8 == 0 &&
+  if (dtype == RLLM_DT_BF16 && H % 8 == 0 && H <= 256 * 8 * GRN_KEEP && (H >= 2048 || (H >= 1024 && T <= 512)) && g_stride % 8 == 0 &&
       (((uintptr_t)x | (uintptr_t)g | (uintptr_t)w | (uintptr_t)out) & 15) == 0) {
     RLLM_DISPATCH_DTYPE(w_dtype, TW, (rllm_launch_pdl(gated_rmsnorm8_kernel<TW>, dim3(T), dim3(256), (size_t)H * 4, stream,
                                                       x, (const bf16*)g, g_stride, (const TW*)w, (bf16*)out, H, eps)));
