@@ -122,7 +122,7 @@ causal_conv_run_kernel(const T* x, int stride, const TW* w, const TW* bias, floa
 
 // Four taps, bfloat16 rows in steps of four channels on 8-byte boundaries (prompt portions): a thread takes four channels and
 // CV_RUN tokens.  Where a run lies in one sequence, which is nearly always, all its inputs are asked for at once; a token at
-// a time behind the last one's arithmetic, one channel a thread, 2,048 x 4,608 took 37 us, 29 so (38 MB; 6 us at the copy rate;
+// a time behind the last one's arithmetic, one channel a thread, 2,048 x 4,608 took 33 us, 29 so (38 MB; 6 us at the copy rate;
 // the exponential and the division of silu bound it).  The same sums in the same order and the same silu as
 // causal_conv_run_kernel: a decoded token has the same bits whether or not another sequence of the step brings a prompt.
 template <typename TW>
@@ -401,7 +401,10 @@ RLLM_EXPORT int rllm_causal_conv(const void* x, int stride, int dtype, const voi
   if (T <= 0) return 0;
   if (E <= 0 || taps <= 0 || taps > 64 || num_slots <= 0) return RLLM_E_BADARG;
   const long long total = (long long)T * E;
-  if (any_long && taps == 4 && dtype == RLLM_DT_BF16 && E % 4 == 0 && stride % 4 == 0 &&
+  // Four channels a thread need work for the GPU and runs within one sequence.  One channel / four, us: 2,048 x 4,608 33 / 29,
+  // 8,192 x 2,880 101 / 70, in portions of 12 tokens 2,040 x 2,880 even; but 64 x 4,608 6.7 / 6.7, 1,020 x 2,880 in portions
+  // of 12 15.4 / 17.2, 64 x 4,608 in portions of 4 7.2 / 9.3.
+  if (any_long && total >= (1ll << 22) && T >= 8ll * num_seqs && taps == 4 && dtype == RLLM_DT_BF16 && E % 4 == 0 && stride % 4 == 0 &&
       (((uintptr_t)x | (uintptr_t)out) & 7) == 0 && (T + CV_RUN - 1) / CV_RUN <= 65535) {
     RLLM_DISPATCH_DTYPE(w_dtype, TW,
       (rllm_launch_pdl(causal_conv4_kernel<TW>, dim3((unsigned)((E + 511) / 512), (unsigned)((T + CV_RUN - 1) / CV_RUN)),

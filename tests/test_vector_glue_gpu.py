@@ -126,17 +126,34 @@ def test_a_decoded_token_of_the_convolution_does_not_depend_on_its_batch(E):
     """The same bits in a step of decoded tokens and beside a prompt portion, and the portion the same bits whether its
     rows are read four channels at a time or one; sums of -100 to 100, where an exponential is least good."""
     r = gen(E)
-    x, w, b = (r(45, E) * 20).bfloat16(), r(E, 4), r(E) * 0.1
+    n = (1 << 22) // E                                     # a portion large enough for four channels a thread
+    x, w, b = (r(5 + n, E) * 20).bfloat16(), r(E, 4), r(E) * 0.1
     alone, mixed, single = (r(6, 3, E) for _ in range(3))
     mixed.copy_(alone)
     single.copy_(alone)
     decoded = conv_of(x[:5], w, b, alone, [1] * 5, False)
-    both = conv_of(x, w, b, mixed, [1] * 5 + [40], True)
+    both = conv_of(x, w, b, mixed, [1] * 5 + [n], True)
     assert torch.equal(decoded, both[:5]) and torch.equal(alone[:5], mixed[:5])
-    odd = torch.zeros(45, E + 1, dtype=torch.bfloat16, device="cuda")[:, 1:]
-    odd.copy_(x)                                           # rows on 2-byte boundaries: one channel a thread
-    assert torch.equal(conv_of(odd, w, b, single, [1] * 5 + [40], True), both) and torch.equal(single, mixed)
+    assert torch.equal(conv_of(shifted(x), w, b, single, [1] * 5 + [n], True), both) and torch.equal(single, mixed)
     assert float(both.float().min()) < -0.2 and float(both.float().max()) > 50
+
+
+@pytest.mark.parametrize("lens", [[128], [2, 1, 1, 30, 3, 100], [9, 17, 103], [1, 7, 8, 1, 120], [5] * 3 + [1] + [113]])
+def test_convolution_with_four_channels_a_thread(lens):
+    """Runs of eight tokens within a sequence, across sequences and behind the last: the bits of the form with one channel."""
+    r, E = gen(sum(lens)), 1 << 15
+    x, w, b = r(sum(lens), E).bfloat16(), r(E, 4) * 0.4, r(E) * 0.1
+    tail = r(len(lens) + 1, 3, E)
+    four, one = tail.clone(), tail.clone()
+    got = conv_of(x, w, b, four, lens, True)
+    assert torch.equal(got, conv_of(shifted(x), w, b, one, lens, True)) and torch.equal(four, one)
+    at = 0
+    for s, n in enumerate(lens):
+        past = torch.cat([tail[s].double(), x[at: at + n].double()])
+        acc = sum(w[:, k].double() * past[k: k + n] for k in range(4)) + b.double()
+        assert close(got[at: at + n], torch.nn.functional.silu(acc), 4.0)
+        assert torch.equal(four[s], past[n:].float())
+        at += n
 
 
 def shifted(t):
@@ -166,7 +183,7 @@ def test_group_rmsnorm_has_the_bits_of_its_single_value_form(T, E, groups):
     assert close(got, want, 8.0)
 
 
-@pytest.mark.parametrize("T,H,wd", [(5, 8, "float32"), (3, 2048, "float32"), (2, 8192, "bfloat16"), (4, 264, "float32"), (33, 1000, "bfloat16")])
+@pytest.mark.parametrize("T,H,wd", [(513, 1024, "float32"), (512, 1024, "float32"), (3, 2056, "float32"), (2, 8192, "bfloat16"), (33, 1032, "bfloat16")])
 def test_gated_rmsnorm_has_the_bits_of_its_single_value_form(T, H, wd):
     from rllm_b200.kernels import ops
     r = gen(H)
