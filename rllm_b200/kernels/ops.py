@@ -962,6 +962,13 @@ def latent_attention_mma_takes(dtype: torch.dtype, dk: int, dv: int) -> bool:
             and os.environ.get("RLLM_LATENT_ATTENTION") != "simt")
 
 
+def latent_attention_mma_splits(num_seqs: int, max_q_len: int, heads: int, max_seq_len: int, window: int) -> bool:
+    """Whether ``latent_attention_mma`` cuts the keys of such a step into splits."""
+    row_tiles = num_seqs * -(-(max_q_len * heads) // 64)
+    keys = min(max_seq_len, window + max_q_len) if window else max_seq_len
+    return row_tiles <= LATENT_SPLIT_MAX_TILES and keys >= LATENT_SPLIT_MIN_KEYS and max_seq_len <= 8192 * LATENT_SPLIT_KEYS
+
+
 def latent_attention_mma(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor,
                          q_start: torch.Tensor, seq_lens: torch.Tensor, num_seqs: int, max_q_len: int, heads: int,
                          dk: int, dv: int, window: int, scale: float, sink: Optional[torch.Tensor],
@@ -972,9 +979,7 @@ def latent_attention_mma(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor
     few rows and long sequences the keys are also cut into splits of 128 that run side by side."""
     lib = build.load_library("latent_attention_mma")
     split_tiles, nsplit, work = 0, 1, None
-    row_tiles = num_seqs * -(-(max_q_len * heads) // 64)
-    keys = min(max_seq_len, window + max_q_len) if window else max_seq_len
-    if row_tiles <= LATENT_SPLIT_MAX_TILES and keys >= LATENT_SPLIT_MIN_KEYS and max_seq_len <= 8192 * LATENT_SPLIT_KEYS:
+    if latent_attention_mma_splits(num_seqs, max_q_len, heads, max_seq_len, window):
         split_tiles = LATENT_SPLIT_KEYS                     # in keys: a multiple of every key tile
         nsplit = -(-max_seq_len // LATENT_SPLIT_KEYS)
         lib.rllm_latent_attention_mma_work.restype = c_longlong
@@ -995,14 +1000,35 @@ def latent_attention_mma(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor
            "latent_attention_mma")
 
 
-# (token, head) rows of prompt portions from which they run on the tcgen05 kernel.  Its CTA walks all keys of 128 rows (2.9 us
-# a tile of 64 keys of 576 values, however few rows there are), while the mma.sync kernel cuts the keys too where there are
-# few rows: 640 rows x 4,096 keys 190 against 115 us, 1,600 rows 189 against 238, 2,048 x 128 17 against 17.
-LATENT_TCGEN05_MIN_ROWS = 1024
+LATENT_TCGEN05_MIN_ROWS = 1024       # (token, head) rows of a step's prompt portions from which the tcgen05 kernel may run
+
+
+def latent_attention_tcgen05_pays(q_lens, seq_lens, heads: int, dv: int, window: int) -> bool:
+    """Whether the tcgen05 kernel is the faster one for prompt portions of these lengths (``seq_lens`` with what the cache
+    holds).  Its CTA takes 128 rows of one sequence and 256 value columns, an SM to itself, and walks all their keys (2.9 us
+    a tile of 64 keys of 576 values, however few rows there are); the mma.sync kernel takes 16 to 64 rows and cuts the keys
+    too where it has few rows.  The lines, in microseconds mma.sync / tcgen05 (885 sizes were measured; none that the rule
+    lets through is more than 3 % slower):
+      few rows and many keys, cut by mma.sync: 16 heads of 576, 4,096 keys, 1,024 rows 156 / 186, 1,152 174 / 186, 1,280 up
+        to equal; 8 heads of 288 92 / 111 at 1,024 rows;
+      tiles not half full: 128 portions of 2 tokens x 16 heads, 2,048 keys, 177 / 243 (256 CTAs); 64 of them 157 / 121;
+        128 portions of 2 x 8 heads of 288, 512 keys, 22 / 29;
+      few keys, where what a CTA costs to start counts: 64 portions of 4 x 16 heads, 128 keys, 16 / 19, 32 of 8 16 / 18, but
+        16 of 32 30 / 17; with one CTA a tile (up to 256 value columns) 8 portions of 64 x 8 heads 17 / 11."""
+    rows = heads * sum(q_lens)
+    tiles = sum(-(-q * heads // 128) for q in q_lens)
+    most_q, most_keys = max(q_lens), max(seq_lens)
+    keys = min(most_keys, window + most_q) if window else most_keys
+    parts = -(-dv // 256)
+    if rows < 1280 and latent_attention_mma_splits(len(q_lens), most_q, heads, most_keys, window):
+        return False
+    if keys < 512:
+        return rows >= 96 * tiles and (parts == 1 or rows > 4096)
+    return rows >= 64 * tiles or (rows >= 24 * tiles and tiles * parts <= 148)
 
 
 def latent_attention_tcgen05_takes(dtype: torch.dtype, dk: int, dv: int, rows: int, cache: torch.Tensor) -> bool:
-    """Whether prompt portions with this many (token, head) rows run on the tcgen05 kernel.
+    """Whether prompt portions with this many (token, head) rows can run on the tcgen05 kernel.
     RLLM_LATENT_ATTENTION=mma keeps them on the mma.sync kernel (simt: on the CUDA cores)."""
     return (dtype is torch.bfloat16 and dk % 8 == 0 and dk <= 576 and dv % 8 == 0 and dv <= min(dk, 512)
             and rows >= LATENT_TCGEN05_MIN_ROWS and cache.data_ptr() % 16 == 0

@@ -156,7 +156,8 @@ class LatentAttention(Mixer):
         o = torch.empty((T, H * self.kv_rank), dtype=x.dtype, device=x.device)
         window = int(self.window or 0)
         nd = ctx.num_decode
-        if T > nd and ops.latent_attention_tcgen05_takes(x.dtype, dk, self.kv_rank, (T - nd) * H, cache.k):
+        if T > nd and ops.latent_attention_tcgen05_takes(x.dtype, dk, self.kv_rank, (T - nd) * H, cache.k) and \
+                ops.latent_attention_tcgen05_pays(ctx.q_lens_host[nd:], ctx.seq_lens_host[nd:], H, self.kv_rank, window):
             ops.latent_attention_tcgen05(qt, o, cache.k, table, ctx.q_start, ctx.seq_lens, nd, ctx.num_seqs, T - nd, H, dk,
                                          self.kv_rank, window, self.scale, self.sink, ctx.err)
             if nd:

@@ -26,3 +26,14 @@ def test_experts_beyond_the_tensor_maps_keep_the_kernels_that_took_them(E, H, F,
     h = torch.empty(4, H, dtype=BF16, device="meta")
     wgu, wd = torch.empty(E, 2 * F, H, dtype=BF16, device="meta"), torch.empty(E, H, F, dtype=BF16, device="meta")
     assert ops.moe_tcgen05_takes(pairs, h, wgu, wd) is takes
+
+
+@pytest.mark.parametrize("q_lens,keys,heads,dv,window,tcgen05", [
+    ([2048], 2048, 16, 512, 0, True), ([80], 4096, 16, 512, 0, True), ([72], 4096, 16, 512, 0, False),
+    ([8] * 8, 4096, 16, 512, 0, False), ([10] * 8, 4096, 16, 512, 0, True), ([64], 512, 16, 512, 0, True),
+    ([64], 4096, 16, 512, 500, True), ([128], 4096, 8, 256, 0, False), ([160], 4096, 8, 256, 0, True),
+    ([2] * 128, 2048, 16, 512, 0, False), ([2] * 64, 2048, 16, 512, 0, True), ([2] * 128, 512, 8, 256, 0, False),
+    ([4] * 64, 128, 16, 512, 0, False), ([8] * 32, 128, 16, 512, 0, False), ([32] * 16, 128, 16, 512, 0, True),
+    ([64] * 8, 128, 8, 256, 0, True), ([2] * 64, 128, 8, 256, 0, False), ([1792, 3], 1792, 16, 512, 0, True)])
+def test_which_prompt_portions_the_tcgen05_latent_attention_pays_for(q_lens, keys, heads, dv, window, tcgen05):
+    assert ops.latent_attention_tcgen05_pays(q_lens, [keys] * len(q_lens), heads, dv, window) is tcgen05
