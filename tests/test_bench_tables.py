@@ -13,7 +13,7 @@ def test_every_attention_of_the_parts_is_timed():
     for path in glob.glob(os.path.join(ROOT, "rllm_b200", "parts", "*.py")):
         with open(path) as f:
             used |= set(re.findall(r"ops\.(\w*attention\w*)\(", f.read()))
-    used = {n for n in used if not n.endswith("_takes") and not n.startswith("use_")}
+    used = {n for n in used if not n.endswith(("_takes", "_pays")) and not n.startswith("use_")}
     # the CUDA-core forms belong to the 32-bit path, which the tables do not run
     used -= {"attention_simt", "latent_attention_simt"}
     assert "latent_attention_tcgen05" in used and used <= set(bench.STEP_KERNELS), used - set(bench.STEP_KERNELS)
