@@ -1065,7 +1065,7 @@ MOE_TCGEN05_FROM = 65     # from this many pairs on they run on the tcgen05 kern
 
 
 def moe_tcgen05_takes(pairs: int, h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor) -> bool:
-    """Whether the experts' products of this many (token, expert) pairs run on the tcgen05 kernels: bfloat16, sizes
+    """Whether the experts' products of this many (token, expert) pairs can run on the tcgen05 kernels: bfloat16, sizes
     and pointers that TMA takes, 2^30 weight rows and tiles at most.  RLLM_TILE_GEMM=simt and
     RLLM_GEMM=library|no_tcgen05 keep them off."""
     E, H, F = w_down.shape
@@ -1075,6 +1075,15 @@ def moe_tcgen05_takes(pairs: int, h: torch.Tensor, w_gate_up: torch.Tensor, w_do
             and (h.data_ptr() | w_gate_up.data_ptr() | w_down.data_ptr()) % 16 == 0
             and not os.environ.get("RLLM_TILE_GEMM", "").startswith("s")
             and os.environ.get("RLLM_GEMM") not in ("library", "no_tcgen05"))
+
+
+def moe_tcgen05_pays(E: int, H: int, F: int) -> bool:
+    """Whether the tcgen05 kernels are the faster ones for these weights.  A tile costs them some 20 us however small H and F
+    are (its pairs are written 32 columns at a time by one warp a quarter), the row tiles of mma.sync about 8 + (H + F) / 70.
+    Microseconds mma.sync / tcgen05: 64 -> 64 -> 64, 8 experts, 1,024 pairs 15 / 26; 512 -> 512, 8 experts, 512 pairs 26 / 27;
+    1,024 -> 512, 1 expert, 256 pairs 29 / 34, 8 experts even or better; 1,024 -> 1,024, 1 expert 33 / 37; 2,048 -> 256 never
+    slower.  RLLM_GEMM=tcgen05 sends all sizes to tcgen05 (used by tests)."""
+    return os.environ.get("RLLM_GEMM") == "tcgen05" or (H * F >= 1 << 19 and (E >= 8 or H >= 2048))
 
 
 def moe_route(h: torch.Tensor, w_router: torch.Tensor, top: int):
@@ -1125,7 +1134,7 @@ def moe_experts(h: torch.Tensor, ids: torch.Tensor, w_gate_up: torch.Tensor, w_d
     P = T * top
     y = torch.empty((P, F), dtype=h.dtype, device=h.device)
     out = torch.empty((P, H), dtype=h.dtype, device=h.device)
-    tcgen05 = moe_tcgen05_takes(P, h, w_gate_up, w_down)
+    tcgen05 = moe_tcgen05_pays(E, H, F) and moe_tcgen05_takes(P, h, w_gate_up, w_down)
     bm = 128 if tcgen05 else (16 if P <= MOE_SMALL_PAIRS else 64)
     max_tiles = min(P, -(-P // bm) + E)
     meta = torch.empty(1 + (E + 1) + P + 2 * max_tiles, dtype=torch.int32, device=h.device)

@@ -37,3 +37,12 @@ def test_experts_beyond_the_tensor_maps_keep_the_kernels_that_took_them(E, H, F,
     ([64] * 8, 128, 8, 256, 0, True), ([2] * 64, 128, 8, 256, 0, False), ([1792, 3], 1792, 16, 512, 0, True)])
 def test_which_prompt_portions_the_tcgen05_latent_attention_pays_for(q_lens, keys, heads, dv, window, tcgen05):
     assert ops.latent_attention_tcgen05_pays(q_lens, [keys] * len(q_lens), heads, dv, window) is tcgen05
+
+
+@pytest.mark.parametrize("E,H,F,pays", [(32, 2048, 1024, True), (16, 1024, 1024, True), (8, 1024, 512, True), (4, 1024, 512, False),
+                                        (1, 2048, 256, True), (1, 1024, 1024, False), (128, 512, 512, False), (8, 64, 64, False)])
+def test_which_experts_the_tcgen05_kernels_pay_for(E, H, F, pays, monkeypatch):
+    monkeypatch.delenv("RLLM_GEMM", raising=False)
+    assert ops.moe_tcgen05_pays(E, H, F) is pays
+    monkeypatch.setenv("RLLM_GEMM", "tcgen05")
+    assert ops.moe_tcgen05_pays(E, H, F)

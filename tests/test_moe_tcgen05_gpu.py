@@ -55,3 +55,15 @@ def test_which_calls_take_the_tcgen05_experts():
     assert not ops.moe_tcgen05_takes(128, h, wgu[:, :44].contiguous(), wd[:, :, :22].contiguous())
     shifted = torch.zeros(64 * 64 + 4, dtype=torch.bfloat16, device="cuda")[4:].view(64, 64)
     assert not ops.moe_tcgen05_takes(128, shifted, wgu, wd)
+
+
+@pytest.mark.parametrize("T,H,F,E,top,one", [
+    (65, 8, 8, 1, 1, None), (128, 64, 128, 1, 1, None), (129, 136, 264, 1, 1, None), (100, 64, 24, 5, 2, None),
+    (257, 200, 136, 40, 3, None), (1000, 128, 520, 4, 1, 870), (65, 1024, 512, 8, 1, None)])
+def test_small_experts_on_tcgen05(T, H, F, E, top, one, monkeypatch):
+    """The sizes that ordinarily take the row tiles, on the tcgen05 kernels all the same."""
+    from rllm_b200.kernels import ops
+    assert (H * F >= 1 << 19) == ops.moe_tcgen05_pays(E, H, F)
+    monkeypatch.setenv("RLLM_GEMM", "tcgen05")
+    assert ops.moe_tcgen05_pays(E, H, F)
+    test_experts_on_tcgen05(T, H, F, E, top, one, 1.5, 1.702, 1.0)
