@@ -31,10 +31,11 @@
 // around it, on which pages hold it, or on how many warps share it.
 //
 // What bounds it is latency: a lane's key and the 32 values of a group are loads
-// that wait for nothing but the block table, so eight keys' worth of them are
-// kept on their way.  Four sequences of 100 to 3,000 keys, one token each, 32
-// heads of 64 in float32: 1,225 us with a warp a row and a load at a time, 616 with
-// loads ahead, 92 with eight warps a row; 6,400 rows of up to 300 keys 264 -> 183.
+// that wait for nothing but the block table, so eight keys' worth of values (four
+// for heads above 64, two above 128) and up to eight pieces of a key are kept on
+// their way.  Four sequences of 100 to 3,000 keys, one token each, 32 heads of 64 in
+// float32: 1,225 us with a warp a row and a load at a time, 616 with loads ahead, 92
+// with eight warps a row; 6,400 rows of up to 300 keys 264 -> 183.
 #include "common.cuh"
 #include <math.h>
 
@@ -63,7 +64,7 @@ template <> struct Vec8<bf16> {
 // d: the size of a query and key head; dv: of a value and output head (they may differ), up to 32 RD.  VEC: d is a
 // multiple of 8 and keys are fetched eight at a time; otherwise one by one.  WPR warps share a row.
 template <typename T, bool VEC, int RD, int WPR>
-__global__ void __launch_bounds__(32 * (WPR == 1 ? ATT_WARPS : WPR))
+__global__ void __launch_bounds__(32 * (WPR == 1 ? ATT_WARPS : WPR), WPR == 1 ? (RD == 2 ? 6 : 8) : 4)
 attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out,
                       const T* __restrict__ kcache, const T* __restrict__ vcache,
                       const int* __restrict__ block_table, int max_blocks,
@@ -72,8 +73,12 @@ attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out
                       int keep_first, int chunk, float softcap, const float* __restrict__ sinks,
                       const T* __restrict__ gate, int gate_stride, int gate_mode,
                       const float* __restrict__ slopes, int shared_keys, int v_ld, int* __restrict__ err) {
-  constexpr int U = WPR == 1 ? 16 / RD : 8;          // keys whose values are on their way together
-  constexpr int UK = WPR == 1 && RD > 2 ? 4 : 8;     // and pieces of a key (many rows: warps hide it, registers cost warps)
+  // keys whose values are on their way together, and pieces of a key.  More of them, or more registers than the bounds above
+  // leave (64; 80 for one warp a row and heads up to 64), cost warps in flight: with 87 to 93 registers heads of 256 took 1.5 to
+  // 1.9 times as long at 4,096 rows as a load at a time did, 0.97 so; eight warps a row with 128 registers 1.4 to 2 times as
+  // long as now.
+  constexpr int U = 16 / RD;
+  constexpr int UK = WPR == 1 && RD > 2 ? 4 : 8;
   extern __shared__ float qs[];  // WPR 1: [ATT_WARPS][d]; else [d] and the warps' partial results [WPR][ATT_RESULT(RD)]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long gw = WPR == 1 ? (long long)blockIdx.x * ATT_WARPS + warp : (long long)blockIdx.x;
@@ -239,6 +244,19 @@ attention_simt_kernel(const T* __restrict__ q, int q_stride, T* __restrict__ out
 
 // keys [pages, nkv, page_size, d], values [pages, nkv, page_size, dv], out [T, nq * dv]; with shared_keys: keys
 // [pages, 1, page_size, d], values [pages, 1, page_size, nkv * v_ld]
+// How many warps share a row, of 1 and 8: eight where rows are few for the keys that they see.  The block table's width bounds
+// the keys, and so do a window (with its kept keys) and a chunk; how long each sequence is, only the device knows (a wide
+// table means a long row, which takes far longer with one warp than all short ones with eight).  Eight warps' time over
+// one's, mean over float32 and bfloat16 heads of 64, 128 and 256: 512 rows x 128 keys 0.86, x 200 0.61; 1,024 x 200 1.03, x 256
+// 0.88; 2,048 x 400 0.98, x 512 0.85; 4,096 x 512 0.95, x 800 0.79 and x 128 2.3.
+RLLM_EXPORT int rllm_attention_simt_warps(long long rows, int max_blocks, int page_size, int window, int keep_first, int chunk) {
+  long long keys = (long long)max_blocks * page_size;
+  if (window > 0 && (long long)window + keep_first < keys) keys = (long long)window + keep_first;
+  if (chunk > 0 && chunk < keys) keys = chunk;
+  const long long enough = rows / 4 < 640 ? rows / 4 : 640;
+  return rows <= 4096 && keys > ATT_PART && keys >= enough ? 8 : 1;
+}
+
 RLLM_EXPORT int rllm_attention_simt_kv(const void* q, int q_stride, void* out, const void* kcache,
                                        const void* vcache, int dtype, const int* block_table,
                                        int max_blocks, const int* positions, const int* token_seq, int T,
@@ -254,11 +272,7 @@ RLLM_EXPORT int rllm_attention_simt_kv(const void* q, int q_stride, void* out, c
   if (dv > ATT_MAX_D || d > 2816) return RLLM_E_UNSUPPORTED;
   const bool vec = d % 8 == 0 && q_stride % 8 == 0 && (((uintptr_t)q | (uintptr_t)kcache) & 31) == 0;
   const long long rows = (long long)T * nq;
-  // Eight warps a row where rows are few and long (the block table's width bounds the keys): 792 rows x 1,033 keys 426 us
-  // with one warp, 227 with eight, 3,200 x 1,000 447 and 327, 32 x 101 27 and 24; but 2,048 rows x 64 keys 24 and 38,
-  // 6,400 x 300 184 and 294.
-  const long long keys = (long long)max_blocks * page_size;
-  const bool share = (rows <= 4096 && keys >= 512) || (rows <= 512 && keys >= 96);
+  const bool share = rllm_attention_simt_warps(rows, max_blocks, page_size, window, keep_first, chunk) == 8;
   const unsigned blocks = (unsigned)(share ? rows : (rows + ATT_WARPS - 1) / ATT_WARPS);
   const int rd = dv <= 64 ? 2 : (dv <= 128 ? 4 : 8);
   const size_t smem = (share ? (size_t)d + 8 * ATT_RESULT(rd) : (size_t)ATT_WARPS * d) * sizeof(float);

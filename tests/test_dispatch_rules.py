@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from rllm_b200.kernels import ops
+from rllm_b200.kernels import build, ops
 
 BF16 = torch.bfloat16
 
@@ -46,3 +46,18 @@ def test_which_experts_the_tcgen05_kernels_pay_for(E, H, F, pays, monkeypatch):
     assert ops.moe_tcgen05_pays(E, H, F) is pays
     monkeypatch.setenv("RLLM_GEMM", "tcgen05")
     assert ops.moe_tcgen05_pays(E, H, F)
+
+
+def test_how_many_warps_share_a_row_of_the_cuda_core_attention():
+    """The keys that a row can see decide, not the width of the table alone."""
+    from ctypes import c_int, c_longlong
+    f = build.load_library("attention_simt").rllm_attention_simt_warps
+    f.argtypes = [c_longlong] + [c_int] * 5
+    page = 16
+    for width in (64, 512, 8192):                          # keys that the table has room for
+        for window, kept, chunk in ((0, 0, 0), (64, 0, 0), (500, 11, 0), (500, 12, 0), (128, 0, 0), (128, 1, 0), (630, 9, 0), (630, 10, 0), (0, 0, 64),
+                                    (4000, 4, 100), (2 ** 31 - 1, 2 ** 31 - 1, 2 ** 31 - 1)):
+            keys = min(width, window + kept if window else width, chunk or width)
+            for rows in (1, 512, 516, 1024, 2044, 2048, 4096, 4097):
+                want = 8 if rows <= 4096 and keys > 128 and keys >= min(rows // 4, 640) else 1
+                assert f(rows, width // page, page, window, kept, chunk) == want
