@@ -1,4 +1,4 @@
-// Sampling over float32 logits [R, V], one block per row, with the reference's
+// Sampling over float32 logits [R, V], a cluster of blocks a row, with the reference's
 // pipeline (crates/rllm-sampling/src/sampler.rs:62-169): penalties and biases
 // (rllm_logit_edits), masks (rllm_logit_mask), then per row: greedy when
 // temperature <= 0 or top_k == 1 (:117), else temperature, top-k, top-p, min-p
@@ -351,6 +351,7 @@ RLLM_EXPORT int rllm_argmax(const float* logits, int R, int V, int ld, int* out_
 #define SC_BINS 2048
 #define SC_SELECT_BYTES (SC_BINS * 8 + SC_BINS * 4 + SC_BINS * 8)      // the last term over the CTAs of a row
 #define SC_STAGED_MAX (176 * 1024)       // bytes of a range that are kept in shared memory; a longer one is read again
+#define SC_WORDS_MAX (1 << 18)           // weights of a range that three words of 14 bits and 32 to count them hold
 
 __device__ __forceinline__ unsigned sc_addr(const void* p, int rank) {
   unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
@@ -396,6 +397,7 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
   const int per = (((V + cs - 1) / cs) + 3) & ~3;
   const int lo = min(V, rank * per), n = min(V, lo + per) - lo;
   x += lo;
+  const bool wide = per > SC_WORDS_MAX;
   auto value = [&](int i) { return staged ? ys[i] : x[i] * inv_t; };
 
   ArgMax best; best.v = -INFINITY; best.i = 0x7fffffff;
@@ -434,8 +436,9 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
     unsigned long long cum = 0;
     for (int pass = 0; pass < 3; ++pass) {
       const int shift = pass == 0 ? 21 : (pass == 1 ? 10 : 0);
-      // A weight's 42 bits are added up as three words of 14, with native 32-bit atomics; two of the words stand where
-      // the bins' sums will.
+      // A weight's 41 bits are added up as three words of 14, with native 32-bit atomics; two of the words stand where
+      // the bins' sums will.  A range of more than 2^18 weights could run over them: it takes two words and the carry, which
+      // an atomic has to come back with.
       unsigned* const w0 = (unsigned*)hist;
       unsigned* const w1 = w0 + SC_BINS;
       for (int b = tid; b < SC_BINS; b += THREADS) w0[b] = w1[b] = third[b] = 0u;
@@ -448,7 +451,11 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
         const unsigned bin = (key >> shift) & (SC_BINS - 1);
         if (by_mass) {
           const unsigned long long w = fx_mass(y, mx);
-          if (w) {
+          if (w && wide) {
+            const unsigned low = (unsigned)w;
+            const unsigned carry = atomicAdd(w0 + bin, low) > ~low ? 1u : 0u;
+            atomicAdd(w1 + bin, (unsigned)(w >> 32) + carry);
+          } else if (w) {
             atomicAdd(w0 + bin, (unsigned)w & 0x3fffu);
             atomicAdd(w1 + bin, (unsigned)(w >> 14) & 0x3fffu);
             atomicAdd(third + bin, (unsigned)(w >> 28));
@@ -463,7 +470,7 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
 #pragma unroll
       for (int q = 0; q < PER; ++q) {
         const int b = tid + q * THREADS;
-        mine[q] = ((unsigned long long)third[b] << 28) + ((unsigned long long)w1[b] << 14) + w0[b];
+        mine[q] = ((unsigned long long)third[b] << 28) + ((unsigned long long)w1[b] << (wide ? 32 : 14)) + w0[b];
       }
       __syncthreads();
 #pragma unroll
@@ -643,11 +650,6 @@ RLLM_EXPORT int rllm_sample(const float* logits, int R, int V, int ld, const flo
                             int select, cudaStream_t stream) {
   if (R <= 0) return 0;
   if (V <= 0 || ld < V || R > 65535) return RLLM_E_BADARG;
-  if (V > (1 << 21)) {                   // 32 bits hold 14-bit parts of 2^18 weights a CTA: a longer row is walked by one
-    sample_kernel<<<R, SAMPLE_THREADS, 0, stream>>>(logits, V, ld, temperature, top_k, top_p, min_p, seeds, gen_index, out_tokens);
-    RLLM_LAUNCH_CHECK();
-    return 0;
-  }
   // While the rows' clusters all fit at one CTA an SM: 1,024 threads (8 rows with top-p: 39 us, 43 with 512); then two
   // CTAs an SM (16 rows: 49 us, 69 with 1,024).
   if (R <= 14)

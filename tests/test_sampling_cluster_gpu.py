@@ -1,6 +1,6 @@
 """Sampling by a cluster of CTAs a row against the one-CTA kernel, token for token: the sizes at which the cluster, its
 threads and where a range is kept change (one, two and eight CTAs a row; up to 14 rows and more; ranges too long for
-shared memory, rows too long for the bins' words), rows that start anywhere, ties across the edges between ranges."""
+shared memory, ranges too long for words of 14 bits), rows that start anywhere, ties across the edges between ranges."""
 import pytest
 import torch
 
@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("V,R", [(2048, 3), (2049, 14), (16385, 15), (128256, 1), (128257, 14), (128256, 33),
-                                 (500003, 3), (2097153, 2)])
+                                 (500003, 3), (2097152, 1), (2097153, 2), (5000001, 1)])
 def test_clusters_draw_the_tokens_of_one_cta(V, R):
     from rllm_b200.kernels import ops
     g = torch.Generator(device="cuda")
