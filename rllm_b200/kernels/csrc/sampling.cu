@@ -621,11 +621,10 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
 template <int THREADS>
 static int sample_cluster_launch(const float* logits, int R, int V, int ld, const float* temperature, const int* top_k,
                                  const float* top_p, const float* min_p, const unsigned long long* seeds,
-                                 const long long* gen_index, int* out_tokens, int select, cudaStream_t stream) {
-  int cs = 8;                            // the portable most; fewer where a row is so short that they hold it at 2,048 each
-  while (cs > 1 && (cs / 2) * 2048 >= V) cs /= 2;
+                                 const long long* gen_index, int* out_tokens, int select, int cs, cudaStream_t stream) {
   const long long range = (long long)((((V + cs - 1) / cs) + 3) & ~3) * 4;
-  const int staged = range <= SC_STAGED_MAX ? 1 : 0;
+  // a long range in shared memory leaves an SM one CTA: plain draws of many rows rather read it again
+  const int staged = range <= SC_STAGED_MAX && (select || R < 64 || V < 200000) ? 1 : 0;
   static SmemLimit limit;
   if (const int e = limit.allow(sample_cluster_kernel<THREADS>, SC_STAGED_MAX + SC_SELECT_BYTES)) return e;
   cudaLaunchConfig_t cfg = {};
@@ -650,11 +649,41 @@ RLLM_EXPORT int rllm_sample(const float* logits, int R, int V, int ld, const flo
                             int select, cudaStream_t stream) {
   if (R <= 0) return 0;
   if (V <= 0 || ld < V || R > 65535) return RLLM_E_BADARG;
-  // While the rows' clusters all fit at one CTA an SM: 1,024 threads (8 rows with top-p: 39 us, 43 with 512); then two
-  // CTAs an SM (16 rows: 49 us, 69 with 1,024).
-  if (R <= 14)
-    return sample_cluster_launch<1024>(logits, R, V, ld, temperature, top_k, top_p, min_p, seeds, gen_index, out_tokens, select, stream);
-  return sample_cluster_launch<512>(logits, R, V, ld, temperature, top_k, top_p, min_p, seeds, gen_index, out_tokens, select, stream);
+  int cs = 8;                            // CTAs a row: the portable most; fewer where a row is so short that they hold it at 2,048 each
+  while (cs > 1 && (cs / 2) * 2048 >= V) cs /= 2;
+  int threads;
+  if (select) {
+    // While the rows' clusters all fit at one CTA an SM: 1,024 threads (8 rows with top-p: 39 us, 43 with 512); then two
+    // CTAs an SM (16 rows: 49 us, 69 with 1,024).
+    threads = R <= 14 ? 1024 : 512;
+    if (R >= 256 && V <= 16384) cs = 1;  // many short rows: 1,024 x 16,384 with top-p 781 us with eight CTAs a row, 164 with one
+  } else {
+    // A plain draw has three barriers and little else: the CTAs are as many and as large as the rows need to fill the GPU
+    // about once.  us, rows x logits, with 8 CTAs of 512 threads / as chosen: 1,024 x 64 22 / 12 (1 of 256), 512 x 4,096 28 / 15 (1 of
+    // 256), 256 x 16,384 62 / 24 and 256 x 32,000 71 / 36 (4 of 256), 256 x 64,000 88 / 61 (8 of 256), 15 x 262,144 31 / 24 and
+    // 15 x 524,288 71 / 46 (8 of 1,024), 256 x 262,144 361 / 257 (8 of 512, read twice).
+    if (V <= 2048) {
+      cs = 1; threads = 256;
+    } else if (V <= 8192) {
+      cs = R <= 128 ? 4 : (R <= 256 ? 2 : 1); threads = 256;
+    } else if (V >= 400000) {
+      threads = 1024;
+    } else if (R <= 32) {
+      threads = V >= 200000 || (V >= 48000 && R <= 15) ? 1024 : 512;
+    } else if (V >= 200000) {
+      threads = R < 64 ? 1024 : 512;
+    } else if (R <= 64) {
+      threads = V >= 100000 ? 512 : 256;
+    } else {
+      if (V < 48000) cs = 4;
+      threads = 256;
+    }
+  }
+#define SC_GO(T_) return sample_cluster_launch<T_>(logits, R, V, ld, temperature, top_k, top_p, min_p, seeds, gen_index, out_tokens, select, cs, stream)
+  if (threads == 1024) SC_GO(1024);
+  if (threads == 512) SC_GO(512);
+  SC_GO(256);
+#undef SC_GO
 }
 
 // ---------------------------------------------------------------------------

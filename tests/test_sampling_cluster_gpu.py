@@ -8,7 +8,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("V,R", [(2048, 3), (2049, 14), (16385, 15), (128256, 1), (128257, 14), (128256, 33),
-                                 (500003, 3), (2097152, 1), (2097153, 2), (5000001, 1)])
+                                 (500003, 3), (2097152, 1), (2097153, 2), (5000001, 1), (64, 300), (3001, 130), (3001, 260),
+                                 (20000, 50), (20000, 70), (50001, 65), (210000, 40), (210001, 64), (420001, 20)])
 def test_clusters_draw_the_tokens_of_one_cta(V, R):
     from rllm_b200.kernels import ops
     g = torch.Generator(device="cuda")
