@@ -152,11 +152,11 @@ template <int W> struct LtcRows {
     }
   }
   template <bool STEPS>
-  __device__ __forceinline__ void store(bf16 (*dst)[W + 8]) const {
+  __device__ __forceinline__ void store(bf16 (*dst)[W + 8], int n) const {
 #pragma unroll
     for (int u = 0; u < N; ++u) {
       const int e = (u * LTC_THREADS + threadIdx.x) * 8, j = e / W, c = e - j * W;
-      if (STEPS) {
+      if (STEPS || j >= n) {                     // (behind the chunk's end: zeros, without the work of activating them)
         *(uint4*)&dst[j][c] = raw[u];
       } else {
         float v[8];
@@ -169,8 +169,8 @@ template <int W> struct LtcRows {
   }
 };
 
-// (d, dv: the head's sizes; without STEPS they are D and DV)
-template <int D, int DV, bool STEPS>
+// (d, dv: the head's sizes; without STEPS they are D and DV.  WHOLE: heads of D x DV whose rows start on 16 bytes)
+template <int D, int DV, bool STEPS, bool WHOLE>
 __global__ void __launch_bounds__(LTC_THREADS)
 lightning_mma_pass1_kernel(const bf16* k, const bf16* v, int stride, int wide, const float* decay, LtSteps steps,
                            float* work, const int* q_start, int max_chunks, int heads, int d_, int dv_) {
@@ -186,10 +186,9 @@ lightning_mma_pass1_kernel(const bf16* k, const bf16* v, int stride, int wide, c
   if (n <= 0) return;
   const float l2 = STEPS ? 0.f : log2f(decay[h]);
   const int hk = STEPS ? h / steps.per : h;
-  const bool fast = wide == 2 && d == D && dv == DV;
   LtcRows<D> rk;
   LtcRows<DV> rv;
-  if (fast) {
+  if (WHOLE) {
     rk.fetch(k + (size_t)hk * D, stride, t0, n);
     rv.fetch(v + (size_t)h * DV, stride, t0, n);
   }
@@ -198,12 +197,16 @@ lightning_mma_pass1_kernel(const bf16* k, const bf16* v, int stride, int wide, c
     __syncthreads();
     if (threadIdx.x == 0) steps.chunk_dt[(size_t)blockIdx.y * heads + h] = -fac.L[n - 1] / (expf(steps.a_log[h]) * 1.4426950408889634f);
   }
-  if (fast) {
+  if (WHOLE) {
 #pragma unroll
     for (int u = 0; u < LtcRows<D>::N; ++u) {
       const int e = (u * LTC_THREADS + threadIdx.x) * 8, j = e / D, i = e - j * D;
-      float w = 0.f;
-      if (j < n) w = STEPS ? exp2f(fac.L[n - 1] - fac.L[j]) * fac.dt[j] : ltc_pow(l2, n - 1 - j);
+      if (j >= n) {                              // zeros, as they were fetched
+        *(uint4*)&sm.kh[j][i] = rk.raw[u];
+        *(uint4*)&sm.kl[j][i] = rk.raw[u];
+        continue;
+      }
+      const float w = STEPS ? exp2f(fac.L[n - 1] - fac.L[j]) * fac.dt[j] : ltc_pow(l2, n - 1 - j);
       float o[8], hi[8], lo[8];
       unpack8(rk.raw[u], o);
 #pragma unroll
@@ -215,7 +218,7 @@ lightning_mma_pass1_kernel(const bf16* k, const bf16* v, int stride, int wide, c
       store8(&sm.kh[j][i], hi);
       store8(&sm.kl[j][i], lo);
     }
-    rv.template store<STEPS>(sm.v);
+    rv.template store<STEPS>(sm.v, n);
   } else {
 #pragma unroll
   for (int e0 = 0; e0 < LTC_CHUNK * D; e0 += LTC_THREADS * 4) {
@@ -279,8 +282,8 @@ lightning_mma_pass1_kernel(const bf16* k, const bf16* v, int stride, int wide, c
     }
 }
 
-template <int D, int DV, bool STEPS>
-__global__ void __launch_bounds__(LTC_THREADS)
+template <int D, int DV, bool STEPS, bool WHOLE>
+__global__ void __launch_bounds__(LTC_THREADS, D == 64 && DV == 64 ? 3 : 2)      // blocks an SM
 lightning_mma_pass2_kernel(const bf16* q, const bf16* k, const bf16* v, int stride, int wide, const float* decay,
                            LtSteps steps, const float* work, const int* q_start, int max_chunks, float* out, int heads,
                            int d_, int dv_) {
@@ -300,7 +303,7 @@ lightning_mma_pass2_kernel(const bf16* q, const bf16* k, const bf16* v, int stri
   const int hk = STEPS ? h / steps.per : h;
   const float* s0 = work + ((size_t)blockIdx.y * heads + h) * d * dv;      // the chunk's start state [i][c]
   const bool whole = d == D && dv == DV;
-  if (whole && wide == 2) {
+  if (WHOLE) {
     LtcRows<D> rq, rk;
     LtcRows<DVB> rv;
     constexpr int NS = D * DVB / (LTC_THREADS * 4);
@@ -314,9 +317,9 @@ lightning_mma_pass2_kernel(const bf16* q, const bf16* k, const bf16* v, int stri
       rs[u] = *(const float4*)(s0 + (size_t)i * DV + cb + c);
     }
     if (STEPS) ltc_factors(fac, steps, t0, n, h, heads);
-    rq.template store<STEPS>(sm.q);
-    rk.template store<STEPS>(sm.k);
-    rv.template store<STEPS>(sm.v);
+    rq.template store<STEPS>(sm.q, n);
+    rk.template store<STEPS>(sm.k, n);
+    rv.template store<STEPS>(sm.v, n);
 #pragma unroll
     for (int u = 0; u < NS; ++u) {
       const int e = (u * LTC_THREADS + threadIdx.x) * 4, i = e / DVB, c = e - i * DVB;
@@ -461,22 +464,31 @@ lightning_mma_pass2_kernel(const bf16* q, const bf16* k, const bf16* v, int stri
 
 // Launches the two passes around `chain` (the caller's kernel that turns end-from-zero states into start
 // states).  Returns false if this head shape is not instantiated.
+template <int D, int DV, bool STEPS, bool WHOLE, typename Chain>
+static void ltc_launch_form(const bf16* q, const bf16* k, const bf16* v, int stride, int wide, const float* decay, LtSteps steps,
+                            float* work, const int* q_start, int num_seqs, int max_chunks, float* out, int heads, int d,
+                            int dv, cudaStream_t stream, Chain chain) {
+  const dim3 grid(heads, num_seqs * max_chunks);
+  const size_t s1 = sizeof(LtcSmem1<D, DV>), s2 = sizeof(LtcSmem2<D, DV / LtcSplit<D, DV>::N>);
+  static SmemLimit limit1, limit2;                  // (refused: the launch then says so)
+  limit1.allow(lightning_mma_pass1_kernel<D, DV, STEPS, WHOLE>, s1);
+  limit2.allow(lightning_mma_pass2_kernel<D, DV, STEPS, WHOLE>, s2);
+  rllm_launch_pdl(lightning_mma_pass1_kernel<D, DV, STEPS, WHOLE>, grid, dim3(LTC_THREADS), s1, stream, k, v, stride, wide, decay,
+                  steps, work, q_start, max_chunks, heads, d, dv);
+  chain();
+  rllm_launch_pdl(lightning_mma_pass2_kernel<D, DV, STEPS, WHOLE>, dim3(grid.x, grid.y, LtcSplit<D, DV>::N), dim3(LTC_THREADS), s2, stream, q, k, v, stride, wide, decay,
+                  steps, (const float*)work, q_start, max_chunks, out, heads, d, dv);
+}
 template <int D, int DV, bool STEPS, typename Chain>
 static bool ltc_launch(const bf16* q, const bf16* k, const bf16* v, int stride, const float* decay, LtSteps steps,
                        float* work, const int* q_start, int num_seqs, int max_chunks, float* out, int heads, int d,
                        int dv, cudaStream_t stream, Chain chain) {
-  const dim3 grid(heads, num_seqs * max_chunks);
-  const size_t s1 = sizeof(LtcSmem1<D, DV>), s2 = sizeof(LtcSmem2<D, DV / LtcSplit<D, DV>::N>);
-  static SmemLimit limit1, limit2;                  // (refused: the launch then says so)
-  limit1.allow(lightning_mma_pass1_kernel<D, DV, STEPS>, s1);
-  limit2.allow(lightning_mma_pass2_kernel<D, DV, STEPS>, s2);
   // rows that start on 8-byte boundaries are fetched four values a load, on 16-byte boundaries (whole heads) eight
-  const int wide8 = stride % 8 == 0 && d % 8 == 0 && dv % 8 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) == 0;
-  const int wide = wide8 ? 2 : (stride % 4 == 0 && d % 4 == 0 && dv % 4 == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 7) == 0);
-  rllm_launch_pdl(lightning_mma_pass1_kernel<D, DV, STEPS>, grid, dim3(LTC_THREADS), s1, stream, k, v, stride, wide, decay,
-                  steps, work, q_start, max_chunks, heads, d, dv);
-  chain();
-  rllm_launch_pdl(lightning_mma_pass2_kernel<D, DV, STEPS>, dim3(grid.x, grid.y, LtcSplit<D, DV>::N), dim3(LTC_THREADS), s2, stream, q, k, v, stride, wide, decay,
-                  steps, (const float*)work, q_start, max_chunks, out, heads, d, dv);
+  const uintptr_t at = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v;
+  const int wide = stride % 4 == 0 && d % 4 == 0 && dv % 4 == 0 && (at & 7) == 0;
+  if (d == D && dv == DV && stride % 8 == 0 && (at & 15) == 0)
+    ltc_launch_form<D, DV, STEPS, true>(q, k, v, stride, wide, decay, steps, work, q_start, num_seqs, max_chunks, out, heads, d, dv, stream, chain);
+  else
+    ltc_launch_form<D, DV, STEPS, false>(q, k, v, stride, wide, decay, steps, work, q_start, num_seqs, max_chunks, out, heads, d, dv, stream, chain);
   return true;
 }
