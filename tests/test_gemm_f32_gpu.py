@@ -6,7 +6,8 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("N,K,offset", [(1024, 2048, 0), (8192, 260, 0), (301, 40, 0), (77, 129, 1), (2080, 63, 3)])
+@pytest.mark.parametrize("N,K,offset", [(1024, 2048, 0), (8192, 260, 0), (301, 40, 0), (77, 129, 1), (2080, 63, 3), (8192, 16, 0),
+                                        (8200, 40, 0), (8192, 101, 1), (4100, 520, 2)])
 def test_rows_of_the_float32_product_are_independent(N, K, offset):
     from rllm_b200.kernels import ops
     g = torch.Generator(device="cuda")
