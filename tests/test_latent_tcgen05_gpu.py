@@ -107,3 +107,66 @@ def test_rows_that_the_window_hides_do_not_reach_the_output(heads, dk, dv, windo
     want, size = p @ rows[:, :dv].double(), p @ rows[:, :dv].double().abs()
     got = out.view(m, heads, dv).transpose(0, 1).double()
     assert bool(((got - want).abs() <= 2.0 ** -7 * size + 1e-5).all())       # the bound of the test above
+
+
+@pytest.mark.parametrize("window,sink", [(None, False), (37, True), (None, True)])
+def test_a_step_of_decoded_tokens_and_prompts_through_the_mixer(window, sink, monkeypatch):
+    """The part alone: prompts first, then a step in which three requests decode beside two portions, one of them behind
+    rows of an earlier step.  The portions run on tcgen05, the decoded tokens on mma.sync."""
+    from test_parts_gpu import DEV, context_for, load_part
+
+    from rllm_b200.cache import CacheStorage
+    from rllm_b200.kernels import ops
+    from rllm_b200.models.decoder import CacheLayout
+    from rllm_b200.parts import PartSpec, build_part
+    hidden, H, nope, rot, vdim, kv, dt = 96, 32, 24, 16, 40, 64, torch.bfloat16
+    names = {k: k for k in ("dq", "dq_norm", "uq", "dkv", "dkv_norm", "uk", "uv", "sink", "o")}
+    spec = PartSpec.of("latent_attention", tensor_names=names, hidden_size=hidden, num_heads=H, nope_dim=nope, rot_dim=rot,
+                       v_dim=vdim, q_rank=56, kv_rank=kv, scale=(nope + rot) ** -0.5, eps=1e-6, window=window, sink=sink,
+                       position=PartSpec.of("rotary", head_dim=rot, rotary_dim=rot, theta=5000.0, scaling=None, interleaved=True))
+    part = build_part("mixer", spec)
+    w = load_part(part, dt)
+    storage = CacheStorage(CacheLayout([part.cache_need()], [[0]], [0], [0]), 16, [64], 8, dt, DEV)
+    torch.manual_seed(3)
+    before, new = {"a": 70, "b": 9, "c": 130, "d": 50, "e": 0}, {"a": 1, "b": 1, "c": 1, "d": 64, "e": 41}
+    xs = {r: (torch.randn(before[r] + new[r], hidden) * 2).to(dt) for r in before}
+    ctx, cache = context_for([part.cache_need()], 16, 64, [(r, [0] * n, 0) for r, n in before.items() if n], dt)
+    part.forward(torch.cat([xs[r][: before[r]] for r in "abcd"]).to(DEV), ctx, storage.view(0))
+    ran = []
+    for name in ("latent_attention_tcgen05", "latent_attention_mma"):
+        real = getattr(ops, name)
+        monkeypatch.setattr(ops, name, lambda *a, _f=real, _n=name, **k: (ran.append(_n), _f(*a, **k))[1])
+    ctx, cache = context_for([part.cache_need()], 16, 64, [(r, [0] * n, before[r]) for r, n in new.items()], dt, cache)
+    assert ctx.num_decode == 3
+    got = part.forward(torch.cat([xs[r][before[r]:] for r in new]).to(DEV), ctx, storage.view(0)).double().cpu()
+    assert ran == ["latent_attention_tcgen05", "latent_attention_mma"] and int(ctx.err.item()) == 0
+
+    def norm(x, g):
+        return x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-6) * g
+
+    def turn(x, pos):                                      # pairs (2 i, 2 i + 1)
+        a = pos[:, None] * 5000.0 ** (-torch.arange(0, rot, 2, dtype=torch.float64) / rot)
+        c, s = a.cos().view(len(pos), *([1] * (x.ndim - 2)), -1), a.sin().view(len(pos), *([1] * (x.ndim - 2)), -1)
+        u, v = x[..., ::2], x[..., 1::2]
+        return torch.stack([u * c - v * s, v * c + u * s], -1).flatten(-2)
+
+    at = 0
+    for r, m in new.items():
+        x, n = xs[r].double(), before[r] + m
+        pos = torch.arange(n, dtype=torch.float64)
+        q = (norm(x @ w["dq"].t(), w["dq_norm"]) @ w["uq"].t()).view(n, H, nope + rot)
+        a = x @ w["dkv"].t()
+        rows = torch.cat([norm(a[:, :kv], w["dkv_norm"]), turn(a[:, kv:], pos)], 1)
+        qt = torch.cat([torch.einsum("thn,hnk->thk", q[..., :nope], w["uk"].view(H, nope, kv)), turn(q[..., nope:], pos)], 2)
+        sc = torch.einsum("thk,jk->htj", qt, rows) * (nope + rot) ** -0.5
+        hidden_keys = pos[None] > pos[:, None]
+        if window:
+            hidden_keys |= pos[None] <= pos[:, None] - window
+        sc = sc.masked_fill(hidden_keys, -math.inf)
+        if sink:
+            sc = torch.cat([sc, w["sink"].view(H, 1, 1).expand(H, n, 1)], 2)
+        o = torch.einsum("htj,jk->thk", torch.softmax(sc, 2)[:, :, :n], rows[:, :kv])
+        want = torch.einsum("thk,hvk->thv", o, w["uv"].view(H, vdim, kv)).reshape(n, H * vdim) @ w["o"].t()
+        # a dozen roundings to bfloat16 one after the other, as the parts' other tests allow for: 2 % of the largest result
+        assert float((got[at: at + m] - want[before[r]:]).abs().max()) <= 2e-2 * float(want.abs().max()), r
+        at += m
