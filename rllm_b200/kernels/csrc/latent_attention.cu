@@ -111,6 +111,15 @@ RLLM_EXPORT int rllm_latent_prep(const void* a, int a_stride, int q_rank, int kv
 // ---------------------------------------------------------------------------
 // the queries' rotated part: q[t, h, dim : dim+rot] rotated -> qt[t, h, kv_rank : kv_rank+rot]
 // ---------------------------------------------------------------------------
+// The turn of a pair with its roundings spelled out, the same in every kernel: left to fuse the products itself, the compiler
+// chose differently for the two forms below, and a token's bits depended on how many came with it.  (Which product keeps its
+// rounding differs by type as it always has.)
+template <typename T>
+__device__ __forceinline__ void rot_turn(float u, float v, float c, float sn, float* x, float* y) {
+  *x = __fmaf_rn(u, c, -__fmul_rn(v, sn));
+  *y = sizeof(T) == 4 ? __fmaf_rn(u, sn, __fmul_rn(v, c)) : __fmaf_rn(v, c, __fmul_rn(u, sn));
+}
+
 // a thread a pair and head
 template <typename T>
 __global__ void latent_q_rot_pair_kernel(const T* q, T* qt, const int* positions,
@@ -132,8 +141,10 @@ __global__ void latent_q_rot_pair_kernel(const T* q, T* qt, const int* positions
     float c, sn;
     rot_cos_sin<T>(positions[t], inv_freq[i], &c, &sn);
     c *= mag; sn *= mag;
-    dst[2 * i] = from_f32<T>(u * c - v * sn);
-    dst[2 * i + 1] = from_f32<T>(v * c + u * sn);
+    float tu, tv;
+    rot_turn<T>(u, v, c, sn, &tu, &tv);
+    dst[2 * i] = from_f32<T>(tu);
+    dst[2 * i + 1] = from_f32<T>(tv);
   } else {
     dst[2 * i] = from_f32<T>(u);
     dst[2 * i + 1] = from_f32<T>(v);
@@ -161,8 +172,10 @@ __global__ void latent_q_rot_kernel(const T* q, T* qt, const int* positions,
       const T* src = q + ((size_t)t * heads + h) * (dim + rot) + dim;
       T* dst = qt + ((size_t)t * heads + h) * (kv_rank + rot) + kv_rank;
       const float u = to_f32(src[2 * i]), v = to_f32(src[2 * i + 1]);
-      dst[2 * i] = turns ? from_f32<T>(u * c - v * sn) : from_f32<T>(u);
-      dst[2 * i + 1] = turns ? from_f32<T>(v * c + u * sn) : from_f32<T>(v);
+      float tu = u, tv = v;
+      if (turns) rot_turn<T>(u, v, c, sn, &tu, &tv);
+      dst[2 * i] = from_f32<T>(tu);
+      dst[2 * i + 1] = from_f32<T>(tv);
     }
   }
 }
