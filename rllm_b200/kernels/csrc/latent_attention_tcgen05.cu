@@ -288,7 +288,9 @@ latent_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, bf16* out, cons
       ok = pair_exchange(x_mine + (it & 1), x_theirs + (it & 1), &xbar[quarter], it, mx, &mx_other, err);
       if (!ok) break;
       mx = fmaxf(mx, mx_other) * scale_log2;
-      const bool moves = mx > m_ref + 8.0f;          // the reference point moves only when the max has grown by 2^8
+      // The reference point is the row's largest score so far, so that its weight is 1 and has no rounding.  (Moved only when the
+      // max has grown by 2^8, as in attention_tcgen05.cu, results are further from float64 than the mma.sync kernel's.)
+      const bool moves = mx > m_ref;
       float corr = 1.0f;
       if (moves) {
         corr = at_ex2(m_ref - mx);
