@@ -16,10 +16,11 @@
 // Q takes 147 KB at 576 values, which leaves room for one tile's value panels and six slots.  What bounds it there is a
 // cycle: P V gives the value panels back, the next ones come in (about 1,700 cycles), the scores are finished, the softmax
 // runs.  Rows of up to 448 values have two sets of value panels.
-// Measured against the mma.sync kernel: 2,048 tokens x 16 heads, rows of 576: 627 -> 205 us (8,192 tokens 9.3 -> 2.65 ms,
-// 441 TFLOP/s); 8 heads, rows of 288: 189 -> 62 us (8,192: 2.58 -> 0.40 ms, 722 TFLOP/s).  One warp issuing all products:
-// 312 us; the panels shared by all producer warps, one panel at a time: 410 us; the value panels brought twice, so that
-// the scores need not wait for P V: 205 us (what the copies add is what the wait cost).
+// Measured against the mma.sync kernel: 2,048 tokens x 16 heads, rows of 576: 625 -> 213 us (8,192 tokens 9.3 -> 2.90 ms,
+// 403 TFLOP/s); 8 heads, rows of 288: 188 -> 68 us (8,192: 2.57 -> 0.45 ms, 645 TFLOP/s).  With a reference point that lagged the
+// running maximum 205 us, and there: one warp issuing all products 312 us; the panels shared by all producer warps, one panel
+// at a time: 410 us; the value panels brought twice, so that the scores need not wait for P V: 205 us (what the copies add is
+// what the wait cost).
 // Every wait on an mbarrier is bounded (bit 16 of the error word, then wind-down).  No cluster, no multicast.
 #include "attention_tcgen05.cuh"
 

@@ -1007,10 +1007,13 @@ def latent_attention_tcgen05_pays(q_lens, seq_lens, heads: int, dv: int, window:
     """Whether the tcgen05 kernel is the faster one for prompt portions of these lengths (``seq_lens`` with what the cache
     holds).  Its CTA takes 128 rows of one sequence and 256 value columns, an SM to itself, and walks all their keys (2.9 us
     a tile of 64 keys of 576 values, however few rows there are); the mma.sync kernel takes 16 to 64 rows and cuts the keys
-    too where it has few rows.  The lines, in microseconds mma.sync / tcgen05 (885 sizes were measured; none that the rule
-    lets through is more than 3 % slower):
-      few rows and many keys, cut by mma.sync: 16 heads of 576, 4,096 keys, 1,024 rows 156 / 186, 1,152 174 / 186, 1,280 up
-        to equal; 8 heads of 288 92 / 111 at 1,024 rows;
+    too where it has few rows.  The lines, in microseconds mma.sync / tcgen05 (2,700 sizes of 4 to 128 heads of 144 to 576
+    values were measured; 5 of those that the rule lets through are more than 3 % slower, by 10 % at most):
+      few rows and many keys, cut by mma.sync: 16 heads of 576, 4,096 keys, 1,280 rows 197 / 215, 1,600 238 / 215; 8 heads of
+        288 110 / 128 at 1,280 rows; 32 heads of 192, 1,280 rows 59 / 94; 4 heads of 144, 8,192 keys, 1,536 rows
+        112 / 180, 2,048 79 / 103 at 4,096 keys;
+      one tile of keys on many CTAs: 64 portions of 16 x 8 heads of 288, 16 keys, 12 / 15; few keys and many sequences of a tile, among
+        which a CTA looks for its own: 300 portions of 4 x 32 heads of 192, 104 keys, 45 / 90;
       tiles not half full: 128 portions of 2 tokens x 16 heads, 2,048 keys, 177 / 243 (256 CTAs); 64 of them 157 / 121;
         128 portions of 2 x 8 heads of 288, 512 keys, 22 / 29;
       few keys, where what a CTA costs to start counts: 64 portions of 4 x 16 heads, 128 keys, 16 / 19, 32 of 8 16 / 18, but
@@ -1020,7 +1023,10 @@ def latent_attention_tcgen05_pays(q_lens, seq_lens, heads: int, dv: int, window:
     most_q, most_keys = max(q_lens), max(seq_lens)
     keys = min(most_keys, window + most_q) if window else most_keys
     parts = -(-dv // 256)
-    if rows < 1280 and latent_attention_mma_splits(len(q_lens), most_q, heads, most_keys, window):
+    few_rows = 1408 if parts > 1 else (2048 if dv > 128 else 3072)
+    if rows < few_rows and latent_attention_mma_splits(len(q_lens), most_q, heads, most_keys, window):
+        return False
+    if (keys <= 64 and tiles * parts > 32) or (keys < 256 and tiles <= len(q_lens) > 100):
         return False
     if keys < 512:
         return rows >= 96 * tiles and (parts == 1 or rows > 4096)

@@ -29,12 +29,14 @@ def test_experts_beyond_the_tensor_maps_keep_the_kernels_that_took_them(E, H, F,
 
 
 @pytest.mark.parametrize("q_lens,keys,heads,dv,window,tcgen05", [
-    ([2048], 2048, 16, 512, 0, True), ([80], 4096, 16, 512, 0, True), ([72], 4096, 16, 512, 0, False),
-    ([8] * 8, 4096, 16, 512, 0, False), ([10] * 8, 4096, 16, 512, 0, True), ([64], 512, 16, 512, 0, True),
-    ([64], 4096, 16, 512, 500, True), ([128], 4096, 8, 256, 0, False), ([160], 4096, 8, 256, 0, True),
+    ([2048], 2048, 16, 512, 0, True), ([80], 4096, 16, 512, 0, False), ([88], 4096, 16, 512, 0, True),
+    ([8] * 8, 4096, 16, 512, 0, False), ([10] * 8, 4096, 16, 512, 0, False), ([11] * 8, 4096, 16, 512, 0, True), ([64], 512, 16, 512, 0, True),
+    ([64], 4096, 16, 512, 500, True), ([128], 4096, 8, 256, 0, False), ([160], 4096, 8, 256, 0, False), ([256], 4096, 8, 256, 0, True),
     ([2] * 128, 2048, 16, 512, 0, False), ([2] * 64, 2048, 16, 512, 0, True), ([2] * 128, 512, 8, 256, 0, False),
     ([4] * 64, 128, 16, 512, 0, False), ([8] * 32, 128, 16, 512, 0, False), ([32] * 16, 128, 16, 512, 0, True),
-    ([64] * 8, 128, 8, 256, 0, True), ([2] * 64, 128, 8, 256, 0, False), ([1792, 3], 1792, 16, 512, 0, True)])
+    ([64] * 8, 128, 8, 256, 0, True), ([2] * 64, 128, 8, 256, 0, False), ([1792, 3], 1792, 16, 512, 0, True),
+    ([40], 4136, 32, 128, 0, False), ([100], 4096, 32, 128, 0, True), ([512], 4608, 4, 128, 0, False), ([4] * 300, 4, 32, 128, 0, False),
+    ([4] * 300, 204, 32, 128, 0, False), ([32] * 16, 64, 16, 512, 0, False), ([64] * 8, 64, 8, 256, 0, True), ([64] * 8, 164, 32, 128, 0, True)])
 def test_which_prompt_portions_the_tcgen05_latent_attention_pays_for(q_lens, keys, heads, dv, window, tcgen05):
     assert ops.latent_attention_tcgen05_pays(q_lens, [keys] * len(q_lens), heads, dv, window) is tcgen05
 
