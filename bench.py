@@ -566,7 +566,8 @@ BIKOVIK_SIZES = {
 
 # entry points of ``ops`` whose launches the step tables of ``--design`` time one by one
 STEP_KERNELS = (
-    "latent_attention_mma", "latent_attention_tcgen05", "attention_prefill_tcgen05", "attention_prefill_bf16",
+    "latent_attention_mma", "latent_attention_tcgen05", "latent_expanded_tcgen05", "latent_expand_prep",
+    "attention_prefill_tcgen05", "attention_prefill_bf16",
     "attention_decode_bf16", "moe_experts", "moe_route", "head_gemm", "mingru_scan", "gated_postnorm_add",
     "depth_average", "rmsnorm", "silu_mul", "latent_prep", "latent_q_rot", "rope_kv_write", "gemm_small_m",
     "moe_choose", "gemm_small_m_residual", "gemm_small_m_rstd", "gemm_tcgen05", "embedding", "lightning_scan",
@@ -614,6 +615,12 @@ def compare_designs(args):
             vis = sum(min(p + 1, window or p + 1) for p in range(ctx - Tn // S, ctx)) * S
             keys = S * min(ctx, (window or ctx) + Tn // S)
             return 2.0 * (dk + dv) * heads * vis, 2.0 * (keys * dk + q.numel() + a[1].numel())
+        if name == "latent_expanded_tcgen05":
+            q, kv, rows, out, (heads, nope, rot, v, _, window) = a[0], a[1], a[2], a[3], a[9:15]
+            vis = sum(min(p + 1, window or p + 1) for p in range(ctx - Tn // S, ctx)) * S
+            return 2.0 * (nope + rot + v) * heads * vis, 2.0 * (q.numel() + kv.numel() + rows.shape[0] * rot + out.numel())
+        if name == "latent_expand_prep":
+            return 0.0, 4.0 * (a[2].numel() + a[0].shape[0] * a[11] * a[13])
         if name in ("attention_prefill_tcgen05", "attention_prefill_bf16", "attention_decode_bf16"):
             nq, nkv, d, window = (a[11], a[12], a[13], a[14]) if name != "attention_decode_bf16" else \
                 (a[9], a[10], a[11], a[12])

@@ -37,7 +37,7 @@ NVCC_FLAGS = [
 ]
 
 SOURCES = ["elementwise", "attention_simt", "attention_mma", "attention_tcgen05", "gemm_f32", "gemm_small_m", "gemm_tcgen05", "sampling", "weights_rng",
-           "layer_glue", "mingru", "latent_attention", "latent_attention_mma", "latent_attention_tcgen05", "moe", "moe_tcgen05",
+           "layer_glue", "mingru", "latent_attention", "latent_attention_mma", "latent_attention_tcgen05", "latent_expanded_tcgen05", "moe", "moe_tcgen05",
            "hyper_streams", "mixer_glue", "lightning", "selective_scan", "layernorm", "mlstm",
            "ssd", "channel_delta", "linear_state", "talking_heads", "shared_key_attention"]
 

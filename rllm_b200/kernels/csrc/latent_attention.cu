@@ -201,6 +201,85 @@ RLLM_EXPORT int rllm_latent_q_rot(const void* q, void* qt, const int* positions,
 }
 
 // ---------------------------------------------------------------------------
+// What latent_expanded_tcgen05.cu reads, for the prompt portions of sequences seq_begin .. seq_end - 1: the visible cached
+// rows of every sequence, gathered from their pages one sequence behind the other (each from the oldest key of its first
+// query rounded down to 128; what lies ahead of that key is zeros), and the queries' last rot dims rotated in place.
+// Blocks 0 .. gather_blocks - 1 gather, a warp a row; the rest rotate, a block a token.  Both are copies of memory (2,048
+// rows of 576 and 16 heads of 64: 13 MB), together a launch less.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256)
+latent_expand_prep_kernel(bf16* q, const bf16* cache, bf16* rows, const int* block_table, int max_blocks,
+                          const int* q_start, const int* seq_lens, int seq_begin, int seq_end, const int* positions,
+                          const double* inv_freq, float mag, int first_token, int heads, int dim, int rot, int rot_dims,
+                          int dk, int num_rows, int gather_blocks, int page_size, int num_pages, int window, int* err) {
+  pdl_wait();
+  pdl_launch();
+  if ((int)blockIdx.x >= gather_blocks) {
+    const int half = rot / 2, t = first_token + blockIdx.x - gather_blocks;
+    const int turned = rot_dims / 2;                              // the pairs behind these stay as they are
+    const int per = max(1, (int)blockDim.x / max(1, turned));     // heads side by side
+    for (int w = threadIdx.x; w < per * turned; w += blockDim.x) {
+      const int i = w % turned;
+      float c, sn;
+      rot_cos_sin<bf16>(positions[t], inv_freq[i], &c, &sn);
+      c *= mag; sn *= mag;
+      for (int h = w / turned; h < heads; h += per) {
+        __nv_bfloat162* at = (__nv_bfloat162*)(q + ((size_t)t * heads + h) * (dim + 2 * half) + dim) + i;
+        const float2 uv = __bfloat1622float2(*at);
+        float tu, tv;
+        rot_turn<bf16>(uv.x, uv.y, c, sn, &tu, &tv);
+        *at = __floats2bfloat162_rn(tu, tv);
+      }
+    }
+    return;
+  }
+  const int lane = threadIdx.x & 31;
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (row >= num_rows) return;
+  int s = -1, j = 0, oldest = 0;
+  {
+    int left = row;
+    for (int i = seq_begin; i < seq_end; ++i) {
+      const int p = seq_lens[i] - (q_start[i + 1] - q_start[i]);              // the first query's position
+      oldest = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
+      const int lo = oldest / 128 * 128, n = seq_lens[i] - lo;
+      if (left < n) { s = i; j = lo + left; break; }
+      left -= n;
+    }
+  }
+  if (s < 0) return;
+  const bf16* src = nullptr;
+  if (j >= oldest) {
+    const int page = block_table[(size_t)s * max_blocks + j / page_size];
+    if (page >= 0 && page < num_pages) src = cache + ((size_t)page * page_size + j % page_size) * dk;
+    else if (lane == 0) atomicOr(err, 4);                         // a visible key without a page
+  }
+  uint4* to = (uint4*)(rows + (size_t)row * dk);
+  for (int i = lane; i < dk / 8; i += 32) to[i] = src ? ((const uint4*)src)[i] : make_uint4(0u, 0u, 0u, 0u);
+}
+
+// q [., heads (dim + rot)], rotated in place from row first_token on (num_tokens rows); cache [pages, 1, page_size, dk]; rows [num_rows, dk], num_rows
+// what the sequences' visible rows come to.  dk and dim + rot multiples of 8; rot and rot_dims even.
+RLLM_EXPORT int rllm_latent_expand_prep(void* q, const void* cache, void* rows, const int* block_table, int max_blocks,
+                                        const int* q_start, const int* seq_lens, int seq_begin, int seq_end,
+                                        const int* positions, const double* inv_freq, float mag, int first_token,
+                                        int num_tokens, int heads, int dim, int rot, int rot_dims, int dk, int num_rows,
+                                        int page_size, int num_pages, int window, int* err, cudaStream_t stream) {
+  if (seq_end <= seq_begin || num_tokens <= 0) return 0;
+  if (heads <= 0 || dim <= 0 || rot < 0 || (rot & 1) || (rot_dims & 1) || rot_dims < 0 || rot_dims > rot || dk <= 0 || num_rows <= 0 || page_size <= 0 ||
+      num_pages <= 0 || max_blocks <= 0 || window < 0 || first_token < 0 || !err)
+    return RLLM_E_BADARG;
+  if (dk % 8 || (dim & 1) || (((uintptr_t)cache | (uintptr_t)rows) & 15) || ((uintptr_t)q & 3)) return RLLM_E_UNSUPPORTED;
+  const int gather_blocks = (num_rows + 7) / 8;
+  rllm_launch_pdl(latent_expand_prep_kernel, dim3((unsigned)(gather_blocks + (rot_dims ? num_tokens : 0))), dim3(256), (size_t)0,
+                  stream, (bf16*)q, (const bf16*)cache, (bf16*)rows, block_table, max_blocks, q_start, seq_lens, seq_begin,
+                  seq_end, positions, inv_freq, mag, first_token, heads, dim, rot, rot_dims, dk, num_rows, gather_blocks,
+                  page_size, num_pages, window, err);
+  RLLM_LAUNCH_CHECK();
+  return 0;
+}
+
+// ---------------------------------------------------------------------------
 // products per head: C[m, h, 0:N] = A[m, h, 0:K] . B[h], with B[h] either [N, K] or [K, N];
 // A, B and C are slices with their own row and head strides (elements)
 // ---------------------------------------------------------------------------

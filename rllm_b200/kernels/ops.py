@@ -1061,6 +1061,100 @@ def latent_attention_tcgen05(q: torch.Tensor, out: torch.Tensor, cache: torch.Te
         "latent_attention_tcgen05")
 
 
+def latent_expanded_rows(q_lens, seq_lens, window: int) -> int:
+    """How many cached rows ``latent_expand_prep`` gathers for prompt portions of these lengths."""
+    n = 0
+    for q, k in zip(q_lens, seq_lens):
+        n += k - (max(0, k - q - window + 1) // 128 * 128 if window else 0)
+    return n
+
+
+def latent_expanded_shapes(dtype: torch.dtype, nope: int, rot: int, v: int, kv_rank: int, scale: float) -> bool:
+    """Whether prompt portions of a mixer of these sizes can run with every head's own keys and values."""
+    return (dtype is torch.bfloat16 and nope in (64, 128) and v in (64, 128) and 0 < rot <= 64 and rot % 8 == 0
+            and kv_rank % 8 == 0 and scale > 0)
+
+
+def latent_expanded_allowed() -> bool:
+    """RLLM_LATENT_ATTENTION (simt, mma, absorbed) and RLLM_GEMM=library|no_tcgen05 keep prompts off that form."""
+    return not os.environ.get("RLLM_LATENT_ATTENTION") and os.environ.get("RLLM_GEMM") not in ("library", "no_tcgen05")
+
+
+LATENT_EXPANDED_SCRATCH = 512 << 20      # bytes of gathered rows, keys and values; more only where the other form needs as much
+
+
+def latent_expanded_pays(q_lens, seq_lens, heads: int, nope: int, v: int, kv_rank: int, rot: int, window: int,
+                         beside: bool = False) -> bool:
+    """Whether prompt portions of these lengths (``seq_lens`` with what the cache holds) are faster with every head's own
+    keys and values than with W_uk and W_uv on the query side.  ``beside``: tokens that decode are in the step too; they
+    keep the query side, which then costs its launches as well.  The lines, in microseconds a mixer, query side / own
+    (A: 16 heads of 128 + 64 | 128 over rows of 512 + 64; B: 8 of 64 + 32 | 64 over 256 + 32; C: A with 64 heads; D: 4
+    heads of B's over 128 + 32), prompts from position 0 of 1,800 tokens A 264 / 110, B 98 / 54:
+      few rows: B 2 tokens 21 / 23, D 8 tokens 22 / 23, but B 8 tokens 29 / 25;
+      few rows and many keys, where a CTA walks all its keys and the query side cuts them: 4,096 keys A 17 tokens 86 / 113,
+        33 120 / 114, B 33 63 / 72, 64 76 / 72, D 128 48 / 69, 300 75 / 72; beside 8 tokens that decode D 83 behind
+        1,024 46 / 72, A 64 122 / 102;
+      a product over the rows that costs more than it saves: 1,024 keys, 8 tokens A 45 / 48, C 68 / 72;
+      tiles of 128 tokens not filled, by many sequences or on more CTAs than run at once: 64 portions of 4 A 61 / 75, D
+        27 / 40, of 16 behind 200 A 111 / 169; 16 of 33 behind 1,000 C 348 / 489, but A (256 CTAs) 171 / 156."""
+    own, absorbed = nope + rot + v, 2 * kv_rank + rot          # multiplications a query, key and head
+    tokens, most, tiles, pairs, padded = sum(q_lens), 0, 0, 0, 0
+    for q, k in zip(q_lens, seq_lens):
+        keys, t = min(k, window + q) if window else k, -(-q // 128)
+        most, tiles, pairs, padded = max(most, keys), tiles + t, pairs + q * keys, padded + 128 * t * keys
+    rows = latent_expanded_rows(q_lens, seq_lens, window)
+    if 2 * rows * (heads * (nope + v) + kv_rank + rot) > max(LATENT_EXPANDED_SCRATCH, 2 * tokens * heads * absorbed):
+        return False
+    if tokens * heads < 64 or (most > 512 and tokens * heads * absorbed < (1.0 if beside else 0.4) * most * own):
+        return False
+    product = rows * kv_rank * heads * (nope + v)
+    if product > 1.5e9 and product > 6 * pairs * heads * (absorbed - own):
+        return False
+    return (tiles * heads <= 296 and tiles <= 32) or padded * own <= pairs * absorbed
+
+
+def latent_expand_prep(q: torch.Tensor, cache: torch.Tensor, rows: torch.Tensor, block_table: torch.Tensor,
+                       q_start: torch.Tensor, seq_lens: torch.Tensor, seq_begin: int, seq_end: int, positions: torch.Tensor,
+                       inv_freq: Optional[torch.Tensor], first_token: int, heads: int, nope: int, rot: int, rot_dims: int,
+                       window: int, err: torch.Tensor, magnitude: float = 1.0) -> None:
+    """For the prompt portions of sequences seq_begin .. seq_end-1: gathers their visible cached rows into ``rows``
+    [latent_expanded_rows, dk] and rotates the last rot values of every head of q [T, heads * (nope + rot)] in place
+    (tokens first_token .. T-1)."""
+    lib = build.load_library("latent_attention")
+    T, dk = q.shape[0], cache.shape[3]
+    assert q.dtype is torch.bfloat16 and cache.dtype is torch.bfloat16 and rows.dtype is torch.bfloat16
+    assert q.shape[1] == heads * (nope + rot) and rows.shape[1] == dk and cache.shape[1] == 1
+    _contig(q, "q"); _contig(cache, "cache"); _contig(rows, "rows"); _contig(block_table, "block_table")
+    if rot_dims:
+        assert inv_freq is not None and inv_freq.dtype is torch.float64 and inv_freq.numel() == rot_dims // 2
+    _check(lib.rllm_latent_expand_prep(
+        _ptr(q), _ptr(cache), _ptr(rows), _ptr(block_table), c_int(block_table.shape[1]), _ptr(q_start), _ptr(seq_lens),
+        c_int(seq_begin), c_int(seq_end), _ptr(positions), _ptr(inv_freq), c_float(magnitude), c_int(first_token),
+        c_int(T - first_token), c_int(heads), c_int(nope), c_int(rot), c_int(rot_dims), c_int(dk), c_int(rows.shape[0]),
+        c_int(cache.shape[2]), c_int(cache.shape[0]), c_int(window), _ptr(err), _stream()), "latent_expand_prep")
+
+
+def latent_expanded_tcgen05(q: torch.Tensor, kv: torch.Tensor, rows: torch.Tensor, out: torch.Tensor, q_start: torch.Tensor,
+                            seq_lens: torch.Tensor, seq_begin: int, seq_end: int, num_tokens: int, heads: int, nope: int,
+                            rot: int, v: int, kv_rank: int, window: int, scale: float, sink: Optional[torch.Tensor],
+                            err: torch.Tensor) -> None:
+    """Attention of prompt portions (``num_tokens`` tokens of sequences seq_begin .. seq_end-1) with every head's own keys
+    and values: q [T, heads * (nope + rot)] rotated, ``rows`` as ``latent_expand_prep`` leaves them, kv [rows, heads nope +
+    heads v] the product of their first kv_rank values with [W_uk; W_uv]; out [T, heads * v]."""
+    lib = build.load_library("latent_expanded_tcgen05")
+    T = q.shape[0]
+    assert q.shape == (T, heads * (nope + rot)) and out.shape == (T, heads * v)
+    assert kv.shape == (rows.shape[0], heads * (nope + v)) and rows.shape[1] == kv_rank + rot
+    assert all(t.dtype is torch.bfloat16 for t in (q, kv, rows, out))
+    _contig(q, "q"); _contig(kv, "kv"); _contig(rows, "rows"); _contig(out, "out")
+    if sink is not None:
+        assert sink.dtype is torch.float32 and sink.numel() == heads
+    _check(lib.rllm_latent_expanded_tcgen05(
+        _ptr(q), c_int(T), _ptr(kv), _ptr(rows), c_int(rows.shape[0]), c_int(rows.shape[1]), c_int(kv_rank), _ptr(out),
+        _ptr(q_start), _ptr(seq_lens), c_int(seq_begin), c_int(seq_end), c_int(num_tokens), c_int(heads), c_int(nope),
+        c_int(rot), c_int(v), c_int(window), c_float(scale), _ptr(sink), _ptr(err), _stream()), "latent_expanded_tcgen05")
+
+
 # ---------------------------------------------------------------------------
 # routed experts (moe.cu)
 # ---------------------------------------------------------------------------

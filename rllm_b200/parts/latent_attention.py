@@ -8,10 +8,12 @@ encoding rotates the queries' rot part and the shared key part.  A token keeps c
 the rotated shared part, nothing else: one row of kv_rank + rot_dim values
 (``KVPagesNeed(1, kv_rank + rot_dim, window, values=False)``).
 
-The products with W_uk and W_uv are moved to the query side, so that the cached
-rows are read as they are, by prompts and by decoding alike:
+Decoded tokens, and prompts where it pays, have the products with W_uk and W_uv on the query side, so that the cached
+rows are read as they are:
     q~[h] = [W_uk[h]^T q_nope[h] | rotated q_rot[h]],  score = q~[h] . row * scale,
     o~[h] = sum_j p_j c_j,  head output = W_uv[h] o~[h],  y = W_o [head outputs].
+Other prompt portions make every head's keys and values of the visible rows (``ops.latent_expanded_pays``): more
+products before the attention, a third of the multiplications in it.
 Scores, softmax and the sums over keys are float32.  ``window`` (None: every key up
 to the query; w: the query's own position and the w - 1 before it) masks; with
 ``sink`` a learned number per head joins the softmax's denominator as exp(sink[h]),
@@ -78,7 +80,7 @@ class LatentAttention(Mixer):
             raise ValueError("the latent attention kernels rotate pairs (2i, 2i+1): the position part must be interleaved")
         if self.rot_dims > self.rot:
             raise ValueError(f"the rotation covers {self.rot_dims} dimensions, the rotated part has {self.rot}")
-        self.w_down = self.w_uq = self.w_uk = self.w_uv = self.w_o = None
+        self.w_down = self.w_uq = self.w_uk = self.w_uv = self.w_ukv = self.w_o = None
         self.w_qn = self.w_kvn = self.sink = None
         self.magnitude = float(getattr(self.position, "magnitude", 1.0)) if self.rot_dims else 1.0
 
@@ -120,7 +122,12 @@ class LatentAttention(Mixer):
         self.w_uq = tensors[n["uq"]]
         # W_uk[h]^T, [h, n = kv_rank, k = nope]: the query-side product reads it along k
         self.w_uk = tensors[n["uk"]].view(H, self.nope, self.kv_rank).transpose(1, 2).contiguous()
-        self.w_uv = tensors[n["uv"]].contiguous().view(H, self.vdim, self.kv_rank)      # [h, n = vdim, k = kv_rank]
+        uv = tensors[n["uv"]].contiguous()
+        if ops.latent_expanded_shapes(uv.dtype, self.nope, self.rot, self.vdim, self.kv_rank, self.scale):
+            # [W_uk; W_uv]: one product gives all heads' keys and values of cached rows; W_uv is its second half
+            self.w_ukv = torch.cat([tensors[n["uk"]], uv], dim=0).contiguous()
+            uv = self.w_ukv[H * self.nope:]
+        self.w_uv = uv.view(H, self.vdim, self.kv_rank)                                 # [h, n = vdim, k = kv_rank]
         self.w_o = tensors[n["o"]]
         self.sink = tensors[n["sink"]].float().contiguous() if self.has_sink else None
 
@@ -147,34 +154,59 @@ class LatentAttention(Mixer):
                         cache.k if writes else None, table, ctx.positions, ctx.token_seq, inv_freq, ctx.err,
                         magnitude=self.magnitude)
         q = linear(cq, self.w_uq)                                    # [T, H (nope + rot)]
-        qt = torch.empty((T, H * dk), dtype=x.dtype, device=x.device)
-        ops.head_gemm(q.view(T, H, self.nope + self.rot)[:, :, : self.nope], self.w_uk,
-                      qt.view(T, H, dk)[:, :, : self.kv_rank], b_kn=False)
-        if self.rot:
-            ops.latent_q_rot(q, qt, ctx.positions, inv_freq, H, self.nope, self.rot, self.rot_dims, self.kv_rank,
-                             magnitude=self.magnitude)
-        o = torch.empty((T, H * self.kv_rank), dtype=x.dtype, device=x.device)
+        ov = torch.empty((T, H * self.vdim), dtype=x.dtype, device=x.device)
         window = int(self.window or 0)
         nd = ctx.num_decode
-        if T > nd and ops.latent_attention_tcgen05_takes(x.dtype, dk, self.kv_rank, (T - nd) * H, cache.k) and \
-                ops.latent_attention_tcgen05_pays(ctx.q_lens_host[nd:], ctx.seq_lens_host[nd:], H, self.kv_rank, window):
-            ops.latent_attention_tcgen05(qt, o, cache.k, table, ctx.q_start, ctx.seq_lens, nd, ctx.num_seqs, T - nd, H, dk,
-                                         self.kv_rank, window, self.scale, self.sink, ctx.err)
+        if T > nd and self.w_ukv is not None and ops.latent_expanded_allowed() and \
+                ops.latent_expanded_pays(ctx.q_lens_host[nd:], ctx.seq_lens_host[nd:], H, self.nope, self.vdim,
+                                         self.kv_rank, self.rot, window, nd > 0):
+            self._expanded(q, ov, ctx, cache, table, inv_freq, window)
             if nd:
-                ops.latent_attention_mma(qt[:nd], o[:nd], cache.k, table, ctx.q_start, ctx.seq_lens, nd, 1, H, dk,
-                                         self.kv_rank, window, self.scale, self.sink, ctx.err,
-                                         max_seq_len=max(ctx.seq_lens_host[:nd]))
-        elif ops.latent_attention_mma_takes(x.dtype, dk, self.kv_rank):
-            ops.latent_attention_mma(qt, o, cache.k, table, ctx.q_start, ctx.seq_lens, ctx.num_seqs, ctx.max_q_len, H,
-                                     dk, self.kv_rank, window, self.scale, self.sink, ctx.err,
-                                     max_seq_len=ctx.max_seq_len)
+                self._absorbed(q[:nd], ov[:nd], ctx, cache, table, inv_freq, window, nd, 1, max(ctx.seq_lens_host[:nd]))
         else:
-            ops.latent_attention_simt(qt, o, cache.k, table, ctx.positions, ctx.token_seq, H, dk, self.kv_rank,
-                                      window, self.scale, self.sink, ctx.err)
-        ov = torch.empty((T, H * self.vdim), dtype=x.dtype, device=x.device)
-        ops.head_gemm(o.view(T, H, self.kv_rank), self.w_uv, ov.view(T, H, self.vdim), b_kn=False)
+            self._absorbed(q, ov, ctx, cache, table, inv_freq, window, ctx.num_seqs, ctx.max_q_len, ctx.max_seq_len)
         if self.gate:
             at = self._down_rows() - H * self.vdim
             ops.sigmoid_gate(ov, a[:, at: at + H * self.vdim], ov)
         y = linear(ov, self.w_o)
         return (y, a[:, self._down_rows():]) if side else y
+
+    def _expanded(self, q, ov, ctx, cache, table, inv_freq, window):
+        """The prompt portions with every head's own keys and values, made of the visible rows; rotates their q in place."""
+        H, dk, nd = self.heads, self.kv_rank + self.rot, ctx.num_decode
+        n = ops.latent_expanded_rows(ctx.q_lens_host[nd:], ctx.seq_lens_host[nd:], window)
+        rows = torch.empty((n, dk), dtype=q.dtype, device=q.device)
+        ops.latent_expand_prep(q, cache.k, rows, table, ctx.q_start, ctx.seq_lens, nd, ctx.num_seqs, ctx.positions, inv_freq,
+                               nd, H, self.nope, self.rot, self.rot_dims, window, ctx.err, magnitude=self.magnitude)
+        kv = torch.empty((n, H * (self.nope + self.vdim)), dtype=q.dtype, device=q.device)
+        ops.gemm_tcgen05(rows[:, : self.kv_rank], self.w_ukv, kv)
+        ops.latent_expanded_tcgen05(q, kv, rows, ov, ctx.q_start, ctx.seq_lens, nd, ctx.num_seqs, q.shape[0] - nd, H,
+                                    self.nope, self.rot, self.vdim, self.kv_rank, window, self.scale, self.sink, ctx.err)
+
+    def _absorbed(self, q, ov, ctx, cache, table, inv_freq, window, num_seqs, max_q_len, max_seq_len):
+        """The first ``num_seqs`` sequences' tokens (all of q's) over the cached rows as they are, W_uk and W_uv on the
+        query side."""
+        T, H, nd = q.shape[0], self.heads, ctx.num_decode
+        dk = self.kv_rank + self.rot
+        qt = torch.empty((T, H * dk), dtype=q.dtype, device=q.device)
+        ops.head_gemm(q.view(T, H, self.nope + self.rot)[:, :, : self.nope], self.w_uk,
+                      qt.view(T, H, dk)[:, :, : self.kv_rank], b_kn=False)
+        if self.rot:
+            ops.latent_q_rot(q, qt, ctx.positions, inv_freq, H, self.nope, self.rot, self.rot_dims, self.kv_rank,
+                             magnitude=self.magnitude)
+        o = torch.empty((T, H * self.kv_rank), dtype=q.dtype, device=q.device)
+        if T > nd and ops.latent_attention_tcgen05_takes(q.dtype, dk, self.kv_rank, (T - nd) * H, cache.k) and \
+                ops.latent_attention_tcgen05_pays(ctx.q_lens_host[nd:], ctx.seq_lens_host[nd:], H, self.kv_rank, window):
+            ops.latent_attention_tcgen05(qt, o, cache.k, table, ctx.q_start, ctx.seq_lens, nd, num_seqs, T - nd, H, dk,
+                                         self.kv_rank, window, self.scale, self.sink, ctx.err)
+            if nd:
+                ops.latent_attention_mma(qt[:nd], o[:nd], cache.k, table, ctx.q_start, ctx.seq_lens, nd, 1, H, dk,
+                                         self.kv_rank, window, self.scale, self.sink, ctx.err,
+                                         max_seq_len=max(ctx.seq_lens_host[:nd]))
+        elif ops.latent_attention_mma_takes(q.dtype, dk, self.kv_rank):
+            ops.latent_attention_mma(qt, o, cache.k, table, ctx.q_start, ctx.seq_lens, num_seqs, max_q_len, H,
+                                     dk, self.kv_rank, window, self.scale, self.sink, ctx.err, max_seq_len=max_seq_len)
+        else:
+            ops.latent_attention_simt(qt, o, cache.k, table, ctx.positions, ctx.token_seq, H, dk, self.kv_rank,
+                                      window, self.scale, self.sink, ctx.err)
+        ops.head_gemm(o.view(T, H, self.kv_rank), self.w_uv, ov.view(T, H, self.vdim), b_kn=False)

@@ -41,6 +41,30 @@ def test_which_prompt_portions_the_tcgen05_latent_attention_pays_for(q_lens, key
     assert ops.latent_attention_tcgen05_pays(q_lens, [keys] * len(q_lens), heads, dv, window) is tcgen05
 
 
+@pytest.mark.parametrize("q_lens,starts,sizes,window,pays", [
+    ([2048], 0, "A", 0, True), ([33], 4096, "A", 0, True), ([17], 4096, "A", 0, False), ([8], 0, "A", 0, True), ([2], 0, "A", 0, False),
+    ([8], 1024, "A", 0, False), ([300], 4096, "A", 512, True), ([33], 4096, "B", 0, False), ([64], 4096, "B", 0, True),
+    ([128], 4096, "D", 0, False), ([300], 4096, "D", 0, True), ([4] * 64, 0, "A", 0, False), ([16] * 64, 200, "D", 0, False),
+    ([33] * 16, 1000, "A", 0, True), ([33] * 16, 1000, "C", 0, False), ([350] * 5, 0, "C", 0, True), ([512], 30000, "A", 0, True), ([512], 60000, "A", 0, False),
+    ([4096], 30000, "A", 0, True)])
+def test_which_prompt_portions_run_with_every_heads_own_keys_and_values(q_lens, starts, sizes, window, pays):
+    sizes = {"A": (16, 128, 128, 512, 64), "B": (8, 64, 64, 256, 32), "C": (64, 128, 128, 512, 64), "D": (4, 64, 64, 128, 32)}[sizes]
+    assert ops.latent_expanded_pays(q_lens, [q + starts for q in q_lens], *sizes, window) is pays
+
+
+@pytest.mark.parametrize("dtype,nope,rot,v,kv,scale,ok", [
+    (BF16, 128, 64, 128, 512, 0.1, True), (BF16, 64, 8, 128, 40, 0.1, True), (torch.float32, 128, 64, 128, 512, 0.1, False),
+    (BF16, 96, 64, 128, 512, 0.1, False), (BF16, 128, 64, 96, 512, 0.1, False), (BF16, 128, 0, 128, 512, 0.1, False),
+    (BF16, 128, 72, 128, 512, 0.1, False), (BF16, 128, 12, 128, 512, 0.1, False), (BF16, 128, 64, 128, 500, 0.1, False),
+    (BF16, 128, 64, 128, 512, -0.1, False)])
+def test_which_mixers_have_that_form(dtype, nope, rot, v, kv, scale, ok, monkeypatch):
+    assert ops.latent_expanded_shapes(dtype, nope, rot, v, kv, scale) is ok
+    monkeypatch.delenv("RLLM_LATENT_ATTENTION", raising=False)
+    assert ops.latent_expanded_allowed()
+    monkeypatch.setenv("RLLM_LATENT_ATTENTION", "mma")
+    assert not ops.latent_expanded_allowed()
+
+
 @pytest.mark.parametrize("E,H,F,pays", [(32, 2048, 1024, True), (16, 1024, 1024, True), (8, 1024, 512, True), (4, 1024, 512, False),
                                         (1, 2048, 256, True), (1, 1024, 1024, False), (128, 512, 512, False), (8, 64, 64, False)])
 def test_which_experts_the_tcgen05_kernels_pay_for(E, H, F, pays, monkeypatch):
