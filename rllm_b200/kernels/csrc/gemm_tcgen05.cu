@@ -9,16 +9,17 @@
 //   * tcgen05.commit hands a stage back to the TMA producer when the MMAs that
 //     read it are done, and at the end tells the epilogue warps that the
 //     accumulator is complete;
-//   * four epilogue warps read their 32 TMEM lanes with tcgen05.ld, round to
+//   * eight epilogue warps (two a quarter of the 128 lanes) read their 32 TMEM lanes with tcgen05.ld, round to
 //     bfloat16 (or keep float32) and store; with the SiLU-gate epilogue the tile
 //     holds 128 gate and 128 up features of [Wgate; Wup] side by side and
 //     silu(gate) * up is applied to the accumulators
 //     (crates/rllm-model/src/layers.rs:214-220), so the [T, 2I] intermediate
 //     never exists.
-// Warp 0: TMA producer.  Warp 1: TMEM allocation and MMA issue.  Warps 2-5:
+// Warp 0: TMA producer.  Warp 1: TMEM allocation and MMA issue.  Warps 2-9:
 // epilogue.  The kernel is persistent (one CTA per SM walks over output tiles) and
 // keeps two accumulators in TMEM, so that the epilogue of a tile overlaps the
-// MMAs of the next.  No cluster, no multicast.
+// MMAs of the next.  No multicast.  Larger products run on pairs of CTAs (cta_group::2) that share a tile of 256 rows:
+// gemm_tcgen05_pair_kernel below.
 //
 // Every wait on an mbarrier is bounded: after the limit the thread sets bit 16
 // of the error word and the CTA winds down (gives its TMEM columns back) instead
@@ -31,7 +32,8 @@
 
 #define TG_BM 128
 #define TG_BK 64
-#define TG_THREADS 192
+#define TG_EPI_WARPS 8                  // two a quarter of the lanes, half of the columns each
+#define TG_THREADS (64 + 32 * TG_EPI_WARPS)
 #define TG_EPI_BF16 0
 #define TG_EPI_F32 1
 #define TG_EPI_SILU 2
@@ -40,6 +42,61 @@ template <int BN> constexpr int tg_stages() { return BN == 256 ? 4 : (BN == 192 
 template <int BN> constexpr int tg_tmem_cols() { return BN > 128 ? 512 : 256; }
 template <int BN> constexpr int tg_stage_bytes() { return (TG_BM + BN) * TG_BK * 2; }
 template <int BN> constexpr int tg_smem_bytes() { return tg_stages<BN>() * tg_stage_bytes<BN>() + 1024 + 256; }
+
+// One warp's 32 rows and half of a tile's columns: from tensor memory (lane_addr: its lanes' first column) to row m,
+// columns n0 .. of out.
+template <int BN, int EPI>
+__device__ __forceinline__ void tg_epilogue(unsigned lane_addr, int half, void* __restrict__ out, size_t at, int ldo, int m, int n0,
+                                            int M, int N, const GateAct& ga) {
+  constexpr int NOUT = (EPI == TG_EPI_SILU) ? BN / 2 : BN, SPLIT = NOUT / 64 * 32;      // 192 columns: 96 and 96
+#pragma unroll 1
+  for (int c0 = half ? SPLIT : 0; c0 < (half ? NOUT : SPLIT); c0 += 32) {
+    unsigned r[32];
+    tmem_ld32(lane_addr + c0, r);
+    if (EPI == TG_EPI_SILU) {
+      unsigned u[32];
+      tmem_ld32(lane_addr + NOUT + c0, u);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        const float g = fminf(__uint_as_float(r[j]), ga.limit);
+        const float up = fminf(fmaxf(__uint_as_float(u[j]), -ga.limit), ga.limit);
+        r[j] = __float_as_uint(__fdividef(g, 1.0f + __expf(-ga.slope * g)) * (up + ga.shift));
+      }
+    } else {
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    }
+    if (m < M) {
+      const int n = n0 + c0;
+      if (EPI == TG_EPI_F32) {
+        float* o = (float*)out + at + (size_t)m * ldo + n;
+        if (n + 32 <= N && (((uintptr_t)o) & 15) == 0) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 4)
+            *(float4*)(o + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
+                                            __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
+        } else {
+          for (int j = 0; j < 32; ++j) if (n + j < N) o[j] = __uint_as_float(r[j]);
+        }
+      } else {
+        bf16* o = (bf16*)out + at + (size_t)m * ldo + n;
+        if (n + 32 <= N && (((uintptr_t)o) & 15) == 0) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 8) {
+            uint4 v;
+            __nv_bfloat162* p = (__nv_bfloat162*)&v;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              p[q] = __floats2bfloat162_rn(__uint_as_float(r[j + 2 * q]), __uint_as_float(r[j + 2 * q + 1]));
+            *(uint4*)(o + j) = v;
+          }
+        } else {
+          for (int j = 0; j < 32; ++j) if (n + j < N) o[j] = __float2bfloat16_rn(__uint_as_float(r[j]));
+        }
+      }
+    }
+  }
+}
 
 // EPI: 0 bfloat16 out, 1 float32 out, 2 SiLU-gate (BN must be 256; W rows n and up_offset + n pair up).
 // Persistent: CTA b takes the output tiles b, b + gridDim.x, ... (rows of tiles first, so that CTAs
@@ -68,7 +125,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], TG_EPI_WARPS); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"((unsigned long long)&map_a) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"((unsigned long long)&map_w) : "memory");
@@ -81,18 +138,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const unsigned tmem_base = *tmem_slot;
+  pdl_wait();                                        // what lies above overlaps the kernel ahead; nothing of global memory is read there
+  pdl_launch();
 
   if (warp == 0) {
     if (lane == 0) {
-      unsigned it = 0;
+      int s = -1;
+      unsigned phase = 1;                                  // a fresh barrier passes the wait for parity 1
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         const int m0 = (tile % tiles_m) * TG_BM, tn = tile / tiles_m, n0 = (HEADS ? tn % tiles_n : tn) * NOUT;
         const int head = HEADS ? tn / tiles_n : 0;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % STAGES;
-          const unsigned phase = (it / STAGES) & 1;
-          ok = mbar_wait(&empty[s], phase ^ 1, err);       // a fresh barrier passes the wait for parity 1
+        for (int kb = 0; kb < num_kb; ++kb) {
+          if (++s == STAGES) { s = 0; phase ^= 1; }
+          ok = mbar_wait(&empty[s], phase, err);
           if (!ok) break;
           unsigned char* sa = stage_mem + s * tg_stage_bytes<BN>();
           unsigned char* sb = sa + TG_BM * TG_BK * 2;
@@ -117,27 +176,32 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     if (lane == 0) {
       // instruction descriptor: float32 accumulate, bfloat16 A and B, both K-major, N = BN, M = 128
       const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(TG_BM >> 4) << 24);
-      unsigned it = 0, ti = 0;
-      bool ok = true;
+      // The thread that issues is what a step of k waits for (a product about 55 cycles, a commit 66, a look at a barrier
+      // 130; the tensor cores need 2 BN cycles a step), so it looks at the next stage's barrier before it issues this
+      // stage's products and finds the answer there afterwards.
+      int s = 0;
+      unsigned phase = 0, ti = 0;
+      bool ok = true, ready = false;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++ti) {
         const unsigned buf = ti & 1, use = ti >> 1;
         ok = mbar_wait(&acc_empty[buf], (use & 1) ^ 1, err);   // the epilogue has drained this accumulator
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const unsigned tmem_acc = tmem_base + buf * BN;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % STAGES;
-          const unsigned phase = (it / STAGES) & 1;
-          ok = mbar_wait(&full[s], phase, err);
+        for (int kb = 0; kb < num_kb; ++kb) {
+          if (!ready) ok = mbar_wait(&full[s], phase, err);
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           unsigned char* sa = stage_mem + s * tg_stage_bytes<BN>();
           unsigned char* sb = sa + TG_BM * TG_BK * 2;
           const unsigned long long da = umma_desc(sa), db = umma_desc(sb);
+          unsigned long long* const here = &empty[s];
+          if (++s == STAGES) { s = 0; phase ^= 1; }
+          ready = mbar_test(&full[s], phase);
 #pragma unroll
           for (int k = 0; k < TG_BK / 16; ++k)     // 16 bf16 = 32 bytes further along K: + 2 in the address field
             umma_bf16(tmem_acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-          umma_commit(&empty[s]);                  // the stage is free once these MMAs have read it
+          umma_commit(here);                       // the stage is free once these MMAs have read it
         }
         if (ok) umma_commit(&acc_full[buf]);       // the accumulator is complete once all MMAs are done
       }
@@ -158,53 +222,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const unsigned lane_addr = tmem_base + buf * BN + ((unsigned)(quarter * 32) << 16);
-#pragma unroll 1
-      for (int c0 = 0; c0 < NOUT; c0 += 32) {
-        unsigned r[32];
-        tmem_ld32(lane_addr + c0, r);
-        if (EPI == TG_EPI_SILU) {
-          unsigned u[32];
-          tmem_ld32(lane_addr + NOUT + c0, u);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float g = fminf(__uint_as_float(r[j]), ga.limit);
-            const float up = fminf(fmaxf(__uint_as_float(u[j]), -ga.limit), ga.limit);
-            r[j] = __float_as_uint(__fdividef(g, 1.0f + __expf(-ga.slope * g)) * (up + ga.shift));
-          }
-        } else {
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        }
-        if (m < M) {
-          const int n = n0 + c0;
-          if (EPI == TG_EPI_F32) {
-            float* o = (float*)out + at + (size_t)m * ldo + n;
-            if (n + 32 <= N && (((uintptr_t)o) & 15) == 0) {
-#pragma unroll
-              for (int j = 0; j < 32; j += 4)
-                *(float4*)(o + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
-                                                __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-            } else {
-              for (int j = 0; j < 32; ++j) if (n + j < N) o[j] = __uint_as_float(r[j]);
-            }
-          } else {
-            bf16* o = (bf16*)out + at + (size_t)m * ldo + n;
-            if (n + 32 <= N && (((uintptr_t)o) & 15) == 0) {
-#pragma unroll
-              for (int j = 0; j < 32; j += 8) {
-                uint4 v;
-                __nv_bfloat162* p = (__nv_bfloat162*)&v;
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                  p[q] = __floats2bfloat162_rn(__uint_as_float(r[j + 2 * q]), __uint_as_float(r[j + 2 * q + 1]));
-                *(uint4*)(o + j) = v;
-              }
-            } else {
-              for (int j = 0; j < 32; ++j) if (n + j < N) o[j] = __float2bfloat16_rn(__uint_as_float(r[j]));
-            }
-          }
-        }
-      }
+      tg_epilogue<BN, EPI>(lane_addr, (warp - 2) >> 2, out, at, ldo, m, n0, M, N, ga);
       // this warp has read its lanes of the accumulator: hand it back to the MMA warp
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -215,6 +233,196 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   __syncthreads();
   if (warp == 1) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tg_tmem_cols<BN>()) : "memory");
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The same product by pairs of CTAs (tcgen05 cta_group::2): a pair has a tile of 256 rows by BN columns, each CTA 128 of
+// the rows.  The instruction takes its A operand from both CTAs (each its own rows) and its B operand half from each, so a
+// CTA brings (128 + BN / 2) x 64 operand values a step of k instead of (128 + BN) x 64: a tile of 128 x 256 asks 96 bytes a
+// cycle of L2 at the tensor cores' full rate, a pair's CTA 64.
+//
+// Both CTAs load their part (TMA, no multicast) into the same offsets of their own shared memory; the leader's (rank 0)
+// barrier `full` counts the bytes of both.  The leader issues the instructions; tcgen05.commit arrives at both CTAs' `empty`
+// and `acc_full`, and the epilogue warps of both arrive at the leader's `acc_empty`.  The pair leaves together: nothing
+// arrives at a CTA that has gone.
+// ---------------------------------------------------------------------------
+#define TGP_BK 128                       // two panels of 64
+template <int BN> constexpr int tgp_stage_bytes() { return (TG_BM + BN / 2) * TGP_BK * 2; }
+template <int BN> constexpr int tgp_stages() { return BN == 128 ? 4 : 3; }
+template <int BN> constexpr int tgp_smem_bytes() { return tgp_stages<BN>() * tgp_stage_bytes<BN>() + 1024 + 256; }
+
+__device__ __forceinline__ unsigned tgp_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// the address of the leader's copy of a barrier
+__device__ __forceinline__ unsigned tgp_leaders(const void* bar) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(tg_smem(bar)));
+  return r;
+}
+__device__ __forceinline__ void tgp_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tgp_load_2d(void* dst, const CUtensorMap* map, int x, int y, unsigned leaders_bar) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+               ::"r"(tg_smem(dst)), "l"((unsigned long long)map), "r"(x), "r"(y), "r"(leaders_bar) : "memory");
+}
+__device__ __forceinline__ void tgp_umma(unsigned tmem_d, unsigned long long da, unsigned long long db, unsigned idesc, unsigned accumulate) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+               "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+               ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tgp_commit(void* bar) {      // at this barrier in both CTAs
+  const unsigned short both = 3;
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(tg_smem(bar)), "h"(both) : "memory");
+}
+// mbar_wait for barriers at which the other CTA's threads arrive
+__device__ __forceinline__ bool tgp_wait(void* bar, unsigned parity, int* err) {
+  const unsigned addr = tg_smem(bar);
+  for (unsigned spin = 0; spin < TG_SPIN_LIMIT; ++spin) {
+    unsigned done;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(addr), "r"(parity) : "memory");
+    if (done) return true;
+  }
+  atomicOr(err, 16);
+  return false;
+}
+
+template <int BN, int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TG_THREADS)
+gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
+                         void* __restrict__ out, int ldo, int M, int N, int K, int up_offset, int tiles_m, int num_tiles,
+                         int* __restrict__ err, GateAct ga) {
+  constexpr int STAGES = tgp_stages<BN>();
+  constexpr int NOUT = (EPI == TG_EPI_SILU) ? BN / 2 : BN;     // output columns of a tile
+  extern __shared__ unsigned char tg_raw[];
+  unsigned char* base = (unsigned char*)(((uintptr_t)tg_raw + 1023) & ~(uintptr_t)1023);   // the same offset in both CTAs
+  unsigned char* stage_mem = base;
+  unsigned long long* bars = (unsigned long long*)(base + STAGES * tgp_stage_bytes<BN>());
+  unsigned long long* full = bars;                   // [STAGES]  leader's: both CTAs' TMA -> MMA
+  unsigned long long* empty = bars + STAGES;         // [STAGES]  MMA -> each CTA's TMA
+  unsigned long long* acc_full = bars + 2 * STAGES;  // [2]       MMA -> each CTA's epilogue
+  unsigned long long* acc_empty = acc_full + 2;      // [2]       leader's: both CTAs' epilogues -> MMA
+  unsigned* tmem_slot = (unsigned*)(acc_empty + 2);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = (int)tgp_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int num_kb = (K + TGP_BK - 1) / TGP_BK;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 2 * TG_EPI_WARPS); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"((unsigned long long)&map_a) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"((unsigned long long)&map_w) : "memory");
+  }
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tg_smem(tmem_slot)), "r"(tg_tmem_cols<BN>()) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  tgp_cluster_sync();                                // both CTAs' barriers and tensor memory are there
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const unsigned tmem_base = *tmem_slot;
+  pdl_wait();                                        // what lies above overlaps the kernel ahead; nothing of global memory is read there
+  pdl_launch();
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int s = -1;
+      unsigned phase = 1, uses = 0;                      // a fresh barrier passes the wait for parity 1
+      bool ok = true;
+      for (int tile = pair; tile < num_tiles && ok; tile += pairs) {
+        const int m0 = (tile % tiles_m) * 2 * TG_BM + rank * TG_BM, n0 = tile / tiles_m * NOUT;
+        // this CTA's half of the weight rows: with the gate, rank 0 has the gate rows and rank 1 the up rows
+        const int w0 = EPI == TG_EPI_SILU ? n0 + rank * up_offset : n0 + rank * (BN / 2);
+        for (int kb = 0; kb < num_kb; ++kb, ++uses) {
+          if (++s == STAGES) { s = 0; phase ^= 1; }
+          ok = mbar_wait(&empty[s], phase, err);
+          if (!ok) break;
+          unsigned char* sa = stage_mem + s * tgp_stage_bytes<BN>();
+          unsigned char* sb = sa + TG_BM * TGP_BK * 2;
+          const int x = kb * TGP_BK;
+          const bool two = x + 64 < K;                     // the second panel has values
+          if (rank == 0) mbar_expect_tx(&full[s], (two ? 2u : 1u) * tgp_stage_bytes<BN>());
+          const unsigned bar = tgp_leaders(&full[s]);
+          tgp_load_2d(sa, &map_a, x, m0, bar);
+          tgp_load_2d(sb, &map_w, x, w0, bar);
+          if (two) {
+            tgp_load_2d(sa + TG_BM * 128, &map_a, x + 64, m0, bar);
+            tgp_load_2d(sb + BN / 2 * 128, &map_w, x + 64, w0, bar);
+          }
+        }
+      }
+      // the last uses of the stages: their commits have arrived here before this CTA leaves
+      for (unsigned i = 1; i <= (unsigned)STAGES && i <= uses && ok; ++i)
+        ok = mbar_wait(&empty[(uses - i) % STAGES], ((uses - i) / STAGES) & 1, err);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (rank == 0 && lane == 0) {
+      // instruction descriptor: float32 accumulate, bfloat16 A and B, both K-major, N = BN, M = 256
+      const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(2 * TG_BM >> 4) << 24);
+      int s = 0;
+      unsigned phase = 0, ti = 0;
+      bool ok = true, ready = false;
+      for (int tile = pair; tile < num_tiles && ok; tile += pairs, ++ti) {
+        const unsigned buf = ti & 1, use = ti >> 1;
+        ok = tgp_wait(&acc_empty[buf], (use & 1) ^ 1, err);   // both epilogues have drained this accumulator
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const unsigned tmem_acc = tmem_base + buf * BN;
+        for (int kb = 0; kb < num_kb; ++kb) {
+          if (!ready) ok = mbar_wait(&full[s], phase, err);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          unsigned char* sa = stage_mem + s * tgp_stage_bytes<BN>();
+          const unsigned long long da = umma_desc(sa), db = umma_desc(sa + TG_BM * TGP_BK * 2);
+          unsigned long long* const here = &empty[s];
+          if (++s == STAGES) { s = 0; phase ^= 1; }
+          ready = mbar_test(&full[s], phase);      // the next stage's: see gemm_tcgen05_kernel
+#pragma unroll
+          for (int k = 0; k < 4; ++k)              // 16 bf16 = 32 bytes further along K: + 2 in the address field
+            tgp_umma(tmem_acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+          if (kb * TGP_BK + 64 < K) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              tgp_umma(tmem_acc, da + (TG_BM * 128 >> 4) + 2 * k, db + (BN / 2 * 128 >> 4) + 2 * k, idesc, 1u);
+          }
+          tgp_commit(here);
+        }
+        if (ok) tgp_commit(&acc_full[buf]);
+      }
+    }
+    __syncwarp();
+  } else {
+    const int quarter = warp & 3;
+    unsigned ti = 0;
+    bool ok = true;
+    for (int tile = pair; tile < num_tiles && ok; tile += pairs, ++ti) {
+      const int m0 = (tile % tiles_m) * 2 * TG_BM + rank * TG_BM, n0 = tile / tiles_m * NOUT;
+      const unsigned buf = ti & 1, use = ti >> 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[buf], use & 1, err));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      tg_epilogue<BN, EPI>(tmem_base + buf * BN + ((unsigned)(quarter * 32) << 16), (warp - 2) >> 2, out, (size_t)0, ldo, m0 + quarter * 32 + lane, n0, M, N, ga);
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(tgp_leaders(&acc_empty[buf])) : "memory");
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  tgp_cluster_sync();
+  if (warp == 1) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tg_tmem_cols<BN>()) : "memory");
   }
 }
 
@@ -233,8 +441,29 @@ static int tg_run(const CUtensorMap& ma, const CUtensorMap& mw, void* out, int l
   if (num_tiles > (1ll << 30)) return RLLM_E_UNSUPPORTED;
   const int num_sms = tg_num_sms();
   const int grid = (int)(num_tiles < num_sms ? num_tiles : num_sms);
-  gemm_tcgen05_kernel<BN, EPI, HEADS><<<grid, TG_THREADS, tg_smem_bytes<BN>(), stream>>>(
-      ma, mw, out, ldo, M, N, K, up_offset, tiles_m, (int)num_tiles, err, ga, tiles_n, c_head);
+  rllm_launch_pdl(gemm_tcgen05_kernel<BN, EPI, HEADS>, dim3(grid), dim3(TG_THREADS), (size_t)tg_smem_bytes<BN>(), stream, ma, mw, out,
+                  ldo, M, N, K, up_offset, tiles_m, (int)num_tiles, err, ga, tiles_n, c_head);
+  RLLM_LAUNCH_CHECK();
+  return 0;
+}
+
+template <int BN, int EPI>
+static int tgp_launch(const void* a, int lda, const void* w, int ldw, int w_rows, void* out, int ldo, int M, int N, int K,
+                      int up_offset, int* err, cudaStream_t stream, GateAct ga = GateAct{INFINITY, 1.f, 0.f}) {
+  constexpr int NOUT = (EPI == TG_EPI_SILU) ? BN / 2 : BN;
+  CUtensorMap ma, mw;
+  int rc = tg_make_map(&ma, a, M, K, lda, TG_BM);
+  if (!rc) rc = tg_make_map(&mw, w, w_rows, K, ldw, BN / 2);
+  if (rc) return rc;
+  static SmemLimit limit;
+  if (const int e = limit.allow(gemm_tcgen05_pair_kernel<BN, EPI>, tgp_smem_bytes<BN>())) return e;
+  const int tiles_m = (M + 2 * TG_BM - 1) / (2 * TG_BM), tiles_n = (N + NOUT - 1) / NOUT;
+  const long long num_tiles = (long long)tiles_m * tiles_n;
+  if (num_tiles > (1ll << 29)) return RLLM_E_UNSUPPORTED;
+  const int pairs = tg_num_sms() / 2;
+  const int grid = 2 * (int)(num_tiles < pairs ? num_tiles : pairs);
+  rllm_launch_pdl(gemm_tcgen05_pair_kernel<BN, EPI>, dim3(grid), dim3(TG_THREADS), (size_t)tgp_smem_bytes<BN>(), stream, ma, mw, out,
+                  ldo, M, N, K, up_offset, tiles_m, (int)num_tiles, err, ga);
   RLLM_LAUNCH_CHECK();
   return 0;
 }
@@ -255,10 +484,9 @@ static int tg_launch(const void* a, int lda, const void* w, int ldw, int w_rows,
 // Tile width 256, 192 or 128 for N columns of `rows` tiles of rows: the one with the least estimated time = rounds of the
 // persistent CTAs x width x a factor for what a narrower tile costs (A is read again more often, the epilogue overlaps
 // less).
-static int tg_width(long long rows, int N) {
+static int tg_width(long long rows, int N, long long sms) {
   int bn = N > 192 ? 256 : (N > 128 ? 192 : 128);
   if (N > 128) {
-    const long long sms = tg_num_sms();
     double best = 1e30;
     const int widths[3] = {256, 192, 128};
     const double factor[3] = {1.0, 1.05, 1.3};
@@ -271,6 +499,36 @@ static int tg_width(long long rows, int N) {
   return bn;
 }
 
+// The form for a product: the width of a pair's tile, or 0 for CTAs on their own.  A launch of pairs costs a microsecond
+// more (two cluster barriers), so only products of 64 steps of 64 k or more a CTA (rounds times k) take them, and of those
+// the ones that the estimate favours, in microseconds of one launch after another: single CTAs 4.5 and 0.35 a step whatever
+// the width (the loads, not the products, set the pace), pairs 5.3 and 0.32, 0.30 or 0.235 at 256, 192 or 128 columns.
+// Single / pairs, M x N x K: 2,047 x 3,072 x 2,048 24.9 / 24.2 (192 wide), 2,047 x 2,048 x 4,096 27.5 / 26.3,
+// 6,327 x 3,072 x 2,048 70 / 62, 2,048 x 8,512 x 2,048 63 / 54, 1,024 x 2,048 x 8,192 49 / 42 (128 wide), 8,192 cubed 813 / 754;
+// with the gate 512 x 4,096 x 2,048 31 / 28.5, 2,047 x 4,096 x 2,048 54 / 50, 4,096 x 8,192 x 2,048 197 / 176.  Below the line
+// 2,047 x 2,048 x 2,048 15.7 / 16.1, 384 x 6,144 x 2,048 13.4 / 15.4, 2,048 x 3,072 x 768 13.4 / 14.3, 2,048 x 1,024 x 1,024
+// 7.9 / 8.8.
+static int tg_pair_width(int M, int N, int K, int epilogue, long long sms) {
+  if (sms < 2) return 0;
+  const long long steps = (K + TG_BK - 1) / TG_BK;
+  const bool gate = epilogue == TG_EPI_SILU;
+  const int single = gate ? 128 : tg_width((M + TG_BM - 1) / TG_BM, N, sms);             // output columns
+  const auto rounds = [](long long tiles, long long at_once) { return (tiles + at_once - 1) / at_once; };
+  const long long alone = steps * rounds((long long)((M + TG_BM - 1) / TG_BM) * ((N + single - 1) / single), sms);
+  if (alone < 64) return 0;
+  double best = 4.5 + 0.35 * alone;
+  int width = 0;
+  const int widths[3] = {256, 192, 128};
+  const double step[3] = {0.32, 0.30, 0.235};
+  for (int i = 0; i < (gate ? 1 : 3); ++i) {
+    const int cols = gate ? 128 : widths[i];
+    const double t = 5.3 + step[i] * steps * rounds((long long)((M + 2 * TG_BM - 1) / (2 * TG_BM)) * ((N + cols - 1) / cols), sms / 2);
+    if (t < best) { best = t; width = widths[i]; }
+  }
+  return width;
+}
+RLLM_EXPORT int rllm_gemm_tcgen05_pair_width(int M, int N, int K, int epilogue, int sms) { return tg_pair_width(M, N, K, epilogue, sms); }
+
 // epilogue 0: out bfloat16 [M, N]; 1: out float32 [M, N]; 2: W = [gate rows (N); up rows (N)] stacked,
 // out bfloat16 [M, N] = silu(A . gate^T) * (A . up^T), with the gate's constants limit, slope, shift (GateAct).  err:
 // the engine's error word (bit 16: a wait ran out).
@@ -281,17 +539,22 @@ RLLM_EXPORT int rllm_gemm_tcgen05(const void* a, int lda, const void* w, int ldw
   if (K <= 0 || lda < K || ldw < K || ldo < N || !err) return RLLM_E_BADARG;
   // TMA: 16-byte aligned bases and row strides
   if (K % 8 || lda % 8 || ldw % 8 || (((uintptr_t)a | (uintptr_t)w) & 15)) return RLLM_E_UNSUPPORTED;
-  const int bn = tg_width((M + TG_BM - 1) / TG_BM, N);
+  const int bn = tg_width((M + TG_BM - 1) / TG_BM, N, tg_num_sms());
+  const int pair = tg_pair_width(M, N, K, epilogue, tg_num_sms());
 #define TG_BY_WIDTH(EPI_)                                                                                      \
+  if (pair == 256) return tgp_launch<256, EPI_>(a, lda, w, ldw, N, out, ldo, M, N, K, 0, err, stream);         \
+  if (pair == 192) return tgp_launch<192, EPI_>(a, lda, w, ldw, N, out, ldo, M, N, K, 0, err, stream);         \
+  if (pair == 128) return tgp_launch<128, EPI_>(a, lda, w, ldw, N, out, ldo, M, N, K, 0, err, stream);         \
   if (bn == 256) return tg_launch<256, EPI_>(a, lda, w, ldw, N, out, ldo, M, N, K, 0, err, stream);            \
   if (bn == 192) return tg_launch<192, EPI_>(a, lda, w, ldw, N, out, ldo, M, N, K, 0, err, stream);            \
   return tg_launch<128, EPI_>(a, lda, w, ldw, N, out, ldo, M, N, K, 0, err, stream)
+  const GateAct ga{limit, slope, shift};
   switch (epilogue) {
     case TG_EPI_BF16: TG_BY_WIDTH(TG_EPI_BF16);
     case TG_EPI_F32: TG_BY_WIDTH(TG_EPI_F32);
     case TG_EPI_SILU:
-      return tg_launch<256, TG_EPI_SILU>(a, lda, w, ldw, 2 * N, out, ldo, M, N, K, N, err, stream,
-                                         GateAct{limit, slope, shift});
+      if (pair) return tgp_launch<256, TG_EPI_SILU>(a, lda, w, ldw, 2 * N, out, ldo, M, N, K, N, err, stream, ga);
+      return tg_launch<256, TG_EPI_SILU>(a, lda, w, ldw, 2 * N, out, ldo, M, N, K, N, err, stream, ga);
   }
   return RLLM_E_BADARG;
 }
@@ -313,7 +576,7 @@ RLLM_EXPORT int rllm_head_gemm_tcgen05(const void* a, long long lda, long long a
   if (M <= 0 || N <= 0 || heads <= 0) return 0;
   if (K <= 0 || !err) return RLLM_E_BADARG;
   if (K % 8 || lda % 8 || a_head % 8 || ldw % 8 || w_head % 8 || (((uintptr_t)a | (uintptr_t)w) & 15)) return RLLM_E_UNSUPPORTED;
-  const int bn = tg_width((long long)((M + TG_BM - 1) / TG_BM) * heads, N);
+  const int bn = tg_width((long long)((M + TG_BM - 1) / TG_BM) * heads, N, tg_num_sms());
   if (bn == 256) return tg_launch_heads<256>(a, lda, a_head, w, ldw, w_head, out, ldo, c_head, M, N, K, heads, err, stream);
   if (bn == 192) return tg_launch_heads<192>(a, lda, a_head, w, ldw, w_head, out, ldo, c_head, M, N, K, heads, err, stream);
   return tg_launch_heads<128>(a, lda, a_head, w, ldw, w_head, out, ldo, c_head, M, N, K, heads, err, stream);

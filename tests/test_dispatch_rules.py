@@ -87,3 +87,13 @@ def test_how_many_warps_share_a_row_of_the_cuda_core_attention():
             for rows in (1, 512, 516, 1024, 2044, 2048, 4096, 4097):
                 want = 8 if rows <= 4096 and keys > 128 and keys >= min(rows // 4, 640) else 1
                 assert f(rows, width // page, page, window, kept, chunk) == want
+
+
+@pytest.mark.parametrize("M,N,K,epilogue,sms,width", [
+    (2047, 3072, 2048, 0, 148, 192), (2047, 2048, 4096, 0, 148, 256), (2047, 2048, 2048, 0, 148, 0), (2047, 4096, 2048, 2, 148, 256),
+    (1024, 2048, 8192, 0, 148, 128), (6327, 2048, 2048, 1, 148, 256), (2048, 1024, 1024, 0, 148, 0), (100, 200, 64, 0, 148, 0),
+    (2047, 2048, 4096, 0, 1, 0)])
+def test_which_products_run_on_pairs_of_ctas(M, N, K, epilogue, sms, width):
+    from ctypes import c_int
+    f = build.load_library("gemm_tcgen05").rllm_gemm_tcgen05_pair_width
+    assert f(c_int(M), c_int(N), c_int(K), c_int(epilogue), c_int(sms)) == width
