@@ -42,6 +42,7 @@ RLLM_EXPORT int rllm_latent_attention_mma(const void* q, void* out, const void* 
   if (dv <= 64) LAM_PICK(2, 4, 4);
   if (dv <= 128) LAM_PICK(2, 4, 8);
   if (dv <= 256) LAM_PICK(4, 4, 8);
+  if (mt == 1 && split_keys > 0) LAM_GO(1, 16, 4);
   LAM_PICK(8, 2, 8);
 #undef LAM_PICK
 #undef LAM_GO
