@@ -31,7 +31,7 @@ template <int V> struct __align__(4 * V) LtVec { float v[V]; };
 #define LT_TILE 8            // a thread's tile of S is LT_TILE x LT_TILE
 #define LT_MAX_COLS 256      // value columns a block covers at most
 
-__device__ __forceinline__ float lt_silu(float v) { return v / (1.0f + expf(-v)); }
+__device__ __forceinline__ float lt_silu(float v) { return div_1_plus_exp(v, 1.0f + expf(-v)); }
 template <bool STEPS> __device__ __forceinline__ float lt_act(float v) { return STEPS ? v : lt_silu(v); }
 
 // mode 0: whole portion from the slot's state, state written back

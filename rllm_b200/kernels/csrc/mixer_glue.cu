@@ -322,11 +322,13 @@ RLLM_EXPORT int rllm_rms_mean2(const void* a, const void* b, const void* wa, con
 // The same for bfloat16 rows of up to 8,192 values that start on 16 bytes: eight values an access, all of a thread's loads
 // on their way before the sum, nothing read twice.  The sum runs over shared memory in the order of the form below (256
 // threads), so that a row has the same bits wherever it starts.  Single values / eight an access, in a graph: 33 x 2,048 6.1 /
-// 2.8 us, 2,048 x 2,048 13.1 / 13.2, 2,048 x 4,096 27 / 21, 2,048 x 8,192 81 / 37, 300 x 1,024 3.8 / 3.1; short rows leave most
+// 1.9 us, 2,048 x 2,048 13.1 / 8.7, 2,048 x 4,096 27 / 13.8, 2,048 x 8,192 81 / 32, 300 x 1,024 3.8 / 2.0; short rows leave most
 // of the 256 threads without a value: 2,048 x 1,024 8.1 / 10.8, 2,048 x 512 5.5 / 9.8, 8 x 512 2.4 / 2.5: they take single values.
+// KEEP, the groups of eight that a thread holds, follows the row: with registers for 32 values a thread whatever the row,
+// three blocks shared an SM and each waited for its loads and its sum (2,048 x 2,048 13.0 -> 8.7 us, 34 MB).
 #define GRN_KEEP 4
-template <typename TW>
-__global__ void __launch_bounds__(256)
+template <typename TW, int KEEP, int BLOCKS>
+__global__ void __launch_bounds__(256, BLOCKS)
 gated_rmsnorm8_kernel(const float* x, const bf16* g, int g_stride, const TW* w, bf16* out, int H, float eps) {
   __shared__ float red[32];
   extern __shared__ __align__(16) float grn_x[];        // [H]
@@ -334,11 +336,11 @@ gated_rmsnorm8_kernel(const float* x, const bf16* g, int g_stride, const TW* w, 
   pdl_launch();
   const size_t base = (size_t)blockIdx.x * H;
   const bf16* gr = g + (size_t)blockIdx.x * g_stride;
-  float v[GRN_KEEP][8];
-  uint4 gate[GRN_KEEP];
+  float v[KEEP][8];
+  uint4 gate[KEEP];
   float ss = 0.f;
 #pragma unroll
-  for (int u = 0; u < GRN_KEEP; ++u) {
+  for (int u = 0; u < KEEP; ++u) {
     const int i = (threadIdx.x + u * blockDim.x) * 8;
     if (i < H) {
       load8(x + base + i, v[u]);
@@ -346,26 +348,28 @@ gated_rmsnorm8_kernel(const float* x, const bf16* g, int g_stride, const TW* w, 
     }
   }
 #pragma unroll
-  for (int u = 0; u < GRN_KEEP; ++u) {
+  for (int u = 0; u < KEEP; ++u) {
     const int i = (threadIdx.x + u * blockDim.x) * 8;
     if (i < H) {
       *(float4*)(grn_x + i) = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
       *(float4*)(grn_x + i + 4) = make_float4(v[u][4], v[u][5], v[u][6], v[u][7]);
     }
   }
+  float first_w[8];                                     // (asked for ahead of the sum where a thread has registers for it)
+  if (KEEP == 1 && threadIdx.x * 8 < H) load8(w + threadIdx.x * 8, first_w);
   __syncthreads();
   for (int i = threadIdx.x; i < H; i += blockDim.x) ss = fmaf(grn_x[i], grn_x[i], ss);
   ss = block_sum(ss, red);
   const float r = 1.0f / sqrtf(ss / (float)H + eps);
 #pragma unroll
-  for (int u = 0; u < GRN_KEEP; ++u) {
+  for (int u = 0; u < KEEP; ++u) {
     const int i = (threadIdx.x + u * blockDim.x) * 8;
     if (i < H) {
       float wv[8], gv[8];
-      load8(w + i, wv);
+      if (KEEP > 1) load8(w + i, wv);
       unpack8(gate[u], gv);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[u][j] = v[u][j] * r * wv[j] * (1.0f / (1.0f + expf(-gv[j])));
+      for (int j = 0; j < 8; ++j) v[u][j] = v[u][j] * r * (KEEP > 1 ? wv[j] : first_w[j]) * div_1_plus_exp(1.0f, 1.0f + expf(-gv[j]));
       store8(out + base + i, v[u]);
     }
   }
@@ -385,7 +389,7 @@ gated_rmsnorm_kernel(const float* x, const T* g, int g_stride, const TW* w, T* o
   ss = block_sum(ss, red);
   const float r = 1.0f / sqrtf(ss / (float)H + eps);
   for (int i = threadIdx.x; i < H; i += blockDim.x) {
-    const float gate = 1.0f / (1.0f + expf(-to_f32(gr[i])));
+    const float gate = div_1_plus_exp(1.0f, 1.0f + expf(-to_f32(gr[i])));
     out[base + i] = from_f32<T>(x[base + i] * r * to_f32(w[i]) * gate);
   }
 }
@@ -396,8 +400,14 @@ RLLM_EXPORT int rllm_gated_rmsnorm(const float* x, const void* g, int g_stride, 
   if (H <= 0) return RLLM_E_BADARG;
   if (dtype == RLLM_DT_BF16 && H % 8 == 0 && H <= 256 * 8 * GRN_KEEP && (H >= 2048 || (H >= 1024 && T <= 512)) && g_stride % 8 == 0 &&
       (((uintptr_t)x | (uintptr_t)g | (uintptr_t)w | (uintptr_t)out) & 15) == 0) {
-    RLLM_DISPATCH_DTYPE(w_dtype, TW, (rllm_launch_pdl(gated_rmsnorm8_kernel<TW>, dim3(T), dim3(256), (size_t)H * 4, stream,
-                                                      x, (const bf16*)g, g_stride, (const TW*)w, (bf16*)out, H, eps)));
+#define GRN_GO(KEEP_, BLOCKS_)                                                                                                 \
+    RLLM_DISPATCH_DTYPE(w_dtype, TW, (rllm_launch_pdl(gated_rmsnorm8_kernel<TW, KEEP_, BLOCKS_>, dim3(T), dim3(256), (size_t)H * 4, stream, \
+                                                      x, (const bf16*)g, g_stride, (const TW*)w, (bf16*)out, H, eps)))
+    if (H <= 2048) GRN_GO(1, 6);
+    else if (H <= 4096) GRN_GO(2, 4);
+    else if (T >= 512) GRN_GO(GRN_KEEP, 4);              // (fewer rows: no four blocks for an SM, and all registers help)
+    else GRN_GO(GRN_KEEP, 1);
+#undef GRN_GO
     RLLM_LAUNCH_CHECK();
     return 0;
   }

@@ -21,7 +21,7 @@
 #define SS_TOKENS 8
 #define SS_CHUNK 64
 
-__device__ __forceinline__ float ss_silu(float v) { return v / (1.0f + expf(-v)); }
+__device__ __forceinline__ float ss_silu(float v) { return div_1_plus_exp(v, 1.0f + expf(-v)); }
 __device__ __forceinline__ float ss_softplus(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 
 // x: T rows with stride `stride` (the first E columns are read).  One thread a (token, channel).
@@ -121,103 +121,130 @@ causal_conv_run_kernel(const T* x, int stride, const TW* w, const TW* bias, floa
 }
 
 // Four taps, bfloat16 rows in steps of four channels on 8-byte boundaries (prompt portions): a thread takes four channels and
-// CV_RUN tokens.  Where a run lies in one sequence, which is nearly always, all its inputs are asked for at once; a token at
-// a time behind the last one's arithmetic, one channel a thread, 2,048 x 4,608 took 33 us, 29 so (38 MB; 6 us at the copy rate;
-// the exponential and the division of silu bound it).  The same sums in the same order and the same silu as
+// CV4_RUN tokens.  Where a run lies in one sequence, which is nearly always, all its inputs are asked for at once.  A
+// channel's four weights come in one load: one value a load, the lanes' 64 bytes apart, the 20 loads of weights and bias
+// were most of the wavefronts of a run of eight tokens.  2,048 x 4,608 (38 MB; 6 us at the copy rate): one channel a
+// thread 33 us, four and eight tokens 28, so 16.6.  The same sums in the same order and the same silu as
 // causal_conv_run_kernel: a decoded token has the same bits whether or not another sequence of the step brings a prompt.
-template <typename TW>
-__global__ void __launch_bounds__(128)
-causal_conv4_kernel(const bf16* x, int stride, const TW* w, const TW* bias, float* tail, const int* q_start,
-                    const int* token_seq, const int* slots, int num_slots, bf16* out, int E, int T_tokens, int* err) {
-  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
-  if (c >= E) return;
-  float wv[4][4], b[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k) wv[i][k] = to_f32(w[(size_t)(c + i) * 4 + k]);
-    b[i] = bias ? to_f32(bias[c + i]) : 0.f;
-  }
-  pdl_wait();
-  pdl_launch();
-  const int ta = blockIdx.y * CV_RUN, tb = min(T_tokens, ta + CV_RUN);
-  auto unpack = [](const uint2& raw, float (&v)[4]) {
-    const float2 lo = __bfloat1622float2(*(const __nv_bfloat162*)&raw.x), hi = __bfloat1622float2(*(const __nv_bfloat162*)&raw.y);
-    v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
-  };
-  auto finish = [&](int t, const float (&win)[4][4]) {          // win[k]: the inputs of the taps, the token's own last
+#define CV4_RUN 16
+__device__ __forceinline__ void cv4_load(const float* p, float (&v)[4]) {
+  const float4 r = *(const float4*)p;
+  v[0] = r.x; v[1] = r.y; v[2] = r.z; v[3] = r.w;
+}
+__device__ __forceinline__ void cv4_unpack(const uint2& raw, float (&v)[4]) {
+  const float2 lo = __bfloat1622float2(*(const __nv_bfloat162*)&raw.x), hi = __bfloat1622float2(*(const __nv_bfloat162*)&raw.y);
+  v[0] = lo.x; v[1] = lo.y; v[2] = hi.x; v[3] = hi.y;
+}
+__device__ __forceinline__ void cv4_load(const bf16* p, float (&v)[4]) { cv4_unpack(*(const uint2*)p, v); }
+
+struct Cv4 {                                       // four channels' weights and bias
+  float w[4][4], b[4];
+  // win[k]: the inputs of the taps, the token's own last
+  __device__ __forceinline__ void finish(bf16* to, const float (&win)[4][4]) const {
     float o[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       float acc = b[i];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) acc = fmaf(wv[i][k], win[k][i], acc);
+      for (int k = 0; k < 4; ++k) acc = fmaf(w[i][k], win[k][i], acc);
       o[i] = ss_silu(acc);
     }
     uint2 raw;
     *(__nv_bfloat162*)&raw.x = __floats2bfloat162_rn(o[0], o[1]);
     *(__nv_bfloat162*)&raw.y = __floats2bfloat162_rn(o[2], o[3]);
-    *(uint2*)(out + (size_t)t * E + c) = raw;
-  };
-  const int s0 = token_seq[ta], first0 = q_start[s0], qlen0 = q_start[s0 + 1] - first0;
-  if (token_seq[tb - 1] == s0 && qlen0 > 1) {
-    const int slot = slots[s0];
-    if (slot < 0 || slot >= num_slots) {
-      atomicOr(err, 8);
-      return;
-    }
-    const float* tl = tail + (size_t)slot * 3 * E + c;
-    const int li = ta - first0;
-    uint2 raw[CV_RUN + 3];
+    *(uint2*)to = raw;
+  }
+  // tokens ta .. tb - 1 (at most RUN) of one sequence, of which token ta is number li; x, tl and out at the first channel
+  template <int RUN>
+  __device__ __forceinline__ void run(const bf16* x, int stride, const float* tl, bf16* out, int E, int ta, int tb, int li) const {
+    uint2 raw[RUN + 3];
 #pragma unroll
-    for (int k = 0; k < CV_RUN + 3; ++k) {
+    for (int k = 0; k < RUN + 3; ++k) {
       const int t = ta - 3 + k;
-      raw[k] = (li - 3 + k >= 0 && t < tb) ? *(const uint2*)(x + (size_t)t * stride + c) : make_uint2(0u, 0u);
+      raw[k] = (li - 3 + k >= 0 && t < tb) ? *(const uint2*)(x + (size_t)t * stride) : make_uint2(0u, 0u);
     }
     float win[4][4];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      unpack(raw[k], win[k]);
+      cv4_unpack(raw[k], win[k]);
       if (li - 3 + k < 0) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) win[k][i] = tl[(size_t)(li + k) * E + i];       // input li - 3 + k of the sequence
       }
     }
 #pragma unroll
-    for (int k = 0; k < CV_RUN; ++k) {
+    for (int k = 0; k < RUN; ++k) {
       if (ta + k >= tb) break;
-      unpack(raw[k + 3], win[3]);
-      finish(ta + k, win);
+      cv4_unpack(raw[k + 3], win[3]);
+      finish(out + (size_t)(ta + k) * E, win);
 #pragma unroll
       for (int i = 0; i < 4; ++i) { win[0][i] = win[1][i]; win[1][i] = win[2][i]; win[2][i] = win[3][i]; }
     }
-    return;
   }
-  for (int t = ta; t < tb; ++t) {
-    const int s = token_seq[t], first = q_start[s], qlen = q_start[s + 1] - first, slot = slots[s];
-    if (slot < 0 || slot >= num_slots) {
-      atomicOr(err, 8);
-      return;
+};
+
+// (w rows and bias start on 16 bytes, 8 of bfloat16: E is a multiple of four, and the host has looked at the bases)
+template <typename TW>
+__global__ void __launch_bounds__(128)
+causal_conv4_kernel(const bf16* x, int stride, const TW* w, const TW* bias, float* tail, const int* q_start,
+                    const int* token_seq, const int* slots, int num_slots, bf16* out, int E, int T_tokens, int* err) {
+  const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  if (c >= E) return;
+  Cv4 cv;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) cv4_load(w + (size_t)(c + i) * 4, cv.w[i]);
+  if (bias) cv4_load(bias + c, cv.b);
+  else cv.b[0] = cv.b[1] = cv.b[2] = cv.b[3] = 0.f;
+  pdl_wait();
+  pdl_launch();
+  x += c;
+  out += c;
+  tail += c;
+  const int t0 = blockIdx.y * CV4_RUN, t1 = min(T_tokens, t0 + CV4_RUN);
+  const int last = token_seq[t1 - 1];
+  for (int ta = t0; ta < t1;) {
+    const int s0 = token_seq[ta], first0 = q_start[s0], qlen0 = q_start[s0 + 1] - first0;
+    const bool whole = s0 == last;                       // what is left of the run lies in one sequence
+    const int tb = whole ? t1 : min(t1, ta + 8);
+    if (qlen0 > 1 && (whole || token_seq[tb - 1] == s0)) {
+      const int slot = slots[s0];
+      if (slot < 0 || slot >= num_slots) {
+        atomicOr(err, 8);
+        return;
+      }
+      const float* tl = tail + (size_t)slot * 3 * E;
+      if (tb - ta > 8) cv.run<CV4_RUN>(x, stride, tl, out, E, ta, tb, ta - first0);
+      else cv.run<8>(x, stride, tl, out, E, ta, tb, ta - first0);
+      ta = tb;
+      continue;
     }
-    float* tl = tail + (size_t)slot * 3 * E + c;
-    float win[4][4];
+    for (int t = ta; t < tb; ++t) {
+      const int s = token_seq[t], first = q_start[s], qlen = q_start[s + 1] - first, slot = slots[s];
+      if (slot < 0 || slot >= num_slots) {
+        atomicOr(err, 8);
+        return;
+      }
+      float* tl = tail + (size_t)slot * 3 * E;
+      float win[4][4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int src = t - first - 3 + k;
-      if (src >= 0) {
-        unpack(*(const uint2*)(x + (size_t)(first + src) * stride + c), win[k]);
-      } else {
+      for (int k = 0; k < 4; ++k) {
+        const int src = t - first - 3 + k;
+        if (src >= 0) {
+          cv4_unpack(*(const uint2*)(x + (size_t)(first + src) * stride), win[k]);
+        } else {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) win[k][i] = tl[(size_t)(3 + src) * E + i];
+          for (int i = 0; i < 4; ++i) win[k][i] = tl[(size_t)(3 + src) * E + i];
+        }
+      }
+      cv.finish(out + (size_t)t * E, win);
+      if (qlen == 1) {                     // the only reader of this sequence's tail: move it on by one input
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) tl[(size_t)k * E + i] = win[k + 1][i];
       }
     }
-    finish(t, win);
-    if (qlen == 1) {                     // the only reader of this sequence's tail: move it on by one input
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) tl[(size_t)k * E + i] = win[k + 1][i];
-    }
+    ta = tb;
   }
 }
 
@@ -401,13 +428,14 @@ RLLM_EXPORT int rllm_causal_conv(const void* x, int stride, int dtype, const voi
   if (T <= 0) return 0;
   if (E <= 0 || taps <= 0 || taps > 64 || num_slots <= 0) return RLLM_E_BADARG;
   const long long total = (long long)T * E;
-  // Four channels a thread need work for the GPU and runs within one sequence.  One channel / four, us: 2,048 x 4,608 33 / 29,
-  // 8,192 x 2,880 101 / 70, in portions of 12 tokens 2,040 x 2,880 even; but 64 x 4,608 6.7 / 6.7, 1,020 x 2,880 in portions
+  // Four channels a thread need work for the GPU and runs within one sequence.  One channel / four, us: 2,048 x 4,608 33 / 16.6,
+  // 8,192 x 2,880 101 / 44.5, in portions of 12 tokens 2,040 x 2,880 25 / 22; but 64 x 4,608 6.7 / 6.7, 1,020 x 2,880 in portions
   // of 12 15.4 / 17.2, 64 x 4,608 in portions of 4 7.2 / 9.3.
   if (any_long && total >= (1ll << 22) && T >= 8ll * num_seqs && taps == 4 && dtype == RLLM_DT_BF16 && E % 4 == 0 && stride % 4 == 0 &&
-      (((uintptr_t)x | (uintptr_t)out) & 7) == 0 && (T + CV_RUN - 1) / CV_RUN <= 65535) {
+      (((uintptr_t)x | (uintptr_t)out) & 7) == 0 && (((uintptr_t)w | (uintptr_t)bias) & (w_dtype == RLLM_DT_F32 ? 15 : 7)) == 0 &&
+      (T + CV4_RUN - 1) / CV4_RUN <= 65535) {
     RLLM_DISPATCH_DTYPE(w_dtype, TW,
-      (rllm_launch_pdl(causal_conv4_kernel<TW>, dim3((unsigned)((E + 511) / 512), (unsigned)((T + CV_RUN - 1) / CV_RUN)),
+      (rllm_launch_pdl(causal_conv4_kernel<TW>, dim3((unsigned)((E + 511) / 512), (unsigned)((T + CV4_RUN - 1) / CV4_RUN)),
                        dim3(128), (size_t)0, stream, (const bf16*)x, stride, (const TW*)w, (const TW*)bias, tail, q_start,
                        token_seq, slots, num_slots, (bf16*)out, E, T, err)));
   } else if (taps <= CV_TAPS && (T + CV_RUN - 1) / CV_RUN <= 65535) {

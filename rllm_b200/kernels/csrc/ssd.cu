@@ -101,8 +101,11 @@ silu_gated_group_rmsnorm_kernel(const float* y, const T* z, int z_stride, const 
 // thread's loads on their way before the sum.  The sum runs over shared memory in the order of the form above, so that a
 // row has the same bits wherever it starts.  2,048 x 4,096 in two groups, 67 MB: 44.6 us with single values, 10 at the copy
 // rate; the gates' exponentials and divisions bound it.
+// KEEP, the groups of eight that a thread holds, follows the row: with registers for 32 values a thread whatever the row,
+// three blocks shared an SM and each waited for its loads and its sum (21.9 -> 14.9 us).
 #define SGN_KEEP 4
-__global__ void __launch_bounds__(256)
+template <int KEEP, int BLOCKS>
+__global__ void __launch_bounds__(256, BLOCKS)
 silu_gated_group_rmsnorm8_kernel(const float* y, const bf16* z, int z_stride, const float* w, bf16* out, int E, int size,
                                  float eps) {
   __shared__ float red[32];
@@ -112,11 +115,11 @@ silu_gated_group_rmsnorm8_kernel(const float* y, const bf16* z, int z_stride, co
   const size_t base = (size_t)blockIdx.x * E + (size_t)blockIdx.y * size;
   const bf16* zr = z + (size_t)blockIdx.x * z_stride + (size_t)blockIdx.y * size;
   const float* wr = w + (size_t)blockIdx.y * size;
-  float v[SGN_KEEP][8];
-  uint4 gate[SGN_KEEP];
+  float v[KEEP][8];
+  uint4 gate[KEEP];
   float ss = 0.f;
 #pragma unroll
-  for (int u = 0; u < SGN_KEEP; ++u) {
+  for (int u = 0; u < KEEP; ++u) {
     const int i = (threadIdx.x + u * blockDim.x) * 8;
     if (i < size) {
       load8(y + base + i, v[u]);
@@ -124,7 +127,7 @@ silu_gated_group_rmsnorm8_kernel(const float* y, const bf16* z, int z_stride, co
     }
   }
 #pragma unroll
-  for (int u = 0; u < SGN_KEEP; ++u) {
+  for (int u = 0; u < KEEP; ++u) {
     const int i = (threadIdx.x + u * blockDim.x) * 8;
     if (i < size) {
       float zv[8];
@@ -135,18 +138,20 @@ silu_gated_group_rmsnorm8_kernel(const float* y, const bf16* z, int z_stride, co
       *(float4*)(sgn_x + i + 4) = make_float4(v[u][4], v[u][5], v[u][6], v[u][7]);
     }
   }
+  float first_w[8];                                     // (asked for ahead of the sum where a thread has registers for it)
+  if (KEEP == 1 && threadIdx.x * 8 < size) load8(wr + threadIdx.x * 8, first_w);
   __syncthreads();
   for (int i = threadIdx.x; i < size; i += blockDim.x) ss = fmaf(sgn_x[i], sgn_x[i], ss);
   ss = block_sum(ss, red);
   const float r = 1.0f / sqrtf(ss / (float)size + eps);
 #pragma unroll
-  for (int u = 0; u < SGN_KEEP; ++u) {
+  for (int u = 0; u < KEEP; ++u) {
     const int i = (threadIdx.x + u * blockDim.x) * 8;
     if (i < size) {
       float wv[8];
-      load8(wr + i, wv);
+      if (KEEP > 1) load8(wr + i, wv);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[u][j] = v[u][j] * r * wv[j];
+      for (int j = 0; j < 8; ++j) v[u][j] = v[u][j] * r * (KEEP > 1 ? wv[j] : first_w[j]);
       store8(out + base + i, v[u]);
     }
   }
@@ -162,8 +167,14 @@ RLLM_EXPORT int rllm_silu_gated_group_rmsnorm(const float* y, const void* z, int
   threads = threads < 32 ? 32 : (threads > 256 ? 256 : threads);
   if (dtype == RLLM_DT_BF16 && size % 8 == 0 && size <= 256 * 8 * SGN_KEEP && z_stride % 8 == 0 &&
       (((uintptr_t)y | (uintptr_t)z | (uintptr_t)w | (uintptr_t)out) & 15) == 0) {
-    rllm_launch_pdl(silu_gated_group_rmsnorm8_kernel, dim3(T, groups), dim3(threads), (size_t)size * 4, stream, y, (const bf16*)z,
-                    z_stride, w, (bf16*)out, E, size, eps);
+#define SGN_GO(KEEP_, BLOCKS_)                                                                                                \
+    rllm_launch_pdl(silu_gated_group_rmsnorm8_kernel<KEEP_, BLOCKS_>, dim3(T, groups), dim3(threads), (size_t)size * 4, stream, y, \
+                    (const bf16*)z, z_stride, w, (bf16*)out, E, size, eps)
+    if (size <= 2048) SGN_GO(1, 6);
+    else if (size <= 4096) SGN_GO(2, 4);
+    else if ((long long)T * groups >= 512) SGN_GO(SGN_KEEP, 4);      // (fewer: no four blocks for an SM, and all registers help)
+    else SGN_GO(SGN_KEEP, 1);
+#undef SGN_GO
     RLLM_LAUNCH_CHECK();
     return 0;
   }
