@@ -98,7 +98,7 @@ __device__ __forceinline__ void tg_epilogue(unsigned lane_addr, int half, void* 
   }
 }
 
-// EPI: 0 bfloat16 out, 1 float32 out, 2 SiLU-gate (BN must be 256; W rows n and up_offset + n pair up).
+// EPI: 0 bfloat16 out, 1 float32 out, 2 SiLU-gate (half of BN columns are gate rows; W rows n and up_offset + n pair up).
 // Persistent: CTA b takes the output tiles b, b + gridDim.x, ... (rows of tiles first, so that CTAs
 // running side by side share a weight tile in L2).  Two accumulators in TMEM: the epilogue of a
 // tile runs while the tensor cores work on the next.
@@ -120,7 +120,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   unsigned long long* acc_full = bars + 2 * STAGES;  // [2]       MMA -> epilogue
   unsigned long long* acc_empty = acc_full + 2;      // [2]       epilogue -> MMA
   unsigned* tmem_slot = (unsigned*)(acc_empty + 2);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int num_kb = (K + TG_BK - 1) / TG_BK;
 
   if (threadIdx.x == 0) {
@@ -137,7 +137,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const unsigned tmem_base = *tmem_slot;
+  const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   pdl_wait();                                        // what lies above overlaps the kernel ahead; nothing of global memory is read there
   pdl_launch();
 
@@ -173,38 +173,43 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      // instruction descriptor: float32 accumulate, bfloat16 A and B, both K-major, N = BN, M = 128
-      const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(TG_BM >> 4) << 24);
-      // The thread that issues is what a step of k waits for (a product about 55 cycles, a commit 66, a look at a barrier
-      // 130; the tensor cores need 2 BN cycles a step), so it looks at the next stage's barrier before it issues this
-      // stage's products and finds the answer there afterwards.
-      int s = 0;
-      unsigned phase = 0, ti = 0;
-      bool ok = true, ready = false;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++ti) {
-        const unsigned buf = ti & 1, use = ti >> 1;
-        ok = mbar_wait(&acc_empty[buf], (use & 1) ^ 1, err);   // the epilogue has drained this accumulator
+    // instruction descriptor: float32 accumulate, bfloat16 A and B, both K-major, N = BN, M = 128
+    const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(TG_BM >> 4) << 24);
+    // The whole warp walks and one lane issues, with the warp's number and the accumulator's address taken from lane 0:
+    // the compiler then knows the instruction's operands to be the same in all lanes, and a product costs the warp half
+    // of the 100 cycles that a lane on its own took (tiles of 128 columns, 1,024 x 2,048 x 8,192: 40.5 -> 31.5 us, pairs
+    // 39.1 -> 28.8; of 256 columns unchanged: there a step's 96 KB into and out of shared memory, 80 of a pair's CTA,
+    // set the pace, at 135 to 140 bytes a cycle).  The next stage's barrier is looked at before this stage's products are
+    // issued, so that the answer is there afterwards.
+    int s = 0;
+    unsigned phase = 0, ti = 0;
+    bool ok = true, ready = false;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++ti) {
+      const unsigned buf = ti & 1, use = ti >> 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], (use & 1) ^ 1, err));   // the epilogue has drained this accumulator
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const unsigned tmem_acc = tmem_base + buf * BN;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!ready) ok = __all_sync(0xffffffffu, mbar_wait(&full[s], phase, err));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const unsigned tmem_acc = tmem_base + buf * BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!ready) ok = mbar_wait(&full[s], phase, err);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          unsigned char* sa = stage_mem + s * tg_stage_bytes<BN>();
-          unsigned char* sb = sa + TG_BM * TG_BK * 2;
-          const unsigned long long da = umma_desc(sa), db = umma_desc(sb);
-          unsigned long long* const here = &empty[s];
-          if (++s == STAGES) { s = 0; phase ^= 1; }
-          ready = mbar_test(&full[s], phase);
+        unsigned char* sa = stage_mem + s * tg_stage_bytes<BN>();
+        unsigned char* sb = sa + TG_BM * TG_BK * 2;
+        const unsigned long long da = umma_desc(sa), db = umma_desc(sb);
+        unsigned long long* const here = &empty[s];
+        if (++s == STAGES) { s = 0; phase ^= 1; }
+        ready = __all_sync(0xffffffffu, mbar_test(&full[s], phase));
+        if (umma_elect()) {
 #pragma unroll
-          for (int k = 0; k < TG_BK / 16; ++k)     // 16 bf16 = 32 bytes further along K: + 2 in the address field
+          for (int k = 0; k < TG_BK / 16; ++k)   // 16 bf16 = 32 bytes further along K: + 2 in the address field
             umma_bf16(tmem_acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-          umma_commit(here);                       // the stage is free once these MMAs have read it
+          umma_commit(here);                     // the stage is free once these MMAs have read it
         }
-        if (ok) umma_commit(&acc_full[buf]);       // the accumulator is complete once all MMAs are done
+        __syncwarp();
       }
+      if (ok && umma_elect()) umma_commit(&acc_full[buf]);       // the accumulator is complete once all MMAs are done
+      __syncwarp();
     }
     __syncwarp();
   } else {
@@ -309,8 +314,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   unsigned long long* acc_full = bars + 2 * STAGES;  // [2]       MMA -> each CTA's epilogue
   unsigned long long* acc_empty = acc_full + 2;      // [2]       leader's: both CTAs' epilogues -> MMA
   unsigned* tmem_slot = (unsigned*)(acc_empty + 2);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = (int)tgp_rank(), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int rank = __shfl_sync(0xffffffffu, (int)tgp_rank(), 0), pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int num_kb = (K + TGP_BK - 1) / TGP_BK;
 
   if (threadIdx.x == 0) {
@@ -329,7 +334,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   __syncthreads();
   tgp_cluster_sync();                                // both CTAs' barriers and tensor memory are there
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const unsigned tmem_base = *tmem_slot;
+  const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   pdl_wait();                                        // what lies above overlaps the kernel ahead; nothing of global memory is read there
   pdl_launch();
 
@@ -366,7 +371,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (rank == 0 && lane == 0) {
+    if (rank == 0) {
       // instruction descriptor: float32 accumulate, bfloat16 A and B, both K-major, N = BN, M = 256
       const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(2 * TG_BM >> 4) << 24);
       int s = 0;
@@ -374,30 +379,34 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       bool ok = true, ready = false;
       for (int tile = pair; tile < num_tiles && ok; tile += pairs, ++ti) {
         const unsigned buf = ti & 1, use = ti >> 1;
-        ok = tgp_wait(&acc_empty[buf], (use & 1) ^ 1, err);   // both epilogues have drained this accumulator
+        ok = __all_sync(0xffffffffu, tgp_wait(&acc_empty[buf], (use & 1) ^ 1, err));   // both epilogues have drained this accumulator
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const unsigned tmem_acc = tmem_base + buf * BN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!ready) ok = mbar_wait(&full[s], phase, err);
+          if (!ready) ok = __all_sync(0xffffffffu, mbar_wait(&full[s], phase, err));
           if (!ok) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           unsigned char* sa = stage_mem + s * tgp_stage_bytes<BN>();
           const unsigned long long da = umma_desc(sa), db = umma_desc(sa + TG_BM * TGP_BK * 2);
           unsigned long long* const here = &empty[s];
           if (++s == STAGES) { s = 0; phase ^= 1; }
-          ready = mbar_test(&full[s], phase);      // the next stage's: see gemm_tcgen05_kernel
+          ready = __all_sync(0xffffffffu, mbar_test(&full[s], phase));      // the next stage's: see gemm_tcgen05_kernel
+          if (umma_elect()) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k)              // 16 bf16 = 32 bytes further along K: + 2 in the address field
-            tgp_umma(tmem_acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
-          if (kb * TGP_BK + 64 < K) {
+            for (int k = 0; k < 4; ++k)            // 16 bf16 = 32 bytes further along K: + 2 in the address field
+              tgp_umma(tmem_acc, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+            if (kb * TGP_BK + 64 < K) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-              tgp_umma(tmem_acc, da + (TG_BM * 128 >> 4) + 2 * k, db + (BN / 2 * 128 >> 4) + 2 * k, idesc, 1u);
+              for (int k = 0; k < 4; ++k)
+                tgp_umma(tmem_acc, da + (TG_BM * 128 >> 4) + 2 * k, db + (BN / 2 * 128 >> 4) + 2 * k, idesc, 1u);
+            }
+            tgp_commit(here);
           }
-          tgp_commit(here);
+          __syncwarp();
         }
-        if (ok) tgp_commit(&acc_full[buf]);
+        if (ok && umma_elect()) tgp_commit(&acc_full[buf]);
+        __syncwarp();
       }
     }
     __syncwarp();
@@ -449,7 +458,7 @@ static int tg_run(const CUtensorMap& ma, const CUtensorMap& mw, void* out, int l
 
 template <int BN, int EPI>
 static int tgp_launch(const void* a, int lda, const void* w, int ldw, int w_rows, void* out, int ldo, int M, int N, int K,
-                      int up_offset, int* err, cudaStream_t stream, GateAct ga = GateAct{INFINITY, 1.f, 0.f}) {
+                      int up_offset, int* err, cudaStream_t stream, GateAct ga) {
   constexpr int NOUT = (EPI == TG_EPI_SILU) ? BN / 2 : BN;
   CUtensorMap ma, mw;
   int rc = tg_make_map(&ma, a, M, K, lda, TG_BM);
@@ -470,8 +479,7 @@ static int tgp_launch(const void* a, int lda, const void* w, int ldw, int w_rows
 
 template <int BN, int EPI>
 static int tg_launch(const void* a, int lda, const void* w, int ldw, int w_rows, void* out, int ldo, int M, int N,
-                     int K, int up_offset, int* err, cudaStream_t stream,
-                     GateAct ga = GateAct{INFINITY, 1.f, 0.f}) {
+                     int K, int up_offset, int* err, cudaStream_t stream, GateAct ga) {
   constexpr int NOUT = (EPI == TG_EPI_SILU) ? BN / 2 : BN;
   CUtensorMap ma, mw;
   int rc = tg_make_map(&ma, a, M, K, lda, TG_BM);
@@ -481,53 +489,44 @@ static int tg_launch(const void* a, int lda, const void* w, int ldw, int w_rows,
   return tg_run<BN, EPI, false>(ma, mw, out, ldo, M, N, K, up_offset, 1, 0, err, stream, ga);
 }
 
-// Tile width 256, 192 or 128 for N columns of `rows` tiles of rows: the one with the least estimated time = rounds of the
-// persistent CTAs x width x a factor for what a narrower tile costs (A is read again more often, the epilogue overlaps
-// less).
-static int tg_width(long long rows, int N, long long sms) {
-  int bn = N > 192 ? 256 : (N > 128 ? 192 : 128);
-  if (N > 128) {
-    double best = 1e30;
-    const int widths[3] = {256, 192, 128};
-    const double factor[3] = {1.0, 1.05, 1.3};
-    for (int i = 0; i < 3; ++i) {
-      const long long tiles = rows * ((N + widths[i] - 1) / widths[i]);
-      const double cost = (double)((tiles + sms - 1) / sms) * widths[i] * factor[i];
-      if (cost < best * 0.999) { best = cost; bn = widths[i]; }
-    }
+// Which form a product of `rows` rows takes, and how wide its tile is: the least estimated time, a launch + a step of 64 k
+// times the steps times the rounds of the persistent CTAs, in microseconds (one launch after another on a B200):
+//   CTAs on their own   4.6 + 0.37, 0.30 or 0.22 a step of 256, 192 or 128 columns
+//   pairs               6.3 + 0.32, 6.0 + 0.275 or 5.8 + 0.19 (a tile of twice the rows; two cluster barriers more a launch)
+// A step costs by the bytes that pass through shared memory, so narrow tiles pay where wide ones would leave the last round
+// empty.  Measured, single 256 / 192 / 128 and pairs 256 / 192 / 128, M x N x K:
+//   2,048 x 2,048 x 2,048 16.3 / 22.2 / 18.6, 16.7 / 21.3 / 17.2;    x 4,096 28.2 / 37.6 / 32.1, 26.6 / 37.6 / 28.7
+//   2,047 x 3,072 x 2,048 30.5 / 24.4 / 27.4, 27.9 / 23.7 / 24.4;    700 x 3,072 x 2,048 17.6 / 14.1 / 11.6, 17.3 / 14.7 / 11.8
+//   2,048 x 1,344 x 2,048 17.2 / 13.7 / 17.8, 17.2 / 14.0 / 16.2;    1,024 x 2,048 x 8,192 49 / 40 / 31.5, 42 / 39 / 28.8
+//   6,327 x 3,072 x 2,048 69 / 67 / 76, 61 / 63 / 68
+// With the gate a tile has half as many output columns.
+struct TgForm { int width; bool pair; };
+static TgForm tg_form(long long tiles_rows, long long tiles_rows2, int N, int K, bool gate, bool pairs, long long sms) {
+  static const int widths[3] = {256, 192, 128};
+  static const double single[2][3] = {{4.6, 4.6, 4.6}, {0.37, 0.30, 0.22}}, both[2][3] = {{6.3, 6.0, 5.8}, {0.32, 0.275, 0.19}};
+  const double steps = (K + TG_BK - 1) / TG_BK;
+  TgForm best{256, false};
+  double least = 1e30;
+  for (int i = 0; i < 3; ++i) {
+    const long long cols = gate ? widths[i] / 2 : widths[i], across = (N + cols - 1) / cols;
+    const double t = single[0][i] + single[1][i] * steps * (double)((tiles_rows * across + sms - 1) / sms);
+    if (t < least) { least = t; best = TgForm{widths[i], false}; }
   }
-  return bn;
-}
-
-// The form for a product: the width of a pair's tile, or 0 for CTAs on their own.  A launch of pairs costs a microsecond
-// more (two cluster barriers), so only products of 64 steps of 64 k or more a CTA (rounds times k) take them, and of those
-// the ones that the estimate favours, in microseconds of one launch after another: single CTAs 4.5 and 0.35 a step whatever
-// the width (the loads, not the products, set the pace), pairs 5.3 and 0.32, 0.30 or 0.235 at 256, 192 or 128 columns.
-// Single / pairs, M x N x K: 2,047 x 3,072 x 2,048 24.9 / 24.2 (192 wide), 2,047 x 2,048 x 4,096 27.5 / 26.3,
-// 6,327 x 3,072 x 2,048 70 / 62, 2,048 x 8,512 x 2,048 63 / 54, 1,024 x 2,048 x 8,192 49 / 42 (128 wide), 8,192 cubed 813 / 754;
-// with the gate 512 x 4,096 x 2,048 31 / 28.5, 2,047 x 4,096 x 2,048 54 / 50, 4,096 x 8,192 x 2,048 197 / 176.  Below the line
-// 2,047 x 2,048 x 2,048 15.7 / 16.1, 384 x 6,144 x 2,048 13.4 / 15.4, 2,048 x 3,072 x 768 13.4 / 14.3, 2,048 x 1,024 x 1,024
-// 7.9 / 8.8.
-static int tg_pair_width(int M, int N, int K, int epilogue, long long sms) {
-  if (sms < 2) return 0;
-  const long long steps = (K + TG_BK - 1) / TG_BK;
-  const bool gate = epilogue == TG_EPI_SILU;
-  const int single = gate ? 128 : tg_width((M + TG_BM - 1) / TG_BM, N, sms);             // output columns
-  const auto rounds = [](long long tiles, long long at_once) { return (tiles + at_once - 1) / at_once; };
-  const long long alone = steps * rounds((long long)((M + TG_BM - 1) / TG_BM) * ((N + single - 1) / single), sms);
-  if (alone < 64) return 0;
-  double best = 4.5 + 0.35 * alone;
-  int width = 0;
-  const int widths[3] = {256, 192, 128};
-  const double step[3] = {0.32, 0.30, 0.235};
-  for (int i = 0; i < (gate ? 1 : 3); ++i) {
-    const int cols = gate ? 128 : widths[i];
-    const double t = 5.3 + step[i] * steps * rounds((long long)((M + 2 * TG_BM - 1) / (2 * TG_BM)) * ((N + cols - 1) / cols), sms / 2);
-    if (t < best) { best = t; width = widths[i]; }
+  for (int i = 0; i < 3 && pairs && sms >= 2; ++i) {
+    const long long cols = gate ? widths[i] / 2 : widths[i], across = (N + cols - 1) / cols;
+    const double t = both[0][i] + both[1][i] * steps * (double)((tiles_rows2 * across + sms / 2 - 1) / (sms / 2));
+    if (t < least) { least = t; best = TgForm{widths[i], true}; }
   }
-  return width;
+  return best;
 }
-RLLM_EXPORT int rllm_gemm_tcgen05_pair_width(int M, int N, int K, int epilogue, int sms) { return tg_pair_width(M, N, K, epilogue, sms); }
+static TgForm tg_form_of(int M, int N, int K, int epilogue, long long sms) {
+  return tg_form((M + TG_BM - 1) / TG_BM, (M + 2 * TG_BM - 1) / (2 * TG_BM), N, K, epilogue == TG_EPI_SILU, true, sms);
+}
+// the width of the tiles, negative for pairs (the host's rule alone, for tests)
+RLLM_EXPORT int rllm_gemm_tcgen05_form(int M, int N, int K, int epilogue, int sms) {
+  const TgForm f = tg_form_of(M, N, K, epilogue, sms);
+  return f.pair ? -f.width : f.width;
+}
 
 // epilogue 0: out bfloat16 [M, N]; 1: out float32 [M, N]; 2: W = [gate rows (N); up rows (N)] stacked,
 // out bfloat16 [M, N] = silu(A . gate^T) * (A . up^T), with the gate's constants limit, slope, shift (GateAct).  err:
@@ -539,22 +538,22 @@ RLLM_EXPORT int rllm_gemm_tcgen05(const void* a, int lda, const void* w, int ldw
   if (K <= 0 || lda < K || ldw < K || ldo < N || !err) return RLLM_E_BADARG;
   // TMA: 16-byte aligned bases and row strides
   if (K % 8 || lda % 8 || ldw % 8 || (((uintptr_t)a | (uintptr_t)w) & 15)) return RLLM_E_UNSUPPORTED;
-  const int bn = tg_width((M + TG_BM - 1) / TG_BM, N, tg_num_sms());
-  const int pair = tg_pair_width(M, N, K, epilogue, tg_num_sms());
-#define TG_BY_WIDTH(EPI_)                                                                                      \
-  if (pair == 256) return tgp_launch<256, EPI_>(a, lda, w, ldw, N, out, ldo, M, N, K, 0, err, stream);         \
-  if (pair == 192) return tgp_launch<192, EPI_>(a, lda, w, ldw, N, out, ldo, M, N, K, 0, err, stream);         \
-  if (pair == 128) return tgp_launch<128, EPI_>(a, lda, w, ldw, N, out, ldo, M, N, K, 0, err, stream);         \
-  if (bn == 256) return tg_launch<256, EPI_>(a, lda, w, ldw, N, out, ldo, M, N, K, 0, err, stream);            \
-  if (bn == 192) return tg_launch<192, EPI_>(a, lda, w, ldw, N, out, ldo, M, N, K, 0, err, stream);            \
-  return tg_launch<128, EPI_>(a, lda, w, ldw, N, out, ldo, M, N, K, 0, err, stream)
+  const TgForm form = tg_form_of(M, N, K, epilogue, tg_num_sms());
+  const bool gate = epilogue == TG_EPI_SILU;
+  const int w_rows = gate ? 2 * N : N, up = gate ? N : 0;
   const GateAct ga{limit, slope, shift};
+#define TG_GO(F_, BN_, EPI_) return F_<BN_, EPI_>(a, lda, w, ldw, w_rows, out, ldo, M, N, K, up, err, stream, ga)
+#define TG_BY_FORM(EPI_)                                                          \
+  if (form.pair && form.width == 256) TG_GO(tgp_launch, 256, EPI_);              \
+  if (form.pair && form.width == 192) TG_GO(tgp_launch, 192, EPI_);              \
+  if (form.pair) TG_GO(tgp_launch, 128, EPI_);                                   \
+  if (form.width == 256) TG_GO(tg_launch, 256, EPI_);                            \
+  if (form.width == 192) TG_GO(tg_launch, 192, EPI_);                            \
+  TG_GO(tg_launch, 128, EPI_)
   switch (epilogue) {
-    case TG_EPI_BF16: TG_BY_WIDTH(TG_EPI_BF16);
-    case TG_EPI_F32: TG_BY_WIDTH(TG_EPI_F32);
-    case TG_EPI_SILU:
-      if (pair) return tgp_launch<256, TG_EPI_SILU>(a, lda, w, ldw, 2 * N, out, ldo, M, N, K, N, err, stream, ga);
-      return tg_launch<256, TG_EPI_SILU>(a, lda, w, ldw, 2 * N, out, ldo, M, N, K, N, err, stream, ga);
+    case TG_EPI_BF16: TG_BY_FORM(TG_EPI_BF16);
+    case TG_EPI_F32: TG_BY_FORM(TG_EPI_F32);
+    case TG_EPI_SILU: TG_BY_FORM(TG_EPI_SILU);
   }
   return RLLM_E_BADARG;
 }
@@ -576,7 +575,7 @@ RLLM_EXPORT int rllm_head_gemm_tcgen05(const void* a, long long lda, long long a
   if (M <= 0 || N <= 0 || heads <= 0) return 0;
   if (K <= 0 || !err) return RLLM_E_BADARG;
   if (K % 8 || lda % 8 || a_head % 8 || ldw % 8 || w_head % 8 || (((uintptr_t)a | (uintptr_t)w) & 15)) return RLLM_E_UNSUPPORTED;
-  const int bn = tg_width((long long)((M + TG_BM - 1) / TG_BM) * heads, N, tg_num_sms());
+  const int bn = tg_form((long long)((M + TG_BM - 1) / TG_BM) * heads, 0, N, K, false, false, tg_num_sms()).width;
   if (bn == 256) return tg_launch_heads<256>(a, lda, a_head, w, ldw, w_head, out, ldo, c_head, M, N, K, heads, err, stream);
   if (bn == 192) return tg_launch_heads<192>(a, lda, a_head, w, ldw, w_head, out, ldo, c_head, M, N, K, heads, err, stream);
   return tg_launch_heads<128>(a, lda, a_head, w, ldw, w_head, out, ldo, c_head, M, N, K, heads, err, stream);

@@ -89,11 +89,12 @@ def test_how_many_warps_share_a_row_of_the_cuda_core_attention():
                 assert f(rows, width // page, page, window, kept, chunk) == want
 
 
-@pytest.mark.parametrize("M,N,K,epilogue,sms,width", [
-    (2047, 3072, 2048, 0, 148, 192), (2047, 2048, 4096, 0, 148, 256), (2047, 2048, 2048, 0, 148, 0), (2047, 4096, 2048, 2, 148, 256),
-    (1024, 2048, 8192, 0, 148, 128), (6327, 2048, 2048, 1, 148, 256), (2048, 1024, 1024, 0, 148, 0), (100, 200, 64, 0, 148, 0),
-    (2047, 2048, 4096, 0, 1, 0)])
-def test_which_products_run_on_pairs_of_ctas(M, N, K, epilogue, sms, width):
+@pytest.mark.parametrize("M,N,K,epilogue,sms,form", [
+    (2047, 3072, 2048, 0, 148, -192), (2047, 2048, 4096, 0, 148, -256), (2047, 2048, 2048, 0, 148, 256), (2047, 4096, 2048, 2, 148, -256),
+    (1024, 2048, 8192, 0, 148, -128), (6327, 2048, 2048, 1, 148, -256), (2048, 1024, 1024, 0, 148, 128), (100, 200, 64, 0, 148, 128),
+    (700, 3072, 2048, 0, 148, 128), (2047, 2048, 4096, 0, 1, 256)])
+def test_which_tile_a_product_takes(M, N, K, epilogue, sms, form):
+    """The tile's width, negative for pairs of CTAs; a device of one SM has no pairs."""
     from ctypes import c_int
-    f = build.load_library("gemm_tcgen05").rllm_gemm_tcgen05_pair_width
-    assert f(c_int(M), c_int(N), c_int(K), c_int(epilogue), c_int(sms)) == width
+    f = build.load_library("gemm_tcgen05").rllm_gemm_tcgen05_form
+    assert f(c_int(M), c_int(N), c_int(K), c_int(epilogue), c_int(sms)) == form

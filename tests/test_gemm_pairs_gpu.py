@@ -1,5 +1,5 @@
-"""The tcgen05 product by pairs of CTAs: remainders of its tiles in rows (a pair's second CTA with no row), columns and k
-(a stage whose second half is empty), every tile width and epilogue, more tiles than pairs, strided rows."""
+"""The tcgen05 product on CTAs of their own and on pairs: remainders of its tiles in rows (a pair's second CTA with no row),
+columns and k (a stage whose second half is empty), every tile width and epilogue, more tiles than CTAs, strided rows."""
 from ctypes import c_int
 
 import pytest
@@ -8,17 +8,19 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("M,N,K,epilogue,width", [
-    (2047, 3072, 2056, "store", 192), (1100, 2040, 4160, "store", 192), (1025, 2048, 8192, "store", 192), (6327, 2048, 2056, "store", 256),
-    (6300, 2050, 2048, "store", 192), (4100, 2048, 4096, "f32", 256), (129, 389, 5000, "f32", 128), (2047, 3070, 2048, "f32", 192),
-    (1100, 120, 4200, "store", 128), (300, 8200, 2048, "silu_mul", 256), (513, 4090, 2184, "silu_mul", 256),
-    (1, 100, 4104, "silu_mul", 256)])
-def test_products_on_pairs_of_ctas(M, N, K, epilogue, width):
+@pytest.mark.parametrize("M,N,K,epilogue,form", [
+    (2047, 3072, 2056, "store", -192), (1100, 2040, 4160, "store", 128), (6327, 2048, 2056, "store", -256), (6300, 2050, 2048, "store", -192),
+    (4100, 2048, 4096, "f32", -256), (129, 389, 5000, "f32", -128), (2047, 3070, 2048, "f32", -192), (2048, 1344, 2048, "f32", 192),
+    (1100, 120, 4200, "store", -128), (300, 8200, 2048, "silu_mul", 192), (513, 4090, 2184, "silu_mul", -192),
+    (1, 100, 4104, "silu_mul", -128), (257, 1000, 4096, "silu_mul", -128), (4097, 3000, 2048, "silu_mul", -256),
+    (700, 3072, 2040, "store", 128), (1024, 4100, 4096, "silu_mul", -256)])
+def test_products_on_every_form_of_tile(M, N, K, epilogue, form):
+    """``form``: the tile's width, negative for pairs of CTAs."""
     from rllm_b200.kernels import build, ops
     code = {"store": 0, "f32": 1, "silu_mul": 2}[epilogue]
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    f = build.load_library("gemm_tcgen05").rllm_gemm_tcgen05_pair_width
-    assert f(c_int(M), c_int(N), c_int(K), c_int(code), c_int(sms)) == width
+    f = build.load_library("gemm_tcgen05").rllm_gemm_tcgen05_form
+    assert f(c_int(M), c_int(N), c_int(K), c_int(code), c_int(sms)) == form
     g = torch.Generator(device="cuda")
     g.manual_seed(M + N + K)
     rows = N * (2 if code == 2 else 1)
