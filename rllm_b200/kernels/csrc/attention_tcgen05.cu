@@ -94,7 +94,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   unsigned long long* xbar = bars + 13;           // [4] the two warps of a row quarter, one another
   unsigned* tmem_slot = (unsigned*)(bars + 17);
   int* s_pages = (int*)(bars + 18);               // [4 tiles][8 boxes]: the producer's page numbers, from K's request to V's
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int g = nq / nkv;
   const int bq = AT_BM / g;                        // query tokens per tile
   const int kvh = blockIdx.x % nkv;
@@ -153,7 +153,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const unsigned tmem_s = *tmem_slot, tmem_o = tmem_s + AT_BN, tmem_p = tmem_o + AT_D;   // BN + D + BN / 2 <= 256 columns
+  const unsigned tmem_s = __shfl_sync(0xffffffffu, *tmem_slot, 0), tmem_o = tmem_s + AT_BN, tmem_p = tmem_o + AT_D;   // BN + D + BN / 2 <= 256 columns
 
   if (warp == 0) {
     if (lane == 0) {
@@ -221,49 +221,55 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      // S: float32 accumulate, bf16 x bf16, A and B K-major, M 128, N BN.
-      // PV: the same with N = D, A (P) in tensor memory and B (V) MN-major.
-      const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(AT_BN >> 3) << 17) | ((unsigned)(AT_BM >> 4) << 24);
-      // (all D dims in one instruction: for D = 128 the two panels of V are a leading-dimension step apart)
-      const unsigned idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((unsigned)(AT_D >> 3) << 17) | ((unsigned)(AT_BM >> 4) << 24);
-      const int ntiles = num_tiles;
-      const unsigned long long dq = umma_desc(sQ);
-      // scores of the tile in stage st: D / 16 steps along the head dims, panel by panel
-      auto scores = [&](int st) {
-        const unsigned long long dk = umma_desc(sK + st * AT_STAGE);
+    // S: float32 accumulate, bf16 x bf16, A and B K-major, M 128, N BN.
+    // PV: the same with N = D, A (P) in tensor memory and B (V) MN-major.
+    // The whole warp walks and one lane issues, with what the instructions take from lane 0: the compiler then knows their
+    // operands to be the same in all lanes, and a product costs the warp half as much (see gemm_tcgen05.cu).  Against a
+    // lane that walks alone: 8,192 tokens, 32/8 heads of 64 373 -> 358 us, 16/4 of 128 320 -> 302; 2,048 tokens 41.2 -> 39.5
+    // and 45.6 -> 43.3.
+    const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(AT_BN >> 3) << 17) | ((unsigned)(AT_BM >> 4) << 24);
+    // (all D dims in one instruction: for D = 128 the two panels of V are a leading-dimension step apart)
+    const unsigned idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((unsigned)(AT_D >> 3) << 17) | ((unsigned)(AT_BM >> 4) << 24);
+    const int ntiles = __shfl_sync(0xffffffffu, num_tiles, 0);
+    const unsigned long long dq = umma_desc(sQ);
+    auto wait = [&](unsigned long long* bar, unsigned parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)) != 0; };
+    // scores of the tile in stage st: D / 16 steps along the head dims, panel by panel
+    auto scores = [&](int st) {
+      const unsigned long long dk = umma_desc(sK + st * AT_STAGE);
+      if (umma_elect()) {
 #pragma unroll
         for (int k = 0; k < AT_D / 16; ++k) {
           const unsigned long long a = dq + (unsigned long long)((k >> 2) * (16384 >> 4) + 2 * (k & 3));
           const unsigned long long b = dk + (unsigned long long)((k >> 2) * (KPANEL >> 4) + 2 * (k & 3));
           umma_bf16(tmem_s, a, b, idesc_s, k != 0);
         }
-      };
-      bool ok = mbar_wait(q_full, 0, err) && mbar_wait(&k_full[0], 0, err);
-      if (ok) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        scores(0);
         umma_commit(s_full);
-        umma_commit(&k_empty[0]);
+        umma_commit(&k_empty[st]);
       }
-      for (int it = 0; it < ntiles && ok; ++it) {
-        const int st = it & 1;
-        if (it + 1 < ntiles) {
-          // the next tile's scores, as soon as its keys are here and the softmax warps hold this tile's scores
-          const int sn = (it + 1) & 1;
-          ok = mbar_wait(&k_full[sn], ((it + 1) >> 1) & 1, err) && mbar_wait(s_free, it & 1, err);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          scores(sn);
-          umma_commit(s_full);
-          umma_commit(&k_empty[sn]);
-        }
-        ok = mbar_wait(&v_full[st], (it >> 1) & 1, err) && mbar_wait(p_full, it & 1, err);   // P is in tensor memory, O is rescaled
+      __syncwarp();
+    };
+    bool ok = wait(q_full, 0) && wait(&k_full[0], 0);
+    if (ok) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      scores(0);
+    }
+    for (int it = 0; it < ntiles && ok; ++it) {
+      const int st = it & 1;
+      if (it + 1 < ntiles) {
+        // the next tile's scores, as soon as its keys are here and the softmax warps hold this tile's scores
+        const int sn = (it + 1) & 1;
+        ok = wait(&k_full[sn], ((it + 1) >> 1) & 1) && wait(s_free, it & 1);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // V is the MN-major operand: 64 dims x 8 keys a swizzle atom, 8 keys on 1024 bytes further (stride
-        // field), 64 dims on a panel further (leading-dimension field)
-        const unsigned long long dv = (umma_desc(sV + st * AT_STAGE) & ~(0x3FFFull << 16)) | ((unsigned long long)(KPANEL >> 4) << 16);
+        scores(sn);
+      }
+      ok = wait(&v_full[st], (it >> 1) & 1) && wait(p_full, it & 1);   // P is in tensor memory, O is rescaled
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // V is the MN-major operand: 64 dims x 8 keys a swizzle atom, 8 keys on 1024 bytes further (stride
+      // field), 64 dims on a panel further (leading-dimension field)
+      const unsigned long long dv = (umma_desc(sV + st * AT_STAGE) & ~(0x3FFFull << 16)) | ((unsigned long long)(KPANEL >> 4) << 16);
+      if (umma_elect()) {
 #pragma unroll
         for (int kk = 0; kk < AT_BN / 16; ++kk)         // 16 keys a step: 8 columns of P on, V two row groups on
           umma_bf16_tmem_a(tmem_o, tmem_p + kk * 8, dv + (unsigned long long)(kk * (2048 >> 4)), idesc_pv,
@@ -271,8 +277,8 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         umma_commit(pv_full);
         umma_commit(&v_empty[st]);
       }
+      __syncwarp();
     }
-    __syncwarp();
   } else {
     // Two threads a row: warps 2-5 take the first half of the tile's keys (and of the output dims),
     // warps 6-9 the second; warp w and warp w + 4 own the same 32 rows (TMEM lanes) and exchange

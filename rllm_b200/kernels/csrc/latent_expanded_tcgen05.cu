@@ -14,8 +14,8 @@
 //              in tensor memory and V as the MN-major operand.
 //   warps 2-9  softmax, two threads a row, as in attention_tcgen05.cu; the reference point is the running maximum, as in
 //              latent_attention_tcgen05.cu.
-// Measured, 2,048 tokens, 16 heads of 128 + 64 | 128 over rows of 512 + 64: attention 221 -> 45 us (475 TFLOP/s of visible
-// pairs), gather 7 and product 16 us in place of the query side's products 21 + 16; the mixer 320 -> 126 us, its distance
+// Measured, 2,048 tokens, 16 heads of 128 + 64 | 128 over rows of 512 + 64: attention 221 -> 39 us (550 TFLOP/s of visible
+// pairs), gather 7 and product 16 us in place of the query side's products 21 + 16; the mixer 320 -> 120 us, its distance
 // from float64 0.0052 -> 0.0051 of the result's norm.  The longest CTAs (32 tiles of keys, 1 us each) are what is left.
 // K has two stages; V one or two, what the 113 KB of half an SM leave: V of a tile is asked for when the product of the
 // tile before is through, which the tile's softmax hides.
@@ -67,7 +67,7 @@ latent_expanded_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   unsigned long long* s_free = bars + 12;         // softmax (8 warps) -> MMA
   unsigned long long* xbar = bars + 13;           // [4] the two warps of a row quarter, one another
   unsigned* tmem_slot = (unsigned*)(bars + 17);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int head = blockIdx.x % heads;
   // which (sequence, tile): the tiles that see the most keys first; where the sequence's gathered rows begin
   int s = -1, tile = 0, row0 = 0;
@@ -110,7 +110,7 @@ latent_expanded_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const unsigned tmem_s = *tmem_slot, tmem_o = tmem_s + BN, tmem_p = tmem_o + DV;   // BN + DV + BN / 2 <= 256 columns
+  const unsigned tmem_s = __shfl_sync(0xffffffffu, *tmem_slot, 0), tmem_o = tmem_s + BN, tmem_p = tmem_o + DV;   // BN + DV + BN / 2 <= 256 columns
 
   if (warp == 0) {
     if (lane == 0) {
@@ -144,52 +144,57 @@ latent_expanded_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(LE_BM >> 4) << 24);
-      const unsigned idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((unsigned)(DV >> 3) << 17) | ((unsigned)(LE_BM >> 4) << 24);
-      const unsigned long long dq = umma_desc(sQ);
-      const int rot_steps = (rot + 15) / 16;       // the shared part's dims behind `rot` are zeros
-      auto scores = [&](int st) {
-        const unsigned long long dk = umma_desc(sK + st * Shape::K_STAGE);
+    // The whole warp walks and one lane issues, with what the instructions take from lane 0: the compiler then knows their
+    // operands to be the same in all lanes, and a product costs the warp half as much (see gemm_tcgen05.cu; 45 -> 39 us).
+    const unsigned idesc_s = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(BN >> 3) << 17) | ((unsigned)(LE_BM >> 4) << 24);
+    const unsigned idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((unsigned)(DV >> 3) << 17) | ((unsigned)(LE_BM >> 4) << 24);
+    const unsigned long long dq = umma_desc(sQ);
+    const int rot_steps = (rot + 15) / 16;         // the shared part's dims behind `rot` are zeros
+    const int tiles = __shfl_sync(0xffffffffu, ntiles, 0);
+    auto scores = [&](int st) {
+      const unsigned long long dk = umma_desc(sK + st * Shape::K_STAGE);
+      if (umma_elect()) {
 #pragma unroll
         for (int k = 0; k < NQ * 4; ++k) {
           if (k >= (NQ - 1) * 4 + rot_steps) break;
           umma_bf16(tmem_s, dq + (unsigned long long)((k >> 2) * (16384 >> 4) + 2 * (k & 3)),
                     dk + (unsigned long long)((k >> 2) * (PANEL >> 4) + 2 * (k & 3)), idesc_s, k != 0);
         }
-      };
-      bool ok = mbar_wait(q_full, 0, err) && mbar_wait(&k_full[0], 0, err);
-      if (ok) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        scores(0);
         umma_commit(s_full);
-        umma_commit(&k_empty[0]);
+        umma_commit(&k_empty[st]);
       }
-      for (int it = 0; it < ntiles && ok; ++it) {
-        if (it + 1 < ntiles) {                     // the next tile's scores, as soon as the softmax warps hold this tile's
-          const int sn = (it + 1) & 1;
-          ok = mbar_wait(&k_full[sn], ((it + 1) >> 1) & 1, err) && mbar_wait(s_free, it & 1, err);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          scores(sn);
-          umma_commit(s_full);
-          umma_commit(&k_empty[sn]);
-        }
-        const int sv = it % NV;
-        ok = mbar_wait(&v_full[sv], (it / NV) & 1, err) && mbar_wait(p_full, it & 1, err);   // P is in tensor memory, O is rescaled
+      __syncwarp();
+    };
+    auto wait = [&](unsigned long long* bar, unsigned parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)) != 0; };
+    bool ok = wait(q_full, 0) && wait(&k_full[0], 0);
+    if (ok) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      scores(0);
+    }
+    for (int it = 0; it < tiles && ok; ++it) {
+      if (it + 1 < tiles) {                        // the next tile's scores, as soon as the softmax warps hold this tile's
+        const int sn = (it + 1) & 1;
+        ok = wait(&k_full[sn], ((it + 1) >> 1) & 1) && wait(s_free, it & 1);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // V: 64 dims x 8 keys a swizzle atom, 8 keys on 1024 bytes further (stride field), 64 dims on a panel further
-        // (leading-dimension field)
-        const unsigned long long dv = (umma_desc(sV + sv * Shape::V_STAGE) & ~(0x3FFFull << 16)) | ((unsigned long long)(PANEL >> 4) << 16);
+        scores(sn);
+      }
+      const int sv = it % NV;
+      ok = wait(&v_full[sv], (it / NV) & 1) && wait(p_full, it & 1);   // P is in tensor memory, O is rescaled
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // V: 64 dims x 8 keys a swizzle atom, 8 keys on 1024 bytes further (stride field), 64 dims on a panel further
+      // (leading-dimension field)
+      const unsigned long long dv = (umma_desc(sV + sv * Shape::V_STAGE) & ~(0x3FFFull << 16)) | ((unsigned long long)(PANEL >> 4) << 16);
+      if (umma_elect()) {
 #pragma unroll
         for (int kk = 0; kk < BN / 16; ++kk)
           umma_bf16_tmem_a(tmem_o, tmem_p + kk * 8, dv + (unsigned long long)(kk * (2048 >> 4)), idesc_pv, (it | kk) != 0);
         umma_commit(&v_empty[sv]);
         umma_commit(pv_full);
       }
+      __syncwarp();
     }
-    __syncwarp();
   } else {
     const int quarter = warp & 3, half = (warp - 2) >> 2;
     const int r = quarter * 32 + lane;               // this thread's row of the tile
