@@ -27,7 +27,6 @@
 #define MT_STAGE (3 * MT_PANEL)          // two weight panels, one panel of pairs
 #define MT_STAGES 4
 #define MT_SMEM (MT_STAGES * MT_STAGE + 1024 + 256)
-#define MT_LAG 2                         // a gathered stage is handed over when the second one behind it is on its way
 
 struct MoeTile { int e, r0, rows; };
 
@@ -78,11 +77,11 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   unsigned long long* acc_full = bars + 2 * MT_STAGES;  // [2]      MMA -> epilogue
   unsigned long long* acc_empty = acc_full + 2;         // [2]      epilogue -> MMA
   unsigned* tmem_slot = (unsigned*)(acc_empty + 2);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int num_kb = (K + 63) / 64;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < MT_STAGES; ++i) { mbar_init(&full[i], GATE ? 5 : 1); mbar_init(&empty[i], 1); }
+    for (int i = 0; i < MT_STAGES; ++i) { mbar_init(&full[i], GATE ? 129 : 1); mbar_init(&empty[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"((unsigned long long)&map_w) : "memory");
@@ -95,11 +94,11 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const unsigned tmem_base = *tmem_slot;
+  const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   pdl_wait_on(h, offsets, sorted, tile_expert, tile_row0, meta);
   pdl_launch();
   const int m_tiles = meta[0];
-  const int num_tiles = m_tiles * tiles_f;
+  const int num_tiles = __shfl_sync(0xffffffffu, m_tiles * tiles_f, 0);
 
   if (warp == 0) {
     if (lane == 0) {
@@ -123,32 +122,41 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
     __syncwarp();
   } else if (warp == 1) {
-    // the whole warp walks the loop, one lane issues (154 -> 151 us against a lane that walks alone)
-    unsigned it = 0, ti = 0;
-    bool ok = true;
+    // The whole warp walks and one lane issues, with what the instructions take from lane 0, and the next stage is looked at
+    // ahead: see gemm_tcgen05.cu.
+    int s = 0;
+    unsigned phase = 0, ti = 0;
+    bool ok = true, ready = false;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++ti) {
       const MoeTile t = moe_tile(tile_expert, tile_row0, offsets, tile % m_tiles, m_tiles);
       // instruction descriptor: float32 accumulate, bfloat16 A and B, both K-major, M = 128, N = the tile's pairs
-      const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)((t.rows + 15) >> 4) << 18) | ((128u >> 4) << 24);
+      const unsigned wide = __shfl_sync(0xffffffffu, (unsigned)((t.rows + 15) >> 4), 0);
+      const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | (wide << 18) | ((128u >> 4) << 24);
       const unsigned buf = ti & 1, use = ti >> 1;
       ok = __all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], (use & 1) ^ 1, err));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const unsigned acc = tmem_base + buf * 256;
-      for (int kb = 0; kb < num_kb; ++kb, ++it) {
-        const int s = it % MT_STAGES;
-        ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (it / MT_STAGES) & 1, err));
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!ready) ok = __all_sync(0xffffffffu, mbar_wait(&full[s], phase, err));
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // The gathered rows were written by cp.async, and the instructions read them through the async proxy.  (Each stage
+        // arrives with its copies; handed over by the copying warps when the second stage behind it was on its way, with the
+        // fence there: 2,048 tokens, top 4 of 32, 162.7 us, so 159.6; top 2 of 16, 1,024 wide 84.3 -> 81.4.)
+        if (GATE) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         unsigned char* sa = base + s * MT_STAGE;
         const unsigned long long d0 = umma_desc(sa), d1 = umma_desc(sa + MT_PANEL), db = umma_desc(sa + 2 * MT_PANEL);
+        unsigned long long* const here = &empty[s];
+        if (++s == MT_STAGES) { s = 0; phase ^= 1; }
+        ready = __all_sync(0xffffffffu, mbar_test(&full[s], phase));
         if (umma_elect()) {
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             umma_bf16(acc, d0 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
             umma_bf16(acc + 128, d1 + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
           }
-          umma_commit(&empty[s]);
+          umma_commit(here);
         }
         __syncwarp();
       }
@@ -199,11 +207,6 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int tid = threadIdx.x - 192, chunk = tid & 7, g = tid >> 3;
     unsigned it = 0;
     bool ok = true;
-    auto hand_over = [&](unsigned stage) {      // after this thread's copies of that stage have landed
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tensor cores read it through the async proxy
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&full[stage]);
-    };
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
       const MoeTile t = moe_tile(tile_expert, tile_row0, offsets, tile % m_tiles, m_tiles);
       const bf16* src[8];
@@ -223,16 +226,11 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         for (int i = 0; i < 8; ++i)
           if (src[i])                                         // rows behind the tile's pairs: columns no one reads
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + i * 2048), "l"(n ? src[i] + kb * 64 : src[i]), "r"(n) : "memory");
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (it >= MT_LAG) {
-          asm volatile("cp.async.wait_group %0;" ::"n"(MT_LAG) : "memory");
-          hand_over((it - MT_LAG) % MT_STAGES);
-        }
+        // this thread's arrival, when its copies have landed
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tg_smem(&full[s])) : "memory");
       }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (ok)
-      for (unsigned k = it < MT_LAG ? 0 : it - MT_LAG; k < it; ++k) hand_over(k % MT_STAGES);
+    asm volatile("cp.async.wait_all;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
