@@ -11,6 +11,7 @@ from typing import Optional
 
 import torch
 
+from ..native import build as native_build
 from . import build
 
 DT_F32, DT_BF16 = 0, 1
@@ -56,6 +57,117 @@ def _check(code: int, what: str) -> None:
     raise KernelError(f"{what}: CUDA error {code}")
 
 
+# The entry points by name: the library that holds each, its arguments (see native/csrc/launch.cc: p tensor or None, i int,
+# l long long, f float; the stream, which comes last everywhere, is added) and what a refusal calls it.
+_TABLE = {
+    "rllm_softcap": ("elementwise", "plf", "softcap_rows"),
+    "rllm_shared_key_attention_mma": ("shared_key_attention", "pppppippiiiiiiiiiiifiipp", "shared_key_attention_mma"),
+    "rllm_shared_key_attention_tcgen05": ("shared_key_attention", "pippppippiiiiiiiiiiiifp", "shared_key_attention_tcgen05"),
+    "rllm_talking_prep": ("talking_heads", "piipppppipipppippiiiiiiiiipp", "talking_prep"),
+    "rllm_linear_state_walk": ("linear_state", "piippifpppfippppiiiiiippip", "linear_state_walk"),
+    "rllm_linear_state_chunked": ("linear_state", "pippifpppfipppppiiiiiiipp", "linear_state_chunked"),
+    "rllm_rotation_table": ("linear_state", "ppiip", "rotation_table"),
+    "rllm_channel_delta_step": ("channel_delta", "pippippppipppppppiiiiiiiiiiiiifffip", "channel_delta_step"),
+    "rllm_channel_delta_walk": ("channel_delta", "pppppiipppiipiiiip", "channel_delta_walk"),
+    "rllm_channel_delta_prepare": ("channel_delta", "piippppppppiiiiff", "channel_delta_prepare"),
+    "rllm_channel_delta_chunked": ("channel_delta", "pippppffpppiiiippiiiip", "channel_delta_chunked"),
+    "rllm_silu_gated_group_rmsnorm": ("ssd", "ppippiiiif", "silu_gated_group_rmsnorm"),
+    "rllm_ssd_scan": ("ssd", "piipppppppppiiipiiiip", "ssd_scan"),
+    "rllm_head_gated_rmsnorm": ("mlstm", "ppipipiiiif", "head_gated_rmsnorm"),
+    "rllm_mlstm_scan": ("mlstm", "pppiipppffppppiiiiiiippp", "mlstm_scan"),
+    "rllm_add_row_bias": ("layernorm", "ppiii", "add_row_bias"),
+    "rllm_add_rows": ("layernorm", "ppppiii", "add_rows"),
+    "rllm_layernorm": ("layernorm", "ppppppppiiifi", "layernorm"),
+    "rllm_selective_scan": ("selective_scan", "ppppiiipppiiipppppiiipiip", "selective_scan"),
+    "rllm_causal_conv": ("selective_scan", "piippippppiiipiiip", "causal_conv"),
+    "rllm_lightning_scan": ("lightning", "pppiipppppiiipiiip", "lightning_scan"),
+    "rllm_gated_rmsnorm": ("mixer_glue", "ppipipiiif", "gated_rmsnorm"),
+    "rllm_rms_mean2": ("mixer_glue", "ppppipiiif", "rms_mean2"),
+    "rllm_attention_simt_kv": ("attention_simt", "pipppipippiiiiiiiifiifppiipiip", "attention_simt_kv"),
+    "rllm_head_norm_kv_write": ("mixer_glue", "piippppifpippiiiiiiipiiippififiip", "head_norm_kv_write"),
+    "rllm_dyt": ("hyper_streams", "ppppppipiiii", "dyt"),
+    "rllm_hs_write": ("hyper_streams", "ppipppppppippili", "streams_write"),
+    "rllm_hs_read": ("hyper_streams", "ppppppipiilii", "streams_read"),
+    "rllm_act_mul": ("elementwise", "ppiiii", "act_mul"),
+    "rllm_sigmoid_gate": ("elementwise", "ppipiii", "sigmoid_gate"),
+    "rllm_act": ("elementwise", "ppili", "act"),
+    "rllm_moe_choose_sigmoid": ("moe", "ppfppiii", "moe_choose_sigmoid"),
+    "rllm_weighted_slot_sum": ("moe", "pppiiippi", "weighted_slot_sum"),
+    "rllm_moe_experts": ("moe", "ppppppppppiiiiifffi", "moe_experts"),
+    "rllm_moe_experts_tcgen05": ("moe_tcgen05", "ppppppppppiiiiiifffp", "moe_experts_tcgen05"),
+    "rllm_moe_sort": ("moe", "piiippppp", "moe_sort"),
+    "rllm_moe_choose": ("moe", "pppiiiiii", "moe_choose"),
+    "rllm_moe_route": ("moe", "ppppiiiii", "moe_route"),
+    "rllm_latent_expanded_tcgen05": ("latent_expanded_tcgen05", "pippiiipppiiiiiiiifpp", "latent_expanded_tcgen05"),
+    "rllm_latent_expand_prep": ("latent_attention", "ppppippiippfiiiiiiiiiiip", "latent_expand_prep"),
+    "rllm_latent_attention_tcgen05": ("latent_attention_tcgen05", "pipppippiiiiiiiiifpp", "latent_attention_tcgen05"),
+    "rllm_latent_attention_mma": ("latent_attention_mma", "ppppippiiiiiiiifpiipp", "latent_attention_mma"),
+    "rllm_latent_attention_simt": ("latent_attention", "pppipippiiiiiiifpp", "latent_attention_simt"),
+    "rllm_head_gemm": ("latent_attention", "pllplliplliiiii", "head_gemm"),
+    "rllm_head_gemm_tcgen05": ("gemm_tcgen05", "pllpllpiliiiip", "head_gemm_tcgen05"),
+    "rllm_latent_q_rot": ("latent_attention", "ppppfiiiiiii", "latent_q_rot"),
+    "rllm_latent_prep": ("latent_attention", "piiiiippfpppipppfiiiiiip", "latent_prep"),
+    "rllm_mingru_scan": ("mingru", "pipppppipiiiip", "mingru_scan"),
+    "rllm_mingru_scan_chunked": ("mingru", "pipppppipiiipiip", "mingru_scan_chunked"),
+    "rllm_depth_average": ("layer_glue", "plipppppfiiii", "depth_average"),
+    "rllm_scaled_sum2": ("layer_glue", "ppffpil", "scaled_sum2"),
+    "rllm_activation_rows": ("layer_glue", "ppl", "activation_rows"),
+    "rllm_postnorm_add": ("layer_glue", "pppffpffpiiii", "postnorm_add"),
+    "rllm_gated_postnorm_add": ("layer_glue", "pppippippfppfplippiiii", "gated_postnorm_add"),
+    "rllm_attention_decode_bf16": ("attention_mma", "pippppipiiiiiiiifpiippp", "attention_decode_bf16"),
+    "rllm_attention_decode_bf16_opts": ("attention_mma", "pippppipiiiiiiiifiifppiipiipfpppp", "attention_decode_bf16_opts"),
+    "rllm_attention_prefill_tcgen05": ("attention_tcgen05", "piippppippiiiiiiiiifp", "attention_prefill_tcgen05"),
+    "rllm_attention_prefill_tcgen05_opts": ("attention_tcgen05", "piippppippiiiiiiiiifiifppiipp", "attention_prefill_tcgen05_opts"),
+    "rllm_attention_prefill_bf16": ("attention_mma", "pippppippiiiiiiiiifp", "attention_prefill_bf16"),
+    "rllm_attention_prefill_bf16_opts": ("attention_mma", "pippppippiiiiiiiiifiifppiipp", "attention_prefill_bf16_opts"),
+    "rllm_logit_mask": ("sampling", "piiippipp", "logit_mask"),
+    "rllm_logit_edits": ("sampling", "piiippppppp", "logit_edits"),
+    "rllm_sample_one_cta": ("sampling", "piiippppppp", "sample_one_cta"),
+    "rllm_sample": ("sampling", "piiipppppppi", "sample"),
+    "rllm_argmax": ("sampling", "piiippp", "argmax"),
+    "rllm_gemm_tcgen05": ("gemm_tcgen05", "pipipiiiiifffp", "gemm_tcgen05"),
+    "rllm_gemm_small_m_rstd": ("gemm_small_m", "pipifpipiiiiifff", "gemm_small_m_rstd"),
+    "rllm_gemm_small_m_residual": ("gemm_small_m", "pipipippipippiii", "gemm_small_m_residual"),
+    "rllm_gemm_small_m": ("gemm_small_m", "pipipiiiiifff", "gemm_small_m"),
+    "rllm_gemm_f32": ("gemm_f32", "pipipiiii", "gemm_f32"),
+    "rllm_attention_simt": ("attention_simt", "pipppipippiiiiiiifp", "attention_simt"),
+    "rllm_silu_mul": ("elementwise", "ppiiifff", "silu_mul"),
+    "rllm_rope_kv_write": ("elementwise", "pipppipippiiiiiiip", "rope_kv_write"),
+    "rllm_residual_add": ("elementwise", "ppil", "residual_add"),
+    "rllm_rmsnorm": ("elementwise", "ppppipiiifi", "rmsnorm"),
+    "rllm_embedding": ("elementwise", "ppipiiifip", "embedding"),
+}
+
+
+class _Entries:
+    """An entry point as an attribute, made when it is first asked for (which compiles what is missing, its library with its
+    first call)."""
+
+    def __getattr__(self, symbol: str):
+        library, signature, what = _TABLE[symbol]
+
+        def find() -> int:
+            return ctypes.cast(getattr(build.load_library(library), symbol), c_void_p).value
+
+        entry = _launch().entry(signature, find, what)
+        setattr(self, symbol, entry)
+        return entry
+
+
+_entries = _Entries()
+_launch_module = None
+
+
+def _launch():
+    """The extension module that calls entry points."""
+    global _launch_module
+    if _launch_module is None:
+        module = native_build.load_extension("launch")
+        module.setup(KernelError, LAUNCHES)
+        _launch_module = module
+    return _launch_module
+
+
 def _contig(t: torch.Tensor, name: str) -> None:
     if not t.is_contiguous():
         raise KernelError(f"{name} must be contiguous")
@@ -65,14 +177,11 @@ def _contig(t: torch.Tensor, name: str) -> None:
 def embedding(ids: torch.Tensor, table: torch.Tensor, out: torch.Tensor, err: torch.Tensor,
               scale: float = 1.0) -> None:
     """out[t] = table[ids[t]] * scale as float32; ids int32 [T], out float32 [T, H], or [C, T, H]: C copies."""
-    lib = build.load_library("elementwise")
     T, (V, H) = ids.numel(), table.shape
     copies = out.shape[0] if out.dim() == 3 else 1
     assert ids.dtype is torch.int32 and out.dtype is torch.float32 and out.shape[-2:] == (T, H)
     _contig(table, "table"); _contig(out, "out")
-    _check(lib.rllm_embedding(_ptr(ids), _ptr(table), c_int(dtype_code(table.dtype)), _ptr(out),
-                              c_int(T), c_int(H), c_int(V), c_float(scale), c_int(copies), _ptr(err), _stream()),
-           "embedding")
+    _entries.rllm_embedding(ids, table, dtype_code(table.dtype), out, T, H, V, scale, copies, err)
 
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor,
@@ -81,7 +190,6 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor
     """out = rmsnorm(x [+ delta]) * weight; x float32 [., H]; out [R, H] in the
     activation dtype.  ``writeback`` stores x + delta into x.  ``rows`` (int32
     [R]) picks the input row of each output row."""
-    lib = build.load_library("elementwise")
     H = x.shape[-1]
     R = out.shape[0]
     assert x.dtype is torch.float32 and out.shape[-1] == H and weight.numel() == H
@@ -93,18 +201,14 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor
         assert rows.dtype is torch.int32 and rows.numel() == R
     else:
         assert x.shape[0] == R
-    _check(lib.rllm_rmsnorm(_ptr(x), _ptr(delta), _ptr(rows), _ptr(weight),
-                            c_int(dtype_code(weight.dtype)), _ptr(out), c_int(dtype_code(out.dtype)),
-                            c_int(R), c_int(H), c_float(eps), c_int(1 if writeback else 0), _stream()),
-           "rmsnorm")
+    _entries.rllm_rmsnorm(x, delta, rows, weight, dtype_code(weight.dtype), out, dtype_code(out.dtype), R, H, eps, 1 if
+                          writeback else 0)
 
 
 def residual_add(x: torch.Tensor, delta: torch.Tensor) -> None:
-    lib = build.load_library("elementwise")
     assert x.dtype is torch.float32 and x.shape == delta.shape
     _contig(x, "x"); _contig(delta, "delta")
-    _check(lib.rllm_residual_add(_ptr(x), _ptr(delta), c_int(dtype_code(delta.dtype)),
-                                 c_longlong(x.numel()), _stream()), "residual_add")
+    _entries.rllm_residual_add(x, delta, dtype_code(delta.dtype), x.numel())
 
 
 def rope_kv_write(qkv: torch.Tensor, positions: torch.Tensor, token_seq: torch.Tensor,
@@ -115,7 +219,6 @@ def rope_kv_write(qkv: torch.Tensor, positions: torch.Tensor, token_seq: torch.T
 
     qkv [T, (nq + 2 nkv) d]; caches [pages, nkv, page_size, d]; inv_freq float64
     [rotary_dim / 2]; block_table int32 [S, max_blocks]."""
-    lib = build.load_library("elementwise")
     T = qkv.shape[0]
     assert qkv.shape[1] == (nq + 2 * nkv) * d
     _contig(qkv, "qkv")
@@ -128,12 +231,8 @@ def rope_kv_write(qkv: torch.Tensor, positions: torch.Tensor, token_seq: torch.T
         pages, page_size, max_blocks = kcache.shape[0], kcache.shape[2], block_table.shape[1]
     else:
         pages = page_size = max_blocks = 0
-    _check(lib.rllm_rope_kv_write(_ptr(qkv), c_int(dtype_code(qkv.dtype)), _ptr(positions),
-                                  _ptr(token_seq), _ptr(inv_freq), c_int(rotary_dim),
-                                  _ptr(block_table), c_int(max_blocks), _ptr(kcache), _ptr(vcache),
-                                  c_int(T), c_int(nq), c_int(nkv), c_int(d), c_int(page_size),
-                                  c_int(pages), c_int(1 if write_kv else 0), _ptr(err), _stream()),
-           "rope_kv_write")
+    _entries.rllm_rope_kv_write(qkv, dtype_code(qkv.dtype), positions, token_seq, inv_freq, rotary_dim, block_table,
+                                max_blocks, kcache, vcache, T, nq, nkv, d, page_size, pages, 1 if write_kv else 0, err)
 
 
 PLAIN_GATE = (float("inf"), 1.0, 0.0)
@@ -148,12 +247,10 @@ def _gate_args(gate):
 
 def silu_mul(gate_up: torch.Tensor, out: torch.Tensor, gate=PLAIN_GATE) -> None:
     """out[t, i] = silu(gate_up[t, i]) * gate_up[t, I + i] (``gate``: other constants, see ``_gate_args``)."""
-    lib = build.load_library("elementwise")
     T, I = out.shape
     assert gate_up.shape == (T, 2 * I) and gate_up.dtype is out.dtype
     _contig(gate_up, "gate_up"); _contig(out, "out")
-    _check(lib.rllm_silu_mul(_ptr(gate_up), _ptr(out), c_int(dtype_code(out.dtype)), c_int(T), c_int(I),
-                             *_gate_args(gate), _stream()), "silu_mul")
+    _entries.rllm_silu_mul(gate_up, out, dtype_code(out.dtype), T, I, *gate)
 
 
 def attention_simt(q: torch.Tensor, q_stride: int, out: torch.Tensor, kcache: torch.Tensor,
@@ -163,28 +260,22 @@ def attention_simt(q: torch.Tensor, q_stride: int, out: torch.Tensor, kcache: to
     """Paged causal attention of T query tokens, one warp per (token, head).
 
     q: T rows of nq*d values with row stride q_stride (elements); out [T, nq*d]."""
-    lib = build.load_library("attention_simt")
     T = out.shape[0]
     _contig(out, "out"); _contig(kcache, "kcache"); _contig(vcache, "vcache"); _contig(block_table, "block_table")
     assert kcache.dtype is q.dtype and out.dtype is q.dtype
-    _check(lib.rllm_attention_simt(_ptr(q), c_int(q_stride), _ptr(out), _ptr(kcache), _ptr(vcache),
-                                   c_int(dtype_code(q.dtype)), _ptr(block_table),
-                                   c_int(block_table.shape[1]), _ptr(positions), _ptr(token_seq),
-                                   c_int(T), c_int(nq), c_int(nkv), c_int(d), c_int(kcache.shape[2]),
-                                   c_int(kcache.shape[0]), c_int(window), c_float(scale), _ptr(err),
-                                   _stream()), "attention_simt")
+    _entries.rllm_attention_simt(q, q_stride, out, kcache, vcache, dtype_code(q.dtype), block_table,
+                                 block_table.shape[1], positions, token_seq, T, nq, nkv, d, kcache.shape[2],
+                                 kcache.shape[0], window, scale, err)
 
 
 def gemm_f32(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     """out[M, N] = a[M, K] . w[N, K]^T, float32 FFMA."""
-    lib = build.load_library("gemm_f32")
     M, K = a.shape
     N = w.shape[0]
     assert a.dtype is torch.float32 and w.dtype is torch.float32 and out.dtype is torch.float32
     assert w.shape[1] == K and out.shape == (M, N)
     assert a.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
-    _check(lib.rllm_gemm_f32(_ptr(a), c_int(a.stride(0)), _ptr(w), c_int(w.stride(0)), _ptr(out),
-                             c_int(out.stride(0)), c_int(M), c_int(N), c_int(K), _stream()), "gemm_f32")
+    _entries.rllm_gemm_f32(a, a.stride(0), w, w.stride(0), out, out.stride(0), M, N, K)
 
 
 SMALL_M_MAX = 8       # up to here the weight-streaming GEMM beats the library's on a B200 (it takes 16)
@@ -199,7 +290,6 @@ def gemm_small_m(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: 
     """out = x . w^T for M <= 16 rows of bfloat16, bound by one read of w.
     epilogue "store": out [M, N] bfloat16 or float32.  "silu_mul": w = [gate rows;
     up rows] stacked (2 N rows), out [M, N] bfloat16 = silu(x gate^T) * (x up^T)."""
-    lib = build.load_library("gemm_small_m")
     M, K = x.shape
     assert x.dtype is torch.bfloat16 and w.dtype is torch.bfloat16 and w.shape[1] == K
     assert x.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
@@ -212,9 +302,7 @@ def gemm_small_m(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: 
         assert out.shape == (M, N)
         code = 1 if out.dtype is torch.float32 else 0
         assert out.dtype in (torch.float32, torch.bfloat16)
-    _check(lib.rllm_gemm_small_m(_ptr(x), c_int(x.stride(0)), _ptr(w), c_int(w.stride(0)), _ptr(out),
-                                 c_int(out.stride(0)), c_int(M), c_int(N), c_int(K), c_int(code), *_gate_args(gate),
-                                 _stream()), "gemm_small_m")
+    _entries.rllm_gemm_small_m(x, x.stride(0), w, w.stride(0), out, out.stride(0), M, N, K, code, *gate)
 
 
 def gemm_small_m_residual(x: torch.Tensor, w: torch.Tensor, h: torch.Tensor,
@@ -239,12 +327,9 @@ def gemm_small_m_residual(x: torch.Tensor, w: torch.Tensor, h: torch.Tensor,
     if w_next is not None:
         assert w_next.numel() == N and w_next.is_contiguous() and w_next.dtype in (torch.float32, torch.bfloat16)
         scaled = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
-    _check(lib.rllm_gemm_small_m_residual(_ptr(x), c_int(x.stride(0)), _ptr(w), c_int(w.stride(0)), _ptr(h),
-                                          c_int(h.stride(0)), _ptr(parts), _ptr(w_next),
-                                          c_int(1 if w_next is not None and w_next.dtype is torch.float32 else 0),
-                                          _ptr(scaled), c_int(N), _ptr(alpha), _ptr(shift), c_int(M), c_int(N), c_int(K),
-                                          _stream()),
-           "gemm_small_m_residual")
+    _entries.rllm_gemm_small_m_residual(x, x.stride(0), w, w.stride(0), h, h.stride(0), parts, w_next, 1 if w_next is
+                                        not None and w_next.dtype is torch.float32 else 0, scaled, N, alpha, shift, M,
+                                        N, K)
     return parts, scaled
 
 
@@ -253,7 +338,6 @@ def gemm_small_m_rstd(x: torch.Tensor, parts: torch.Tensor, eps: float, w: torch
     """out = (x . w^T) with row m scaled by 1 / sqrt(sum(parts[:, m]) / K + eps): with
     x and parts from ``gemm_small_m_residual`` this is rmsnorm(h) . w^T.  Epilogues
     as in ``gemm_small_m`` (bfloat16 out)."""
-    lib = build.load_library("gemm_small_m")
     M, K = x.shape
     assert x.dtype is torch.bfloat16 and w.dtype is torch.bfloat16 and w.shape[1] == K and out.dtype is torch.bfloat16
     assert parts.dtype is torch.float32 and parts.is_contiguous() and parts.shape[1] == M
@@ -264,9 +348,8 @@ def gemm_small_m_rstd(x: torch.Tensor, parts: torch.Tensor, eps: float, w: torch
     else:
         N, code = w.shape[0], 0
     assert out.shape == (M, N)
-    _check(lib.rllm_gemm_small_m_rstd(_ptr(x), c_int(x.stride(0)), _ptr(parts), c_int(parts.shape[0]), c_float(eps),
-                                      _ptr(w), c_int(w.stride(0)), _ptr(out), c_int(out.stride(0)), c_int(M),
-                                      c_int(N), c_int(K), c_int(code), *_gate_args(gate), _stream()), "gemm_small_m_rstd")
+    _entries.rllm_gemm_small_m_rstd(x, x.stride(0), parts, parts.shape[0], eps, w, w.stride(0), out, out.stride(0), M,
+                                    N, K, code, *gate)
 
 
 _one_wave_tiles = {}
@@ -305,7 +388,24 @@ def gemm_error_word(device: torch.device) -> torch.Tensor:
     t = _gemm_err.get(device)
     if t is None:
         t = _gemm_err[device] = torch.zeros(1, dtype=torch.int32, device=device)
+        if t.is_cuda:
+            _launch().error_word(t.get_device(), t)
     return t
+
+
+_product = None
+
+
+def product(x: torch.Tensor, w: torch.Tensor, out_f32: bool = False, silu: bool = False, gate=PLAIN_GATE) -> Optional[torch.Tensor]:
+    """x . w^T on the bfloat16 kernels where the call is a plain one that ``small_m_takes`` or ``tcgen05_takes`` let through
+    (checked, allocated and launched by the extension module in one go), else None: the caller's own way, which refuses what
+    has to be refused.  ``silu``: silu(x gate^T) * (x up^T) of w = [gate rows; up rows]."""
+    global _product
+    if _product is None:
+        module = _launch()
+        module.products(_entries.rllm_gemm_small_m, _entries.rllm_gemm_tcgen05, SMALL_M_MAX, TCGEN05_MIN_TILES)
+        _product = module.product
+    return _product(x, w, out_f32, silu, *gate)
 
 
 def check_gemm_errors(device: torch.device) -> None:
@@ -324,7 +424,6 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: 
     """out = x . w^T for bfloat16 on the tcgen05 tensor cores (TMA in, TMEM accumulators).
     epilogue "store": out [M, N] bfloat16 or float32.  "silu_mul": w = [gate rows;
     up rows] stacked (2 N rows), out [M, N] bfloat16 = silu(x gate^T) * (x up^T)."""
-    lib = build.load_library("gemm_tcgen05")
     M, K = x.shape
     assert x.dtype is torch.bfloat16 and w.dtype is torch.bfloat16 and w.shape[1] == K
     assert x.stride(1) == 1 and w.stride(1) == 1 and out.stride(1) == 1
@@ -336,9 +435,8 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: 
         N = w.shape[0]
         assert out.shape == (M, N) and out.dtype in (torch.float32, torch.bfloat16)
         code = 1 if out.dtype is torch.float32 else 0
-    _check(lib.rllm_gemm_tcgen05(_ptr(x), c_int(x.stride(0)), _ptr(w), c_int(w.stride(0)), _ptr(out),
-                                 c_int(out.stride(0)), c_int(M), c_int(N), c_int(K), c_int(code), *_gate_args(gate),
-                                 _ptr(gemm_error_word(x.device)), _stream()), "gemm_tcgen05")
+    _entries.rllm_gemm_tcgen05(x, x.stride(0), w, w.stride(0), out, out.stride(0), M, N, K, code, *gate,
+                               gemm_error_word(x.device))
 
 
 TCGEN05_MIN_TILES = 96    # below this many 128 x 256 output tiles the GPU is not filled: the library's
@@ -415,8 +513,7 @@ def argmax(logits: torch.Tensor, out: torch.Tensor) -> None:
         scratch = (torch.empty(rows * 64 * 2, dtype=torch.int32, device=logits.device),
                    torch.zeros(rows, dtype=torch.int32, device=logits.device))
         _argmax_scratch[logits.device] = scratch
-    _check(lib.rllm_argmax(_ptr(logits), c_int(R), c_int(V), c_int(logits.stride(0)), _ptr(out),
-                           _ptr(scratch[0]), _ptr(scratch[1]), _stream()), "argmax")
+    _entries.rllm_argmax(logits, R, V, logits.stride(0), out, scratch[0], scratch[1])
 
 
 def _sample_asserts(logits, temperature, top_k, top_p, min_p, seeds, gen_index, out):
@@ -432,44 +529,34 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
     """out[r] = the next token of row r: argmax for greedy rows, else a draw after temperature, top-k,
     top-p and min-p.  A cluster of CTAs works on every row.
     ``with_select=False`` leaves top-k and top-p out (the caller knows that no row uses them)."""
-    lib = build.load_library("sampling")
     R, V = logits.shape
     _sample_asserts(logits, temperature, top_k, top_p, min_p, seeds, gen_index, out)
-    _check(lib.rllm_sample(_ptr(logits), c_int(R), c_int(V), c_int(logits.stride(0)), _ptr(temperature),
-                           _ptr(top_k), _ptr(top_p), _ptr(min_p), _ptr(seeds), _ptr(gen_index), _ptr(out),
-                           c_int(1 if with_select else 0), _stream()), "sample")
+    _entries.rllm_sample(logits, R, V, logits.stride(0), temperature, top_k, top_p, min_p, seeds, gen_index, out, 1 if
+                         with_select else 0)
 
 
 def sample_one_cta(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor, top_p: torch.Tensor,
                    min_p: torch.Tensor, seeds: torch.Tensor, gen_index: torch.Tensor, out: torch.Tensor) -> None:
     """The same sampling with one CTA a row in one kernel (slow for large vocabularies; kept as the
     simple form that the clusters are checked against)."""
-    lib = build.load_library("sampling")
     R, V = logits.shape
     _sample_asserts(logits, temperature, top_k, top_p, min_p, seeds, gen_index, out)
-    _check(lib.rllm_sample_one_cta(_ptr(logits), c_int(R), c_int(V), c_int(logits.stride(0)), _ptr(temperature),
-                                   _ptr(top_k), _ptr(top_p), _ptr(min_p), _ptr(seeds), _ptr(gen_index),
-                                   _ptr(out), _stream()), "sample_one_cta")
+    _entries.rllm_sample_one_cta(logits, R, V, logits.stride(0), temperature, top_k, top_p, min_p, seeds, gen_index,
+                                 out)
 
 
 def logit_edits(logits: torch.Tensor, rows: torch.Tensor, tokens: torch.Tensor, counts: torch.Tensor,
                 bias: torch.Tensor, rep: torch.Tensor, freq: torch.Tensor, pres: torch.Tensor) -> None:
-    lib = build.load_library("sampling")
     R, V = logits.shape
-    _check(lib.rllm_logit_edits(_ptr(logits), c_int(V), c_int(logits.stride(0)), c_int(rows.numel()),
-                                _ptr(rows), _ptr(tokens), _ptr(counts), _ptr(bias), _ptr(rep),
-                                _ptr(freq), _ptr(pres), _stream()), "logit_edits")
+    _entries.rllm_logit_edits(logits, V, logits.stride(0), rows.numel(), rows, tokens, counts, bias, rep, freq, pres)
 
 
 def logit_mask(logits: torch.Tensor, allowed_start: Optional[torch.Tensor],
                allowed: Optional[torch.Tensor], sup_rows: Optional[torch.Tensor],
                sup_tokens: Optional[torch.Tensor]) -> None:
-    lib = build.load_library("sampling")
     R, V = logits.shape
     n = 0 if sup_rows is None else sup_rows.numel()
-    _check(lib.rllm_logit_mask(_ptr(logits), c_int(R), c_int(V), c_int(logits.stride(0)),
-                               _ptr(allowed_start), _ptr(allowed), c_int(n), _ptr(sup_rows),
-                               _ptr(sup_tokens), _stream()), "logit_mask")
+    _entries.rllm_logit_mask(logits, R, V, logits.stride(0), allowed_start, allowed, n, sup_rows, sup_tokens)
 
 
 def attention_prefill_bf16(q: torch.Tensor, q_stride: int, out: torch.Tensor, kcache: torch.Tensor,
@@ -481,25 +568,19 @@ def attention_prefill_bf16(q: torch.Tensor, q_stride: int, out: torch.Tensor, kc
                            slopes: Optional[torch.Tensor] = None) -> None:
     """Tensor-core attention of the prompt portions of sequences seq_begin .. seq_end-1.  ``keep_first``,
     ``chunk``, ``softcap``, ``sinks``, ``gate`` and ``slopes`` as in ``attention_simt_kv`` (gate: a row per row of q)."""
-    lib = build.load_library("attention_mma")
     _contig(out, "out"); _contig(kcache, "kcache"); _contig(vcache, "vcache"); _contig(block_table, "block_table")
     assert q.dtype is torch.bfloat16 and kcache.dtype is torch.bfloat16 and out.dtype is torch.bfloat16
     if keep_first or chunk or softcap or sinks is not None or gate is not None or slopes is not None:
         gate_mode = _attention_opts_asserts(sinks, gate, gate_per_head, nq, d, slopes)
-        _check(lib.rllm_attention_prefill_bf16_opts(
-            _ptr(q), c_int(q_stride), _ptr(out), _ptr(kcache), _ptr(vcache), _ptr(block_table),
-            c_int(block_table.shape[1]), _ptr(q_start), _ptr(seq_lens), c_int(seq_begin), c_int(seq_end),
-            c_int(num_tokens), c_int(nq), c_int(nkv), c_int(d), c_int(kcache.shape[2]), c_int(kcache.shape[0]),
-            c_int(window), c_float(scale), c_int(keep_first), c_int(chunk), c_float(softcap), _ptr(sinks), _ptr(gate),
-            c_int(gate.stride(0) if gate is not None else 0), c_int(gate_mode), _ptr(slopes), _ptr(err), _stream()),
-            "attention_prefill_bf16_opts")
+        _entries.rllm_attention_prefill_bf16_opts(q, q_stride, out, kcache, vcache, block_table, block_table.shape[1],
+                                                  q_start, seq_lens, seq_begin, seq_end, num_tokens, nq, nkv, d,
+                                                  kcache.shape[2], kcache.shape[0], window, scale, keep_first, chunk,
+                                                  softcap, sinks, gate, gate.stride(0) if gate is not None else 0,
+                                                  gate_mode, slopes, err)
         return
-    _check(lib.rllm_attention_prefill_bf16(_ptr(q), c_int(q_stride), _ptr(out), _ptr(kcache), _ptr(vcache),
-                                           _ptr(block_table), c_int(block_table.shape[1]), _ptr(q_start),
-                                           _ptr(seq_lens), c_int(seq_begin), c_int(seq_end), c_int(num_tokens),
-                                           c_int(nq), c_int(nkv), c_int(d), c_int(kcache.shape[2]),
-                                           c_int(kcache.shape[0]), c_int(window), c_float(scale), _ptr(err),
-                                           _stream()), "attention_prefill_bf16")
+    _entries.rllm_attention_prefill_bf16(q, q_stride, out, kcache, vcache, block_table, block_table.shape[1], q_start,
+                                         seq_lens, seq_begin, seq_end, num_tokens, nq, nkv, d, kcache.shape[2],
+                                         kcache.shape[0], window, scale, err)
 
 
 def attention_prefill_tcgen05_supported(nq: int, nkv: int, d: int, page_size: int) -> bool:
@@ -520,25 +601,19 @@ def attention_prefill_tcgen05(q: torch.Tensor, q_stride: int, out: torch.Tensor,
     """Attention of the prompt portions of sequences seq_begin .. seq_end-1 on the
     tcgen05 tensor cores (same contract and options as ``attention_prefill_bf16``; ``q`` is the
     first of ``q.shape[0]`` rows of ``q_stride`` elements)."""
-    lib = build.load_library("attention_tcgen05")
     _contig(out, "out"); _contig(kcache, "kcache"); _contig(vcache, "vcache"); _contig(block_table, "block_table")
     assert q.dtype is torch.bfloat16 and kcache.dtype is torch.bfloat16 and out.dtype is torch.bfloat16
     if keep_first or chunk or softcap or sinks is not None or gate is not None or slopes is not None:
         gate_mode = _attention_opts_asserts(sinks, gate, gate_per_head, nq, d, slopes)
-        _check(lib.rllm_attention_prefill_tcgen05_opts(
-            _ptr(q), c_int(q_stride), c_int(q.shape[0]), _ptr(out), _ptr(kcache), _ptr(vcache), _ptr(block_table),
-            c_int(block_table.shape[1]), _ptr(q_start), _ptr(seq_lens), c_int(seq_begin), c_int(seq_end),
-            c_int(num_tokens), c_int(nq), c_int(nkv), c_int(d), c_int(kcache.shape[2]), c_int(kcache.shape[0]),
-            c_int(window), c_float(scale), c_int(keep_first), c_int(chunk), c_float(softcap), _ptr(sinks), _ptr(gate),
-            c_int(gate.stride(0) if gate is not None else 0), c_int(gate_mode), _ptr(slopes), _ptr(err), _stream()),
-            "attention_prefill_tcgen05_opts")
+        _entries.rllm_attention_prefill_tcgen05_opts(q, q_stride, q.shape[0], out, kcache, vcache, block_table,
+                                                     block_table.shape[1], q_start, seq_lens, seq_begin, seq_end,
+                                                     num_tokens, nq, nkv, d, kcache.shape[2], kcache.shape[0], window,
+                                                     scale, keep_first, chunk, softcap, sinks, gate, gate.stride(0) if
+                                                     gate is not None else 0, gate_mode, slopes, err)
         return
-    _check(lib.rllm_attention_prefill_tcgen05(_ptr(q), c_int(q_stride), c_int(q.shape[0]), _ptr(out), _ptr(kcache),
-                                              _ptr(vcache), _ptr(block_table), c_int(block_table.shape[1]),
-                                              _ptr(q_start), _ptr(seq_lens), c_int(seq_begin), c_int(seq_end),
-                                              c_int(num_tokens), c_int(nq), c_int(nkv), c_int(d),
-                                              c_int(kcache.shape[2]), c_int(kcache.shape[0]), c_int(window),
-                                              c_float(scale), _ptr(err), _stream()), "attention_prefill_tcgen05")
+    _entries.rllm_attention_prefill_tcgen05(q, q_stride, q.shape[0], out, kcache, vcache, block_table,
+                                            block_table.shape[1], q_start, seq_lens, seq_begin, seq_end, num_tokens, nq,
+                                            nkv, d, kcache.shape[2], kcache.shape[0], window, scale, err)
 
 
 _decode_counters = {}
@@ -593,7 +668,6 @@ def attention_decode_bf16(qkv: torch.Tensor, q_stride: int, out: torch.Tensor, k
     ``gate`` as in ``attention_simt_kv`` (gate: a row per sequence).  With any of them, and the rotation and
     cache write in the kernel, ``bias`` (float32 over a row's q, k and v heads) is added first and cosine and sine
     are multiplied by ``magnitude``, as ``head_norm_kv_write`` does for prompt portions."""
-    lib = build.load_library("attention_mma")
     _contig(out, "out"); _contig(kcache, "kcache"); _contig(vcache, "vcache"); _contig(block_table, "block_table")
     assert qkv.dtype is torch.bfloat16 and kcache.dtype is torch.bfloat16 and out.dtype is torch.bfloat16
     need = attention_decode_workspace(num_seqs, nq, d, max_seq_len)
@@ -608,22 +682,16 @@ def attention_decode_bf16(qkv: torch.Tensor, q_stride: int, out: torch.Tensor, k
         gate_mode = _attention_opts_asserts(sinks, gate, gate_per_head, nq, d, slopes)
         if bias is not None:
             assert write_kv and bias.dtype is torch.float32 and bias.is_contiguous() and bias.numel() == (nq + 2 * nkv) * d
-        _check(lib.rllm_attention_decode_bf16_opts(
-            _ptr(qkv), c_int(q_stride), _ptr(out), _ptr(kcache), _ptr(vcache), _ptr(block_table),
-            c_int(block_table.shape[1]), _ptr(seq_lens), c_int(num_seqs), c_int(max_seq_len), c_int(nq), c_int(nkv),
-            c_int(d), c_int(kcache.shape[2]), c_int(kcache.shape[0]), c_int(window), c_float(scale), c_int(keep_first),
-            c_int(chunk), c_float(softcap), _ptr(sinks), _ptr(gate), c_int(gate.stride(0) if gate is not None else 0),
-            c_int(gate_mode), _ptr(inv_freq if rotary_dim else None), c_int(rotary_dim), c_int(1 if write_kv else 0),
-            _ptr(bias), c_float(magnitude), _ptr(slopes), _ptr(workspace), _ptr(counters), _ptr(err), _stream()),
-            "attention_decode_bf16_opts")
+        _entries.rllm_attention_decode_bf16_opts(qkv, q_stride, out, kcache, vcache, block_table, block_table.shape[1],
+                                                 seq_lens, num_seqs, max_seq_len, nq, nkv, d, kcache.shape[2],
+                                                 kcache.shape[0], window, scale, keep_first, chunk, softcap, sinks,
+                                                 gate, gate.stride(0) if gate is not None else 0, gate_mode, inv_freq if
+                                                 rotary_dim else None, rotary_dim, 1 if write_kv else 0, bias,
+                                                 magnitude, slopes, workspace, counters, err)
         return
-    _check(lib.rllm_attention_decode_bf16(_ptr(qkv), c_int(q_stride), _ptr(out), _ptr(kcache), _ptr(vcache),
-                                          _ptr(block_table), c_int(block_table.shape[1]), _ptr(seq_lens),
-                                          c_int(num_seqs), c_int(max_seq_len), c_int(nq), c_int(nkv), c_int(d),
-                                          c_int(kcache.shape[2]), c_int(kcache.shape[0]), c_int(window),
-                                          c_float(scale), _ptr(inv_freq), c_int(rotary_dim),
-                                          c_int(1 if write_kv else 0), _ptr(workspace), _ptr(counters),
-                                          _ptr(err), _stream()), "attention_decode_bf16")
+    _entries.rllm_attention_decode_bf16(qkv, q_stride, out, kcache, vcache, block_table, block_table.shape[1], seq_lens,
+                                        num_seqs, max_seq_len, nq, nkv, d, kcache.shape[2], kcache.shape[0], window,
+                                        scale, inv_freq, rotary_dim, 1 if write_kv else 0, workspace, counters, err)
 
 
 def attention_decode_workspace(num_seqs: int, nq: int, d: int, max_seq_len: int) -> int:
@@ -699,7 +767,6 @@ def gated_postnorm_add(x_in: torch.Tensor, x_out: torch.Tensor, y: torch.Tensor,
     ``depth`` = (history float32 [L, T, H] whose level ``levels - 1`` is ``x_out``, levels, coeff [levels],
     stream_out float32 [T, H]): the depth average sum_j coeff[j] history[j] is written to ``stream_out`` in the
     same kernel, and the returned norm is the norm of that sum."""
-    lib = build.load_library("layer_glue")
     T, H = x_in.shape
     hist = coeff = stream_out = None
     level_stride = levels = 0
@@ -726,12 +793,10 @@ def gated_postnorm_add(x_in: torch.Tensor, x_out: torch.Tensor, y: torch.Tensor,
     if next_weight is not None:
         assert next_weight.dtype is norm_weight.dtype and next_weight.numel() == H
         nxt = torch.empty((T, H), dtype=y.dtype, device=y.device)
-    _check(lib.rllm_gated_postnorm_add(_ptr(x_in), _ptr(x_out), _ptr(y), c_int(slots), _ptr(slot_weights),
-                                       _ptr(gate), c_int(g_stride), _ptr(gate_bias if gate is not None else None), _ptr(norm_weight), c_float(eps), _ptr(next_weight),
-                                       _ptr(nxt), c_float(next_eps), _ptr(hist), c_longlong(level_stride),
-                                       c_int(levels), _ptr(coeff), _ptr(stream_out), c_int(T), c_int(H),
-                                       c_int(dtype_code(y.dtype)), c_int(dtype_code(norm_weight.dtype)),
-                                       _stream()), "gated_postnorm_add")
+    _entries.rllm_gated_postnorm_add(x_in, x_out, y, slots, slot_weights, gate, g_stride, gate_bias if gate is not None
+                                     else None, norm_weight, eps, next_weight, nxt, next_eps, hist, level_stride,
+                                     levels, coeff, stream_out, T, H, dtype_code(y.dtype),
+                                     dtype_code(norm_weight.dtype))
     return nxt
 
 
@@ -740,7 +805,6 @@ def postnorm_add(x: torch.Tensor, y, weight: torch.Tensor, eps: float, multiplie
     """x += multiplier * rmsnorm(y) * weight in place (x float32 [T, H]; y [T, H] in the activation dtype, or a
     ``WeightedSum`` of two such terms, added up in float32 before the norm).  Returns the new x in the activation
     dtype (x itself for float32)."""
-    lib = build.load_library("layer_glue")
     terms, scales = ((y,), (1.0, 0.0)) if isinstance(y, torch.Tensor) else (tuple(y.terms), tuple(y.scales))
     T, H = x.shape
     assert x.dtype is torch.float32 and weight.numel() == H
@@ -749,10 +813,8 @@ def postnorm_add(x: torch.Tensor, y, weight: torch.Tensor, eps: float, multiplie
         assert t.shape == (T, H) and t.dtype is act_dtype
         _contig(t, "y")
     out = None if act_dtype is torch.float32 else torch.empty((T, H), dtype=act_dtype, device=x.device)
-    _check(lib.rllm_postnorm_add(_ptr(x), _ptr(terms[0]), _ptr(terms[1] if len(terms) > 1 else None),
-                                 c_float(scales[0]), c_float(scales[1]), _ptr(weight), c_float(eps),
-                                 c_float(multiplier), _ptr(out), c_int(T), c_int(H), c_int(dtype_code(act_dtype)),
-                                 c_int(dtype_code(weight.dtype)), _stream()), "postnorm_add")
+    _entries.rllm_postnorm_add(x, terms[0], terms[1] if len(terms) > 1 else None, scales[0], scales[1], weight, eps,
+                               multiplier, out, T, H, dtype_code(act_dtype), dtype_code(weight.dtype))
     return x if out is None else out
 
 
@@ -761,21 +823,18 @@ def activation_rows(x: torch.Tensor, act_dtype: torch.dtype) -> torch.Tensor:
     assert x.dtype is torch.float32
     if act_dtype is torch.float32:
         return x
-    lib = build.load_library("layer_glue")
     _contig(x, "x")
     out = torch.empty(x.shape, dtype=act_dtype, device=x.device)
-    _check(lib.rllm_activation_rows(_ptr(x), _ptr(out), c_longlong(x.numel()), _stream()), "activation_rows")
+    _entries.rllm_activation_rows(x, out, x.numel())
     return out
 
 
 def scaled_sum2(a: torch.Tensor, b: torch.Tensor, scale_a: float, scale_b: float) -> torch.Tensor:
     """scale_a * a + scale_b * b, added in float32."""
-    lib = build.load_library("layer_glue")
     assert a.shape == b.shape and a.dtype is b.dtype
     _contig(a, "a"); _contig(b, "b")
     out = torch.empty_like(a)
-    _check(lib.rllm_scaled_sum2(_ptr(a), _ptr(b), c_float(scale_a), c_float(scale_b), _ptr(out),
-                                c_int(dtype_code(a.dtype)), c_longlong(a.numel()), _stream()), "scaled_sum2")
+    _entries.rllm_scaled_sum2(a, b, scale_a, scale_b, out, dtype_code(a.dtype), a.numel())
     return out
 
 
@@ -785,7 +844,6 @@ def depth_average(history: torch.Tensor, levels: int, coeff: torch.Tensor, strea
     """s = sum_j coeff[j] * history[j] over the first ``levels`` levels; history float32 [L, T, H].
     Writes s to ``stream_out`` (float32 [T, H]) if given and returns rmsnorm(s) * norm_weight in
     ``act_dtype`` if a weight is given.  ``rows`` (int32 [R]): only these rows (no ``stream_out`` then)."""
-    lib = build.load_library("layer_glue")
     L, T, H = history.shape
     assert history.dtype is torch.float32 and 1 <= levels <= L and coeff.numel() == levels
     _contig(history, "history"); _contig(coeff, "coeff")
@@ -799,10 +857,8 @@ def depth_average(history: torch.Tensor, levels: int, coeff: torch.Tensor, strea
     if norm_weight is not None:
         assert norm_weight.dtype is coeff.dtype and norm_weight.numel() == H
         out = torch.empty((R, H), dtype=act_dtype, device=history.device)
-    _check(lib.rllm_depth_average(_ptr(history), c_longlong(history.stride(0)), c_int(levels), _ptr(coeff),
-                                  _ptr(rows), _ptr(stream_out), _ptr(norm_weight), _ptr(out), c_float(eps),
-                                  c_int(R), c_int(H), c_int(dtype_code(act_dtype)),
-                                  c_int(dtype_code(coeff.dtype)), _stream()), "depth_average")
+    _entries.rllm_depth_average(history, history.stride(0), levels, coeff, rows, stream_out, norm_weight, out, eps, R,
+                                H, dtype_code(act_dtype), dtype_code(coeff.dtype))
     return out
 
 
@@ -818,7 +874,6 @@ def mingru_scan(zxg: torch.Tensor, bias_z: torch.Tensor, bias_x: torch.Tensor, s
     """zxg [T, >= 3 W]: a token's z, x and g projections side by side; state float32 [slots, W], updated in
     place for the sequences' slots; out [T, W] = S_t * silu(g).  ``max_q_len``: the most tokens a sequence
     brings; long portions are scanned in chunks of 64 that run side by side."""
-    lib = build.load_library("mingru")
     T, W = out.shape
     if max_q_len >= MINGRU_CHUNKED_FROM and num_seqs * -(-max_q_len // 64) <= 65535:
         assert zxg.shape[0] == T and zxg.stride(1) == 1 and zxg.shape[1] >= 3 * W and out.dtype is zxg.dtype
@@ -826,20 +881,16 @@ def mingru_scan(zxg: torch.Tensor, bias_z: torch.Tensor, bias_x: torch.Tensor, s
         _contig(out, "out"); _contig(state, "state")
         chunks = -(-max_q_len // 64)
         work = torch.empty(num_seqs * chunks * 2 * W + num_seqs * W, dtype=torch.float32, device=out.device)
-        _check(lib.rllm_mingru_scan_chunked(_ptr(zxg), c_int(zxg.stride(0)), _ptr(bias_z), _ptr(bias_x), _ptr(state),
-                                            _ptr(q_start), _ptr(slots), c_int(state.shape[0]), _ptr(out),
-                                            c_int(num_seqs), c_int(W), c_int(max_q_len), _ptr(work),
-                                            c_int(dtype_code(out.dtype)), c_int(dtype_code(bias_z.dtype)),
-                                            _ptr(err), _stream()), "mingru_scan_chunked")
+        _entries.rllm_mingru_scan_chunked(zxg, zxg.stride(0), bias_z, bias_x, state, q_start, slots, state.shape[0],
+                                          out, num_seqs, W, max_q_len, work, dtype_code(out.dtype),
+                                          dtype_code(bias_z.dtype), err)
         return
     assert zxg.shape[0] == T and zxg.stride(1) == 1 and zxg.shape[1] >= 3 * W and out.dtype is zxg.dtype
     assert state.dtype is torch.float32 and state.shape[1] == W
     assert bias_z.dtype is bias_x.dtype and bias_z.numel() == W and bias_x.numel() == W
     _contig(out, "out"); _contig(state, "state")
-    _check(lib.rllm_mingru_scan(_ptr(zxg), c_int(zxg.stride(0)), _ptr(bias_z), _ptr(bias_x), _ptr(state),
-                                _ptr(q_start), _ptr(slots), c_int(state.shape[0]), _ptr(out), c_int(num_seqs),
-                                c_int(W), c_int(dtype_code(out.dtype)), c_int(dtype_code(bias_z.dtype)),
-                                _ptr(err), _stream()), "mingru_scan")
+    _entries.rllm_mingru_scan(zxg, zxg.stride(0), bias_z, bias_x, state, q_start, slots, state.shape[0], out, num_seqs,
+                              W, dtype_code(out.dtype), dtype_code(bias_z.dtype), err)
 
 
 # ---------------------------------------------------------------------------
@@ -853,7 +904,6 @@ def latent_prep(a: torch.Tensor, q_rank: int, kv_rank: int, rot: int, rot_dims: 
     rmsnorm(a[:, :q_rank]) * wq.  With a cache ([pages, 1, page_size, kv_rank + rot]) the token's row is
     written: rmsnorm of the next kv_rank values times wkv, then the last rot values, the first rot_dims
     of them rotated by position (pairs 2i, 2i+1), cosine and sine times ``magnitude``."""
-    lib = build.load_library("latent_attention")
     T = a.shape[0]
     write = cache is not None
     assert a.stride(1) == 1 and cq.shape == (T, q_rank) and cq.dtype is a.dtype
@@ -867,27 +917,20 @@ def latent_prep(a: torch.Tensor, q_rank: int, kv_rank: int, rot: int, rot_dims: 
         pages, page_size, max_blocks = cache.shape[0], cache.shape[2], block_table.shape[1]
     else:
         pages = page_size = max_blocks = 0
-    _check(lib.rllm_latent_prep(_ptr(a), c_int(a.stride(0)), c_int(q_rank), c_int(kv_rank), c_int(rot),
-                                c_int(rot_dims), _ptr(wq), _ptr(wkv), c_float(eps), _ptr(cq), _ptr(cache),
-                                _ptr(block_table), c_int(max_blocks), _ptr(positions), _ptr(token_seq),
-                                _ptr(inv_freq), c_float(magnitude), c_int(page_size), c_int(pages),
-                                c_int(1 if write else 0),
-                                c_int(T), c_int(dtype_code(a.dtype)), c_int(dtype_code(wq.dtype)), _ptr(err),
-                                _stream()), "latent_prep")
+    _entries.rllm_latent_prep(a, a.stride(0), q_rank, kv_rank, rot, rot_dims, wq, wkv, eps, cq, cache, block_table,
+                              max_blocks, positions, token_seq, inv_freq, magnitude, page_size, pages, 1 if write else
+                              0, T, dtype_code(a.dtype), dtype_code(wq.dtype), err)
 
 
 def latent_q_rot(q: torch.Tensor, qt: torch.Tensor, positions: torch.Tensor, inv_freq: Optional[torch.Tensor],
                  heads: int, dim: int, rot: int, rot_dims: int, kv_rank: int, magnitude: float = 1.0) -> None:
     """qt[t, h, kv_rank:] = q[t, h, dim:] with its first rot_dims values rotated by position (cosine and sine
     times ``magnitude``)."""
-    lib = build.load_library("latent_attention")
     T = q.shape[0]
     assert q.shape == (T, heads * (dim + rot)) and qt.shape == (T, heads * (kv_rank + rot)) and qt.dtype is q.dtype
     _contig(q, "q"); _contig(qt, "qt")
-    _check(lib.rllm_latent_q_rot(_ptr(q), _ptr(qt), _ptr(positions), _ptr(inv_freq), c_float(magnitude), c_int(T),
-                                 c_int(heads),
-                                 c_int(dim), c_int(rot), c_int(rot_dims), c_int(kv_rank),
-                                 c_int(dtype_code(q.dtype)), _stream()), "latent_q_rot")
+    _entries.rllm_latent_q_rot(q, qt, positions, inv_freq, magnitude, T, heads, dim, rot, rot_dims, kv_rank,
+                               dtype_code(q.dtype))
 
 
 # results from which the products per head run on the tcgen05 kernel.  16 heads: 2,048 rows x 512 of 128 61 -> 21 us,
@@ -911,23 +954,17 @@ def head_gemm_tcgen05_takes(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor) -
 def head_gemm(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, b_kn: bool) -> None:
     """c[m, h, :] = a[m, h, :] . b[h] for every head h.  a [M, heads, K], c [M, heads, N]: views with unit
     stride in the last dim; b [heads, K, N] (``b_kn``) or [heads, N, K], contiguous."""
-    lib = build.load_library("latent_attention")
     M, heads, K = a.shape
     N = c.shape[2]
     assert c.shape[:2] == (M, heads) and a.stride(2) == 1 and c.stride(2) == 1 and a.dtype is b.dtype is c.dtype
     assert b.shape == ((heads, K, N) if b_kn else (heads, N, K))
     _contig(b, "b")
     if M * heads * N >= HEAD_GEMM_TCGEN05_FROM and not b_kn and head_gemm_tcgen05_takes(a, b, c):
-        lib = build.load_library("gemm_tcgen05")
-        _check(lib.rllm_head_gemm_tcgen05(
-            _ptr(a), c_longlong(a.stride(0)), c_longlong(a.stride(1)), _ptr(b), c_longlong(b.stride(1)),
-            c_longlong(b.stride(0)), _ptr(c), c_int(c.stride(0)), c_longlong(c.stride(1)), c_int(M), c_int(N), c_int(K),
-            c_int(heads), _ptr(gemm_error_word(a.device)), _stream()), "head_gemm_tcgen05")
+        _entries.rllm_head_gemm_tcgen05(a, a.stride(0), a.stride(1), b, b.stride(1), b.stride(0), c, c.stride(0),
+                                        c.stride(1), M, N, K, heads, gemm_error_word(a.device))
         return
-    _check(lib.rllm_head_gemm(_ptr(a), c_longlong(a.stride(0)), c_longlong(a.stride(1)), _ptr(b),
-                              c_longlong(b.stride(1)), c_longlong(b.stride(0)), c_int(1 if b_kn else 0), _ptr(c),
-                              c_longlong(c.stride(0)), c_longlong(c.stride(1)), c_int(M), c_int(N), c_int(K),
-                              c_int(heads), c_int(dtype_code(a.dtype)), _stream()), "head_gemm")
+    _entries.rllm_head_gemm(a, a.stride(0), a.stride(1), b, b.stride(1), b.stride(0), 1 if b_kn else 0, c, c.stride(0),
+                            c.stride(1), M, N, K, heads, dtype_code(a.dtype))
 
 
 def latent_attention_simt(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor,
@@ -936,19 +973,15 @@ def latent_attention_simt(q: torch.Tensor, out: torch.Tensor, cache: torch.Tenso
     """q [T, heads * dk], cache [pages, 1, page_size, dk], out [T, heads * dv]: softmax(q . row * scale) over
     the visible rows (``window`` 0: all up to the query's position), times the rows' first dv values.
     ``sink`` float32 [heads]: exp(sink[h]) joins the denominator."""
-    lib = build.load_library("latent_attention")
     T = q.shape[0]
     assert q.shape == (T, heads * dk) and out.shape == (T, heads * dv) and cache.shape[3] == dk
     assert cache.dtype is q.dtype and out.dtype is q.dtype
     _contig(q, "q"); _contig(out, "out"); _contig(cache, "cache"); _contig(block_table, "block_table")
     if sink is not None:
         assert sink.dtype is torch.float32 and sink.numel() == heads
-    _check(lib.rllm_latent_attention_simt(_ptr(q), _ptr(out), _ptr(cache), c_int(dtype_code(q.dtype)),
-                                          _ptr(block_table), c_int(block_table.shape[1]), _ptr(positions),
-                                          _ptr(token_seq), c_int(T), c_int(heads), c_int(dk), c_int(dv),
-                                          c_int(cache.shape[2]), c_int(cache.shape[0]), c_int(window),
-                                          c_float(scale), _ptr(sink), _ptr(err), _stream()),
-           "latent_attention_simt")
+    _entries.rllm_latent_attention_simt(q, out, cache, dtype_code(q.dtype), block_table, block_table.shape[1],
+                                        positions, token_seq, T, heads, dk, dv, cache.shape[2], cache.shape[0], window,
+                                        scale, sink, err)
 
 
 LATENT_SPLIT_MAX_TILES = 64      # at most this many row tiles in a launch (they fill less than half the GPU) ...
@@ -992,12 +1025,9 @@ def latent_attention_mma(q: torch.Tensor, out: torch.Tensor, cache: torch.Tensor
     _contig(q, "q"); _contig(out, "out"); _contig(cache, "cache"); _contig(block_table, "block_table")
     if sink is not None:
         assert sink.dtype is torch.float32 and sink.numel() == heads
-    _check(lib.rllm_latent_attention_mma(_ptr(q), _ptr(out), _ptr(cache), _ptr(block_table),
-                                         c_int(block_table.shape[1]), _ptr(q_start), _ptr(seq_lens), c_int(num_seqs),
-                                         c_int(max_q_len), c_int(heads), c_int(dk), c_int(dv), c_int(cache.shape[2]),
-                                         c_int(cache.shape[0]), c_int(window), c_float(scale), _ptr(sink),
-                                         c_int(split_tiles), c_int(nsplit), _ptr(work), _ptr(err), _stream()),
-           "latent_attention_mma")
+    _entries.rllm_latent_attention_mma(q, out, cache, block_table, block_table.shape[1], q_start, seq_lens, num_seqs,
+                                       max_q_len, heads, dk, dv, cache.shape[2], cache.shape[0], window, scale, sink,
+                                       split_tiles, nsplit, work, err)
 
 
 LATENT_TCGEN05_MIN_ROWS = 1024       # (token, head) rows of a step's prompt portions from which the tcgen05 kernel may run
@@ -1047,18 +1077,15 @@ def latent_attention_tcgen05(q: torch.Tensor, out: torch.Tensor, cache: torch.Te
                              err: torch.Tensor) -> None:
     """The attention of ``latent_attention_simt`` on the tcgen05 tensor cores, for the prompt portions (``num_tokens``
     tokens) of sequences seq_begin .. seq_end-1 of the step; q and out hold all of the step's tokens."""
-    lib = build.load_library("latent_attention_tcgen05")
     T = q.shape[0]
     assert q.shape == (T, heads * dk) and out.shape == (T, heads * dv) and cache.shape[3] == dk
     assert q.dtype is torch.bfloat16 and cache.dtype is torch.bfloat16 and out.dtype is torch.bfloat16
     _contig(q, "q"); _contig(out, "out"); _contig(cache, "cache"); _contig(block_table, "block_table")
     if sink is not None:
         assert sink.dtype is torch.float32 and sink.numel() == heads
-    _check(lib.rllm_latent_attention_tcgen05(
-        _ptr(q), c_int(T), _ptr(out), _ptr(cache), _ptr(block_table), c_int(block_table.shape[1]), _ptr(q_start),
-        _ptr(seq_lens), c_int(seq_begin), c_int(seq_end), c_int(num_tokens), c_int(heads), c_int(dk), c_int(dv),
-        c_int(cache.shape[2]), c_int(cache.shape[0]), c_int(window), c_float(scale), _ptr(sink), _ptr(err), _stream()),
-        "latent_attention_tcgen05")
+    _entries.rllm_latent_attention_tcgen05(q, T, out, cache, block_table, block_table.shape[1], q_start, seq_lens,
+                                           seq_begin, seq_end, num_tokens, heads, dk, dv, cache.shape[2],
+                                           cache.shape[0], window, scale, sink, err)
 
 
 def latent_expanded_rows(q_lens, seq_lens, window: int) -> int:
@@ -1120,18 +1147,15 @@ def latent_expand_prep(q: torch.Tensor, cache: torch.Tensor, rows: torch.Tensor,
     """For the prompt portions of sequences seq_begin .. seq_end-1: gathers their visible cached rows into ``rows``
     [latent_expanded_rows, dk] and rotates the last rot values of every head of q [T, heads * (nope + rot)] in place
     (tokens first_token .. T-1)."""
-    lib = build.load_library("latent_attention")
     T, dk = q.shape[0], cache.shape[3]
     assert q.dtype is torch.bfloat16 and cache.dtype is torch.bfloat16 and rows.dtype is torch.bfloat16
     assert q.shape[1] == heads * (nope + rot) and rows.shape[1] == dk and cache.shape[1] == 1
     _contig(q, "q"); _contig(cache, "cache"); _contig(rows, "rows"); _contig(block_table, "block_table")
     if rot_dims:
         assert inv_freq is not None and inv_freq.dtype is torch.float64 and inv_freq.numel() == rot_dims // 2
-    _check(lib.rllm_latent_expand_prep(
-        _ptr(q), _ptr(cache), _ptr(rows), _ptr(block_table), c_int(block_table.shape[1]), _ptr(q_start), _ptr(seq_lens),
-        c_int(seq_begin), c_int(seq_end), _ptr(positions), _ptr(inv_freq), c_float(magnitude), c_int(first_token),
-        c_int(T - first_token), c_int(heads), c_int(nope), c_int(rot), c_int(rot_dims), c_int(dk), c_int(rows.shape[0]),
-        c_int(cache.shape[2]), c_int(cache.shape[0]), c_int(window), _ptr(err), _stream()), "latent_expand_prep")
+    _entries.rllm_latent_expand_prep(q, cache, rows, block_table, block_table.shape[1], q_start, seq_lens, seq_begin,
+                                     seq_end, positions, inv_freq, magnitude, first_token, T - first_token, heads, nope,
+                                     rot, rot_dims, dk, rows.shape[0], cache.shape[2], cache.shape[0], window, err)
 
 
 def latent_expanded_tcgen05(q: torch.Tensor, kv: torch.Tensor, rows: torch.Tensor, out: torch.Tensor, q_start: torch.Tensor,
@@ -1141,7 +1165,6 @@ def latent_expanded_tcgen05(q: torch.Tensor, kv: torch.Tensor, rows: torch.Tenso
     """Attention of prompt portions (``num_tokens`` tokens of sequences seq_begin .. seq_end-1) with every head's own keys
     and values: q [T, heads * (nope + rot)] rotated, ``rows`` as ``latent_expand_prep`` leaves them, kv [rows, heads nope +
     heads v] the product of their first kv_rank values with [W_uk; W_uv]; out [T, heads * v]."""
-    lib = build.load_library("latent_expanded_tcgen05")
     T = q.shape[0]
     assert q.shape == (T, heads * (nope + rot)) and out.shape == (T, heads * v)
     assert kv.shape == (rows.shape[0], heads * (nope + v)) and rows.shape[1] == kv_rank + rot
@@ -1149,10 +1172,8 @@ def latent_expanded_tcgen05(q: torch.Tensor, kv: torch.Tensor, rows: torch.Tenso
     _contig(q, "q"); _contig(kv, "kv"); _contig(rows, "rows"); _contig(out, "out")
     if sink is not None:
         assert sink.dtype is torch.float32 and sink.numel() == heads
-    _check(lib.rllm_latent_expanded_tcgen05(
-        _ptr(q), c_int(T), _ptr(kv), _ptr(rows), c_int(rows.shape[0]), c_int(rows.shape[1]), c_int(kv_rank), _ptr(out),
-        _ptr(q_start), _ptr(seq_lens), c_int(seq_begin), c_int(seq_end), c_int(num_tokens), c_int(heads), c_int(nope),
-        c_int(rot), c_int(v), c_int(window), c_float(scale), _ptr(sink), _ptr(err), _stream()), "latent_expanded_tcgen05")
+    _entries.rllm_latent_expanded_tcgen05(q, T, kv, rows, rows.shape[0], rows.shape[1], kv_rank, out, q_start, seq_lens,
+                                          seq_begin, seq_end, num_tokens, heads, nope, rot, v, window, scale, sink, err)
 
 
 # ---------------------------------------------------------------------------
@@ -1189,15 +1210,13 @@ def moe_tcgen05_pays(E: int, H: int, F: int) -> bool:
 def moe_route(h: torch.Tensor, w_router: torch.Tensor, top: int):
     """(ids int32 [T, top], scores float32 [T, top]): softmax over all experts of the float32 logits
     h . w_router^T, the ``top`` largest in falling order (lowest index first among equals)."""
-    lib = build.load_library("moe")
     T, H = h.shape
     E = w_router.shape[0]
     assert w_router.shape == (E, H) and w_router.dtype is h.dtype
     _contig(h, "h"); _contig(w_router, "w_router")
     ids = torch.empty((T, top), dtype=torch.int32, device=h.device)
     scores = torch.empty((T, top), dtype=torch.float32, device=h.device)
-    _check(lib.rllm_moe_route(_ptr(h), _ptr(w_router), _ptr(ids), _ptr(scores), c_int(T), c_int(H), c_int(E),
-                              c_int(top), c_int(dtype_code(h.dtype)), _stream()), "moe_route")
+    _entries.rllm_moe_route(h, w_router, ids, scores, T, H, E, top, dtype_code(h.dtype))
     return ids, scores
 
 
@@ -1206,14 +1225,12 @@ def moe_choose(logits: torch.Tensor, top: int, groups: int = 0, keep: int = 0, r
     experts form that many equal groups of neighbours, a group's score is its largest expert score, and only
     experts of the ``keep`` best groups can be chosen.  ``renormalise``: the chosen scores are divided by their
     sum + 1e-20."""
-    lib = build.load_library("moe")
     T, E = logits.shape
     assert logits.dtype is torch.float32
     _contig(logits, "logits")
     ids = torch.empty((T, top), dtype=torch.int32, device=logits.device)
     scores = torch.empty((T, top), dtype=torch.float32, device=logits.device)
-    _check(lib.rllm_moe_choose(_ptr(logits), _ptr(ids), _ptr(scores), c_int(T), c_int(E), c_int(top), c_int(groups),
-                               c_int(keep), c_int(1 if renormalise else 0), _stream()), "moe_choose")
+    _entries.rllm_moe_choose(logits, ids, scores, T, E, top, groups, keep, 1 if renormalise else 0)
     return ids, scores
 
 
@@ -1223,7 +1240,6 @@ def moe_experts(h: torch.Tensor, ids: torch.Tensor, w_gate_up: torch.Tensor, w_d
     W_down (g' sigmoid(alpha g') (u' + up_shift)), g' = min(W_gate h, limit), u' = clamp(W_up h, +-limit)
     (limit inf, alpha 1, up_shift 0: silu(W_gate h) * W_up h).
     w_gate_up [E, 2 F, H] (gate rows, then up rows), w_down [E, H, F]."""
-    lib = build.load_library("moe")
     T, H = h.shape
     top = ids.shape[1]
     E, F2, _ = w_gate_up.shape
@@ -1241,21 +1257,14 @@ def moe_experts(h: torch.Tensor, ids: torch.Tensor, w_gate_up: torch.Tensor, w_d
     m_tiles, offsets, sorted_pairs = meta[0:1], meta[1:E + 2], meta[E + 2:E + 2 + P]
     tile_expert = meta[E + 2 + P:E + 2 + P + max_tiles]
     tile_row0 = meta[E + 2 + P + max_tiles:]
-    _check(lib.rllm_moe_sort(_ptr(ids), c_int(P), c_int(E), c_int(bm), _ptr(offsets), _ptr(sorted_pairs),
-                             _ptr(tile_expert), _ptr(tile_row0), _ptr(m_tiles), _stream()), "moe_sort")
+    _entries.rllm_moe_sort(ids, P, E, bm, offsets, sorted_pairs, tile_expert, tile_row0, m_tiles)
     if tcgen05:
-        lib = build.load_library("moe_tcgen05")
-        _check(lib.rllm_moe_experts_tcgen05(
-            _ptr(h), _ptr(w_gate_up), _ptr(w_down), _ptr(y), _ptr(out), _ptr(offsets), _ptr(sorted_pairs),
-            _ptr(tile_expert), _ptr(tile_row0), _ptr(m_tiles), c_int(max_tiles), c_int(P), c_int(E), c_int(H), c_int(F),
-            c_int(top), c_float(limit), c_float(alpha), c_float(up_shift), _ptr(gemm_error_word(h.device)), _stream()),
-            "moe_experts_tcgen05")
+        _entries.rllm_moe_experts_tcgen05(h, w_gate_up, w_down, y, out, offsets, sorted_pairs, tile_expert, tile_row0,
+                                          m_tiles, max_tiles, P, E, H, F, top, limit, alpha, up_shift,
+                                          gemm_error_word(h.device))
         return out
-    _check(lib.rllm_moe_experts(_ptr(h), _ptr(w_gate_up), _ptr(w_down), _ptr(y), _ptr(out), _ptr(offsets),
-                                _ptr(sorted_pairs), _ptr(tile_expert), _ptr(tile_row0), _ptr(m_tiles),
-                                c_int(max_tiles), c_int(bm), c_int(H), c_int(F), c_int(top), c_float(limit),
-                                c_float(alpha), c_float(up_shift), c_int(dtype_code(h.dtype)), _stream()),
-           "moe_experts")
+    _entries.rllm_moe_experts(h, w_gate_up, w_down, y, out, offsets, sorted_pairs, tile_expert, tile_row0, m_tiles,
+                              max_tiles, bm, H, F, top, limit, alpha, up_shift, dtype_code(h.dtype))
     return out
 
 
@@ -1263,7 +1272,6 @@ def weighted_slot_sum(y: torch.Tensor, coeff: torch.Tensor, out: torch.Tensor, e
                       extra_gate: Optional[torch.Tensor] = None) -> None:
     """out[t] = sum_k coeff[t, k] * y[t * K + k] (+ sigmoid(extra_gate[t]) * extra[t]); y [T * K, H], coeff
     float32 [T, K], out and extra [T, H], extra_gate float32 [T] (absent: the extra row is added as it is)."""
-    lib = build.load_library("moe")
     T, H = out.shape
     K = coeff.shape[1]
     assert y.shape == (T * K, H) and coeff.shape == (T, K) and coeff.dtype is torch.float32 and y.dtype is out.dtype
@@ -1273,16 +1281,14 @@ def weighted_slot_sum(y: torch.Tensor, coeff: torch.Tensor, out: torch.Tensor, e
         _contig(extra, "extra")
         if extra_gate is not None:
             assert extra_gate.dtype is torch.float32 and extra_gate.numel() == T and extra_gate.is_contiguous()
-    _check(lib.rllm_weighted_slot_sum(_ptr(y), _ptr(coeff), _ptr(out), c_int(T), c_int(K), c_int(H), _ptr(extra),
-                                      _ptr(extra_gate if extra is not None else None),
-                                      c_int(dtype_code(out.dtype)), _stream()), "weighted_slot_sum")
+    _entries.rllm_weighted_slot_sum(y, coeff, out, T, K, H, extra, extra_gate if extra is not None else None,
+                                    dtype_code(out.dtype))
 
 
 def moe_choose_sigmoid(logits: torch.Tensor, top: int, bias: Optional[torch.Tensor], scale: float):
     """(ids int32 [T, top], weights float32 [T, top]) from float32 router logits [T, E]: s = sigmoid(z); the
     ``top`` experts with the largest s + bias (float32 [E] or None; lowest index among equals), in falling
     order; weights s * scale without the bias."""
-    lib = build.load_library("moe")
     T, E = logits.shape
     assert logits.dtype is torch.float32
     _contig(logits, "logits")
@@ -1290,8 +1296,7 @@ def moe_choose_sigmoid(logits: torch.Tensor, top: int, bias: Optional[torch.Tens
         assert bias.dtype is torch.float32 and bias.numel() == E and bias.is_contiguous()
     ids = torch.empty((T, top), dtype=torch.int32, device=logits.device)
     weights = torch.empty((T, top), dtype=torch.float32, device=logits.device)
-    _check(lib.rllm_moe_choose_sigmoid(_ptr(logits), _ptr(bias), c_float(scale), _ptr(ids), _ptr(weights), c_int(T),
-                                       c_int(E), c_int(top), _stream()), "moe_choose_sigmoid")
+    _entries.rllm_moe_choose_sigmoid(logits, bias, scale, ids, weights, T, E, top)
     return ids, weights
 
 
@@ -1302,32 +1307,27 @@ PLAIN_ACTIVATIONS = {"silu": 0, "gelu_tanh": 1, "relu_squared": 2}
 def act(x: torch.Tensor, out: torch.Tensor, activation: str) -> None:
     """out = act(x) element by element (float32 arithmetic); act "silu", "gelu_tanh" or "relu_squared"
     (max(z, 0)^2); ``out`` may be ``x``."""
-    lib = build.load_library("elementwise")
     assert x.shape == out.shape and x.dtype is out.dtype
     _contig(x, "x"); _contig(out, "out")
-    _check(lib.rllm_act(_ptr(x), _ptr(out), c_int(dtype_code(out.dtype)), c_longlong(x.numel()),
-                        c_int(PLAIN_ACTIVATIONS[activation]), _stream()), "act")
+    _entries.rllm_act(x, out, dtype_code(out.dtype), x.numel(), PLAIN_ACTIVATIONS[activation])
 
 
 def sigmoid_gate(x: torch.Tensor, gate: torch.Tensor, out: torch.Tensor) -> None:
     """out[t, i] = x[t, i] * sigmoid(gate[t, i]); gate may be a column slice (row stride >= its width)."""
-    lib = build.load_library("elementwise")
     T, W = x.shape
     assert out.shape == x.shape and gate.shape == x.shape and gate.dtype is x.dtype and out.dtype is x.dtype
     assert gate.stride(1) == 1
     _contig(x, "x"); _contig(out, "out")
-    _check(lib.rllm_sigmoid_gate(_ptr(x), _ptr(gate), c_int(gate.stride(0) if T > 1 else max(W, gate.stride(0))),
-                                 _ptr(out), c_int(dtype_code(x.dtype)), c_int(T), c_int(W), _stream()), "sigmoid_gate")
+    _entries.rllm_sigmoid_gate(x, gate, gate.stride(0) if T > 1 else max(W, gate.stride(0)), out, dtype_code(x.dtype),
+                               T, W)
 
 
 def act_mul(gate_up: torch.Tensor, out: torch.Tensor, activation: str) -> None:
     """out[t, i] = act(gate_up[t, i]) * gate_up[t, I + i]; act "silu" or "gelu_tanh"."""
-    lib = build.load_library("elementwise")
     T, I = out.shape
     assert gate_up.shape == (T, 2 * I) and gate_up.dtype is out.dtype
     _contig(gate_up, "gate_up"); _contig(out, "out")
-    _check(lib.rllm_act_mul(_ptr(gate_up), _ptr(out), c_int(dtype_code(out.dtype)), c_int(T), c_int(I),
-                            c_int(ACTIVATIONS[activation]), _stream()), "act_mul")
+    _entries.rllm_act_mul(gate_up, out, dtype_code(out.dtype), T, I, ACTIVATIONS[activation])
 
 
 # ---------------------------------------------------------------------------
@@ -1351,7 +1351,6 @@ def streams_read(xs: torch.Tensor, coeff: Optional[torch.Tensor], norm, out_dtyp
     """out[r] = n(sum_s coeff[s] * xs[s, row(r)]); xs float32 [S, T, H]; coeff float32 [S] (None: ones);
     ``norm`` = (alpha float32 [1], weight [H], shift [H]) applies n(u) = tanh(alpha u) * weight + shift and
     rounds to ``out_dtype``; None: out is the float32 sum.  ``rows`` int32 [R] picks rows."""
-    lib = build.load_library("hyper_streams")
     S, T, H = xs.shape
     assert xs.dtype is torch.float32 and S <= HS_MAX_STREAMS
     _contig(xs, "xs")
@@ -1363,9 +1362,8 @@ def streams_read(xs: torch.Tensor, coeff: Optional[torch.Tensor], norm, out_dtyp
         assert rows.dtype is torch.int32
     od = out_dtype if w is not None else torch.float32
     out = torch.empty((R, H), dtype=od, device=xs.device)
-    _check(lib.rllm_hs_read(_ptr(xs), _ptr(coeff), _ptr(rows), _ptr(alpha), _ptr(w), _ptr(c),
-                            c_int(dtype_code(w.dtype) if w is not None else DT_F32), _ptr(out), c_int(dtype_code(od)),
-                            c_int(S), c_longlong(T), c_int(R), c_int(H), _stream()), "streams_read")
+    _entries.rllm_hs_read(xs, coeff, rows, alpha, w, c, dtype_code(w.dtype) if w is not None else DT_F32, out,
+                          dtype_code(od), S, T, R, H)
     return out
 
 
@@ -1377,7 +1375,6 @@ def streams_write(xs: torch.Tensor, y: torch.Tensor, scale: Optional[torch.Tenso
     ``next_read`` (float32 [S]) the next read comes back too: n(sum_t next_read[t] x_t) with ``norm`` as in
     ``streams_read`` (in y's dtype), or the float32 sum without one.  ``sum_out`` float32 [T, H], if given,
     receives the plain sum of the new streams."""
-    lib = build.load_library("hyper_streams")
     S, T, H = xs.shape
     assert xs.dtype is torch.float32 and S <= HS_MAX_STREAMS and y.shape == (T, H)
     assert mix.dtype is torch.float32 and mix.shape == (S, S) and write.dtype is torch.float32 and write.numel() == S
@@ -1392,16 +1389,14 @@ def streams_write(xs: torch.Tensor, y: torch.Tensor, scale: Optional[torch.Tenso
         out = torch.empty((T, H), dtype=y.dtype if w is not None else torch.float32, device=xs.device)
     if sum_out is not None:
         assert sum_out.dtype is torch.float32 and sum_out.shape == (T, H) and sum_out.is_contiguous()
-    _check(lib.rllm_hs_write(_ptr(xs), _ptr(y), c_int(dtype_code(y.dtype)), _ptr(scale), _ptr(mix), _ptr(write),
-                             _ptr(next_read), _ptr(alpha), _ptr(w), _ptr(c), c_int(dtype_code(wd)), _ptr(out),
-                             _ptr(sum_out), c_int(S), c_longlong(T), c_int(H), _stream()), "streams_write")
+    _entries.rllm_hs_write(xs, y, dtype_code(y.dtype), scale, mix, write, next_read, alpha, w, c, dtype_code(wd), out,
+                           sum_out, S, T, H)
     return out
 
 
 def dyt(x: torch.Tensor, alpha: torch.Tensor, weight: torch.Tensor, shift: torch.Tensor, out: torch.Tensor,
         delta: Optional[torch.Tensor] = None, rows: Optional[torch.Tensor] = None, writeback: bool = False) -> None:
     """out = tanh(alpha * (x [+ delta])) * weight + shift; x float32 [., H]; the arguments of ``rmsnorm``."""
-    lib = build.load_library("hyper_streams")
     H, R = x.shape[-1], out.shape[0]
     assert x.dtype is torch.float32 and alpha.dtype is torch.float32 and weight.dtype is shift.dtype
     _contig(x, "x"); _contig(out, "out")
@@ -1410,9 +1405,8 @@ def dyt(x: torch.Tensor, alpha: torch.Tensor, weight: torch.Tensor, shift: torch
         _contig(delta, "delta")
     if rows is not None:
         assert rows.dtype is torch.int32 and rows.numel() == R
-    _check(lib.rllm_dyt(_ptr(x), _ptr(delta), _ptr(rows), _ptr(alpha), _ptr(weight), _ptr(shift),
-                        c_int(dtype_code(weight.dtype)), _ptr(out), c_int(dtype_code(out.dtype)), c_int(R), c_int(H),
-                        c_int(1 if writeback else 0), _stream()), "dyt")
+    _entries.rllm_dyt(x, delta, rows, alpha, weight, shift, dtype_code(weight.dtype), out, dtype_code(out.dtype), R, H,
+                      1 if writeback else 0)
 
 
 # ---------------------------------------------------------------------------
@@ -1436,7 +1430,6 @@ def head_norm_kv_write(qkv: torch.Tensor, positions: torch.Tensor, token_seq: to
     position p is multiplied by 1 + coef * ln(floor((p + 1) / every) + 1).  ``row_norm``: one root mean square over all
     of a token's queries and one over its keys, with weights [nq dk] and [nkv dk] (it wants ``write_kv``).  Columns of
     qkv behind the value heads are left alone."""
-    lib = build.load_library("mixer_glue")
     T = qkv.shape[0]
     assert qkv.shape[1] >= nq * dk + nkv * (dk + dv) and qkv.stride(1) == 1
     if bias is not None:
@@ -1459,17 +1452,12 @@ def head_norm_kv_write(qkv: torch.Tensor, positions: torch.Tensor, token_seq: to
         pages, page_size, max_blocks = kcache.shape[0], kcache.shape[2], block_table.shape[1]
     else:
         pages = page_size = max_blocks = 0
-    _check(lib.rllm_head_norm_kv_write(_ptr(qkv), c_int(dtype_code(qkv.dtype)), c_int(qkv.stride(0)), _ptr(positions),
-                                       _ptr(token_seq), _ptr(q_weight), _ptr(k_weight), c_int(dtype_code(wd)),
-                                       c_float(eps), _ptr(block_table), c_int(max_blocks),
-                                       _ptr(kcache if write_kv else None), _ptr(vcache if write_kv else None),
-                                       c_int(T), c_int(nq), c_int(nkv if write_kv else 0), c_int(dk), c_int(dv),
-                                       c_int(dkp), c_int(dvp), _ptr(q_out),
-                                       c_int(page_size), c_int(pages), c_int(1 if write_kv else 0), _ptr(bias),
-                                       _ptr(inv_freq if rotary_dim else None), c_int(rotary_dim), c_float(magnitude),
-                                       c_int(1 if unit_norm else 0), c_float(q_temp[0] if q_temp else 0.0),
-                                       c_int(int(q_temp[1]) if q_temp else 0), c_int(1 if row_norm else 0),
-                                       _ptr(err), _stream()), "head_norm_kv_write")
+    _entries.rllm_head_norm_kv_write(qkv, dtype_code(qkv.dtype), qkv.stride(0), positions, token_seq, q_weight,
+                                     k_weight, dtype_code(wd), eps, block_table, max_blocks, kcache if write_kv else
+                                     None, vcache if write_kv else None, T, nq, nkv if write_kv else 0, dk, dv, dkp,
+                                     dvp, q_out, page_size, pages, 1 if write_kv else 0, bias, inv_freq if rotary_dim
+                                     else None, rotary_dim, magnitude, 1 if unit_norm else 0, q_temp[0] if q_temp else
+                                     0.0, int(q_temp[1]) if q_temp else 0, 1 if row_norm else 0, err)
 
 
 def attention_simt_kv(q: torch.Tensor, q_stride: int, out: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor,
@@ -1486,7 +1474,6 @@ def attention_simt_kv(q: torch.Tensor, q_stride: int, out: torch.Tensor, kcache:
     stride: the result is multiplied by its sigmoid; ``slopes`` float32 [nq]: slopes[h] * (query position - key
     position) is taken off every score.  ``shared_keys`` = dv: all heads read one key row a token ([pages, 1, page, dk])
     and a token's value row holds the kv heads' values side by side ([pages, 1, page, nkv * places], dv of each)."""
-    lib = build.load_library("attention_simt")
     T, dk, dv = out.shape[0], kcache.shape[3], vcache.shape[3]
     v_ld = 0
     if shared_keys is not None:
@@ -1498,40 +1485,32 @@ def attention_simt_kv(q: torch.Tensor, q_stride: int, out: torch.Tensor, kcache:
         assert sinks.dtype is torch.float32 and sinks.numel() == nq and sinks.is_contiguous()
     if gate is not None:
         assert gate.dtype is q.dtype and gate.stride(1) == 1 and gate.shape == (T, nq if gate_per_head else nq * dv)
-    _check(lib.rllm_attention_simt_kv(_ptr(q), c_int(q_stride), _ptr(out), _ptr(kcache), _ptr(vcache),
-                                      c_int(dtype_code(q.dtype)), _ptr(block_table), c_int(block_table.shape[1]),
-                                      _ptr(positions), _ptr(token_seq), c_int(T), c_int(nq), c_int(nkv), c_int(dk),
-                                      c_int(dv), c_int(kcache.shape[2]), c_int(kcache.shape[0]), c_int(window),
-                                      c_float(scale), c_int(keep_first), c_int(chunk), c_float(softcap), _ptr(sinks),
-                                      _ptr(gate), c_int(gate.stride(0) if gate is not None else 0),
-                                      c_int(0 if gate is None else (1 if gate_per_head else 2)), _ptr(slopes),
-                                      c_int(0 if shared_keys is None else 1), c_int(v_ld), _ptr(err), _stream()),
-           "attention_simt_kv")
+    _entries.rllm_attention_simt_kv(q, q_stride, out, kcache, vcache, dtype_code(q.dtype), block_table,
+                                    block_table.shape[1], positions, token_seq, T, nq, nkv, dk, dv, kcache.shape[2],
+                                    kcache.shape[0], window, scale, keep_first, chunk, softcap, sinks, gate,
+                                    gate.stride(0) if gate is not None else 0, 0 if gate is None else (1 if
+                                    gate_per_head else 2), slopes, 0 if shared_keys is None else 1, v_ld, err)
 
 
 def rms_mean2(a: torch.Tensor, b: torch.Tensor, wa: torch.Tensor, wb: torch.Tensor, eps: float) -> torch.Tensor:
     """(rms(a) * wa + rms(b) * wb) / 2 row by row, rms(x) = x / sqrt(mean(x^2) + eps); a, b [T, H]."""
-    lib = build.load_library("mixer_glue")
     T, H = a.shape
     assert b.shape == a.shape and b.dtype is a.dtype and wa.dtype is wb.dtype and wa.numel() == H and wb.numel() == H
     _contig(a, "a"); _contig(b, "b"); _contig(wa, "wa"); _contig(wb, "wb")
     out = torch.empty_like(a)
-    _check(lib.rllm_rms_mean2(_ptr(a), _ptr(b), _ptr(wa), _ptr(wb), c_int(dtype_code(wa.dtype)), _ptr(out),
-                              c_int(dtype_code(a.dtype)), c_int(T), c_int(H), c_float(eps), _stream()), "rms_mean2")
+    _entries.rllm_rms_mean2(a, b, wa, wb, dtype_code(wa.dtype), out, dtype_code(a.dtype), T, H, eps)
     return out
 
 
 def gated_rmsnorm(x: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, eps: float,
                   out_dtype: torch.dtype) -> torch.Tensor:
     """rms(x) * weight * sigmoid(gate); x float32 [T, H]; gate [T, H] (a column slice of a wider tensor will do)."""
-    lib = build.load_library("mixer_glue")
     T, H = x.shape
     assert x.dtype is torch.float32 and gate.shape == (T, H) and gate.stride(1) == 1 and gate.dtype is out_dtype
     _contig(x, "x"); _contig(weight, "weight")
     out = torch.empty((T, H), dtype=out_dtype, device=x.device)
-    _check(lib.rllm_gated_rmsnorm(_ptr(x), _ptr(gate), c_int(gate.stride(0)), _ptr(weight),
-                                  c_int(dtype_code(weight.dtype)), _ptr(out), c_int(dtype_code(out_dtype)), c_int(T),
-                                  c_int(H), c_float(eps), _stream()), "gated_rmsnorm")
+    _entries.rllm_gated_rmsnorm(x, gate, gate.stride(0), weight, dtype_code(weight.dtype), out, dtype_code(out_dtype),
+                                T, H, eps)
     return out
 
 
@@ -1565,10 +1544,8 @@ def lightning_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: tor
     out = torch.empty((T, heads * dv), dtype=torch.float32, device=q.device)
     chunks = _chunks_for(int(lib.rllm_lightning_chunk()), max_q_len, num_seqs)
     work = torch.empty(num_seqs * chunks * heads * d * dv, dtype=torch.float32, device=q.device) if chunks else None
-    _check(lib.rllm_lightning_scan(_ptr(q), _ptr(k), _ptr(v), c_int(q.stride(0)), c_int(dtype_code(q.dtype)),
-                                   _ptr(decay), _ptr(state), _ptr(work), _ptr(q_start), _ptr(slots),
-                                   c_int(state.shape[0]), c_int(num_seqs), c_int(chunks), _ptr(out), c_int(heads),
-                                   c_int(d), c_int(dv), _ptr(err), _stream()), "lightning_scan")
+    _entries.rllm_lightning_scan(q, k, v, q.stride(0), dtype_code(q.dtype), decay, state, work, q_start, slots,
+                                 state.shape[0], num_seqs, chunks, out, heads, d, dv, err)
     return out
 
 
@@ -1578,7 +1555,6 @@ def causal_conv(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     """silu(bias + causal convolution per channel; ``bias`` may be None); x [T, E] (a column slice will do); weight [E, taps], the
     last column the current token's; tail float32 [slots, taps - 1, E]: a request's last inputs, read for the
     places before this step and moved on.  ``any_long``: some sequence brings more than one token."""
-    lib = build.load_library("selective_scan")
     T, E = x.shape
     taps = weight.shape[1]
     assert weight.shape == (E, taps) and x.stride(1) == 1
@@ -1586,10 +1562,9 @@ def causal_conv(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     assert tail.dtype is torch.float32 and tuple(tail.shape[1:]) == (max(taps - 1, 0), E)
     _contig(weight, "weight"); _contig(tail, "tail")
     out = torch.empty((T, E), dtype=x.dtype, device=x.device)
-    _check(lib.rllm_causal_conv(_ptr(x), c_int(x.stride(0)), c_int(dtype_code(x.dtype)), _ptr(weight), _ptr(bias),
-                                c_int(dtype_code(weight.dtype)), _ptr(tail), _ptr(q_start), _ptr(token_seq),
-                                _ptr(slots), c_int(tail.shape[0]), c_int(num_seqs), c_int(1 if any_long else 0),
-                                _ptr(out), c_int(T), c_int(E), c_int(taps), _ptr(err), _stream()), "causal_conv")
+    _entries.rllm_causal_conv(x, x.stride(0), dtype_code(x.dtype), weight, bias, dtype_code(weight.dtype), tail,
+                              q_start, token_seq, slots, tail.shape[0], num_seqs, 1 if any_long else 0, out, T, E, taps,
+                              err)
     return out
 
 
@@ -1614,12 +1589,9 @@ def selective_scan(xc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: torch.Tensor
     chunks = _chunks_for(int(lib.rllm_scan_chunk()), max_q_len, num_seqs)
     work = torch.empty(num_seqs * chunks * (N + 1) * E, dtype=torch.float32, device=xc.device) if chunks else None
     work_dt = work[num_seqs * chunks * N * E:] if chunks else None
-    _check(lib.rllm_selective_scan(_ptr(xc), _ptr(dt_raw), _ptr(dt_bias), _ptr(bc), c_int(bc.stride(0)), c_int(b_off),
-                                   c_int(c_off), _ptr(a_log), _ptr(dskip), _ptr(z), c_int(z.stride(0)),
-                                   c_int(dtype_code(xc.dtype)), c_int(dtype_code(a_log.dtype)), _ptr(state),
-                                   _ptr(work), _ptr(work_dt), _ptr(q_start), _ptr(slots), c_int(state.shape[0]),
-                                   c_int(num_seqs), c_int(chunks), _ptr(out), c_int(E), c_int(N), _ptr(err),
-                                   _stream()), "selective_scan")
+    _entries.rllm_selective_scan(xc, dt_raw, dt_bias, bc, bc.stride(0), b_off, c_off, a_log, dskip, z, z.stride(0),
+                                 dtype_code(xc.dtype), dtype_code(a_log.dtype), state, work, work_dt, q_start, slots,
+                                 state.shape[0], num_seqs, chunks, out, E, N, err)
     return out
 
 
@@ -1632,7 +1604,6 @@ def layernorm(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, eps: fl
     """out = (v - mean) / sqrt(mean of squared deviations + eps) * weight + bias, row by row in float32, with
     v = x + the sum of ``deltas`` (up to two [T, H] in out's dtype) + ``row_bias`` (float32 [H], every row).
     ``writeback``: x becomes v.  ``rows`` int32 [R]: out[r] is made from row rows[r]."""
-    lib = build.load_library("layernorm")
     H = x.shape[-1]
     R = rows.numel() if rows is not None else x.shape[0]
     assert x.dtype is torch.float32 and x.is_contiguous() and out.is_contiguous() and out.shape == (R, H)
@@ -1645,31 +1616,26 @@ def layernorm(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, eps: fl
         assert row_bias.dtype is torch.float32 and row_bias.numel() == H and row_bias.is_contiguous()
     d0 = deltas[0] if deltas else None
     d1 = deltas[1] if len(deltas) > 1 else None
-    _check(lib.rllm_layernorm(_ptr(x), _ptr(d0), _ptr(d1), _ptr(row_bias), _ptr(rows), _ptr(weight), _ptr(bias),
-                              _ptr(out), c_int(dtype_code(out.dtype)), c_int(R), c_int(H), c_float(eps),
-                              c_int(1 if writeback else 0), _stream()), "layernorm")
+    _entries.rllm_layernorm(x, d0, d1, row_bias, rows, weight, bias, out, dtype_code(out.dtype), R, H, eps, 1 if
+                            writeback else 0)
 
 
 def add_rows(x: torch.Tensor, deltas, row_bias: Optional[torch.Tensor] = None) -> None:
     """x (float32 [T, H]) += the sum of ``deltas`` (one or two [T, H]) + ``row_bias`` (float32 [H])."""
-    lib = build.load_library("layernorm")
     deltas = tuple(deltas)
     assert 1 <= len(deltas) <= 2 and x.dtype is torch.float32 and x.is_contiguous()
     for d in deltas:
         assert d.shape == x.shape and d.is_contiguous() and d.dtype is deltas[0].dtype
     if row_bias is not None:
         assert row_bias.dtype is torch.float32 and row_bias.numel() == x.shape[1] and row_bias.is_contiguous()
-    _check(lib.rllm_add_rows(_ptr(x), _ptr(deltas[0]), _ptr(deltas[1] if len(deltas) > 1 else None), _ptr(row_bias),
-                             c_int(dtype_code(deltas[0].dtype)), c_int(x.shape[0]), c_int(x.shape[1]), _stream()),
-           "add_rows")
+    _entries.rllm_add_rows(x, deltas[0], deltas[1] if len(deltas) > 1 else None, row_bias, dtype_code(deltas[0].dtype),
+                           x.shape[0], x.shape[1])
 
 
 def add_row_bias(y: torch.Tensor, bias: torch.Tensor) -> None:
     """y [T, N] (bfloat16 or float32) += ``bias`` (float32 [N]) on every row, in place."""
-    lib = build.load_library("layernorm")
     assert y.dim() == 2 and y.is_contiguous() and bias.dtype is torch.float32 and bias.numel() == y.shape[1]
-    _check(lib.rllm_add_row_bias(_ptr(y), _ptr(bias), c_int(dtype_code(y.dtype)), c_int(y.shape[0]),
-                                 c_int(y.shape[1]), _stream()), "add_row_bias")
+    _entries.rllm_add_row_bias(y, bias, dtype_code(y.dtype), y.shape[0], y.shape[1])
 
 
 # ---------------------------------------------------------------------------
@@ -1697,7 +1663,6 @@ def mlstm_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gates: torch.T
     sequences' token counts of this step, host integers): if the longest has ``MLSTM_CHUNKED_FROM`` tokens or
     more, the sequences are cut into chunks of ``MLSTM_CHUNK`` tokens that run side by side (three launches);
     the results differ from the token-by-token walk by rounding only."""
-    lib = build.load_library("mlstm")
     T = q.shape[0]
     assert q.shape == (T, heads * d) and k.shape == (T, heads * d) and v.shape == (T, heads * dv)
     assert q.dtype is k.dtype and k.dtype is v.dtype and q.stride(0) == k.stride(0) == v.stride(0)
@@ -1715,11 +1680,8 @@ def mlstm_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gates: torch.T
         else:
             local = torch.empty((chunks, heads, per + 1), dtype=torch.float32, device=q.device)
             start = torch.empty((chunks, heads, per), dtype=torch.float32, device=q.device)
-    _check(lib.rllm_mlstm_scan(_ptr(q), _ptr(k), _ptr(v), c_int(q.stride(0)), c_int(dtype_code(q.dtype)), _ptr(gates),
-                               _ptr(bias_i), _ptr(bias_f), c_float(cap), c_float(qscale), _ptr(state), _ptr(q_start),
-                               _ptr(slots), _ptr(out), c_int(T), c_int(num_seqs), c_int(heads), c_int(d), c_int(dv),
-                               c_int(state.shape[0]), c_int(chunks), _ptr(local), _ptr(start), _ptr(err), _stream()),
-           "mlstm_scan")
+    _entries.rllm_mlstm_scan(q, k, v, q.stride(0), dtype_code(q.dtype), gates, bias_i, bias_f, cap, qscale, state,
+                             q_start, slots, out, T, num_seqs, heads, d, dv, state.shape[0], chunks, local, start, err)
     return out
 
 
@@ -1727,16 +1689,13 @@ def head_gated_rmsnorm(x: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor
                        out_dtype: torch.dtype) -> torch.Tensor:
     """out = x / sqrt(mean over a head's values of x^2 + eps) * weight * sigmoid(gate); x float32 [T, heads * dv],
     weight [heads * dv], gate [T, heads * dv] in ``out_dtype`` (may be a column slice)."""
-    lib = build.load_library("mlstm")
     T, W = x.shape
     assert x.dtype is torch.float32 and x.is_contiguous() and W % heads == 0 and weight.numel() == W
     assert gate.shape == (T, W) and gate.dtype is out_dtype and gate.stride(1) == 1
     _contig(weight, "weight")
     out = torch.empty((T, W), dtype=out_dtype, device=x.device)
-    _check(lib.rllm_head_gated_rmsnorm(_ptr(x), _ptr(gate), c_int(gate.stride(0) if T > 1 else max(W, gate.stride(0))),
-                                       _ptr(weight), c_int(dtype_code(weight.dtype)), _ptr(out),
-                                       c_int(dtype_code(out_dtype)), c_int(T), c_int(heads), c_int(W // heads),
-                                       c_float(eps), _stream()), "head_gated_rmsnorm")
+    _entries.rllm_head_gated_rmsnorm(x, gate, gate.stride(0) if T > 1 else max(W, gate.stride(0)), weight,
+                                     dtype_code(weight.dtype), out, dtype_code(out_dtype), T, heads, W // heads, eps)
     return out
 
 
@@ -1763,11 +1722,9 @@ def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: 
     chunks = _chunks_for(int(lib.rllm_ssd_chunk()), max_q_len, num_seqs)
     work = torch.empty(num_seqs * chunks * heads * (n * p + 1), dtype=torch.float32, device=xbc.device) if chunks else None
     chunk_dt = work[num_seqs * chunks * heads * n * p:] if chunks else None
-    _check(lib.rllm_ssd_scan(_ptr(xbc), c_int(xbc.stride(0) if T > 1 else xbc.shape[1]), c_int(dtype_code(xbc.dtype)),
-                             _ptr(dt), _ptr(dt_bias), _ptr(a_log), _ptr(skip), _ptr(state), _ptr(work), _ptr(chunk_dt),
-                             _ptr(q_start), _ptr(slots), c_int(state.shape[0]), c_int(num_seqs), c_int(chunks),
-                             _ptr(out), c_int(heads), c_int(groups), c_int(n), c_int(p), _ptr(err), _stream()),
-           "ssd_scan")
+    _entries.rllm_ssd_scan(xbc, xbc.stride(0) if T > 1 else xbc.shape[1], dtype_code(xbc.dtype), dt, dt_bias, a_log,
+                           skip, state, work, chunk_dt, q_start, slots, state.shape[0], num_seqs, chunks, out, heads,
+                           groups, n, p, err)
     return out
 
 
@@ -1775,15 +1732,13 @@ def silu_gated_group_rmsnorm(y: torch.Tensor, z: torch.Tensor, weight: torch.Ten
                              out_dtype: torch.dtype) -> torch.Tensor:
     """v = y * silu(z); each of ``groups`` equal parts of a row over its own root mean square, times weight.
     y float32 [T, E]; z [T, E] in ``out_dtype`` (may be a column slice); weight float32 [E]."""
-    lib = build.load_library("ssd")
     T, E = y.shape
     assert y.dtype is torch.float32 and weight.dtype is torch.float32 and weight.numel() == E
     assert z.shape == (T, E) and z.dtype is out_dtype and z.stride(1) == 1
     _contig(y, "y"); _contig(weight, "weight")
     out = torch.empty((T, E), dtype=out_dtype, device=y.device)
-    _check(lib.rllm_silu_gated_group_rmsnorm(_ptr(y), _ptr(z), c_int(z.stride(0) if T > 1 else max(E, z.stride(0))),
-                                             _ptr(weight), _ptr(out), c_int(dtype_code(out_dtype)), c_int(T), c_int(E),
-                                             c_int(groups), c_float(eps), _stream()), "silu_gated_group_rmsnorm")
+    _entries.rllm_silu_gated_group_rmsnorm(y, z, z.stride(0) if T > 1 else max(E, z.stride(0)), weight, out,
+                                           dtype_code(out_dtype), T, E, groups, eps)
     return out
 
 
@@ -1827,24 +1782,17 @@ def channel_delta_scan(c: torch.Tensor, step: torch.Tensor, b: torch.Tensor, dt_
             out = torch.empty((T, heads * dv), **f32)
             work = torch.empty(seg * per, dtype=torch.uint8, device=c.device)
             for chunk0 in range(0, chunks, seg):
-                _check(lib.rllm_channel_delta_chunked(_ptr(c), c_int(stride), _ptr(step), _ptr(b), _ptr(dt_bias),
-                                                      _ptr(a_log), c_float(unit_eps), c_float(float(d) ** -0.5),
-                                                      _ptr(state), _ptr(q_start), _ptr(slots), c_int(state.shape[0]),
-                                                      c_int(num_seqs), c_int(chunk0), c_int(seg), _ptr(work), _ptr(out),
-                                                      c_int(heads), c_int(kv), c_int(d), c_int(dv), _ptr(err),
-                                                      _stream()), "channel_delta_chunked")
+                _entries.rllm_channel_delta_chunked(c, stride, step, b, dt_bias, a_log, unit_eps, float(d) ** -0.5,
+                                                    state, q_start, slots, state.shape[0], num_seqs, chunk0, seg, work,
+                                                    out, heads, kv, d, dv, err)
             return out
     qn, kn, g = torch.empty((T, kv, d), **f32), torch.empty((T, kv, d), **f32), torch.empty((T, heads, d), **f32)
     beta, out = torch.empty((T, heads), **f32), torch.empty((T, heads * dv), **f32)
-    _check(lib.rllm_channel_delta_prepare(_ptr(c), c_int(stride), c_int(dtype_code(c.dtype)), _ptr(step), _ptr(b),
-                                          _ptr(dt_bias), _ptr(a_log), _ptr(qn), _ptr(kn), _ptr(g), _ptr(beta), c_int(T),
-                                          c_int(heads), c_int(kv), c_int(d), c_float(unit_eps),
-                                          c_float(float(d) ** -0.5), _stream()), "channel_delta_prepare")
+    _entries.rllm_channel_delta_prepare(c, stride, dtype_code(c.dtype), step, b, dt_bias, a_log, qn, kn, g, beta, T,
+                                        heads, kv, d, unit_eps, float(d) ** -0.5)
     v = c[:, 2 * kv * d:]
-    _check(lib.rllm_channel_delta_walk(_ptr(qn), _ptr(kn), _ptr(g), _ptr(beta), _ptr(v), c_int(stride),
-                                       c_int(dtype_code(c.dtype)), _ptr(state), _ptr(q_start), _ptr(slots),
-                                       c_int(state.shape[0]), c_int(num_seqs), _ptr(out), c_int(heads), c_int(kv),
-                                       c_int(d), c_int(dv), _ptr(err), _stream()), "channel_delta_walk")
+    _entries.rllm_channel_delta_walk(qn, kn, g, beta, v, stride, dtype_code(c.dtype), state, q_start, slots,
+                                     state.shape[0], num_seqs, out, heads, kv, d, dv, err)
     return out
 
 
@@ -1866,7 +1814,6 @@ def channel_delta_step(a: torch.Tensor, c: Optional[torch.Tensor], x: torch.Tens
     norm [>= dv]; state float32 [slots, heads, d, dv], updated in place.  ``early``: the kernel launched directly ahead
     does not write ``state``, so that it may be fetched while that one still runs.  Returns the gated, normalised result
     [S, heads dv] in a's dtype."""
-    lib = build.load_library("channel_delta")
     S, ch = a.shape[0], 2 * kv * d + heads * dv
     assert a.stride(1) == 1 and x.shape[0] == S and x.stride(1) == 1 and x.dtype is a.dtype
     ra, rg = w["a2"].shape[1], w["g2"].shape[1]
@@ -1884,13 +1831,11 @@ def channel_delta_step(a: torch.Tensor, c: Optional[torch.Tensor], x: torch.Tens
     if c is not None:
         assert c.shape == (S, ch) and c.dtype is a.dtype and c.is_contiguous()
     out = torch.empty((S, heads * dv), dtype=a.dtype, device=a.device)
-    _check(lib.rllm_channel_delta_step(
-        _ptr(a), c_int(a.stride(0)), _ptr(c), _ptr(x), c_int(x.stride(0)), _ptr(w["b"]), _ptr(w["a2"]), _ptr(w["g2"]),
-        _ptr(w["conv"]), c_int(dtype_code(w["conv"].dtype)), _ptr(w["dt_bias"]), _ptr(w["a_log"]), _ptr(w["norm"]),
-        _ptr(tail), _ptr(state), _ptr(slots), _ptr(out), c_int(dtype_code(a.dtype)), c_int(S), c_int(at_a), c_int(at_g),
-        c_int(ra), c_int(rg), c_int(x.shape[1]), c_int(taps), c_int(state.shape[0]), c_int(heads), c_int(kv), c_int(d),
-        c_int(dv), c_float(unit_eps), c_float(float(d) ** -0.5), c_float(eps), c_int(1 if early else 0), _ptr(err),
-        _stream()), "channel_delta_step")
+    _entries.rllm_channel_delta_step(a, a.stride(0), c, x, x.stride(0), w["b"], w["a2"], w["g2"], w["conv"],
+                                     dtype_code(w["conv"].dtype), w["dt_bias"], w["a_log"], w["norm"], tail, state,
+                                     slots, out, dtype_code(a.dtype), S, at_a, at_g, ra, rg, x.shape[1], taps,
+                                     state.shape[0], heads, kv, d, dv, unit_eps, float(d) ** -0.5, eps, 1 if early else
+                                     0, err)
     return out
 
 
@@ -1903,12 +1848,10 @@ LINEAR_STATE_WORK_BYTES = 64 << 20
 
 def rotation_table(positions: torch.Tensor, inv_freq: torch.Tensor) -> torch.Tensor:
     """float32 [T, pairs, 2]: cosine and sine of positions[t] * inv_freq[i]."""
-    lib = build.load_library("linear_state")
     T, half = positions.numel(), inv_freq.numel()
     assert positions.dtype is torch.int32 and inv_freq.dtype is torch.float64
     table = torch.empty((T, half, 2), dtype=torch.float32, device=positions.device)
-    _check(lib.rllm_rotation_table(_ptr(positions), _ptr(inv_freq), c_int(T), c_int(half), _ptr(table), _stream()),
-           "rotation_table")
+    _entries.rllm_rotation_table(positions, inv_freq, T, half, table)
     return table
 
 
@@ -1966,20 +1909,16 @@ def linear_state_scan(a: torch.Tensor, state: torch.Tensor, q_start: torch.Tenso
             work = torch.empty(seg * S * heads * d * (dv + 1), dtype=torch.float32, device=a.device)
             gsum = work[seg * S * heads * d * dv:]
             for chunk0 in range(0, chunks, seg):
-                _check(lib.rllm_linear_state_chunked(
-                    _ptr(a), c_int(stride), _ptr(decay), _ptr(table), c_int(rotary_dim), c_float(k_scale), _ptr(f_bias),
-                    _ptr(lower), _ptr(norm), c_float(eps), c_int(1 if gated else 0), _ptr(state), _ptr(work), _ptr(gsum),
-                    _ptr(q_start[num_decode:]), _ptr(slots[num_decode:]), c_int(state.shape[0]), c_int(S), c_int(chunk0),
-                    c_int(seg), c_int(heads), c_int(d), c_int(dv), _ptr(out), _ptr(err), _stream()), "linear_state_chunked")
+                _entries.rllm_linear_state_chunked(a, stride, decay, table, rotary_dim, k_scale, f_bias, lower, norm,
+                                                   eps, 1 if gated else 0, state, work, gsum, q_start[num_decode:],
+                                                   slots[num_decode:], state.shape[0], S, chunk0, seg, heads, d, dv,
+                                                   out, err)
             return out
     raw = torch.empty((T, heads * dv), dtype=torch.float32, device=a.device) \
         if int(lib.rllm_linear_state_needs_raw(c_int(d), c_int(dv))) else None
-    _check(lib.rllm_linear_state_walk(_ptr(a), c_int(stride), c_int(dtype_code(a.dtype)), _ptr(decay),
-                                      _ptr(inv_freq if rotary_dim else None), c_int(rotary_dim), c_float(k_scale),
-                                      _ptr(f_bias), _ptr(lower), _ptr(norm), c_float(eps), c_int(1 if gated else 0),
-                                      _ptr(positions), _ptr(state), _ptr(q_start), _ptr(slots), c_int(state.shape[0]),
-                                      c_int(num_seqs), c_int(T), c_int(heads), c_int(d), c_int(dv), _ptr(out), _ptr(raw),
-                                      c_int(1 if early else 0), _ptr(err), _stream()), "linear_state_walk")
+    _entries.rllm_linear_state_walk(a, stride, dtype_code(a.dtype), decay, inv_freq if rotary_dim else None, rotary_dim,
+                                    k_scale, f_bias, lower, norm, eps, 1 if gated else 0, positions, state, q_start,
+                                    slots, state.shape[0], num_seqs, T, heads, d, dv, out, raw, 1 if early else 0, err)
     return out
 
 
@@ -1997,7 +1936,6 @@ def talking_prep(qkv: torch.Tensor, positions: torch.Tensor, token_seq: torch.Te
     goes to kcache [pages, 1, page, dkp], the values to vcache [pages, 1, page, nkv * places] (zeros behind each head's
     dv).  ``v_other`` [T, nkv dv] (a column slice will do), ``other_bias`` float32 [nkv dv], ``lam`` float32 [1]:
     v <- (1 - lam) v + lam (v_other + other_bias)."""
-    lib = build.load_library("talking_heads")
     T, dkp, vrow = qkv.shape[0], kcache.shape[3], vcache.shape[3]
     assert qkv.stride(1) == 1 and qkv.shape[1] >= nq * dk + nkv * (dk + dv) and vrow % nkv == 0
     assert kcache.shape[1] == vcache.shape[1] == 1 and kcache.dtype is qkv.dtype and vcache.dtype is qkv.dtype
@@ -2011,13 +1949,12 @@ def talking_prep(qkv: torch.Tensor, positions: torch.Tensor, token_seq: torch.Te
         assert other_bias.dtype is torch.float32 and other_bias.numel() == nkv * dv and other_bias.is_contiguous()
         assert lam.dtype is torch.float32 and lam.numel() == 1
     q_out = torch.empty((T, nq * dkp), dtype=qkv.dtype, device=qkv.device)
-    _check(lib.rllm_talking_prep(
-        _ptr(qkv), c_int(qkv.stride(0) if T > 1 else qkv.shape[1]), c_int(dtype_code(qkv.dtype)), _ptr(positions),
-        _ptr(token_seq), _ptr(bias), _ptr(talk), _ptr(inv_freq if rotary_dim else None), c_int(rotary_dim), _ptr(v_other),
-        c_int(v_other.stride(0) if v_other is not None else 0), _ptr(other_bias if v_other is not None else None),
-        _ptr(lam if v_other is not None else None), _ptr(block_table), c_int(block_table.shape[1]), _ptr(kcache),
-        _ptr(vcache), c_int(kcache.shape[2]), c_int(kcache.shape[0]), c_int(T), c_int(nq), c_int(nkv), c_int(dk),
-        c_int(dv), c_int(dkp), c_int(vrow // nkv), _ptr(q_out), _ptr(err), _stream()), "talking_prep")
+    _entries.rllm_talking_prep(qkv, qkv.stride(0) if T > 1 else qkv.shape[1], dtype_code(qkv.dtype), positions,
+                               token_seq, bias, talk, inv_freq if rotary_dim else None, rotary_dim, v_other,
+                               v_other.stride(0) if v_other is not None else 0, other_bias if v_other is not None else
+                               None, lam if v_other is not None else None, block_table, block_table.shape[1], kcache,
+                               vcache, kcache.shape[2], kcache.shape[0], T, nq, nkv, dk, dv, dkp, vrow // nkv, q_out,
+                               err)
     return q_out
 
 
@@ -2042,16 +1979,13 @@ def shared_key_attention_tcgen05(q: torch.Tensor, out: torch.Tensor, kcache: tor
     """Attention of the prompt portions of sequences seq_begin .. seq_end-1 where all heads read one key row a token: q
     [T, nq * dkp], kcache [pages, 1, page, dkp], vcache [pages, 1, page, nkv * places] (dv of each), out [T, nq * dv];
     key j is visible to position i if j <= i and (i - j < window (0: always) or j < keep_first)."""
-    lib = build.load_library("shared_key_attention")
     _contig(q, "q"); _contig(out, "out"); _contig(kcache, "kcache"); _contig(vcache, "vcache"); _contig(block_table, "block_table")
     dkp, dvp = kcache.shape[3], vcache.shape[3] // nkv
     assert q.dtype is kcache.dtype is vcache.dtype is out.dtype is torch.bfloat16
     assert q.shape[1] == nq * dkp and out.shape == (q.shape[0], nq * dv)
-    _check(lib.rllm_shared_key_attention_tcgen05(
-        _ptr(q), c_int(q.shape[0]), _ptr(out), _ptr(kcache), _ptr(vcache), _ptr(block_table), c_int(block_table.shape[1]),
-        _ptr(q_start), _ptr(seq_lens), c_int(seq_begin), c_int(seq_end), c_int(num_tokens), c_int(nq), c_int(nkv), c_int(dkp),
-        c_int(dv), c_int(dvp), c_int(kcache.shape[2]), c_int(kcache.shape[0]), c_int(window), c_int(keep_first),
-        c_float(scale), _ptr(err), _stream()), "shared_key_attention_tcgen05")
+    _entries.rllm_shared_key_attention_tcgen05(q, q.shape[0], out, kcache, vcache, block_table, block_table.shape[1],
+                                               q_start, seq_lens, seq_begin, seq_end, num_tokens, nq, nkv, dkp, dv, dvp,
+                                               kcache.shape[2], kcache.shape[0], window, keep_first, scale, err)
 
 
 def shared_key_attention_mma(q: torch.Tensor, out: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor,
@@ -2079,17 +2013,14 @@ def shared_key_attention_mma(q: torch.Tensor, out: torch.Tensor, kcache: torch.T
             work = torch.empty(n, dtype=torch.float32, device=q.device)
         else:
             split, nsplit = 0, 1
-    _check(lib.rllm_shared_key_attention_mma(
-        _ptr(q), _ptr(out), _ptr(kcache), _ptr(vcache), _ptr(block_table), c_int(block_table.shape[1]), _ptr(q_start),
-        _ptr(seq_lens), c_int(num_seqs), c_int(max_q_len), c_int(nq), c_int(nkv), c_int(dkp), c_int(dv), c_int(dvp),
-        c_int(kcache.shape[2]), c_int(kcache.shape[0]), c_int(window), c_int(keep_first), c_float(scale), c_int(split),
-        c_int(nsplit), _ptr(work), _ptr(err), _stream()), "shared_key_attention_mma")
+    _entries.rllm_shared_key_attention_mma(q, out, kcache, vcache, block_table, block_table.shape[1], q_start, seq_lens,
+                                           num_seqs, max_q_len, nq, nkv, dkp, dv, dvp, kcache.shape[2], kcache.shape[0],
+                                           window, keep_first, scale, split, nsplit, work, err)
 
 
 def softcap_rows(x: torch.Tensor, cap: float) -> torch.Tensor:
     """x <- cap * tanh(x / cap) in place; x float32, contiguous."""
-    lib = build.load_library("elementwise")
     assert x.dtype is torch.float32 and cap > 0
     _contig(x, "x")
-    _check(lib.rllm_softcap(_ptr(x), c_longlong(x.numel()), c_float(cap), _stream()), "softcap_rows")
+    _entries.rllm_softcap(x, x.numel(), cap)
     return x

@@ -39,6 +39,10 @@ def linear(x, weight: torch.Tensor, out_dtype: Optional[torch.dtype] = None, res
         tanh_norm = norm.elementwise() if w_next is not None and hasattr(norm, "elementwise") else None
         parts, scaled = ops.gemm_small_m_residual(x, weight, h, w_next, tanh_norm=tanh_norm)
         return RowSumsq(parts, scaled, w_next)
+    if out_dtype is None or out_dtype is torch.float32 or out_dtype is x.dtype:
+        fast = ops.product(x, weight, out_dtype is torch.float32)
+        if fast is not None:
+            return fast
     assert x.dim() == 2 and weight.dim() == 2 and x.shape[1] == weight.shape[1], (x.shape, weight.shape)
     if not x.is_cuda:
         raise ops.KernelError("linear: CUDA tensors only; the engine has no CPU path")

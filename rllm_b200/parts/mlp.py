@@ -74,6 +74,10 @@ class GatedMLP(FeedForward):
         return self.activation == "silu" and fused_residual_takes(num_rows, dtype, self.w_gate_up, self.w_down)
 
     def forward(self, x, residual=None):
+        if self.activation == "silu" and not isinstance(x, ScaledRows):
+            act = ops.product(x, self.w_gate_up, silu=True, gate=self.gate)
+            if act is not None:
+                return linear(act, self.w_down, residual=residual)
         act = (x.x if isinstance(x, ScaledRows) else x).new_empty((x.shape[0], self.inter))
         if self.activation != "silu":
             ops.act_mul(linear(x, self.w_gate_up), act, self.activation)
