@@ -346,11 +346,16 @@ RLLM_EXPORT int rllm_argmax(const float* logits, int R, int V, int ld, int* out_
 // cut.  What bounds it is the chain of barriers (maximum, mass, two a radix pass) with a few microseconds of work between
 // two of them.  Microseconds at 128,256 logits, against the same chain as separate kernels (4 to 14 launches, every one
 // reading the logits again): 8 rows, temperature 29 -> 16, top-p 151 -> 39, top-k 130 -> 31, all options 208 -> 50;
-// 64 rows 59 -> 41, 465 -> 107, 375 -> 81, 677 -> 127.
+// 64 rows 59 -> 41, 465 -> 107, 375 -> 81, 677 -> 127.  Then with the other CTAs' numbers read a lane a CTA, and a list of the
+// last keys instead of a third pass, one launch after another: 8 rows 14.7 -> 14.0, 37.4 -> 35.0, 30.5 -> 27.6, 49.4 -> 43.9;
+// 64 rows 37.8 -> 36.6, 102.5 -> 96.0, 77.7 -> 71.7, 123.8 -> 108.7; 8 rows of 32,768 9.5 -> 8.4, 26.4 -> 23.2, 25.0 -> 21.5,
+// 40.0 -> 34.8.
 // ---------------------------------------------------------------------------
 #define SC_BINS 2048
 #define SC_SELECT_BYTES (SC_BINS * 8 + SC_BINS * 4 + SC_BINS * 8)      // the last term over the CTAs of a row
 #define SC_STAGED_MAX (176 * 1024)       // bytes of a range that are kept in shared memory; a longer one is read again
+#define SC_CTAS 8                        // the most CTAs of a row
+#define SC_CAND 64                       // keys of a range that are listed behind the second pass
 #define SC_WORDS_MAX (1 << 18)           // weights of a range that three words of 14 bits and 32 to count them hold
 
 __device__ __forceinline__ unsigned sc_addr(const void* p, int rank) {
@@ -361,6 +366,11 @@ __device__ __forceinline__ unsigned sc_addr(const void* p, int rank) {
 __device__ __forceinline__ unsigned long long sc_ld64(const void* p, int rank) {
   unsigned long long v;
   asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(sc_addr(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned sc_ld32(const void* p, int rank) {
+  unsigned v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(sc_addr(p, rank)) : "memory");
   return v;
 }
 __device__ __forceinline__ void sc_barrier() {
@@ -383,8 +393,9 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
   __shared__ ArgMax sm_arg[32];
   __shared__ __align__(8) ArgMax range_best;          // read by the other CTAs as one word of 64 bits
   __shared__ unsigned long long wsum[WARPS], range_sum, slice_sum, sh_cum;
-  __shared__ int sh_pick, sh_bin;
-  __shared__ unsigned long long sh_rest;
+  __shared__ int sh_pick, sh_bin, cand_n;
+  __shared__ unsigned long long sh_rest, all_mass[SC_CAND * SC_CTAS];
+  __shared__ unsigned cand[SC_CAND], all_cand[SC_CAND * SC_CTAS], cand_top;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r = blockIdx.y, cs = gridDim.x, rank = blockIdx.x;       // the cluster is the whole x dimension
   pdl_wait_on(logits, temperature, top_k, top_p, min_p, seeds, gen_index);
@@ -415,9 +426,17 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
   best = block_argmax(best, sm_arg);
   if (tid == 0) range_best = best;
   sc_barrier();
-  for (int c = 0; c < cs; ++c) {
-    const unsigned long long u = sc_ld64(&range_best, c);
-    ArgMax b; b.v = __uint_as_float((unsigned)u); b.i = (int)(u >> 32);
+  {                                                   // a lane a range: one trip to the others' memory
+    ArgMax b; b.v = -INFINITY; b.i = 0x7fffffff;
+    if (lane < cs) {
+      const unsigned long long u = sc_ld64(&range_best, lane);
+      b.v = __uint_as_float((unsigned)u); b.i = (int)(u >> 32);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      ArgMax c; c.v = __shfl_xor_sync(0xffffffffu, b.v, o); c.i = __shfl_xor_sync(0xffffffffu, b.i, o);
+      b = argmax_better(b, c);
+    }
     best = argmax_better(best, b);
   }
   if (greedy || best.v == -INFINITY) {
@@ -436,6 +455,43 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
     unsigned long long cum = 0;
     for (int pass = 0; pass < 3; ++pass) {
       const int shift = pass == 0 ? 21 : (pass == 1 ? 10 : 0);
+      if (pass == 2) {
+        // The keys that share 22 bits with the threshold are few in a row of unlike values: every range lists its own, and
+        // every CTA adds them up for itself (a barrier and a look at a few dozen keys instead of a pass over bins with two
+        // barriers).  A longer list anywhere: the pass.
+        if (tid == 0) { cand_n = 0; cand_top = 0u; }
+        __syncthreads();
+        for (int i = tid; i < n; i += THREADS) {
+          const unsigned key = f2key(value(i));
+          if (key < floor_key || (key & himask) != prefix) continue;
+          const int at = atomicAdd(&cand_n, 1);
+          if (at < SC_CAND) cand[at] = key;
+        }
+        sc_barrier();
+        const int mine = lane < cs ? (int)sc_ld32(&cand_n, lane) : 0;
+        if (!__any_sync(0xffffffffu, mine > SC_CAND)) {
+          int total = 0;                                // the lists one behind the other, all of them here
+          for (int c = 0; c < cs; ++c) {
+            const int m = __shfl_sync(0xffffffffu, mine, c);
+            if (tid < m) {
+              const unsigned key = sc_ld32(&cand[tid], c);
+              all_cand[total + tid] = key;
+              all_mass[total + tid] = by_mass ? fx_mass(key2f(key), mx) : 1ull;
+            }
+            total += m;
+          }
+          __syncthreads();
+          for (int i = tid; i < total; i += THREADS) {
+            const unsigned key = all_cand[i];
+            unsigned long long w = cum;
+            for (int j = 0; j < total; ++j) w += all_cand[j] >= key ? all_mass[j] : 0ull;
+            if (w >= target) atomicMax(&cand_top, key);
+          }
+          __syncthreads();
+          return max(cand_top, prefix);                 // (none reaches the target: all of them)
+        }
+        sc_barrier();                                   // the lists have been looked at everywhere
+      }
       // A weight's 41 bits are added up as three words of 14, with native 32-bit atomics; two of the words stand where
       // the bins' sums will.  A range of more than 2^18 weights could run over them: it takes two words and the carry, which
       // an atomic has to come back with.
@@ -569,9 +625,15 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
     if (lane == 0) range_sum = t;
   }
   sc_barrier();
-  if (tid == 0) {
-    unsigned long long total = 0;
-    for (int c = 0; c < cs; ++c) total += sc_ld64(&range_sum, c);
+  if (warp == 0) {                                    // a lane a range, then a lane a warp's part
+    const unsigned long long mine = lane < cs ? sc_ld64(&range_sum, lane) : 0ull;
+    unsigned long long upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long v = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += v;
+    }
+    const unsigned long long total = __shfl_sync(0xffffffffu, upto, 31);
     unsigned w[4];
     const unsigned long long seed = seeds[r];
     const unsigned long long ctr = (unsigned long long)gen_index[r];
@@ -579,23 +641,25 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
     const unsigned long long u24 = w[0] >> 8;         // u = u24 / 2^24 in [0, 1)
     const unsigned long long thi = __umul64hi(total, u24), tlo = total * u24;
     const unsigned long long target = (thi << 40) | (tlo >> 24);  // floor(total * u)
-    unsigned long long c = 0;
+    // the first range whose running sum exceeds the target, else the last; in it the first warp's part
+    const unsigned over = __ballot_sync(0xffffffffu, lane < cs && upto > target);
+    const int range = over ? __ffs(over) - 1 : cs - 1;
+    const unsigned long long ahead = __shfl_sync(0xffffffffu, upto - mine, range);
     int pick = -1;
-    for (int q = 0; q < cs && pick < 0; ++q) {
-      const unsigned long long s = sc_ld64(&range_sum, q);
-      if (c + s > target || q == cs - 1) pick = q; else c += s;
-    }
-    if (pick == rank) {
-      int pw = -1;
-      for (int q = 0; q < WARPS && pw < 0; ++q) {
-        if (c + wsum[q] > target || q == WARPS - 1) pw = q; else c += wsum[q];
+    if (range == rank) {
+      const unsigned long long part_sum = lane < WARPS ? wsum[lane] : 0ull;
+      unsigned long long run = part_sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long v = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += v;
       }
-      pick = pw;
-      sh_rest = target - c;                           // what is left to pass inside the picked warp's part
-    } else {
-      pick = -1;
+      const unsigned past = __ballot_sync(0xffffffffu, lane < WARPS && ahead + run > target);
+      pick = past ? __ffs(past) - 1 : WARPS - 1;
+      const unsigned long long before = __shfl_sync(0xffffffffu, run - part_sum, pick);
+      if (lane == 0) sh_rest = target - ahead - before;     // what is left to pass inside the picked warp's part
     }
-    sh_pick = pick;
+    if (lane == 0) sh_pick = pick;
   }
   sc_barrier();                                       // the last read of another CTA's shared memory lies behind this
   if (warp != sh_pick) return;
