@@ -34,21 +34,50 @@ class SamplingRow:
     eos_token_ids: Sequence[int] = ()
 
 
+class _OptionViews:
+    """R rows' options in a pinned buffer and on the device, and the views through which they are written and read: int64
+    first (seeds, token indices), then float32 bits (temperature, top_p, min_p) and int32 (top_k), so that one copy takes
+    them.  Kept, since the views of a batch cost the host as much as its launch."""
+
+    def __init__(self, pinned: torch.Tensor, copied: torch.cuda.Event, device: torch.Tensor, R: int):
+        host = pinned.numpy()
+        ints = host[: 4 * R].view(np.uint64).reshape(2, R)
+        self.copied = copied
+        self.seeds, self.gen = ints[0], ints[1].view(np.int64)
+        self.floats = host[4 * R: 7 * R].view(np.float32).reshape(3, R)
+        self.top_k = host[7 * R: 8 * R]
+        self.pinned, self.device = pinned[: 8 * R], device[: 8 * R]
+        i = device[: 4 * R].view(torch.int64).view(2, R)
+        f = device[4 * R: 7 * R].view(torch.float32).view(3, R)
+        # temperature, top_k, top_p, min_p, seeds, token indices: as ``ops.sample`` takes them
+        self.args = (f[0], device[7 * R: 8 * R], f[1], f[2], i[0], i[1])
+
+    def send(self) -> None:
+        self.device.copy_(self.pinned, non_blocking=True)
+        self.copied.record()
+
+
 class Sampler:
     def __init__(self, device: torch.device):
         self.device = device
 
-    def _option_buffers(self, R: int):
-        """(numpy view of a pinned int32 buffer, device buffer, event of the last copy from it); pinned
-        buffers are used in turn so that filling one does not wait for the copy of the call before."""
+    def _option_buffers(self, R: int) -> "_OptionViews":
+        """Where R rows' options go; pinned buffers are used in turn so that filling one does not wait for the copy of the
+        call before."""
         if not hasattr(self, "_pinned") or self._pinned[0][0].numel() < 8 * R:
             n = max(8 * R, 8 * 256)
             self._pinned = [(torch.zeros(n, dtype=torch.int32, pin_memory=True), torch.cuda.Event()) for _ in range(4)]
             self._devbuf = [torch.zeros(n, dtype=torch.int32, device=self.device) for _ in range(4)]
+            self._views = [{} for _ in range(4)]
             self._slot = 0
         self._slot = (self._slot + 1) % 4
-        t, ev = self._pinned[self._slot]
-        return t.numpy(), self._devbuf[self._slot], ev
+        made = self._views[self._slot]
+        v = made.get(R)
+        if v is None:
+            if len(made) >= 64:                   # as many batch sizes as a server has decode graphs
+                made.clear()
+            v = made[R] = _OptionViews(*self._pinned[self._slot], self._devbuf[self._slot], R)
+        return v
 
     def _dev(self, arr: np.ndarray) -> torch.Tensor:
         return torch.from_numpy(arr).to(self.device, non_blocking=False)
@@ -125,27 +154,22 @@ class Sampler:
         if all(row.params.greedy for row in rows):
             ops.argmax(logits, out)
             return out
-        # all per-row options in one pinned buffer and one copy: int64 first (seeds, token indices),
-        # then float32 bits (temperature, top_p, min_p) and int32 (top_k)
-        host, dev, copied = self._option_buffers(R)
-        copied.synchronize()                      # the copy that last read this pinned buffer is through
-        s = host[: 4 * R].view(np.int64).reshape(2, R)
-        f = host[4 * R: 7 * R].view(np.float32).reshape(3, R)
-        k = host[7 * R: 8 * R]
+        v = self._option_buffers(R)
+        v.copied.synchronize()                    # the copy that last read this pinned buffer is through
         params = [row.params for row in rows]
+        f = v.floats
         f[0], f[1], f[2] = [p.temperature for p in params], [p.top_p for p in params], [p.min_p for p in params]
         for r, p in enumerate(params):
-            k[r] = p.top_k                        # one by one: a number beyond 32 bits is refused
-        s.view(np.uint64)[0] = [row.seed & 0xFFFFFFFFFFFFFFFF for row in rows]
-        s[1] = [row.gen_index for row in rows]
-        with torch.cuda.device(self.device):
-            dev[: 8 * R].copy_(self._pinned[self._slot][0][: 8 * R], non_blocking=True)
-            copied.record()
-        sd = dev[: 4 * R].view(torch.int64).view(2, R)
-        fd = dev[4 * R: 7 * R].view(torch.float32).view(3, R)
-        kd = dev[7 * R: 8 * R]
+            v.top_k[r] = p.top_k                  # one by one: a number beyond 32 bits is refused
+        v.seeds[:] = [row.seed & 0xFFFFFFFFFFFFFFFF for row in rows]
+        v.gen[:] = [row.gen_index for row in rows]
+        if self.device.index is not None and torch.cuda.current_device() == self.device.index:
+            v.send()
+        else:
+            with torch.cuda.device(self.device):
+                v.send()
         V = logits.shape[1]
         # the top-k / top-p kernels are left out when no row uses them
         select = any(1 < row.params.top_k < V or 0.0 < row.params.top_p < 1.0 for row in rows)
-        ops.sample(logits, fd[0], kd, fd[1], fd[2], sd[0], sd[1], out, with_select=select)
+        ops.sample(logits, *v.args, out, with_select=select)
         return out
