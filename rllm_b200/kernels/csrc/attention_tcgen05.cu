@@ -68,7 +68,13 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                          const int* __restrict__ block_table, int max_blocks, const int* __restrict__ q_start,
                          const int* __restrict__ seq_lens, int seq_begin, int seq_end, int nq, int nkv,
                          int page_size, int num_pages, int window, float scale_log2, int* __restrict__ err,
-                         AtOpts opt) {
+                         AtOpts opt, int beside) {
+  // beside: the kernel ahead wrote nothing that this one reads or writes (the attention of the tokens that decode), and
+  // it lets this one in only when the kernel ahead of it is complete: the two run side by side, and this one ends behind it.
+  if (!beside) {
+    pdl_wait();
+    pdl_launch();
+  }
   constexpr int AT_BN = 8192 / AT_D;              // keys a tile
   constexpr int DP = AT_D / 64;                   // panels of head dims (Q, K, V)
   constexpr int KPANEL = AT_BN * 128;             // bytes of a K or V panel: BN rows of 128 bytes
@@ -504,6 +510,10 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   if (warp == 1) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_s), "r"(256) : "memory");
   }
+  if (beside) {
+    pdl_wait();
+    pdl_launch();
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -511,7 +521,7 @@ template <int D, bool OPT>
 static int at_launch(const void* q, int q_stride, int num_q_rows, void* out, const void* kcache, const void* vcache,
                      const int* block_table, int max_blocks, const int* q_start, const int* seq_lens, int seq_begin,
                      int seq_end, int num_tokens, int nq, int nkv, int page_size, int num_pages, int window,
-                     float scale, int* err, cudaStream_t stream, AtOpts opt) {
+                     float scale, int* err, cudaStream_t stream, AtOpts opt, int beside) {
   const int g = nq / nkv;
   CUtensorMap mq, mk, mv;
   {
@@ -537,8 +547,9 @@ static int at_launch(const void* q, int q_stride, int num_q_rows, void* out, con
   const long long tiles = (num_tokens + bq - 1) / bq + (seq_end - seq_begin);
   if (tiles * nkv > 0x7fffffffLL) return RLLM_E_UNSUPPORTED;
   dim3 grid((unsigned)(tiles * nkv));
-  attention_tcgen05_kernel<D, OPT><<<grid, AT_THREADS, at_smem_bytes<D>(), stream>>>(mq, mk, mv, (bf16*)out, block_table, max_blocks,
-      q_start, seq_lens, seq_begin, seq_end, nq, nkv, page_size, num_pages, window, scale * 1.4426950408889634f, err, opt);
+  rllm_launch_pdl(attention_tcgen05_kernel<D, OPT>, grid, dim3(AT_THREADS), (size_t)at_smem_bytes<D>(), stream, mq, mk, mv, (bf16*)out,
+                  block_table, max_blocks, q_start, seq_lens, seq_begin, seq_end, nq, nkv, page_size, num_pages, window,
+                  scale * 1.4426950408889634f, err, opt, beside);
   RLLM_LAUNCH_CHECK();
   return 0;
 }
@@ -552,7 +563,7 @@ static int at_prefill(const void* q, int q_stride, int num_q_rows, void* out,
                       int max_blocks, const int* q_start, const int* seq_lens,
                       int seq_begin, int seq_end, int num_tokens, int nq, int nkv, int d,
                       int page_size, int num_pages, int window, float scale, int* err,
-                      cudaStream_t stream, AtOpts opt) {
+                      cudaStream_t stream, AtOpts opt, int beside = 0) {
   if (seq_end <= seq_begin || num_tokens <= 0) return 0;
   if (nq <= 0 || nkv <= 0 || nq % nkv || num_pages <= 0 || max_blocks <= 0 || window < 0 || !(scale > 0.f) || !err)
     return RLLM_E_BADARG;
@@ -563,20 +574,21 @@ static int at_prefill(const void* q, int q_stride, int num_q_rows, void* out,
     return RLLM_E_UNSUPPORTED;
   if ((long long)num_pages * nkv * page_size > 0x7fffffffLL) return RLLM_E_UNSUPPORTED;   // cache rows are TMA coordinates
 #define AT_LAUNCH(DD) return at_launch<DD, OPT>(q, q_stride, num_q_rows, out, kcache, vcache, block_table, max_blocks, q_start, \
-      seq_lens, seq_begin, seq_end, num_tokens, nq, nkv, page_size, num_pages, window, scale, err, stream, opt)
+      seq_lens, seq_begin, seq_end, num_tokens, nq, nkv, page_size, num_pages, window, scale, err, stream, opt, beside)
   if (d == 64) AT_LAUNCH(64);
   AT_LAUNCH(128);
 }
 
+// beside: see the kernel's; only behind rllm_attention_decode_bf16 on the same stream, of other sequences.
 RLLM_EXPORT int rllm_attention_prefill_tcgen05(const void* q, int q_stride, int num_q_rows, void* out,
                                                const void* kcache, const void* vcache, const int* block_table,
                                                int max_blocks, const int* q_start, const int* seq_lens,
                                                int seq_begin, int seq_end, int num_tokens, int nq, int nkv, int d,
                                                int page_size, int num_pages, int window, float scale, int* err,
-                                               cudaStream_t stream) {
+                                               int beside, cudaStream_t stream) {
   return at_prefill<false>(q, q_stride, num_q_rows, out, kcache, vcache, block_table, max_blocks, q_start, seq_lens,
                            seq_begin, seq_end, num_tokens, nq, nkv, d, page_size, num_pages, window, scale, err, stream,
-                           AtOpts{0, 0, 0.f, nullptr, nullptr, 0, 0, nullptr});
+                           AtOpts{0, 0, 0.f, nullptr, nullptr, 0, 0, nullptr}, beside);
 }
 
 // The same with the options of the head comment; gate [num_q_rows, gate_stride], a row per row of q.

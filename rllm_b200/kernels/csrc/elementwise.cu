@@ -244,6 +244,8 @@ __global__ void rope_kv_write_kernel(T* __restrict__ qkv, const int* __restrict_
                                      int d, int page_size, int num_pages, int write_kv,
                                      int* __restrict__ err) {
   extern __shared__ float cs[];  // cos[rd/2], sin[rd/2]
+  pdl_wait_on(qkv, positions, token_seq, block_table, kcache, vcache);
+  pdl_launch();
   const int t = blockIdx.x;
   const int pos = positions[t];
   const int half = rotary_dim >> 1;
@@ -303,6 +305,8 @@ __global__ void rope_kv_write_bf16x8_kernel(bf16* __restrict__ qkv, const int* _
                                             int d, int page_size, int num_pages, int write_kv,
                                             int* __restrict__ err) {
   extern __shared__ float cs[];  // cos[rd/2], sin[rd/2]
+  pdl_wait_on(qkv, positions, token_seq, block_table, kcache, vcache);
+  pdl_launch();
   const int t = blockIdx.x;
   const int pos = positions[t];
   const int half = rotary_dim >> 1;
@@ -371,13 +375,13 @@ RLLM_EXPORT int rllm_rope_kv_write(void* qkv, int dtype, const int* positions, c
   if (smem > 48 * 1024) return RLLM_E_UNSUPPORTED;
   if (dtype == RLLM_DT_BF16 && d % 16 == 0 && rotary_dim % 16 == 0 && rotary_dim > 0 &&
       (((uintptr_t)qkv | (uintptr_t)kcache | (uintptr_t)vcache) & 15) == 0) {
-    rope_kv_write_bf16x8_kernel<<<T, 128, smem, stream>>>((bf16*)qkv, positions, token_seq, inv_freq, rotary_dim,
-        block_table, max_blocks, (bf16*)kcache, (bf16*)vcache, nq, nkv, d, page_size, num_pages, write_kv, err);
+    rllm_launch_pdl(rope_kv_write_bf16x8_kernel, dim3(T), dim3(128), smem, stream, (bf16*)qkv, positions, token_seq, inv_freq,
+        rotary_dim, block_table, max_blocks, (bf16*)kcache, (bf16*)vcache, nq, nkv, d, page_size, num_pages, write_kv, err);
     RLLM_LAUNCH_CHECK();
     return 0;
   }
   RLLM_DISPATCH_DTYPE(dtype, T_,
-    (rope_kv_write_kernel<T_><<<T, 128, smem, stream>>>((T_*)qkv, positions, token_seq, inv_freq,
+    (rllm_launch_pdl(rope_kv_write_kernel<T_>, dim3(T), dim3(128), smem, stream, (T_*)qkv, positions, token_seq, inv_freq,
         rotary_dim, block_table, max_blocks, (T_*)kcache, (T_*)vcache, nq, nkv, d, page_size,
         num_pages, write_kv, err)));
   RLLM_LAUNCH_CHECK();

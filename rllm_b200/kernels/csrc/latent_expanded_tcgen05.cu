@@ -44,6 +44,8 @@ latent_expanded_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                        const __grid_constant__ CUtensorMap map_r, bf16* __restrict__ out, const int* __restrict__ q_start,
                        const int* __restrict__ seq_lens, int seq_begin, int seq_end, int heads, int rot, int window,
                        float scale_log2, const float* __restrict__ sink, int* __restrict__ err) {
+  pdl_wait();
+  pdl_launch();
   using Shape = LeShape<NQ, DV>;
   constexpr int BN = Shape::BN, PANEL = Shape::PANEL, NV = Shape::NV, VP = DV / 64, NOPE = (NQ - 1) * 64;
   extern __shared__ __align__(1024) unsigned char le_raw[];
@@ -357,8 +359,9 @@ static int le_launch(const CUtensorMap& mq, const CUtensorMap& mkv, const CUtens
                      float scale, const float* sink, int* err, cudaStream_t stream) {
   static SmemLimit limit;
   if (const int e = limit.allow(latent_expanded_kernel<NQ, DV>, LeShape<NQ, DV>::SMEM)) return e;
-  latent_expanded_kernel<NQ, DV><<<dim3((unsigned)(tiles * heads)), LE_THREADS, LeShape<NQ, DV>::SMEM, stream>>>(
-      mq, mkv, mr, (bf16*)out, q_start, seq_lens, seq_begin, seq_end, heads, rot, window, scale * 1.4426950408889634f, sink, err);
+  rllm_launch_pdl(latent_expanded_kernel<NQ, DV>, dim3((unsigned)(tiles * heads)), dim3(LE_THREADS), (size_t)LeShape<NQ, DV>::SMEM, stream,
+                  mq, mkv, mr, (bf16*)out, q_start, seq_lens, seq_begin, seq_end, heads, rot, window, scale * 1.4426950408889634f,
+                  sink, err);
   RLLM_LAUNCH_CHECK();
   return 0;
 }

@@ -116,7 +116,7 @@ _TABLE = {
     "rllm_gated_postnorm_add": ("layer_glue", "pppippippfppfplippiiii", "gated_postnorm_add"),
     "rllm_attention_decode_bf16": ("attention_mma", "pippppipiiiiiiiifpiippp", "attention_decode_bf16"),
     "rllm_attention_decode_bf16_opts": ("attention_mma", "pippppipiiiiiiiifiifppiipiipfpppp", "attention_decode_bf16_opts"),
-    "rllm_attention_prefill_tcgen05": ("attention_tcgen05", "piippppippiiiiiiiiifp", "attention_prefill_tcgen05"),
+    "rllm_attention_prefill_tcgen05": ("attention_tcgen05", "piippppippiiiiiiiiifpi", "attention_prefill_tcgen05"),
     "rllm_attention_prefill_tcgen05_opts": ("attention_tcgen05", "piippppippiiiiiiiiifiifppiipp", "attention_prefill_tcgen05_opts"),
     "rllm_attention_prefill_bf16": ("attention_mma", "pippppippiiiiiiiiifp", "attention_prefill_bf16"),
     "rllm_attention_prefill_bf16_opts": ("attention_mma", "pippppippiiiiiiiiifiifppiipp", "attention_prefill_bf16_opts"),
@@ -597,10 +597,12 @@ def attention_prefill_tcgen05(q: torch.Tensor, q_stride: int, out: torch.Tensor,
                               nkv: int, d: int, window: int, scale: float, err: torch.Tensor, keep_first: int = 0,
                               chunk: int = 0, softcap: float = 0.0, sinks: Optional[torch.Tensor] = None,
                               gate: Optional[torch.Tensor] = None, gate_per_head: bool = False,
-                              slopes: Optional[torch.Tensor] = None) -> None:
+                              slopes: Optional[torch.Tensor] = None, beside_decode: bool = False) -> None:
     """Attention of the prompt portions of sequences seq_begin .. seq_end-1 on the
     tcgen05 tensor cores (same contract and options as ``attention_prefill_bf16``; ``q`` is the
-    first of ``q.shape[0]`` rows of ``q_stride`` elements)."""
+    first of ``q.shape[0]`` rows of ``q_stride`` elements).  ``beside_decode``: the call right ahead on this stream was
+    ``attention_decode_bf16`` of other sequences, and what wrote q and the pages came ahead of that: the two attentions run
+    side by side (without options)."""
     _contig(out, "out"); _contig(kcache, "kcache"); _contig(vcache, "vcache"); _contig(block_table, "block_table")
     assert q.dtype is torch.bfloat16 and kcache.dtype is torch.bfloat16 and out.dtype is torch.bfloat16
     if keep_first or chunk or softcap or sinks is not None or gate is not None or slopes is not None:
@@ -613,7 +615,8 @@ def attention_prefill_tcgen05(q: torch.Tensor, q_stride: int, out: torch.Tensor,
         return
     _entries.rllm_attention_prefill_tcgen05(q, q_stride, q.shape[0], out, kcache, vcache, block_table,
                                             block_table.shape[1], q_start, seq_lens, seq_begin, seq_end, num_tokens, nq,
-                                            nkv, d, kcache.shape[2], kcache.shape[0], window, scale, err)
+                                            nkv, d, kcache.shape[2], kcache.shape[0], window, scale, err,
+                                            1 if beside_decode else 0)
 
 
 _decode_counters = {}

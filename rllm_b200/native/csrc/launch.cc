@@ -96,7 +96,7 @@ struct Row { const char* text; Invoke invoke; };
 const Row kSignatures[] = {
     ROW("piiiiippfpppipppfiiiiiip"), ROW("piiippipp"), ROW("piiippp"), ROW("piiippppp"), ROW("piiippppppp"),
     ROW("piiipppppppi"), ROW("piippifpppfippppiiiiiippip"), ROW("piippippppiiipiiip"),
-    ROW("piippppifpippiiiiiiipiiippififiip"), ROW("piippppippiiiiiiiiifiifppiipp"), ROW("piippppippiiiiiiiiifp"),
+    ROW("piippppifpippiiiiiiipiiippififiip"), ROW("piippppippiiiiiiiiifiifppiipp"), ROW("piippppippiiiiiiiiifpi"),
     ROW("piipppppipipppippiiiiiiiiipp"), ROW("piippppppppiiiiff"), ROW("piipppppppppiiipiiiip"), ROW("pipifpipiiiiifff"),
     ROW("pipipiiii"), ROW("pipipiiiiifff"), ROW("pipipiiiiifffp"), ROW("pipipippipippiii"), ROW("pippifpppfipppppiiiiiiipp"),
     ROW("pippiiipppiiiiiiiifpp"), ROW("pippippppipppppppiiiiiiiiiiiiifffip"), ROW("pipppipippiiiiiiifp"),

@@ -439,19 +439,22 @@ class PagedAttention(Mixer):
         window = int(self.window or 0)
         stride = qkv.shape[1]
         use_mma = ops.use_mma_attention(x.dtype, self.nq, self.nkv, self.d)
-        # sequences with one token: rotation, cache write and attention in one kernel
+        # sequences with one token: rotation, cache write and attention in one kernel.  It stands between the prompts' rotation
+        # and their attention, which runs beside it (on tcgen05: a step of 2,041 and 6 tokens had the GPU for the 6 alone for
+        # 14 us a layer)
         nd = ctx.num_decode if use_mma else 0
+        if T > nd:
+            ops.rope_kv_write(qkv[nd:], ctx.positions[nd:], ctx.token_seq[nd:], inv_freq, rd, table, cache.k,
+                              cache.v, self.nq, nkv_here, self.d, ctx.err, write_kv=writes)
         if nd:
             ops.attention_decode_bf16(qkv, stride, out, cache.k, cache.v, table, ctx.seq_lens, nd,
                                       max(ctx.seq_lens_host[:nd]), self.nq, self.nkv, self.d, window, self.scale,
                                       ctx.err, inv_freq=inv_freq, rotary_dim=rd, write_kv=writes)
         if T > nd:
-            ops.rope_kv_write(qkv[nd:], ctx.positions[nd:], ctx.token_seq[nd:], inv_freq, rd, table, cache.k,
-                              cache.v, self.nq, nkv_here, self.d, ctx.err, write_kv=writes)
             if ops.use_tcgen05_attention(x.dtype, self.nq, self.nkv, self.d, cache.k.shape[2]):
                 ops.attention_prefill_tcgen05(qkv, stride, out, cache.k, cache.v, table, ctx.q_start, ctx.seq_lens,
                                               nd, ctx.num_seqs, T - nd, self.nq, self.nkv, self.d, window,
-                                              self.scale, ctx.err)
+                                              self.scale, ctx.err, beside_decode=nd > 0)
             elif use_mma:
                 ops.attention_prefill_bf16(qkv, stride, out, cache.k, cache.v, table, ctx.q_start, ctx.seq_lens,
                                            nd, ctx.num_seqs, T - nd, self.nq, self.nkv, self.d, window,
