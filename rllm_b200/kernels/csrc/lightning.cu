@@ -18,9 +18,10 @@
 // walks its tokens from its start.  Results differ from the plain walk by rounding only.
 #include "lightning_walk.cuh"
 #include "lightning_mma.cuh"
+#include "lightning_tcgen05.cuh"
 
 // max_chunks 0: the plain walk.  > 0: ceil(longest portion / LT_CHUNK); work then holds
-// num_seqs * max_chunks * heads * d * dv floats.
+// num_seqs * max_chunks * heads * d * dv floats; act null, or (bfloat16) a row of heads (2 d + dv) values a token.
 RLLM_EXPORT int rllm_lightning_chunk() { return LT_CHUNK; }
 
 // RLLM_LIGHTNING=simt keeps the chunk passes on the CUDA cores (for tests and comparisons)
@@ -30,8 +31,8 @@ static inline bool lightning_mma_disabled() {
   return off == 1;
 }
 
-RLLM_EXPORT int rllm_lightning_scan(const void* q, const void* k, const void* v, int stride, int dtype,
-                                    const float* decay, float* state, float* work, const int* q_start,
+RLLM_EXPORT int rllm_lightning_scan(const void* q, const void* k, const void* v, int rows, int stride, int dtype,
+                                    const float* decay, float* state, float* work, void* act, const int* q_start,
                                     const int* slots, int num_slots, int num_seqs, int max_chunks, float* out,
                                     int heads, int d, int dv, int* err, cudaStream_t stream) {
   if (num_seqs <= 0) return 0;
@@ -41,6 +42,9 @@ RLLM_EXPORT int rllm_lightning_scan(const void* q, const void* k, const void* v,
   if ((long long)num_seqs * (max_chunks > 0 ? max_chunks : 1) > 65535) return RLLM_E_UNSUPPORTED;
   static_assert(LT_CHUNK == LTC_CHUNK, "the chain kernel serves both forms of the chunk passes");
   if (dtype == RLLM_DT_BF16 && max_chunks > 0 && !lightning_mma_disabled() && stride % 2 == 0) {
+    const int rc = lg_scan<false>((const bf16*)q, (const bf16*)k, (const bf16*)v, rows, stride, decay, LtSteps{}, state, work, (bf16*)act, q_start,
+                                  slots, num_slots, num_seqs, max_chunks, out, heads, d, dv, err, stream);
+    if (rc >= 0) return rc;
     // long portions of bfloat16 activations: the chunk passes on the tensor cores, where the head's sizes are built
     auto chain = [&]() {
       lightning_chain<false>(decay, LtSteps{}, state, work, q_start, slots, num_slots, num_seqs, max_chunks, heads, d, dv, stream);

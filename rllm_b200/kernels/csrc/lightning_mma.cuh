@@ -1,5 +1,6 @@
 // The lightning recurrence's chunk passes on the tensor cores (bfloat16 activations, mma.sync m16n8k16,
-// float32 accumulators), for heads whose sizes are instantiated below.  For a chunk of C = 64 tokens with
+// float32 accumulators), for heads whose sizes are instantiated below; where there are many of 64 or 128, or the portions are
+// short, lightning_tcgen05.cuh has a faster form (the line is in lg_scan).  For a chunk of C = 64 tokens with
 // start state S_0 (float32 [d, dv]) and decay lambda:
 //   pass 1 (end state from zero):   Z = (K * w)^T V,                 w_j = lambda^(n - 1 - j)
 //   pass 2 (outputs):               O = ((Q K^T) * D) V + diag(lambda^(t + 1)) (Q S_0),

@@ -13,6 +13,7 @@
 //                               square (eps inside the root), times a weight: one block a (token, group)
 #include "lightning_walk.cuh"
 #include "lightning_mma.cuh"
+#include "lightning_tcgen05.cuh"
 
 RLLM_EXPORT int rllm_ssd_chunk() { return LT_CHUNK; }
 
@@ -23,10 +24,10 @@ static inline bool ssd_mma_disabled() {
   return off == 1;
 }
 
-// xbc: rows of [x: heads * P | B: groups * N | C: groups * N] with row stride `stride`.  max_chunks 0: the plain
+// xbc: `rows` rows of [x: heads * P | B: groups * N | C: groups * N] with row stride `stride`.  max_chunks 0: the plain
 // walk.  > 0: ceil(longest portion / LT_CHUNK); work then holds num_seqs * max_chunks * heads * N * P floats and
 // chunk_dt num_seqs * max_chunks * heads.
-RLLM_EXPORT int rllm_ssd_scan(const void* xbc, int stride, int dtype, const float* dt, const float* dt_bias,
+RLLM_EXPORT int rllm_ssd_scan(const void* xbc, int rows, int stride, int dtype, const float* dt, const float* dt_bias,
                               const float* a_log, const float* skip, float* state, float* work, float* chunk_dt,
                               const int* q_start, const int* slots, int num_slots, int num_seqs, int max_chunks,
                               float* out, int heads, int groups, int N, int P, int* err, cudaStream_t stream) {
@@ -39,6 +40,9 @@ RLLM_EXPORT int rllm_ssd_scan(const void* xbc, int stride, int dtype, const floa
   if (dtype == RLLM_DT_BF16 && max_chunks > 0 && !ssd_mma_disabled() && N <= 128 && P <= 128) {
     const bf16* x = (const bf16*)xbc;
     const bf16 *B = x + (size_t)heads * P, *C = B + (size_t)groups * N;
+    const int rc = lg_scan<true>(C, B, x, rows, stride, nullptr, steps, state, work, nullptr, q_start, slots, num_slots, num_seqs, max_chunks, out,
+                                 heads, N, P, err, stream);
+    if (rc >= 0) return rc;
     auto chain = [&]() {
       lightning_chain<true>(nullptr, steps, state, work, q_start, slots, num_slots, num_seqs, max_chunks, heads, N, P, stream);
     };

@@ -72,7 +72,7 @@ _TABLE = {
     "rllm_channel_delta_prepare": ("channel_delta", "piippppppppiiiiff", "channel_delta_prepare"),
     "rllm_channel_delta_chunked": ("channel_delta", "pippppffpppiiiippiiiip", "channel_delta_chunked"),
     "rllm_silu_gated_group_rmsnorm": ("ssd", "ppippiiiif", "silu_gated_group_rmsnorm"),
-    "rllm_ssd_scan": ("ssd", "piipppppppppiiipiiiip", "ssd_scan"),
+    "rllm_ssd_scan": ("ssd", "piiipppppppppiiipiiiip", "ssd_scan"),
     "rllm_head_gated_rmsnorm": ("mlstm", "ppipipiiiif", "head_gated_rmsnorm"),
     "rllm_mlstm_scan": ("mlstm", "pppiipppffppppiiiiiiippp", "mlstm_scan"),
     "rllm_add_row_bias": ("layernorm", "ppiii", "add_row_bias"),
@@ -80,7 +80,7 @@ _TABLE = {
     "rllm_layernorm": ("layernorm", "ppppppppiiifi", "layernorm"),
     "rllm_selective_scan": ("selective_scan", "ppppiiipppiiipppppiiipiip", "selective_scan"),
     "rllm_causal_conv": ("selective_scan", "piippippppiiipiiip", "causal_conv"),
-    "rllm_lightning_scan": ("lightning", "pppiipppppiiipiiip", "lightning_scan"),
+    "rllm_lightning_scan": ("lightning", "pppiiippppppiiipiiip", "lightning_scan"),
     "rllm_gated_rmsnorm": ("mixer_glue", "ppipipiiif", "gated_rmsnorm"),
     "rllm_rms_mean2": ("mixer_glue", "ppppipiiif", "rms_mean2"),
     "rllm_attention_simt_kv": ("attention_simt", "pipppipippiiiiiiiifiifppiipiip", "attention_simt_kv"),
@@ -1547,7 +1547,9 @@ def lightning_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: tor
     out = torch.empty((T, heads * dv), dtype=torch.float32, device=q.device)
     chunks = _chunks_for(int(lib.rllm_lightning_chunk()), max_q_len, num_seqs)
     work = torch.empty(num_seqs * chunks * heads * d * dv, dtype=torch.float32, device=q.device) if chunks else None
-    _entries.rllm_lightning_scan(q, k, v, q.stride(0), dtype_code(q.dtype), decay, state, work, q_start, slots,
+    # room for the activated projections, where the tensor cores read them
+    act = torch.empty((T, heads * (2 * d + dv)), dtype=q.dtype, device=q.device) if chunks and q.dtype is torch.bfloat16 else None
+    _entries.rllm_lightning_scan(q, k, v, T, q.stride(0), dtype_code(q.dtype), decay, state, work, act, q_start, slots,
                                  state.shape[0], num_seqs, chunks, out, heads, d, dv, err)
     return out
 
@@ -1725,7 +1727,7 @@ def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: 
     chunks = _chunks_for(int(lib.rllm_ssd_chunk()), max_q_len, num_seqs)
     work = torch.empty(num_seqs * chunks * heads * (n * p + 1), dtype=torch.float32, device=xbc.device) if chunks else None
     chunk_dt = work[num_seqs * chunks * heads * n * p:] if chunks else None
-    _entries.rllm_ssd_scan(xbc, xbc.stride(0) if T > 1 else xbc.shape[1], dtype_code(xbc.dtype), dt, dt_bias, a_log,
+    _entries.rllm_ssd_scan(xbc, T, xbc.stride(0) if T > 1 else xbc.shape[1], dtype_code(xbc.dtype), dt, dt_bias, a_log,
                            skip, state, work, chunk_dt, q_start, slots, state.shape[0], num_seqs, chunks, out, heads,
                            groups, n, p, err)
     return out

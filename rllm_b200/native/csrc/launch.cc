@@ -97,7 +97,7 @@ const Row kSignatures[] = {
     ROW("piiiiippfpppipppfiiiiiip"), ROW("piiippipp"), ROW("piiippp"), ROW("piiippppp"), ROW("piiippppppp"),
     ROW("piiipppppppi"), ROW("piippifpppfippppiiiiiippip"), ROW("piippippppiiipiiip"),
     ROW("piippppifpippiiiiiiipiiippififiip"), ROW("piippppippiiiiiiiiifiifppiipp"), ROW("piippppippiiiiiiiiifpi"),
-    ROW("piipppppipipppippiiiiiiiiipp"), ROW("piippppppppiiiiff"), ROW("piipppppppppiiipiiiip"), ROW("pipifpipiiiiifff"),
+    ROW("piipppppipipppippiiiiiiiiipp"), ROW("piippppppppiiiiff"), ROW("piiipppppppppiiipiiiip"), ROW("pipifpipiiiiifff"),
     ROW("pipipiiii"), ROW("pipipiiiiifff"), ROW("pipipiiiiifffp"), ROW("pipipippipippiii"), ROW("pippifpppfipppppiiiiiiipp"),
     ROW("pippiiipppiiiiiiiifpp"), ROW("pippippppipppppppiiiiiiiiiiiiifffip"), ROW("pipppipippiiiiiiifp"),
     ROW("pipppipippiiiiiiiifiifppiipiip"), ROW("pipppipippiiiiiiip"), ROW("pipppippiiiiiiiiifpp"),
@@ -106,7 +106,7 @@ const Row kSignatures[] = {
     ROW("pipppppipiiipiip"), ROW("plf"), ROW("plipppppfiiii"), ROW("pllplliplliiiii"), ROW("pllpllpiliiiip"), ROW("ppffpil"),
     ROW("ppfppiii"), ROW("ppiii"), ROW("ppiiifff"), ROW("ppiiii"), ROW("ppiip"), ROW("ppil"), ROW("ppili"), ROW("ppipiii"),
     ROW("ppipiiifip"), ROW("ppipipiiif"), ROW("ppipipiiiif"), ROW("ppippiiiif"), ROW("ppipppppppippili"), ROW("ppl"),
-    ROW("pppffpffpiiii"), ROW("pppiiiiii"), ROW("pppiiippi"), ROW("pppiipppffppppiiiiiiippp"), ROW("pppiipppppiiipiiip"),
+    ROW("pppffpffpiiii"), ROW("pppiiiiii"), ROW("pppiiippi"), ROW("pppiipppffppppiiiiiiippp"), ROW("pppiiippppppiiipiiip"),
     ROW("pppipippiiiiiiifpp"), ROW("pppippippfppfplippiiii"), ROW("ppppfiiiiiii"), ROW("ppppiii"), ROW("ppppiiiii"),
     ROW("ppppiiipppiiipppppiiipiip"), ROW("ppppipiiif"), ROW("ppppipiiifi"), ROW("ppppippiiiiiiiifpiipp"),
     ROW("ppppippiippfiiiiiiiiiiip"), ROW("pppppiipppiipiiiip"), ROW("pppppippiiiiiiiiiiifiipp"), ROW("ppppppipiiii"),
