@@ -12,12 +12,13 @@
 //   chunk costs about 1 us, of which the loads, the products and the factors (a warp or two each) hide behind the arithmetic:
 //   with the arithmetic's own warps doing all of it a chunk took 2.1 us, with copies of 16 bytes in place of TMA 2.8.
 // outputs: persistent CTAs share out the (chunk, head) pairs, chunk by chunk, so that consecutive pairs of a group keep q, k
-//   and Q K^T (in tensor memory) and only bring their values and start state.  The weights pass as the A operand in tensor
-//   memory; between two 32s of tokens they are one factor a row times one a column.  A pair takes 3 us, the workers' warps
-//   one after the other in weights (1,500 cycles), stores of the results (1,100) and the rest.
+//   and Q K^T (in tensor memory) and only bring their values and start state, one to three pairs ahead.  Eight warps make the
+//   weights, which pass as the A operand in tensor memory (between two 32s of tokens they are one factor a row times one a
+//   column), eight the results of the pair before, which leave by TMA; with the same 16 warps at both one after the other a
+//   pair took 5,700 cycles, so 4,500, bound by the instructions of the scheduler whose warps have the chunk's last 32 tokens.
 //   A value that is not finite would reach every token of its chunk (0 times infinity): it is staged as zero and its column
 //   is set to NaN from its token on.
-// Measured, 2,048 tokens: 64 heads of 128 x 64 with steps 122 -> 54 us (states 20), 16 heads of 128 x 128 97 -> 52 us (the
+// Measured, 2,048 tokens: 64 heads of 128 x 64 with steps 122 -> 50 us (states 20), 16 heads of 128 x 128 97 -> 52 us (the
 // activations 13, states 19); the results' distance from float64 2.4e-6 -> 2.3e-6 and 8.5e-7 -> 8.3e-7 of their norm.
 #pragma once
 #include "lightning_walk.cuh"
@@ -26,8 +27,7 @@
 
 #define LG_CHUNK 128
 #define LGS_THREADS 384          // states: 8 warps of arithmetic, one that loads, one that issues products, two for the factors
-#define LGO_WORKERS 512          // outputs: 16 warps of arithmetic, and the latter two
-#define LGO_THREADS 576
+#define LGO_THREADS 608          // outputs: 8 warps for the weights, 8 for the results, and one each of the latter
 #define LG_COLS 32               // value columns a CTA of the states' kernel
 
 __device__ __forceinline__ void lg_tmem_ld16(unsigned taddr, unsigned* r) {
@@ -60,7 +60,9 @@ __device__ __forceinline__ unsigned lg_pack(float a, float b) {
 // two numbers as two pairs of bfloat16: the values and the remainders
 __device__ __forceinline__ void lg_split2(float a, float b, unsigned& hi, unsigned& lo) {
   hi = lg_pack(a, b);
-  lo = lg_pack(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
+  const unsigned long long minus = at_pack2(-1.f, -1.f);
+  at_unpack2(at_fma2(at_pack2(__uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u)), minus, at_pack2(a, b)), a, b);
+  lo = lg_pack(a, b);
 }
 __device__ __forceinline__ int lg_chunks(int len, int most) { return min((len + LG_CHUNK - 1) / LG_CHUNK, most); }
 __device__ __forceinline__ unsigned long long lg_mul2(unsigned long long a, unsigned long long b) {
@@ -331,82 +333,77 @@ lightning_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
 }
 
 // ---------------------------------------------------------------------------
-// What a worker of the outputs' kernel stages of a chunk's rows of W columns: 16 bytes a load, zeros behind the chunk's n
-// tokens (silu(0) = 0).
-template <int W> struct LgRows {
-  static constexpr int N = LG_CHUNK * W / (8 * LGO_WORKERS);
-  uint4 raw[N];
-  __device__ __forceinline__ void fetch(const bf16* src, int stride, int n) {              // src: the chunk's first token
-#pragma unroll
-    for (int u = 0; u < N; ++u) {
-      const int e = u * LGO_WORKERS + threadIdx.x, j = e / (W / 8), c = e % (W / 8);
-      raw[u] = j < n ? *(const uint4*)(src + (size_t)j * stride + c * 8) : make_uint4(0u, 0u, 0u, 0u);
-    }
-  }
-  __device__ __forceinline__ static unsigned char* at(unsigned char* tile, int u) {        // panels of 128 rows
-    const int e = u * LGO_WORKERS + threadIdx.x;
-    return tile + lg_at(e / (W / 8), e % (W / 8), LG_CHUNK * 128);
-  }
-  __device__ __forceinline__ void store(unsigned char* tile) const {
-#pragma unroll
-    for (int u = 0; u < N; ++u) *(uint4*)at(tile, u) = raw[u];
-  }
-  // Where the tile is multiplied by weights that are zero for earlier tokens: a value that is not finite becomes a zero, and
-  // bad[column] remembers its (first) token with the number of the task, the larger the earlier.
-  __device__ __forceinline__ void store_finite(unsigned char* tile, int* bad, int* any, int task) const {
-    store(tile);
+// The outputs' kernel's values as they have landed, by the 256 threads of its results' warps: zeros behind the chunk's n tokens;
+// and as the tile is multiplied by weights that are zero for earlier tokens, a value that is not finite becomes a zero, and
+// bad[column] remembers its (first) token with the number of the task, the larger the earlier.
+template <int W>
+__device__ __noinline__ void lg_make_finite(unsigned char* tile, int n, int tid, int* bad, int* any, int task) {
 #pragma unroll 1
-    for (int u = 0; u < N; ++u) {
-      uint4 w = *(const uint4*)at(tile, u);
-      const unsigned m = 0x7f807f80u, one = 0x00800080u;
-      if ((((w.x & m) + one) | ((w.y & m) + one) | ((w.z & m) + one) | ((w.w & m) + one)) & 0x80008000u) {
-        const int e = u * LGO_WORKERS + threadIdx.x, j = e / (W / 8), c = e % (W / 8);
-        unsigned* x = (unsigned*)&w;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const unsigned bits = 0x7f80u << (16 * (i & 1));
-          if ((x[i >> 1] & bits) == bits) {
-            x[i >> 1] &= ~(0xffffu << (16 * (i & 1)));
-            atomicMax(&bad[c * 8 + i], task << 8 | (255 - j));
-            *any = task;
-          }
-        }
-        *(uint4*)at(tile, u) = w;
+  for (int u = 0; u < LG_CHUNK * W / 2048; ++u) {
+    const int e = u * 256 + tid, j = e / (W / 8), c = e % (W / 8);
+    unsigned* x = (unsigned*)(tile + lg_at(j, c, LG_CHUNK * 128));
+#pragma unroll 1
+    for (int i = 0; i < 8; ++i) {
+      const unsigned bits = 0x7f80u << (16 * (i & 1)), w = x[i >> 1];
+      if (j < n && (w & bits) == bits) {
+        x[i >> 1] = w & ~(0xffffu << (16 * (i & 1)));
+        atomicMax(&bad[c * 8 + i], task << 8 | (255 - j));
+        *any = task;
       }
     }
   }
-};
+}
+template <int W>
+__device__ __forceinline__ bool lg_finite(unsigned char* tile, int n, int tid, int* bad, int* any, int task) {
+  const unsigned m = 0x7f807f80u, one = 0x00800080u;
+  unsigned found = 0u;
+#pragma unroll
+  for (int u = 0; u < LG_CHUNK * W / 2048; ++u) {
+    const int e = u * 256 + tid, j = e / (W / 8);
+    uint4* at = (uint4*)(tile + lg_at(j, e % (W / 8), LG_CHUNK * 128));
+    const uint4 w = *at;
+    if (j >= n) *at = make_uint4(0u, 0u, 0u, 0u);
+    else found |= ((w.x & m) + one) | ((w.y & m) + one) | ((w.z & m) + one) | ((w.w & m) + one);
+  }
+  if (found & 0x80008000u) lg_make_finite<W>(tile, n, tid, bad, any, task);
+  return (found & 0x80008000u) != 0u || n < LG_CHUNK;
+}
 
 // where a task's chunk is
 struct LgPlace { int t0, n, len, s, chunk, h; };
 
 template <int D, int DV> struct LgoShape {
-  static constexpr int Q = (D / 64) * 16384, K = DV * 512; // (K: a task's results pass through it)
-  static constexpr int V = (DV / 64) * 16384, S = D * DV * 4, NST = DV == 64 ? 2 : 1;
-  static constexpr int SMEM = Q + K + NST * (V + S) + 6144;
+  static constexpr int Q = (D / 64) * 16384, V = (DV / 64) * 16384, S = D * DV * 4;
+  static constexpr int NV = DV == 64 ? 3 : 1, NS = DV == 64 ? 2 : 1;                       // stages of values and of start states
+  static constexpr int SMEM = 2 * Q + NV * V + NS * S + 32768 + 6656;
 };
 template <int D, int DV, bool STEPS>
 __global__ void __launch_bounds__(LGO_THREADS, 1)
-lightning_outputs_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v, int stride,
-                         const float* __restrict__ decay, LtSteps steps, const unsigned char* __restrict__ work,
-                         const int* __restrict__ q_start, int num_seqs, int max_chunks, float* __restrict__ out, int heads,
-                         int* __restrict__ err) {
+lightning_outputs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                         const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_out,
+                         const float* __restrict__ decay, LtSteps steps,
+                         const unsigned char* __restrict__ work, const int* __restrict__ q_start, int num_seqs, int max_chunks,
+                         float* __restrict__ out, int heads, int* __restrict__ err) {
   using Shape = LgoShape<D, DV>;
-  constexpr int NST = Shape::NST;
+  constexpr int NV = Shape::NV, NS = Shape::NS, ND = NS;   // (ND: pairs of results in tensor memory)
   extern __shared__ __align__(1024) unsigned char lg_raw[];
-  unsigned char *sQ = lg_raw, *sK = sQ + Shape::Q, *sV = sK + Shape::K, *sS = sV + NST * Shape::V;
+  unsigned char *sQ = lg_raw, *sK = sQ + Shape::Q, *sV = sK + Shape::Q, *sS = sV + NV * Shape::V, *sO = sS + NS * Shape::S;
   // [2] of: log2 of what is left of a token's state since the 32 tokens began [128] | a token's part at the end of its 32
   // [128] | steps [128] | log2 of what the four 32s leave
-  float* fac = (float*)(sS + NST * Shape::S);
-  int* bad = (int*)(fac + 1024);                           // [2][DV] where a column stops to be finite, tasks in turn
-  int* any = bad + 256;                                    // [2] the last task that has such a column
-  unsigned long long* s_full = (unsigned long long*)(any + 2);    // [2] the start state is here
-  unsigned long long* staged_full = s_full + 2;            // workers -> MMA: q, k and values are staged
-  unsigned long long* raw_full = s_full + 3;               // MMA -> workers: Q K^T
-  unsigned long long* p_full = s_full + 4;                 // workers (16 warps) -> MMA: the weights
-  unsigned long long* o_full = s_full + 5;                 // [2] MMA -> workers: a task's products
-  unsigned long long* fac_full = s_full + 7;               // [2] factors -> workers
-  unsigned* tmem_slot = (unsigned*)(s_full + 9);
+  float* fac = (float*)(sO + 32768);
+  int* bad = (int*)(fac + 1024);                           // [3][DV] where a column stops to be finite, tasks in turn
+  int* any = bad + 384;                                    // [3 of 4] the last task that has such a column
+  unsigned long long* v_full = (unsigned long long*)(any + 4);    // [3] loads -> results
+  unsigned long long* s_full = v_full + 3;                 // [2] loads -> MMA: the start state
+  unsigned long long* qk_full = v_full + 5;                // loads -> MMA
+  unsigned long long* raw_full = v_full + 6;               // MMA -> weights: Q K^T
+  unsigned long long* o_full = v_full + 7;                 // [2] MMA -> all: a task's products
+  unsigned long long* v_ready = v_full + 9;                // [2] results (8 warps) -> MMA
+  unsigned long long* raw_read = v_full + 11;              // weights (8 warps) -> MMA
+  unsigned long long* p_full = v_full + 12;                // weights (8 warps) -> MMA
+  unsigned long long* d_free = v_full + 13;                // [3] results (8 warps) -> MMA, loads, factors: through with a task
+  unsigned long long* fac_full = v_full + 16;              // [2] factors (32 lanes) -> weights, results
+  unsigned* tmem_slot = (unsigned*)(v_full + 18);
   pdl_wait();
   pdl_launch();
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
@@ -421,12 +418,15 @@ lightning_outputs_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
   const int last = __shfl_sync(0xffffffffu, (int)(total * (blockIdx.x + 1) / gridDim.x), 0), tasks = last - first;
   if (tasks <= 0) return;
   if (tid == 0) {
-    for (int i = 0; i < 4; ++i) mbar_init(&s_full[i], 1);
-    mbar_init(p_full, 16);
-    for (int i = 0; i < 2; ++i) { mbar_init(&o_full[i], 1); mbar_init(&fac_full[i], 32); }
+    for (int i = 0; i < 9; ++i) mbar_init(&v_full[i], 1);
+    for (int i = 9; i < 16; ++i) mbar_init(&v_full[i], 8);
+    for (int i = 16; i < 18; ++i) mbar_init(&v_full[i], 32);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"((unsigned long long)&map_q) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"((unsigned long long)&map_k) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"((unsigned long long)&map_v) : "memory");
   }
-  for (int e = tid; e < 258; e += LGO_THREADS) bad[e] = 0;                                 // (and `any`)
+  for (int e = tid; e < 388; e += LGO_THREADS) bad[e] = 0;                                 // (and `any`)
   if (warp == 16) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tg_smem(tmem_slot)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -434,8 +434,13 @@ lightning_outputs_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const unsigned tmem_raw = __shfl_sync(0xffffffffu, *tmem_slot, 0), tmem_p = tmem_raw + 128, tmem_s = tmem_raw + 256, tmem_v = tmem_s + DV;
+  // Q K^T: 128 columns, the weights: 128, ND times what the start state gives and what the values give: DV each
+  const unsigned tmem_raw = __shfl_sync(0xffffffffu, *tmem_slot, 0), tmem_p = tmem_raw + 128, tmem_d = tmem_raw + 256;
   auto wait = [&](unsigned long long* bar, unsigned parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)) != 0; };
+  // Task m's of barriers that tasks take in turn.  Whoever waits for a phase is needed for the barrier's next one (so that a
+  // phase is never two behind, where its parity would look unfinished): three of d_free, for which V waits three tasks late.
+  auto wait_task = [&](unsigned long long* bars, int m) { return wait(&bars[m & 1], (m >> 1) & 1); };
+  auto wait_free = [&](int m) { return wait(&d_free[m % 3], (m / 3) & 1); };
   LgPlace p;
   p.h = first % heads;
   p.chunk = first / heads;
@@ -466,30 +471,51 @@ lightning_outputs_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
     p.n = min(LG_CHUNK, p.len - p.chunk * LG_CHUNK);
     return p;
   };
-  // q and k are staged, and Q K^T is made, where the chunk or the group is another than the task's before
-  auto group = [&](const LgPlace& p) { return STEPS ? p.h / steps.per : p.h; };
+  // q and k are loaded, and Q K^T is made, where the chunk or the group is another than the task's before
   auto fresh = [&](const LgPlace& p, int m) { return m == 0 || !STEPS || p.h % steps.per == 0; };
 
-  if (warp == 16) {
-    auto ask_state = [&](const LgPlace& p, int m) {        // task number m's start state
+  if (warp == 18) {
+    for (int m = 0; m < tasks; ++m) {
+      if (m >= NS && !wait_task(o_full, m - NS)) break;    // the stage's last task has used its start state
       if (lane == 0) {
-        void* b = &s_full[m % NST];
-        mbar_expect_tx(b, (unsigned)Shape::S);
+        const int st = m % NS;
+        mbar_expect_tx(&s_full[st], (unsigned)Shape::S);
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                     ::"r"(tg_smem(sS + m % NST * Shape::S)), "l"(work + (((size_t)p.s * max_chunks + p.chunk) * heads + p.h) * Shape::S),
-                       "r"((unsigned)Shape::S), "r"(tg_smem(b)) : "memory");
+                     ::"r"(tg_smem(sS + st * Shape::S)), "l"(work + (((size_t)p.s * max_chunks + p.chunk) * heads + p.h) * Shape::S),
+                       "r"((unsigned)Shape::S), "r"(tg_smem(&s_full[st])) : "memory");
       }
       __syncwarp();
-    };
+      if (m >= NV && !wait_free(m - NV)) break;            // the stage's last task is through
+      if (lane == 0) {
+        const int st = m % NV;
+        mbar_expect_tx(&v_full[st], (unsigned)Shape::V);
+        for (int x = 0; x < DV; x += 64) tma_load_2d(sV + st * Shape::V + (x / 64) * 16384, &map_v, p.h * DV + x, p.t0, &v_full[st]);
+      }
+      __syncwarp();
+      if (fresh(p, m)) {
+        if (m > 0 && !wait_task(o_full, m - 1)) break;     // q's and k's last products are made
+        if (lane == 0) {
+          const int x0 = (STEPS ? p.h / steps.per : p.h) * D;
+          mbar_expect_tx(qk_full, (unsigned)(2 * Shape::Q));
+          for (int x = 0; x < D; x += 64) {
+            tma_load_2d(sQ + (x / 64) * 16384, &map_q, x0 + x, p.t0, qk_full);
+            tma_load_2d(sK + (x / 64) * 16384, &map_k, x0 + x, p.t0, qk_full);
+          }
+        }
+        __syncwarp();
+      }
+      if (m + 1 < tasks) p = advance(p);
+    }
+  } else if (warp == 16) {
     const unsigned idesc_qk = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
     const unsigned idesc_v = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((unsigned)(DV >> 3) << 17) | ((128u >> 4) << 24);
     const unsigned long long dq = umma_desc(sQ), dk = umma_desc(sK);
-    int asked = 1, landed = 0;
-    ask_state(p, 0);
+    int keys = 0;                                          // how many q and k there were
     for (int m = 0; m < tasks; ++m) {
-      if (!wait(staged_full, m & 1)) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (fresh(p, m)) {
+        if (!wait(qk_full, keys & 1) || (m > 0 && !wait(raw_read, (m - 1) & 1))) break;
+        ++keys;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (umma_elect()) {
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk)
@@ -499,14 +525,10 @@ lightning_outputs_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
         }
         __syncwarp();
       }
-      const LgPlace next = m + 1 < tasks ? advance(p) : p;
-      if (NST == 2 && m + 1 < tasks) {                     // (the task before is through with its stage)
-        ask_state(next, m + 1);
-        ++asked;
-      }
-      if (!wait(&s_full[m % NST], (m / NST) & 1)) break;
-      ++landed;
-      const unsigned long long ds = lg_desc_mn(sS + m % NST * Shape::S, D * 128);
+      if (!wait(&s_full[m % NS], (m / NS) & 1) || (m >= ND && !wait_free(m - ND))) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const unsigned tmem_s = tmem_d + m % ND * (2 * DV), tmem_v = tmem_s + DV;
+      const unsigned long long ds = lg_desc_mn(sS + m % NS * Shape::S, D * 128);
       if (umma_elect()) {
 #pragma unroll
         for (int kk = 0; kk < 2 * (D / 16); ++kk) {
@@ -516,9 +538,9 @@ lightning_outputs_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
         }
       }
       __syncwarp();
-      if (!wait(p_full, m & 1)) break;
+      if (!wait_task(v_ready, m) || !wait(p_full, m & 1)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const unsigned long long dv = lg_desc_mn(sV + m % NST * Shape::V, 16384);
+      const unsigned long long dv = lg_desc_mn(sV + m % NV * Shape::V, 16384);
       if (umma_elect()) {
 #pragma unroll
         for (int kk = 0; kk < 16; ++kk)
@@ -526,14 +548,8 @@ lightning_outputs_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
         umma_commit(&o_full[m & 1]);
       }
       __syncwarp();
-      if (NST == 1 && m + 1 < tasks) {
-        if (!wait(&o_full[m & 1], (m >> 1) & 1)) break;
-        ask_state(next, m + 1);
-        ++asked;
-      }
-      p = next;
+      if (m + 1 < tasks) p = advance(p);
     }
-    for (; landed < asked; ++landed) wait(&s_full[landed % NST], (landed / NST) & 1);      // (a wait ran out: copies on their way)
   } else if (warp == 17) {
     // what is left of a token, four tokens a lane
     float next_raw[4];
@@ -580,7 +596,7 @@ lightning_outputs_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
           end[x] = lg_pow(l2, 31 - ((4 * lane + x) & 31));
         }
       }
-      if (m >= 2 && !wait(&o_full[m & 1], ((m - 2) >> 1) & 1)) break;                      // task m - 2 has used its factors
+      if (m >= 2 && !wait_free(m - 2)) break;              // task m - 2 has used its factors
       float* f = fac + (m & 1) * 512;
       *(float4*)(f + 4 * lane) = make_float4(pre[0], pre[1], pre[2], pre[3]);
       *(float4*)(f + 128 + 4 * lane) = make_float4(end[0], end[1], end[2], end[3]);
@@ -592,68 +608,44 @@ lightning_outputs_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
         fetch(p);
       }
     }
-  } else {
-    const int quarter = warp & 3, part = warp >> 2, t = quarter * 32 + lane;               // this thread's token of the chunk
+  } else if (warp < 8) {
+    // the weights of token t and 64 others, as value + remainder, into tensor memory: of those that are later than the warp's
+    // tokens nothing, once; the 32 that are its own tokens with their differences
+    const int quarter = warp & 3, half = warp >> 2, t = quarter * 32 + lane;
     const unsigned lane_sel = (unsigned)(quarter * 32) << 16;
-    const int c0 = part * 32;                              // and its earlier tokens; those of later ones than the warp's weigh nothing
-    if (part > quarter) {
-      unsigned z[16];
+    for (int b = 2 * half; b < 2 * half + 2; ++b) {
+      if (b > quarter) {
+        unsigned z[16];
 #pragma unroll
-      for (int x = 0; x < 16; ++x) z[x] = 0u;
-      tmem_st16(tmem_p + lane_sel + c0 / 2, z);
-      tmem_st16(tmem_p + 64 + lane_sel + c0 / 2, z);
+        for (int x = 0; x < 16; ++x) z[x] = 0u;
+        tmem_st16(tmem_p + lane_sel + b * 16, z);
+        tmem_st16(tmem_p + 64 + lane_sel + b * 16, z);
+      }
     }
-    LgRows<DV> rv;
-    rv.fetch(v + (size_t)p.t0 * stride + (size_t)p.h * DV, stride, p.n);
-    bool ok = true, staged = false;
-    int keys = 0;                                          // how many q and k there were
+    int keys = 0;
     for (int m = 0; m < tasks; ++m) {
-      const bool now = fresh(p, m);
-      if (m > 0 && (now || !staged)) {                     // every warp is through with what is overwritten
-        asm volatile("bar.sync 2, %0;" ::"n"(LGO_WORKERS) : "memory");
-      }
-      if (!staged) rv.store_finite(sV + m % NST * Shape::V, bad + (m & 1) * 128, any + (m & 1), m + 1);
-      if (now) {
-        LgRows<D> rq, rk;
-        rq.fetch(q + (size_t)p.t0 * stride + (size_t)group(p) * D, stride, p.n);
-        rk.fetch(k + (size_t)p.t0 * stride + (size_t)group(p) * D, stride, p.n);
-        rq.store(sQ);
-        rk.store(sK);
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      {
-        unsigned fail;
-        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.or.pred p, 1, %2, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(fail) : "r"(ok ? 0u : 1u), "n"(LGO_WORKERS) : "memory");
-        if (fail) break;
-      }
-      if (tid == 0) mbar_arrive(staged_full);
-      const bool more = m + 1 < tasks;
-      const LgPlace next = more ? advance(p) : p;
-      if (more) rv.fetch(v + (size_t)next.t0 * stride + (size_t)next.h * DV, stride, next.n);
-      ok = wait(&fac_full[m & 1], (m >> 1) & 1) && ok;
-      if (now) {
-        ok = wait(raw_full, keys & 1) && ok;
+      if (!wait_task(fac_full, m)) break;
+      if (fresh(p, m)) {
+        if (!wait(raw_full, keys & 1)) break;
         ++keys;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // the weights, as value + remainder, into tensor memory
       const float* fc = fac + (m & 1) * 512;
       const float l2 = STEPS ? 0.f : log2f(decay[p.h]);
       const float lt = STEPS ? fc[t] : 0.f;
-      auto upto = [&](int from) {                          // log2 of what the tokens from 32 x `from` up to this one leave
-        float sum = lt;
-        for (int i = quarter - 1; i >= from; --i) sum += fc[384 + i];
-        return sum;
-      };
-      if (part <= quarter) {
+      // (every warp waits for the task before, also one without weights: it comes back to these barriers only after the others)
+      bool through = m == 0;
+#pragma unroll 1
+      for (int b = 2 * half; b < 2 * half + 2 && b <= quarter; ++b) {
+        const int c0 = b * 32;
         float sc[32];
         tmem_ld32(tmem_raw + lane_sel + c0, (unsigned*)sc);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (part < quarter) {
+        if (b < quarter) {
           // since the 32 tokens of the columns ended, times what was left of them there: one factor a row, one a column
-          const float since = STEPS ? exp2f(upto(part + 1)) : lg_pow(l2, t - c0 - 31);
+          float sum = lt;
+          if (STEPS) for (int x = quarter - 1; x > b; --x) sum += fc[384 + x];
+          const float since = STEPS ? exp2f(sum) : lg_pow(l2, t - c0 - 31);
           const unsigned long long since2 = at_pack2(since, since);
 #pragma unroll
           for (int j = 0; j < 32; j += 4) {
@@ -680,63 +672,106 @@ lightning_outputs_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k,
         unsigned hi[16], lo[16];
 #pragma unroll
         for (int j = 0; j < 32; j += 2) lg_split2(sc[j], sc[j + 1], hi[j / 2], lo[j / 2]);
-        tmem_st16(tmem_p + lane_sel + c0 / 2, hi);
-        tmem_st16(tmem_p + 64 + lane_sel + c0 / 2, lo);
+        if (!through && !wait_task(o_full, m - 1)) break;  // the task before has read its weights
+        through = true;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem_st16(tmem_p + lane_sel + b * 16, hi);
+        tmem_st16(tmem_p + 64 + lane_sel + b * 16, lo);
       }
-      const float u = STEPS ? exp2f(upto(0)) : lg_pow(l2, t + 1), skip = STEPS ? steps.skip[p.h] : 0.f;
+      if (!through && !wait_task(o_full, m - 1)) break;
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
+      if (lane == 0) mbar_arrive(raw_read);
       if (lane == 0) mbar_arrive(p_full);
-      staged = NST == 2 && more;                           // the next task's values beside this one's products
-      if (staged) rv.store_finite(sV + (m + 1) % NST * Shape::V, bad + (~m & 1) * 128, any + (~m & 1), m + 2);
-      ok = wait(&o_full[m & 1], (m >> 1) & 1) && ok;
+      if (m + 1 < tasks) p = advance(p);
+    }
+  } else {
+    // the values as they land, and the results: out = u (Q S_0) + weights V + skip v
+    const int quarter = warp & 3, half = (warp - 8) >> 2, t = quarter * 32 + lane, id = tid - 256;
+    const unsigned lane_sel = (unsigned)(quarter * 32) << 16;
+    unsigned char* mine = sO + (warp - 8) * 4096;          // 32 columns of the warp's tokens, so that whole lines are stored
+    auto values = [&](const LgPlace& p, int m) {
+      if (!wait(&v_full[m % NV], (m / NV) & 1)) return false;
+      // (the fence waits for stores on their way: only where there is something to be seen)
+      if (__any_sync(0xffffffffu, lg_finite<DV>(sV + m % NV * Shape::V, p.n, id, bad + m % 3 * 128, any + m % 3, m + 1)))
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&v_ready[m & 1]);
+      return true;
+    };
+    bool ok = values(p, 0);
+    for (int m = 0; m < tasks && ok; ++m) {
+      const LgPlace next = m + 1 < tasks ? advance(p) : p;
+      ok = wait_task(fac_full, m);
+      if (!ok) break;
+      const float* fc = fac + (m & 1) * 512;
+      float sum = STEPS ? fc[t] : 0.f;
+      if (STEPS) for (int x = quarter - 1; x >= 0; --x) sum += fc[384 + x];
+      const float u = STEPS ? exp2f(sum) : lg_pow(log2f(decay[p.h]), t + 1), skip = STEPS ? steps.skip[p.h] : 0.f;
+      if (NV > 1 && m + 1 < tasks) ok = values(next, m + 1);
+      ok = ok && wait_task(o_full, m);
+      if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      // out = u (Q S_0) + weights V + skip v; through the warp's part of sK, so that rows of 64 or 128 bytes are stored
-      constexpr int CW = DV / 4, CH = CW / 4;              // columns a warp, its 16 bytes a row
-      const bool holes = *(volatile int*)(any + (m & 1)) == m + 1;
-      unsigned char* mine = sK + warp * (32 * CW * 4);
-      float a[CW], b[CW];
-      if constexpr (CW == 32) {
-        tmem_ld32(tmem_s + lane_sel + part * CW, (unsigned*)a);
-        tmem_ld32(tmem_v + lane_sel + part * CW, (unsigned*)b);
-      } else {
-        lg_tmem_ld16(tmem_s + lane_sel + part * CW, (unsigned*)a);
-        lg_tmem_ld16(tmem_v + lane_sel + part * CW, (unsigned*)b);
-      }
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      const unsigned tmem_s = tmem_d + m % ND * (2 * DV), tmem_v = tmem_s + DV;
+      const bool holes = *(volatile int*)(any + m % 3) == m + 1;
+#pragma unroll 1
+      for (int c0 = half * (DV / 2); c0 < (half + 1) * (DV / 2); c0 += 32) {
+        float a[32], b[32];
+        tmem_ld32(tmem_s + lane_sel + c0, (unsigned*)a);
+        tmem_ld32(tmem_v + lane_sel + c0, (unsigned*)b);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        const unsigned long long u2 = at_pack2(u, u), skip2 = at_pack2(skip, skip);
 #pragma unroll
-      for (int j = 0; j < CW; j += 8) {
-        float x[8];
-        if (STEPS) unpack8(*(const uint4*)(sV + m % NST * Shape::V + lg_at(t, (part * CW + j) / 8, 16384)), x);
+        for (int j = 0; j < 32; j += 8) {
+          uint4 x = make_uint4(0u, 0u, 0u, 0u);
+          if (STEPS) x = *(const uint4*)(sV + m % NV * Shape::V + lg_at(t, (c0 + j) / 8, 16384));
+          const unsigned w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-        for (int y = 0; y < 8; ++y) {
-          float o = fmaf(a[j + y], u, b[j + y]);
-          if (STEPS) o = fmaf(skip, x[y], o);
-          a[j + y] = o;
+          for (int y = 0; y < 4; ++y) {
+            unsigned long long o = at_fma2(at_pack2(a[j + 2 * y], a[j + 2 * y + 1]), u2, at_pack2(b[j + 2 * y], b[j + 2 * y + 1]));
+            if (STEPS) o = at_fma2(skip2, at_pack2(__uint_as_float(w[y] << 16), __uint_as_float(w[y] & 0xffff0000u)), o);
+            at_unpack2(o, a[j + 2 * y], a[j + 2 * y + 1]);
+          }
+        }
+        if (holes) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const int w = bad[m % 3 * 128 + c0 + j];
+            if ((w >> 8) == m + 1 && t >= 255 - (w & 255)) a[j] = __int_as_float(0x7fffffff);
+          }
+        }
+        if (c0 + 32 == (half + 1) * (DV / 2)) {            // the last of the task's tensor memory and values that the warp reads
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&d_free[m % 3]);
+        }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");     // what lay here before is read
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) *(float4*)(mine + lg_at(lane, j, 0)) = make_float4(a[4 * j], a[4 * j + 1], a[4 * j + 2], a[4 * j + 3]);
+        if (p.n == LG_CHUNK) {
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0)
+            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];\n\tcp.async.bulk.commit_group;"
+                         ::"l"((unsigned long long)&map_out), "r"(p.h * DV + c0), "r"(p.t0 + quarter * 32), "r"(tg_smem(mine)) : "memory");
+        } else {
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int row = j * 4 + (lane >> 3), c = lane & 7, tt = quarter * 32 + row;
+            const float4 o = *(const float4*)(mine + lg_at(row, c, 0));
+            if (tt < p.n) *(float4*)(out + ((size_t)(p.t0 + tt) * heads + p.h) * DV + c0 + c * 4) = o;
+          }
+          __syncwarp();
         }
       }
-      if (holes) {
-#pragma unroll
-        for (int j = 0; j < CW; ++j) {
-          const int w = bad[(m & 1) * 128 + part * CW + j];
-          if ((w >> 8) == m + 1 && t >= 255 - (w & 255)) a[j] = __int_as_float(0x7fffffff);
-        }
-      }
-      // (16 bytes j of row r at j ^ r's place among those that share the banks: eight rows of 128 bytes, four pairs of 64)
-      auto place16 = [&](int row, int j) { return mine + row * (CW * 4) + ((j ^ (CH == 8 ? row & 7 : (row >> 1) & 3)) << 4); };
-#pragma unroll
-      for (int j = 0; j < CH; ++j) *(float4*)place16(lane, j) = make_float4(a[4 * j], a[4 * j + 1], a[4 * j + 2], a[4 * j + 3]);
-      __syncwarp();
-#pragma unroll
-      for (int j = 0; j < CH; ++j) {
-        const int row = j * (32 / CH) + lane / CH, c = lane % CH, tt = quarter * 32 + row;
-        const float4 o = *(const float4*)place16(row, c);
-        if (tt < p.n) *(float4*)(out + ((size_t)(p.t0 + tt) * heads + p.h) * DV + part * CW + c * 4) = o;
-      }
-      __syncwarp();
+      if (NV == 1 && m + 1 < tasks) ok = values(next, m + 1);
       p = next;
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    __syncwarp();
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -762,7 +797,17 @@ static int lg_launch(const bf16* q, const bf16* k, const bf16* v, int rows, int 
     k = q + heads * D;
     v = k + heads * D;
   }
-  CUtensorMap mk, mv;
+  CUtensorMap mq, mk, mv, mo;
+  {
+    tg_encode_fn enc = tg_get_encode();
+    if (!enc) return RLLM_E_UNSUPPORTED;
+    cuuint64_t dims[2] = {(cuuint64_t)heads * DV, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)heads * DV * 4};
+    cuuint32_t box[2] = {32, 32}, estr[2] = {1, 1};
+    if (enc(&mo, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, out, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return RLLM_E_BADARG;
+  }
+  if (const int rc = tg_make_map(&mq, q, rows, (STEPS ? heads / steps.per : heads) * D, stride, LG_CHUNK)) return rc;
   if (const int rc = tg_make_map(&mk, k, rows, (STEPS ? heads / steps.per : heads) * D, stride, LG_CHUNK)) return rc;
   if (const int rc = tg_make_map(&mv, v, rows, heads * DV, stride, LG_CHUNK)) return rc;
   rllm_launch_pdl(lightning_states_kernel<D, DV, STEPS>, dim3(heads * (DV / LG_COLS), num_seqs), dim3(LGS_THREADS),
@@ -770,8 +815,8 @@ static int lg_launch(const bf16* q, const bf16* k, const bf16* v, int rows, int 
                   slots, num_slots, max_chunks, heads, stages, err);
   const long long tasks = (long long)num_seqs * max_chunks * heads;
   rllm_launch_pdl(lightning_outputs_kernel<D, DV, STEPS>, dim3((unsigned)(tasks < sms ? tasks : sms)), dim3(LGO_THREADS),
-                  (size_t)LgoShape<D, DV>::SMEM, stream, q, k, v, stride, decay, steps, (const unsigned char*)work, q_start,
-                  num_seqs, max_chunks, out, heads, err);
+                  (size_t)LgoShape<D, DV>::SMEM, stream, mq, mk, mv, mo, decay, steps, (const unsigned char*)work, q_start, num_seqs,
+                  max_chunks, out, heads, err);
   RLLM_LAUNCH_CHECK();
   return 0;
 }
