@@ -86,9 +86,9 @@ __device__ __forceinline__ uint4 lg_act8(const uint4& raw) {
 // its eight columns and walks the rows.
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS)
-lightning_act_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k, const bf16* __restrict__ v, int stride,
-                     const int* __restrict__ q_start, int num_seqs, bf16* __restrict__ act, int kn, int vn) {
-  pdl_wait();
+lightning_act_kernel(const bf16* q, const bf16* k, const bf16* v, int stride, const int* __restrict__ q_start, int num_seqs,
+                     bf16* act, int kn, int vn) {
+  pdl_wait_on(q, k, v);                                    // (the projection ahead wrote them)
   pdl_launch();
   const int c = (blockIdx.x * THREADS + threadIdx.x) * 8, width = 2 * kn + vn;
   if (c >= width) return;
