@@ -71,10 +71,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                          AtOpts opt, int beside) {
   // beside: the kernel ahead wrote nothing that this one reads or writes (the attention of the tokens that decode), and
   // it lets this one in only when the kernel ahead of it is complete: the two run side by side, and this one ends behind it.
-  if (!beside) {
-    pdl_wait();
-    pdl_launch();
-  }
+  if (!beside) pdl_wait();
   constexpr int AT_BN = 8192 / AT_D;              // keys a tile
   constexpr int DP = AT_D / 64;                   // panels of head dims (Q, K, V)
   constexpr int KPANEL = AT_BN * 128;             // bytes of a K or V panel: BN rows of 128 bytes
@@ -159,6 +156,7 @@ attention_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  if (!beside) pdl_launch();                       // behind the allocation: see pdl_launch
   const unsigned tmem_s = __shfl_sync(0xffffffffu, *tmem_slot, 0), tmem_o = tmem_s + AT_BN, tmem_p = tmem_o + AT_D;   // BN + D + BN / 2 <= 256 columns
 
   if (warp == 0) {

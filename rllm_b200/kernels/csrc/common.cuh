@@ -142,6 +142,11 @@ __device__ __forceinline__ void rope_cos_sin(int pos, double inv_freq, float* c,
 // Rule of this code base: a kernel calls pdl_launch only after its own pdl_wait.  Then,
 // when a kernel starts, every kernel but the one directly ahead of it has completed, and
 // what it reads before its own pdl_wait may include what those earlier kernels wrote.
+// A kernel that allocates tensor memory calls pdl_launch behind its allocation too.  The next kernel may allocate before its
+// wait (the products do): on an SM that both fit, its CTA would otherwise hold columns until this kernel ends while a CTA of
+// this kernel waits for columns, and tcgen05.alloc has no limit to its wait.  Behind the allocations of all CTAs the next
+// kernel can only wait for columns that come back.  (Today's shared memory keeps every such pair off one SM; this does not
+// depend on it.)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // A pointer to what the kernel ahead wrote must be taken through pdl_fresh (or pdl_wait_on) after the wait.

@@ -45,7 +45,6 @@ latent_expanded_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                        const int* __restrict__ seq_lens, int seq_begin, int seq_end, int heads, int rot, int window,
                        float scale_log2, const float* __restrict__ sink, int* __restrict__ err) {
   pdl_wait();
-  pdl_launch();
   using Shape = LeShape<NQ, DV>;
   constexpr int BN = Shape::BN, PANEL = Shape::PANEL, NV = Shape::NV, VP = DV / 64, NOPE = (NQ - 1) * 64;
   extern __shared__ __align__(1024) unsigned char le_raw[];
@@ -112,6 +111,7 @@ latent_expanded_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  pdl_launch();                                   // behind the allocation: see pdl_launch
   const unsigned tmem_s = __shfl_sync(0xffffffffu, *tmem_slot, 0), tmem_o = tmem_s + BN, tmem_p = tmem_o + DV;   // BN + DV + BN / 2 <= 256 columns
 
   if (warp == 0) {

@@ -126,7 +126,6 @@ lightning_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   unsigned long long* done = full + 12;                    // [2] MMA -> arithmetic, factors
   unsigned* tmem_slot = (unsigned*)(full + 14);
   pdl_wait();
-  pdl_launch();
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int h = blockIdx.x / SLICES, sl = blockIdx.x % SLICES, s = blockIdx.y;
   const int t0 = q_start[s], len = q_start[s + 1] - t0;
@@ -155,6 +154,7 @@ lightning_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  pdl_launch();                                            // behind the allocation: see pdl_launch
   const unsigned tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   auto wait = [&](unsigned long long* bar, unsigned parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)) != 0; };
 
@@ -405,7 +405,6 @@ lightning_outputs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   unsigned long long* fac_full = v_full + 16;              // [2] factors (32 lanes) -> weights, results
   unsigned* tmem_slot = (unsigned*)(v_full + 18);
   pdl_wait();
-  pdl_launch();
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   if (tg_smem(lg_raw) & 1023u) {
     if (tid == 0) atomicOr(err, 32);
@@ -434,6 +433,7 @@ lightning_outputs_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  pdl_launch();                                            // behind the allocation: see pdl_launch
   // Q K^T: 128 columns, the weights: 128, ND times what the start state gives and what the values give: DV each
   const unsigned tmem_raw = __shfl_sync(0xffffffffu, *tmem_slot, 0), tmem_p = tmem_raw + 128, tmem_d = tmem_raw + 256;
   auto wait = [&](unsigned long long* bar, unsigned parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)) != 0; };

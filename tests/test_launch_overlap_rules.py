@@ -64,3 +64,11 @@ def test_what_the_kernel_ahead_wrote_is_not_declared_unwritten(file, name, param
         fresh |= set(re.findall(r"\w+", args))
     for p in re.findall(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", params):
         assert p in INPUTS | fresh | WEIGHTS.get(name, set()) | BY_ADDRESS.get(name, set()), f"{file}: {name}: {p}"
+
+
+@pytest.mark.parametrize("file,name,params,body", [k for k in kernels() if "tcgen05.alloc" in k[3] and "pdl_launch" in k[3]],
+                         ids=lambda v: v if len(v) < 60 else "")
+def test_the_next_kernel_comes_in_behind_the_allocation_of_tensor_memory(file, name, params, body):
+    """Else its CTAs may hold columns and wait for this kernel's end while a CTA of this kernel waits for columns."""
+    assert body.index("tcgen05.alloc") < body.index("__syncthreads", body.index("tcgen05.alloc")) < body.index("pdl_launch"), f"{file}: {name}"
+    assert body.index("pdl_wait") < body.index("pdl_launch")
