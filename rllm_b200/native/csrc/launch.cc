@@ -14,6 +14,7 @@
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdlib>
@@ -143,20 +144,28 @@ bool finish(int rc, PyObject* what) {
   return false;
 }
 
+// What ATen throws (no strides, no memory) becomes the exception that PyTorch makes of it: nothing of C++ may leave a function
+// that the interpreter calls.
+template <typename F> PyObject* guarded(F&& body) {
+  try {
+    return body();
+  } catch (const std::exception&) {
+    torch::translate_exception_to_python(std::current_exception());
+    return nullptr;
+  }
+}
+
 PyObject* entry_call(PyObject* self, PyObject* const* args, size_t nargsf, PyObject* names) {
   Entry* e = (Entry*)self;
   if ((names && PyTuple_GET_SIZE(names)) || PyVectorcall_NARGS(nargsf) != e->count)
     return PyErr_Format(PyExc_TypeError, "%U takes %zd arguments, by position", e->what, e->count);
   if (!ready(e)) return nullptr;
-  try {
+  return guarded([&]() -> PyObject* {
     bool bad = false;
     const int rc = e->invoke(e->fn, args, bad);
     if (bad || !finish(rc, e->what)) return nullptr;
-  } catch (const std::exception& x) {
-    PyErr_SetString(PyExc_RuntimeError, x.what());
-    return nullptr;
-  }
-  Py_RETURN_NONE;
+    Py_RETURN_NONE;
+  });
 }
 
 void entry_free(PyObject* self) {
@@ -207,17 +216,17 @@ PyObject* set_products(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 // error_word(device index, tensor): the word that the tcgen05 product reports to on that device (the caller keeps it)
 PyObject* set_error_word(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  const long long d = n == 2 ? PyLong_AsLongLong(args[0]) : -1;
-  if (d < 0 || d >= 64 || !THPVariable_Check(args[1])) return PyErr_Occurred() ? nullptr : PyErr_Format(PyExc_TypeError, "error_word(device index, tensor)");
-  g_error_word[d] = THPVariable_Unpack(args[1]).data_ptr();
-  Py_RETURN_NONE;
+  return guarded([&]() -> PyObject* {
+    const long long d = n == 2 ? PyLong_AsLongLong(args[0]) : -1;
+    if (d < 0 || d >= 64 || !THPVariable_Check(args[1])) return PyErr_Occurred() ? nullptr : PyErr_Format(PyExc_TypeError, "error_word(device index, tensor)");
+    g_error_word[d] = THPVariable_Unpack(args[1]).data_ptr();
+    Py_RETURN_NONE;
+  });
 }
 
 bool is(const char* value, const char* text) { return value && !std::strcmp(value, text); }
 
-PyObject* product(PyObject*, PyObject* const* args, Py_ssize_t n) {
-  if (n != 7) return PyErr_Format(PyExc_TypeError, "product(x, w, out_f32, silu, limit, slope, shift)");
-  if (!g_small || !THPVariable_CheckExact(args[0]) || !(THPVariable_CheckExact(args[1]) || THPVariable_Check(args[1]))) Py_RETURN_NONE;
+PyObject* checked_product(PyObject* const* args) {
   const at::Tensor &x = THPVariable_Unpack(args[0]), &w = THPVariable_Unpack(args[1]);
   const bool f32 = args[2] == Py_True, silu = args[3] == Py_True;
   if (!x.is_cuda() || !w.is_cuda() || x.dim() != 2 || w.dim() != 2 || x.scalar_type() != at::kBFloat16 || w.scalar_type() != at::kBFloat16)
@@ -239,29 +248,30 @@ PyObject* product(PyObject*, PyObject* const* args, Py_ssize_t n) {
   Entry* e = small ? g_small : g_tcgen05;
   if (!small && (device < 0 || device >= 64 || !g_error_word[device])) Py_RETURN_NONE;
   if (!ready(e)) return nullptr;
-  try {
-    at::Tensor out = at::empty({M, N}, x.options().dtype(f32 ? at::kFloat : at::kBFloat16));
-    bool bad = false;
-    const float limit = Arg<'f'>::get(args[4], bad), slope = Arg<'f'>::get(args[5], bad), shift = Arg<'f'>::get(args[6], bad);
-    if (bad) return nullptr;
-    void *px = x.data_ptr(), *pw = w.data_ptr(), *po = out.data_ptr();
-    const int code = silu ? 2 : (f32 ? 1 : 0);
-    const cudaStream_t stream = stream_now();
-    int rc;
-    Py_BEGIN_ALLOW_THREADS
-    if (small)
-      rc = reinterpret_cast<int (*)(void*, int, void*, int, void*, int, int, int, int, int, float, float, float, cudaStream_t)>(e->fn)(
-          px, (int)lda, pw, (int)ldw, po, (int)N, (int)M, (int)N, (int)K, code, limit, slope, shift, stream);
-    else
-      rc = reinterpret_cast<int (*)(void*, int, void*, int, void*, int, int, int, int, int, float, float, float, void*, cudaStream_t)>(e->fn)(
-          px, (int)lda, pw, (int)ldw, po, (int)N, (int)M, (int)N, (int)K, code, limit, slope, shift, g_error_word[device], stream);
-    Py_END_ALLOW_THREADS
-    if (!finish(rc, e->what)) return nullptr;
-    return THPVariable_Wrap(std::move(out));
-  } catch (const std::exception& x) {
-    PyErr_SetString(PyExc_RuntimeError, x.what());
-    return nullptr;
-  }
+  at::Tensor out = at::empty({M, N}, x.options().dtype(f32 ? at::kFloat : at::kBFloat16));
+  bool bad = false;
+  const float limit = Arg<'f'>::get(args[4], bad), slope = Arg<'f'>::get(args[5], bad), shift = Arg<'f'>::get(args[6], bad);
+  if (bad) return nullptr;
+  void *px = x.data_ptr(), *pw = w.data_ptr(), *po = out.data_ptr();
+  const int code = silu ? 2 : (f32 ? 1 : 0);
+  const cudaStream_t stream = stream_now();
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  if (small)
+    rc = reinterpret_cast<int (*)(void*, int, void*, int, void*, int, int, int, int, int, float, float, float, cudaStream_t)>(e->fn)(
+        px, (int)lda, pw, (int)ldw, po, (int)N, (int)M, (int)N, (int)K, code, limit, slope, shift, stream);
+  else
+    rc = reinterpret_cast<int (*)(void*, int, void*, int, void*, int, int, int, int, int, float, float, float, void*, cudaStream_t)>(e->fn)(
+        px, (int)lda, pw, (int)ldw, po, (int)N, (int)M, (int)N, (int)K, code, limit, slope, shift, g_error_word[device], stream);
+  Py_END_ALLOW_THREADS
+  if (!finish(rc, e->what)) return nullptr;
+  return THPVariable_Wrap(std::move(out));
+}
+
+PyObject* product(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 7) return PyErr_Format(PyExc_TypeError, "product(x, w, out_f32, silu, limit, slope, shift)");
+  if (!g_small || !THPVariable_CheckExact(args[0]) || !THPVariable_CheckExact(args[1])) Py_RETURN_NONE;      // tensors and parameters
+  return guarded([&] { return checked_product(args); });
 }
 
 // setup(exception class, list of one int)

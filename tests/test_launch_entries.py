@@ -4,6 +4,8 @@ import ctypes
 import glob
 import os
 import re
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -52,6 +54,14 @@ def test_what_is_refused_before_anything_is_called():
     assert ops.product(x, x) is None and ops.product(x.bfloat16(), x.bfloat16()) is None
 
 
+def test_what_the_tensor_library_throws_is_an_exception():
+    """A tensor without memory of its own to point at; in a process of its own, which an exception that leaves the C++ ends."""
+    code = "import torch\nfrom rllm_b200.kernels import ops\ntry:\n    ops._launch().error_word(0, torch.eye(2).to_sparse())\n" \
+           "except RuntimeError as e:\n    print('raised')\n"
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert done.returncode == 0 and done.stdout == "raised\n", done.stderr[-500:]
+
+
 @pytest.mark.gpu
 def test_what_the_arguments_become_and_what_a_refusal_raises():
     seen = []
@@ -72,6 +82,18 @@ def test_what_the_arguments_become_and_what_a_refusal_raises():
         answer[0] = code
         with pytest.raises(ops.KernelError, match=text):
             entry(None, None, 0, 0)
+
+
+@pytest.mark.gpu
+def test_products_that_cannot_be_made_raise():
+    ops.gemm_error_word(torch.device("cuda", 0))
+    x = torch.randn(4, 64, device="cuda").bfloat16()
+    for a, b in ((x.to_sparse_csr(), x), (x, x.to_sparse_csr())):      # (no strides)
+        with pytest.raises(RuntimeError):
+            ops.product(a, b)
+    assert ops.product(x, torch.nn.Parameter(x)) is not None
+    with pytest.raises(torch.OutOfMemoryError):            # 2^22 x 2^16 results
+        ops.product(torch.zeros(1 << 22, 8, device="cuda", dtype=torch.bfloat16), torch.zeros(1 << 16, 8, device="cuda", dtype=torch.bfloat16))
 
 
 @pytest.mark.gpu
