@@ -87,30 +87,6 @@ __device__ __forceinline__ float div_1_plus_exp(float x, float y) {
   const float q = 0.25f * x * r, d = fmaf(fmaf(-q, y, x), 0.25f * r, q);
   return d == d ? d : q;
 }
-// The same of two: x0 / (1 + e0) and x1 / (1 + e1), in the instructions that do two float32 operations (with -y in place of y,
-// which rounds alike); the same bits.
-__device__ __forceinline__ void div_1_plus_exp_2(float& x0, float& x1, float e0, float e1) {
-  unsigned long long x, y, r, q, d;
-  float r0, r1, q0, q1;
-  const unsigned long long minus = 0xbf800000bf800000ull, fourth = 0x3e8000003e800000ull, minus_fourth = 0xbe800000be800000ull;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(x0), "f"(x1));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(e0), "f"(e1));
-  asm("fma.rn.f32x2 %0, %0, %1, %1;" : "+l"(y) : "l"(minus));                  // -(1 + e)
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(y), "l"(minus_fourth));
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r0), "=f"(r1) : "l"(r));
-  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(r0));
-  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(r1));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(r0), "f"(r1));
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(q) : "l"(x), "l"(fourth));
-  asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(q) : "l"(r));
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(q), "l"(y), "l"(x));
-  asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(r) : "l"(fourth));
-  asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(d) : "l"(r), "l"(q));
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x0), "=f"(x1) : "l"(d));
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(q0), "=f"(q1) : "l"(q));
-  x0 = x0 == x0 ? x0 : q0;
-  x1 = x1 == x1 ? x1 : q1;
-}
 
 // The gate of a gated feed-forward: g' sigmoid(slope g') (u' + shift) with g' = min(g, limit) and u' = u kept within
 // +-limit.  {infinity, 1, 0}: silu(g) u.

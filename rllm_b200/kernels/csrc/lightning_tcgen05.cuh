@@ -77,7 +77,7 @@ __device__ __forceinline__ uint4 lg_act8(const uint4& raw) {
   float v[8];
   unpack8(raw, v);
 #pragma unroll
-  for (int x = 0; x < 8; x += 2) div_1_plus_exp_2(v[x], v[x + 1], expf(-v[x]), expf(-v[x + 1]));
+  for (int x = 0; x < 8; ++x) v[x] = lt_silu(v[x]);
   return make_uint4(lg_pack(v[0], v[1]), lg_pack(v[2], v[3]), lg_pack(v[4], v[5]), lg_pack(v[6], v[7]));
 }
 

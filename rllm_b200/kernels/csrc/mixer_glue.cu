@@ -369,12 +369,7 @@ gated_rmsnorm8_kernel(const float* x, const bf16* g, int g_stride, const TW* w, 
       if (KEEP > 1) load8(w + i, wv);
       unpack8(gate[u], gv);
 #pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        float g0 = 1.0f, g1 = 1.0f;
-        div_1_plus_exp_2(g0, g1, expf(-gv[j]), expf(-gv[j + 1]));
-        v[u][j] = v[u][j] * r * (KEEP > 1 ? wv[j] : first_w[j]) * g0;
-        v[u][j + 1] = v[u][j + 1] * r * (KEEP > 1 ? wv[j + 1] : first_w[j + 1]) * g1;
-      }
+      for (int j = 0; j < 8; ++j) v[u][j] = v[u][j] * r * (KEEP > 1 ? wv[j] : first_w[j]) * div_1_plus_exp(1.0f, 1.0f + expf(-gv[j]));
       store8(out + base + i, v[u]);
     }
   }

@@ -147,10 +147,8 @@ struct Cv4 {                                       // four channels' weights and
       float acc = b[i];
 #pragma unroll
       for (int k = 0; k < 4; ++k) acc = fmaf(w[i][k], win[k][i], acc);
-      o[i] = acc;
+      o[i] = ss_silu(acc);
     }
-#pragma unroll
-    for (int i = 0; i < 4; i += 2) div_1_plus_exp_2(o[i], o[i + 1], expf(-o[i]), expf(-o[i + 1]));
     uint2 raw;
     *(__nv_bfloat162*)&raw.x = __floats2bfloat162_rn(o[0], o[1]);
     *(__nv_bfloat162*)&raw.y = __floats2bfloat162_rn(o[2], o[3]);

@@ -137,11 +137,7 @@ silu_gated_group_rmsnorm8_kernel(const float* y, const bf16* z, int z_stride, co
       float zv[8];
       unpack8(gate[u], zv);
 #pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        div_1_plus_exp_2(zv[j], zv[j + 1], expf(-zv[j]), expf(-zv[j + 1]));
-        v[u][j] *= zv[j];
-        v[u][j + 1] *= zv[j + 1];
-      }
+      for (int j = 0; j < 8; ++j) v[u][j] *= lt_silu(zv[j]);
       *(float4*)(sgn_x + i) = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
       *(float4*)(sgn_x + i + 4) = make_float4(v[u][4], v[u][5], v[u][6], v[u][7]);
     }
