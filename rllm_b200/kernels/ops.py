@@ -1521,6 +1521,14 @@ def gated_rmsnorm(x: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, eps
 # recurrences with a state per request (lightning.cu, selective_scan.cu)
 # ---------------------------------------------------------------------------
 SCAN_CHUNKED_FROM = 129       # portions from this many tokens on are scanned as chunks side by side
+# Heads x decoded tokens x value columns from which those tokens are walked by a launch of their own: among the portions each is
+# a padded chunk a head, but a walk takes 8 us by itself.  us with them among the portions / apart, decoded tokens + the prompt:
+#   with steps, 16 heads of 64 x 64: 8 + 129 17.0 / 20.7, 32 + 129 36.6 / 23.2, 64 + 129 64 / 30; 16 of 64 x 128: 8 + 300 + 300
+#   29.9 / 26.3, 64 + 700 113 / 52; 4 of 64 x 64: 32 + 129 17.1 / 20.0, 64 + 129 26.7 / 20.3; 64 of 64 x 64: 1 + 129 16.9 / 23.2,
+#   8 + 129 37.3 / 24.6, 64 + 129 210 / 72
+#   without, 16 heads of 64 x 64: 64 + 129 68 / 33; 4 of 64 x 128: 64 + 129 40.0 / 24.3
+# (Chunk passes without tcgen05, as these sizes had them first: 16 heads of 64 x 64 with steps, 64 + 129 49 us.)
+SCAN_APART_FROM = 1 << 14
 
 
 def _chunks_for(lib_chunk: int, max_q_len: int, num_seqs: int) -> int:
@@ -1532,10 +1540,11 @@ def _chunks_for(lib_chunk: int, max_q_len: int, num_seqs: int) -> int:
 
 def lightning_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, state: torch.Tensor,
                    q_start: torch.Tensor, slots: torch.Tensor, num_seqs: int, err: torch.Tensor,
-                   max_q_len: int = 1) -> torch.Tensor:
+                   max_q_len: int = 1, num_decode: int = 0) -> torch.Tensor:
     """Linear attention with a decay per head.  q, k [T, heads * d] and v [T, heads * dv] are column slices of
     one tensor (the projections before their silu); state float32 [slots, heads, d, dv], updated in place;
-    returns o float32 [T, heads * dv]."""
+    returns o float32 [T, heads * dv].  The first ``num_decode`` sequences bring one token each; beside portions that
+    are scanned as chunks they take the plain walk where they are many (``SCAN_APART_FROM``)."""
     lib = build.load_library("lightning")
     heads, d, dv = state.shape[1:]
     T = q.shape[0]
@@ -1545,7 +1554,12 @@ def lightning_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: tor
     assert decay.numel() == heads
     _contig(state, "state")
     out = torch.empty((T, heads * dv), dtype=torch.float32, device=q.device)
-    chunks = _chunks_for(int(lib.rllm_lightning_chunk()), max_q_len, num_seqs)
+    apart = num_decode if heads * num_decode * dv >= SCAN_APART_FROM else 0
+    chunks = _chunks_for(int(lib.rllm_lightning_chunk()), max_q_len, num_seqs - apart)
+    if chunks and apart:
+        _entries.rllm_lightning_scan(q, k, v, T, q.stride(0), dtype_code(q.dtype), decay, state, None, None, q_start, slots,
+                                     state.shape[0], apart, 0, out, heads, d, dv, err)
+        q_start, slots, num_seqs = q_start[apart:], slots[apart:], num_seqs - apart
     work = torch.empty(num_seqs * chunks * heads * d * dv, dtype=torch.float32, device=q.device) if chunks else None
     # room for the activated projections, where the tensor cores read them
     act = torch.empty((T, heads * (2 * d + dv)), dtype=q.dtype, device=q.device) if chunks and q.dtype is torch.bfloat16 else None
@@ -1709,11 +1723,12 @@ def head_gated_rmsnorm(x: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor
 # ---------------------------------------------------------------------------
 def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: torch.Tensor, skip: torch.Tensor,
              state: torch.Tensor, q_start: torch.Tensor, slots: torch.Tensor, num_seqs: int, heads: int, groups: int,
-             n: int, p: int, err: torch.Tensor, max_q_len: int = 1) -> torch.Tensor:
+             n: int, p: int, err: torch.Tensor, max_q_len: int = 1, num_decode: int = 0) -> torch.Tensor:
     """The Mamba-2 recurrence over this step's tokens.  xbc [T, heads p + 2 groups n]: x | B | C, activated; dt
     float32 [T, heads]: the steps before bias and softplus; dt_bias, a_log, skip float32 [heads]; state float32
     [slots, heads, n, p], updated in place.  Returns y = S^T C + skip x, float32 [T, heads p].  Portions long enough
-    to fill the GPU with chunks are scanned as chunks side by side; the result differs by rounding only."""
+    to fill the GPU with chunks are scanned as chunks side by side; the result differs by rounding only.  ``num_decode`` as
+    in ``lightning_scan``."""
     lib = build.load_library("ssd")
     T = xbc.shape[0]
     assert xbc.shape[1] == heads * p + 2 * groups * n and xbc.stride(1) == 1
@@ -1724,12 +1739,17 @@ def ssd_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, a_log: 
     assert state.dtype is torch.float32 and tuple(state.shape[1:]) == (heads, n, p)
     _contig(dt, "dt"); _contig(state, "state")
     out = torch.empty((T, heads * p), dtype=torch.float32, device=xbc.device)
-    chunks = _chunks_for(int(lib.rllm_ssd_chunk()), max_q_len, num_seqs)
+    stride = xbc.stride(0) if T > 1 else xbc.shape[1]
+    apart = num_decode if heads * num_decode * p >= SCAN_APART_FROM else 0
+    chunks = _chunks_for(int(lib.rllm_ssd_chunk()), max_q_len, num_seqs - apart)
+    if chunks and apart:
+        _entries.rllm_ssd_scan(xbc, T, stride, dtype_code(xbc.dtype), dt, dt_bias, a_log, skip, state, None, None, q_start,
+                               slots, state.shape[0], apart, 0, out, heads, groups, n, p, err)
+        q_start, slots, num_seqs = q_start[apart:], slots[apart:], num_seqs - apart
     work = torch.empty(num_seqs * chunks * heads * (n * p + 1), dtype=torch.float32, device=xbc.device) if chunks else None
     chunk_dt = work[num_seqs * chunks * heads * n * p:] if chunks else None
-    _entries.rllm_ssd_scan(xbc, T, xbc.stride(0) if T > 1 else xbc.shape[1], dtype_code(xbc.dtype), dt, dt_bias, a_log,
-                           skip, state, work, chunk_dt, q_start, slots, state.shape[0], num_seqs, chunks, out, heads,
-                           groups, n, p, err)
+    _entries.rllm_ssd_scan(xbc, T, stride, dtype_code(xbc.dtype), dt, dt_bias, a_log, skip, state, work, chunk_dt, q_start,
+                           slots, state.shape[0], num_seqs, chunks, out, heads, groups, n, p, err)
     return out
 
 

@@ -69,6 +69,7 @@ class LightningAttention(Mixer):
         qk, vv = self.heads * self.d, self.heads * self.dv
         a = linear(x, self.w_in)                                     # [T, 2 qk + 2 vv]: q | k | v | g
         o = ops.lightning_scan(a[:, :qk], a[:, qk:2 * qk], a[:, 2 * qk:2 * qk + vv], self.decay_dev, cache.state,
-                               ctx.q_start, ctx.state_slots, ctx.num_seqs, ctx.err, max_q_len=ctx.max_q_len)
+                               ctx.q_start, ctx.state_slots, ctx.num_seqs, ctx.err, max_q_len=ctx.max_q_len,
+                               num_decode=ctx.num_decode)
         y = ops.gated_rmsnorm(o, a[:, 2 * qk + vv:], self.w_norm, self.eps, x.dtype)
         return linear(y, self.w_o)

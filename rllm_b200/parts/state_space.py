@@ -99,6 +99,6 @@ class StateSpace(Mixer):
                             ctx.state_slots, ctx.num_seqs, ctx.num_tokens > ctx.num_decode, ctx.err)
         y = ops.ssd_scan(c, dt, w["dt_bias"], w["a_log"], w["d"], scan_state.state, ctx.q_start, ctx.state_slots,
                          ctx.num_seqs, self.heads, self.groups, self.state, self.dv, ctx.err,
-                         max_q_len=ctx.max_q_len)                          # float32 [T, inner]
+                         max_q_len=ctx.max_q_len, num_decode=ctx.num_decode)      # float32 [T, inner]
         y = ops.silu_gated_group_rmsnorm(y, a[:, :E], w["norm"], self.eps, self.norm_groups, x.dtype)
         return linear(y, w["o"])

@@ -98,3 +98,30 @@ def test_which_tile_a_product_takes(M, N, K, epilogue, sms, form):
     from ctypes import c_int
     f = build.load_library("gemm_tcgen05").rllm_gemm_tcgen05_form
     assert f(c_int(M), c_int(N), c_int(K), c_int(epilogue), c_int(sms)) == form
+
+
+def test_the_recurrences_are_told_how_many_tokens_decode(monkeypatch):
+    """Their scans walk those apart from the portions that are cut into chunks."""
+    from types import SimpleNamespace
+
+    from rllm_b200.parts import lightning, state_space
+    seen = []
+
+    def scan(*a, num_decode, **k):
+        seen.append(num_decode)
+        return torch.zeros(7, 8)
+    for module in (lightning, state_space):
+        monkeypatch.setattr(module, "linear", lambda x, w, **k: torch.zeros(7, 64))
+    for name in ("lightning_scan", "ssd_scan"):
+        monkeypatch.setattr(ops, name, scan)
+    for name in ("gated_rmsnorm", "silu_gated_group_rmsnorm", "causal_conv"):
+        monkeypatch.setattr(ops, name, lambda *a, **k: None)
+    ctx = SimpleNamespace(q_start=None, state_slots=None, token_seq=None, num_seqs=4, num_tokens=7, num_decode=3, err=None, max_q_len=4)
+    a = lightning.LightningAttention.__new__(lightning.LightningAttention)
+    a.heads, a.d, a.dv, a.eps, a.w_in, a.w_o, a.w_norm, a.decay_dev = 2, 4, 4, 0.0, None, None, None, None
+    a.forward(torch.zeros(7, 8), ctx, SimpleNamespace(state=None))
+    b = state_space.StateSpace.__new__(state_space.StateSpace)
+    b.__dict__.update(w={k: None for k in ("dt", "conv", "conv_bias", "dt_bias", "a_log", "d", "norm", "o")}, inner=8, heads=2, groups=1, state=4,
+                      dv=4, eps=0.0, norm_groups=1, w_in=None)
+    b.forward(torch.zeros(7, 8), ctx, (SimpleNamespace(state=None),) * 2)
+    assert seen == [3, 3]

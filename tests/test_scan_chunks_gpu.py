@@ -39,16 +39,16 @@ def inputs(steps, heads, groups, d, dv, T, seed):
                       torch.ones(T, heads, dtype=F64), torch.zeros(heads, dtype=F64))
 
 
-def scan(steps, heads, groups, d, dv, args, state, lens, slots):
+def scan(steps, heads, groups, d, dv, args, state, lens, slots, **more):
     from rllm_b200.kernels import ops
     err = torch.zeros(1, dtype=torch.int32, device="cuda")
     starts = i32([sum(lens[:i]) for i in range(len(lens) + 1)])
     args = [x.cuda() for x in args]
     if steps:
-        out = ops.ssd_scan(*args, state, starts, i32(slots), len(lens), heads, groups, d, dv, err, max_q_len=max(lens))
+        out = ops.ssd_scan(*args, state, starts, i32(slots), len(lens), heads, groups, d, dv, err, max_q_len=max(lens), **more)
     else:
         q, k, v = torch.split(args[0], [heads * d, heads * d, heads * dv], 1)
-        out = ops.lightning_scan(q, k, v, args[1], state, starts, i32(slots), len(lens), err, max_q_len=max(lens))
+        out = ops.lightning_scan(q, k, v, args[1], state, starts, i32(slots), len(lens), err, max_q_len=max(lens), **more)
     assert int(err.item()) == 0
     return out.view(-1, heads, dv)
 
@@ -92,3 +92,23 @@ def test_a_value_that_is_not_finite_reaches_later_tokens_of_its_column_only(step
     hit[bad:lens[0], 1, 7] = True
     assert not torch.isfinite(got[hit]).any()
     assert torch.equal(got[~hit], clean[~hit])
+
+
+@pytest.mark.parametrize("steps,heads,groups,d,dv,prompts", [(True, 4, 2, 64, 64, [129]), (True, 12, 1, 128, 64, [200, 900]), (True, 2, 1, 24, 40, [300]),
+                                                             (False, 3, 0, 128, 128, [130, 2]), (False, 2, 0, 32, 64, [500]), (False, 2, 0, 48, 20, [140])])
+def test_decoded_tokens_beside_prompts_have_the_bits_of_either_alone(steps, heads, groups, d, dv, prompts):
+    """With as many decoded tokens as are walked apart, and a few more."""
+    from rllm_b200.kernels import ops
+    decode = -(-ops.SCAN_APART_FROM // (heads * dv)) + 2
+    lens = [1] * decode + prompts
+    args, _ = inputs(steps, heads, groups, d, dv, sum(lens), d + dv)
+    g = torch.Generator().manual_seed(d)
+    first = torch.randn(len(lens) + 2, heads, d, dv, generator=g).cuda()
+    slots = torch.randperm(len(lens) + 2, generator=g)[: len(lens)].tolist()
+    both, alone, behind = first.clone(), first.clone(), first.clone()
+    got = scan(steps, heads, groups, d, dv, args, both, lens, slots, num_decode=decode)
+    part = lambda lo, hi: [x[lo:hi] if len(x) == sum(lens) else x for x in args]  # noqa: E731
+    want = torch.cat([scan(steps, heads, groups, d, dv, part(0, decode), alone, [1] * decode, slots[:decode]),
+                      scan(steps, heads, groups, d, dv, part(decode, None), behind, prompts, slots[decode:])])
+    assert torch.equal(got, want)
+    assert torch.equal(both[slots], torch.cat([alone[slots[:decode]], behind[slots[decode:]]]))
