@@ -23,6 +23,10 @@
 // max_chunks 0: the plain walk.  > 0: ceil(longest portion / LT_CHUNK); work then holds
 // num_seqs * max_chunks * heads * d * dv floats; act null, or (bfloat16) a row of heads (2 d + dv) values a token.
 RLLM_EXPORT int rllm_lightning_chunk() { return LT_CHUNK; }
+// the host's rule alone, for tests
+RLLM_EXPORT int rllm_lightning_tcgen05_pays(int chunks, int heads, int num_seqs, int d, int dv) {
+  return lg_pays(false, chunks, heads, num_seqs, d, dv);
+}
 
 // RLLM_LIGHTNING=simt keeps the chunk passes on the CUDA cores (for tests and comparisons)
 static inline bool lightning_mma_disabled() {

@@ -821,6 +821,24 @@ static int lg_launch(const bf16* q, const bf16* k, const bf16* v, int rows, int 
   return 0;
 }
 
+// Whether these kernels are faster than the passes of lightning_mma.cuh, for num_seqs sequences of which the longest has
+// `chunks` chunks of 128.  The states' kernel takes a chunk after the other, 1 us each, whatever the number of heads; the
+// passes take all chunks side by side and are bound by the work.  us there / here:
+//   more than six chunks, 2,048 tokens: 4, 8, 12, 24 heads of 128 x 64 with steps 23.6 / 29.7, 29.7 / 31.7, 39.9 / 33.8, 58 / 40;
+//     2, 4, 6, 12 of 128 x 128 without 35.8 / 33.8, 35.8 / 35.8, 52 / 38, 79 / 50; 4 of 128 x 128 without beside 8 decoded
+//     tokens 38.7 / 31.2, with steps 32.5 / 28.2: those count as sequences too (4 of 64 x 64 are the exception: 22.0 / 24.8)
+//   fewer, with steps: 4 heads of 64 x 64, 300, 512, 768 tokens 11.5 / 12.2, 11.7 / 13.2, 12.5 / 14.8; 10 of them 768 15.2 / 15.3;
+//     4 of 128 x 64 512, 768 tokens 14.3 / 14.3, 14.7 / 15.6; 2 of 64 x 128 768 14.3 / 16.1, 4 of them 15.9 / 15.7; 1 of
+//     128 x 128 768 15.4 / 16.5, 2 of them 16.3 / 15.3
+//   without: 4 heads of 64 x 64, 640 tokens 13.7 / 16.0, 768 13.8 / 16.9
+static inline bool lg_pays(bool steps, int chunks, int heads, int num_seqs, int d, int dv) {
+  const long long work = (long long)heads * num_seqs * d * dv;
+  if (chunks > 6) return work >= 5 << 14;
+  if (!steps) return !(d == 64 && dv == 64 && chunks >= 5 && work < 6 << 12);
+  if (dv == 64 && chunks >= (d == 64 ? 3 : 6)) return work >= 10 << 12;
+  return chunks < 4 || work >= 8 << 12;
+}
+
 // The kernels where the head's sizes are built and rows start on 16 bytes; -1: not taken.  max_chunks: of LT_CHUNK tokens
 // (the start states of half as many chunks lie in `work`).  act (without STEPS): a row of heads (2 d + dv) values a token.
 template <bool STEPS>
@@ -832,11 +850,7 @@ static int lg_scan(const bf16* q, const bf16* k, const bf16* v, int rows, int st
   const int chunks = (max_chunks + 1) / 2;
   if (!(d == 64 || d == 128) || !(dv == 64 || dv == 128) || stride % 8 || (at & 15) || !err || rows <= 0 || (!STEPS && !act)) return -1;
   if ((long long)num_seqs * chunks * heads > 0x3fffffffLL || (long long)heads * 256 > 0x7fffffffLL) return -1;
-  // The states' kernel takes a chunk after the other, 1 us each, whatever the number of heads; the passes of lightning_mma.cuh
-  // take all chunks side by side and are bound by the work.  us there / here, 2,048 tokens: 4, 8, 12, 24 heads of 128 x 64 with
-  // steps 23.6 / 29.7, 29.7 / 31.7, 39.9 / 33.8, 58 / 40; 2, 4, 6, 12 of 128 x 128 without 35.8 / 33.8, 35.8 / 35.8, 52 / 38,
-  // 79 / 50; 700 tokens: 4 heads of 128 x 64 21.5 / 21.5, 12 25.6 / 21.5, 4 of 64 x 64 23.6 / 21.5.
-  if (chunks > 6 && (long long)heads * num_seqs * d * dv < 5 << 14) return -1;
+  if (!lg_pays(STEPS, chunks, heads, num_seqs, d, dv)) return -1;
 #define LG_GO(D_, DV_)                                                                                                    \
   if (d == D_ && dv == DV_)                                                                                               \
     return lg_launch<D_, DV_, STEPS>(q, k, v, rows, stride, decay, steps, state, work, act, q_start, slots, num_slots, num_seqs, chunks, \

@@ -16,6 +16,10 @@
 #include "lightning_tcgen05.cuh"
 
 RLLM_EXPORT int rllm_ssd_chunk() { return LT_CHUNK; }
+// the host's rule alone, for tests
+RLLM_EXPORT int rllm_ssd_tcgen05_pays(int chunks, int heads, int num_seqs, int d, int dv) {
+  return lg_pays(true, chunks, heads, num_seqs, d, dv);
+}
 
 // RLLM_SSD=simt keeps the chunk passes on the CUDA cores (for tests and comparisons)
 static inline bool ssd_mma_disabled() {

@@ -100,6 +100,18 @@ def test_which_tile_a_product_takes(M, N, K, epilogue, sms, form):
     assert f(c_int(M), c_int(N), c_int(K), c_int(epilogue), c_int(sms)) == form
 
 
+@pytest.mark.parametrize("library,chunks,heads,num_seqs,d,dv,pays", [
+    ("ssd", 16, 10, 1, 128, 64, True), ("ssd", 16, 4, 1, 64, 64, False), ("ssd", 7, 4, 5, 64, 64, True), ("ssd", 6, 6, 1, 64, 64, False),
+    ("ssd", 3, 4, 2, 64, 64, False), ("ssd", 3, 10, 1, 64, 64, True), ("ssd", 2, 1, 1, 64, 64, True), ("ssd", 6, 4, 1, 128, 64, False),
+    ("ssd", 5, 4, 1, 128, 64, True), ("ssd", 6, 6, 1, 128, 64, True), ("ssd", 4, 2, 1, 64, 128, False), ("ssd", 4, 4, 1, 64, 128, True),
+    ("ssd", 6, 1, 1, 128, 128, False), ("ssd", 6, 2, 1, 128, 128, True), ("lightning", 6, 1, 1, 128, 128, True),
+    ("lightning", 6, 4, 1, 64, 64, False), ("lightning", 4, 4, 1, 64, 64, True), ("lightning", 16, 4, 1, 128, 128, False),
+    ("lightning", 16, 5, 1, 128, 128, True)])
+def test_which_portions_the_tcgen05_recurrences_pay_for(library, chunks, heads, num_seqs, d, dv, pays):
+    f = getattr(build.load_library(library), f"rllm_{library}_tcgen05_pays")
+    assert bool(f(chunks, heads, num_seqs, d, dv)) is pays
+
+
 def test_the_recurrences_are_told_how_many_tokens_decode(monkeypatch):
     """Their scans walk those apart from the portions that are cut into chunks."""
     from types import SimpleNamespace

@@ -53,10 +53,10 @@ def scan(steps, heads, groups, d, dv, args, state, lens, slots, **more):
     return out.view(-1, heads, dv)
 
 
-# both sides of the line where the chunks of 128 are taken (768 tokens; heads times their size), portions around a chunk,
+# both sides of the line where the chunks of 128 are taken (their number; heads times their size), portions around a chunk,
 # groups of one head, of some and of all, more pairs of chunk and head than an SM each, few and many CTAs a head
 @pytest.mark.parametrize("steps,heads,groups,d,dv,lens", [
-    (True, 4, 2, 128, 64, [129, 128, 1]), (True, 3, 3, 64, 64, [127, 257, 130]), (True, 2, 1, 64, 128, [300, 2]),
+    (True, 4, 2, 128, 64, [129, 128, 1]), (True, 3, 3, 64, 64, [127, 257, 130]), (True, 6, 3, 64, 64, [127, 257, 130]), (True, 2, 1, 64, 128, [300, 2]),
     (True, 2, 1, 128, 128, [511]), (True, 12, 2, 128, 64, [900, 640, 5]), (True, 40, 4, 128, 64, [700]), (True, 2, 1, 128, 64, [900]),
     (False, 3, 0, 128, 128, [129, 128, 1]), (False, 2, 0, 64, 64, [127, 257, 130]), (False, 2, 0, 64, 128, [300, 2]),
     (False, 2, 0, 128, 64, [511]), (False, 6, 0, 128, 128, [900, 3]), (False, 2, 0, 128, 128, [900])])
