@@ -500,27 +500,35 @@ static int tg_launch(const void* a, int lda, const void* w, int ldw, int w_rows,
 //   2,048 x 1,344 x 2,048 17.2 / 13.7 / 17.8, 17.2 / 14.0 / 16.2;    1,024 x 2,048 x 8,192 49 / 40 / 31.5, 42 / 39 / 28.8
 //   6,327 x 3,072 x 2,048 69 / 67 / 76, 61 / 63 / 68
 // With the gate a tile has half as many output columns.
+// Every column of tiles passes over A once more, from HBM where A is larger than what L2 (126 MB) keeps of it: tiles of 128
+// are left out there unless one or two of them span all columns.  Pairs of 256 / 128 columns, M x N x K (A in MB): 8,192 x 1,344 x
+// 8,192 (128) 142 / 161, 16,384 x 1,344 x 4,096 (128) 162 / 222, 16,384 x 1,344 x 8,192 (256) 312 / 426, 8,192 x 1,344 x 6,144 (96)
+// 110 / 123, x 5,120 (80) 93 / 100, x 4,096 (64) 75 / 75; but 8,192 x 200 x 8,192 45 / 37.
 struct TgForm { int width; bool pair; };
-static TgForm tg_form(long long tiles_rows, long long tiles_rows2, int N, int K, bool gate, bool pairs, long long sms) {
+static TgForm tg_form(long long tiles_rows, long long tiles_rows2, int N, int K, bool gate, bool pairs, long long sms, long long a_bytes) {
   static const int widths[3] = {256, 192, 128};
   static const double single[2][3] = {{4.6, 4.6, 4.6}, {0.37, 0.30, 0.22}}, both[2][3] = {{6.3, 6.0, 5.8}, {0.32, 0.275, 0.19}};
   const double steps = (K + TG_BK - 1) / TG_BK;
   TgForm best{256, false};
   double least = 1e30;
+  auto passes = [&](int i, long long across) { return widths[i] == 128 && across > 2 && a_bytes > 72ll << 20; };   // over A, too many
   for (int i = 0; i < 3; ++i) {
     const long long cols = gate ? widths[i] / 2 : widths[i], across = (N + cols - 1) / cols;
+    if (passes(i, across)) continue;
     const double t = single[0][i] + single[1][i] * steps * (double)((tiles_rows * across + sms - 1) / sms);
     if (t < least) { least = t; best = TgForm{widths[i], false}; }
   }
   for (int i = 0; i < 3 && pairs && sms >= 2; ++i) {
     const long long cols = gate ? widths[i] / 2 : widths[i], across = (N + cols - 1) / cols;
+    if (passes(i, across)) continue;
     const double t = both[0][i] + both[1][i] * steps * (double)((tiles_rows2 * across + sms / 2 - 1) / (sms / 2));
     if (t < least) { least = t; best = TgForm{widths[i], true}; }
   }
   return best;
 }
 static TgForm tg_form_of(int M, int N, int K, int epilogue, long long sms) {
-  return tg_form((M + TG_BM - 1) / TG_BM, (M + 2 * TG_BM - 1) / (2 * TG_BM), N, K, epilogue == TG_EPI_SILU, true, sms);
+  return tg_form((M + TG_BM - 1) / TG_BM, (M + 2 * TG_BM - 1) / (2 * TG_BM), N, K, epilogue == TG_EPI_SILU, true, sms,
+                 2ll * M * K);
 }
 // the width of the tiles, negative for pairs (the host's rule alone, for tests)
 RLLM_EXPORT int rllm_gemm_tcgen05_form(int M, int N, int K, int epilogue, int sms) {
@@ -575,7 +583,7 @@ RLLM_EXPORT int rllm_head_gemm_tcgen05(const void* a, long long lda, long long a
   if (M <= 0 || N <= 0 || heads <= 0) return 0;
   if (K <= 0 || !err) return RLLM_E_BADARG;
   if (K % 8 || lda % 8 || a_head % 8 || ldw % 8 || w_head % 8 || (((uintptr_t)a | (uintptr_t)w) & 15)) return RLLM_E_UNSUPPORTED;
-  const int bn = tg_form((long long)((M + TG_BM - 1) / TG_BM) * heads, 0, N, K, false, false, tg_num_sms()).width;
+  const int bn = tg_form((long long)((M + TG_BM - 1) / TG_BM) * heads, 0, N, K, false, false, tg_num_sms(), 2ll * M * K).width;
   if (bn == 256) return tg_launch_heads<256>(a, lda, a_head, w, ldw, w_head, out, ldo, c_head, M, N, K, heads, err, stream);
   if (bn == 192) return tg_launch_heads<192>(a, lda, a_head, w, ldw, w_head, out, ldo, c_head, M, N, K, heads, err, stream);
   return tg_launch_heads<128>(a, lda, a_head, w, ldw, w_head, out, ldo, c_head, M, N, K, heads, err, stream);

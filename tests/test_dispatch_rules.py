@@ -92,7 +92,8 @@ def test_how_many_warps_share_a_row_of_the_cuda_core_attention():
 @pytest.mark.parametrize("M,N,K,epilogue,sms,form", [
     (2047, 3072, 2048, 0, 148, -192), (2047, 2048, 4096, 0, 148, -256), (2047, 2048, 2048, 0, 148, 256), (2047, 4096, 2048, 2, 148, -256),
     (1024, 2048, 8192, 0, 148, -128), (6327, 2048, 2048, 1, 148, -256), (2048, 1024, 1024, 0, 148, 128), (100, 200, 64, 0, 148, 128),
-    (700, 3072, 2048, 0, 148, 128), (2047, 2048, 4096, 0, 1, 256)])
+    (700, 3072, 2048, 0, 148, 128), (2047, 2048, 4096, 0, 1, 256), (8192, 1344, 8192, 0, 148, -256), (16384, 1344, 4096, 0, 148, -256),
+    (8192, 1344, 4096, 0, 148, -128), (8192, 200, 8192, 0, 148, -128), (16384, 672, 4096, 2, 148, -256)])
 def test_which_tile_a_product_takes(M, N, K, epilogue, sms, form):
     """The tile's width, negative for pairs of CTAs; a device of one SM has no pairs."""
     from ctypes import c_int
