@@ -103,6 +103,7 @@ def plan_cache_pages(model: DecoderModel, args: EngineArgs, max_model_len: int, 
     spec = model.spec
     act = args.max_num_batched_tokens * (spec.hidden_size * 16 + 64 * 1024) + \
         min(args.max_num_seqs, args.max_num_batched_tokens) * spec.vocab_size * 8 + (1 << 30)
+    act += model.step_scratch() if hasattr(model, "step_scratch") else 0
     budget = int(total * args.gpu_memory_utilization) - (total - free) - act
     if budget < 4 * sum(nbytes):
         raise RuntimeError(f"no room for a KV cache: {free >> 20} MiB free of {total >> 20} MiB with "

@@ -98,6 +98,10 @@ class DecoderModel:
                     total += v.numel() * v.element_size()
         return total
 
+    def step_scratch(self) -> int:
+        """Bytes that a step may take by what the cache holds; layers run one after the other."""
+        return max((b.mixer.step_scratch() for b in self.blocks), default=0)
+
     # -- cache ------------------------------------------------------------
     def _cache_layout(self) -> CacheLayout:
         groups: List[object] = []

@@ -237,6 +237,10 @@ class Mixer(Part):
     def cache_need(self):
         return None
 
+    def step_scratch(self) -> int:
+        """Bytes that a step may take for a while by what the cache holds, beside those that grow with its tokens."""
+        return 0
+
     def stack_input(self, weight: torch.Tensor) -> bool:
         """A block may hand a mixer one more weight [rows, H] that reads the mixer's own input: a mixer whose
         first step is a matrix product over stacked weights appends it there and returns True; its

@@ -108,6 +108,10 @@ class LatentAttention(Mixer):
         return ([n["dkv"], n["dkv_norm"]] if self.shares_kv else []) + \
             ([] if self.has_sink or "sink" not in n else [n["sink"]])
 
+    def step_scratch(self) -> int:
+        # gathered rows, keys and values of prompt portions grow with the context; one layer's at a time
+        return ops.LATENT_EXPANDED_SCRATCH if self.w_ukv is not None else 0
+
     def load(self, tensors: Dict[str, torch.Tensor]) -> None:
         n, H = self.names, self.heads
         if self.shares_kv:

@@ -52,6 +52,30 @@ def test_counts_from_free_memory(monkeypatch):
         engine_core.plan_cache_pages(m, args, 8192, torch.device("cpu"))
 
 
+def test_what_a_step_takes_by_its_context_is_set_aside(monkeypatch):
+    """The keys and values that a latent mixer makes of a prompt's visible rows: beside them the cache gets less."""
+    from rllm_b200.kernels import ops
+    from rllm_b200.models.decoder import DecoderModel
+    from rllm_b200.parts.base import Mixer
+    from rllm_b200.parts.latent_attention import LatentAttention
+    latent, own = LatentAttention.__new__(LatentAttention), LatentAttention.__new__(LatentAttention)
+    latent.w_ukv, own.w_ukv = None, torch.zeros(1)
+    block = lambda m: SimpleNamespace(mixer=m)  # noqa: E731
+    m = DecoderModel.__new__(DecoderModel)
+    need = KVPagesNeed(1, 576, None, values=False)
+    m.layout, m.dtype, m.spec = SimpleNamespace(groups=[need], owners=[[0, 1]]), torch.bfloat16, SimpleNamespace(hidden_size=64, vocab_size=100)
+    args = EngineArgs(block_size=16, max_num_seqs=1024, max_num_batched_tokens=64, gpu_memory_utilization=0.5)
+    GiB = 1 << 30
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device=None: (4 * GiB, 8 * GiB))
+    args.gpu_memory_utilization = 1.0
+    pages = []
+    for mixers in ([Mixer.__new__(Mixer), latent], [latent, own, own]):
+        m.blocks = [block(x) for x in mixers]
+        pages += engine_core.plan_cache_pages(m, args, 1 << 20, torch.device("cpu"))
+    assert m.step_scratch() == ops.LATENT_EXPANDED_SCRATCH
+    assert abs((pages[0] - pages[1]) * 2 * page_bytes(need, 16, 2) - ops.LATENT_EXPANDED_SCRATCH) <= 2 * page_bytes(need, 16, 2)
+
+
 def test_a_model_without_pages_needs_none():
     m = fake_model([StateNeed((4,))], [[0]])
     assert engine_core.plan_cache_pages(m, EngineArgs(), 128, torch.device("cpu")) == []
