@@ -90,12 +90,12 @@ class DecoderModel:
         self.dtype, self.device = run_dtype, device
 
     def num_weight_bytes(self) -> int:
-        seen, total = set(), 0
-        for part in self.parts():
-            for v in vars(part).values():
-                if isinstance(v, torch.Tensor) and v.data_ptr() not in seen:
-                    seen.add(v.data_ptr())
-                    total += v.numel() * v.element_size()
+        spans = sorted((v.data_ptr(), v.data_ptr() + v.numel() * v.element_size())
+                       for part in self.parts() for v in vars(part).values() if isinstance(v, torch.Tensor))
+        total = end = 0
+        for a, b in spans:                       # (a part may keep a tensor and a view of it)
+            total += max(0, b - max(a, end))
+            end = max(end, b)
         return total
 
     def step_scratch(self) -> int:

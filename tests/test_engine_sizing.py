@@ -76,6 +76,15 @@ def test_what_a_step_takes_by_its_context_is_set_aside(monkeypatch):
     assert abs((pages[0] - pages[1]) * 2 * page_bytes(need, 16, 2) - ops.LATENT_EXPANDED_SCRATCH) <= 2 * page_bytes(need, 16, 2)
 
 
+def test_weights_are_counted_once():
+    from rllm_b200.models.decoder import DecoderModel
+    m = DecoderModel.__new__(DecoderModel)
+    w = torch.zeros(10, 4)
+    parts = [SimpleNamespace(all=w, second=w[5:], name="x", none=None), SimpleNamespace(same=w, own=torch.zeros(3, dtype=torch.bfloat16))]
+    m.parts = lambda: parts
+    assert m.num_weight_bytes() == 160 + 6
+
+
 def test_a_model_without_pages_needs_none():
     m = fake_model([StateNeed((4,))], [[0]])
     assert engine_core.plan_cache_pages(m, EngineArgs(), 128, torch.device("cpu")) == []
