@@ -6,7 +6,7 @@ from __future__ import annotations
 
 import ctypes
 import os
-from ctypes import c_float, c_int, c_longlong, c_void_p
+from ctypes import c_int, c_longlong, c_void_p
 from typing import Optional
 
 import torch
@@ -235,18 +235,12 @@ def rope_kv_write(qkv: torch.Tensor, positions: torch.Tensor, token_seq: torch.T
                                 max_blocks, kcache, vcache, T, nq, nkv, d, page_size, pages, 1 if write_kv else 0, err)
 
 
-PLAIN_GATE = (float("inf"), 1.0, 0.0)
-_PLAIN_GATE_ARGS = tuple(c_float(v) for v in PLAIN_GATE)
-
-
-def _gate_args(gate):
-    """(limit, slope, shift) of a gated product: g' sigmoid(slope g') (u' + shift), g' = min(g, limit), u' = u kept
-    within +-limit; ``PLAIN_GATE`` is silu(g) u."""
-    return _PLAIN_GATE_ARGS if gate is PLAIN_GATE else tuple(c_float(float(v)) for v in gate)
+# A gate is (limit, slope, shift): g' sigmoid(slope g') (u' + shift), g' = min(g, limit), u' = u kept within +-limit.
+PLAIN_GATE = (float("inf"), 1.0, 0.0)       # silu(g) u
 
 
 def silu_mul(gate_up: torch.Tensor, out: torch.Tensor, gate=PLAIN_GATE) -> None:
-    """out[t, i] = silu(gate_up[t, i]) * gate_up[t, I + i] (``gate``: other constants, see ``_gate_args``)."""
+    """out[t, i] = silu(gate_up[t, i]) * gate_up[t, I + i] (``gate``: see ``PLAIN_GATE``)."""
     T, I = out.shape
     assert gate_up.shape == (T, 2 * I) and gate_up.dtype is out.dtype
     _contig(gate_up, "gate_up"); _contig(out, "out")

@@ -113,6 +113,17 @@ def test_products_in_one_go_are_the_products(M, N, K, f32, silu, monkeypatch):
         call = ops.gemm_small_m if ops.small_m_takes(x, w) else ops.gemm_tcgen05
         call(x, w, want, "silu_mul" if silu else "store", gate=(7.0, 1.5, 0.5) if silu else ops.PLAIN_GATE)
         assert got.dtype is want.dtype and torch.equal(got, want)
+    room = torch.zeros(max(M * K, w.numel()) + 8, device="cuda", dtype=torch.bfloat16)
+    off = lambda t: room[1:1 + t.numel()].view_as(t).copy_(t)  # noqa: E731
+    if M > ops.SMALL_M_MAX:                                # off 16 bytes: TMA does not take it
+        assert not ops.tcgen05_takes(off(x), w, silu=silu) and ops.product(room[1:1 + x.numel()].view_as(x), w, f32, silu) is None
+        assert not ops.tcgen05_takes(x, off(w), silu=silu) and ops.product(x, room[1:1 + w.numel()].view_as(w), f32, silu) is None
+    else:                                                  # the kernel refuses it
+        a = off(x)
+        with pytest.raises(ops.KernelError):
+            ops.product(a, w, f32, silu)
+        with pytest.raises(ops.KernelError):
+            ops.gemm_small_m(a, w, torch.empty(M, N, device="cuda", dtype=torch.bfloat16), "silu_mul" if silu else "store")
     for odd in (x[:, :K - 8], x.float(), x.t(), x.cpu(), x[None]):
         assert ops.product(odd, w, f32, silu) is None
     monkeypatch.setenv("RLLM_GEMM", "library")
@@ -121,3 +132,17 @@ def test_products_in_one_go_are_the_products(M, N, K, f32, silu, monkeypatch):
     assert ops.product(x, w, f32, silu) is not None
     monkeypatch.setenv("RLLM_GEMM", "no_tcgen05")
     assert (ops.product(x, w, f32, silu) is not None) == (M <= ops.SMALL_M_MAX)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,silu", [(128 * 12, 256 * 8, False), (128 * 12 - 127, 256 * 7 + 1, False), (128 * 11, 256 * 8, False), (128 * 95, 256, False),
+                                      (128 * 96, 256, False), (128 * 12, 128 * 8, True), (128 * 12, 128 * 7, True), (8, 65537, False), (8, 65536, False), (9, 65537, False)])
+@pytest.mark.parametrize("head", ["", "library"])
+def test_products_in_one_go_follow_the_rule(M, N, silu, head, monkeypatch):
+    """Both sides of the fewest tiles and of the tallest weight that takes few rows whatever the head's switch says."""
+    monkeypatch.setenv("RLLM_HEAD", head)
+    x = torch.zeros(M, 16, device="cuda", dtype=torch.bfloat16)
+    w = torch.zeros(N * (2 if silu else 1), 16, device="cuda", dtype=torch.bfloat16)
+    ops.gemm_error_word(x.device)
+    takes = (ops.small_m_takes(x, w) or ops.tcgen05_takes(x, w, silu=True)) if silu else ops.gemm_bf16(x, w, torch.bfloat16) is not None
+    assert (ops.product(x, w, silu=silu) is not None) == takes
