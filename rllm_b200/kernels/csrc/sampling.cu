@@ -392,7 +392,7 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
   float* const ys = (float*)(sc_raw + (select ? SC_BINS * 12 + SC_BINS * 8 / gridDim.x : 0));
   __shared__ ArgMax sm_arg[32];
   __shared__ __align__(8) ArgMax range_best;          // read by the other CTAs as one word of 64 bits
-  __shared__ unsigned long long wsum[WARPS], range_sum, slice_sum, sh_cum;
+  __shared__ unsigned long long wsum[WARPS], range_sum, slice_sum, sh_cum, sh_weight;
   __shared__ int sh_pick, sh_bin, cand_n;
   __shared__ unsigned long long sh_rest, all_mass[SC_CAND * SC_CTAS];
   __shared__ unsigned cand[SC_CAND], all_cand[SC_CAND * SC_CTAS], cand_top;
@@ -426,14 +426,14 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
   best = block_argmax(best, sm_arg);
   if (tid == 0) range_best = best;
   sc_barrier();
-  {                                                   // a lane a range: one trip to the others' memory
+  if (cs > 1) {                                       // a lane a range (eight lanes, four times): one trip to the others' memory
     ArgMax b; b.v = -INFINITY; b.i = 0x7fffffff;
-    if (lane < cs) {
-      const unsigned long long u = sc_ld64(&range_best, lane);
+    if ((lane & (SC_CTAS - 1)) < cs) {
+      const unsigned long long u = sc_ld64(&range_best, lane & (SC_CTAS - 1));
       b.v = __uint_as_float((unsigned)u); b.i = (int)(u >> 32);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = SC_CTAS / 2; o > 0; o >>= 1) {
       ArgMax c; c.v = __shfl_xor_sync(0xffffffffu, b.v, o); c.i = __shfl_xor_sync(0xffffffffu, b.i, o);
       b = argmax_better(b, c);
     }
@@ -452,13 +452,14 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
   // of all the weight that takes part.
   auto descend = [&](unsigned floor_key, bool by_mass, unsigned long long target, float p) -> unsigned {
     unsigned prefix = 0, himask = 0;
-    unsigned long long cum = 0;
+    unsigned long long cum = 0, weight = 0;           // what the keys above the prefix weigh, and those of the prefix
     for (int pass = 0; pass < 3; ++pass) {
       const int shift = pass == 0 ? 21 : (pass == 1 ? 10 : 0);
-      if (pass == 2) {
+      if (pass == 2 && weight <= SC_CAND * cs * (by_mass ? fx_mass(key2f(prefix | 0x3ffu), mx) : 1ull)) {
         // The keys that share 22 bits with the threshold are few in a row of unlike values: every range lists its own, and
         // every CTA adds them up for itself (a barrier and a look at a few dozen keys instead of a pass over bins with two
-        // barriers).  A longer list anywhere: the pass.
+        // barriers).  A longer list anywhere: the pass.  (Where they weigh more than the longest lists could, in a row of
+        // like values, nothing is listed: 33 rows of 128,256 equal logits with top-k 47 us, 62 with lists that ran over.)
         if (tid == 0) { cand_n = 0; cand_top = 0u; }
         __syncthreads();
         for (int i = tid; i < n; i += THREADS) {
@@ -581,17 +582,21 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
       unsigned long long before = cum + upto - own;
       for (int w = 0; w < warp; ++w) before += wsum[w];
       upto = before;
+      unsigned long long last = 0;
       for (int q = 0; q < per && first - q >= 0; ++q) {      // the highest bin that reaches the target; else bin 0
-        upto += sc_ld64(&slice[first - q], owner);
+        last = sc_ld64(&slice[first - q], owner);
+        upto += last;
         if (upto >= target) { atomicMin(&sh_bin, tid * per + q); break; }
       }
       __syncthreads();
       if (tid == sh_bin / per) {
         for (int q = 0; q < sh_bin % per; ++q) before += sc_ld64(&slice[first - q], owner);
         sh_cum = before;
+        sh_weight = last;
       }
       __syncthreads();
       cum = sh_cum;
+      weight = sh_weight;
       prefix |= (unsigned)(owner * slice_bins + slice_bins - 1 - sh_bin) << shift;
       himask = 0xffffffffu << shift;
       __syncthreads();
@@ -628,12 +633,11 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
   if (warp == 0) {                                    // a lane a range, then a lane a warp's part
     const unsigned long long mine = lane < cs ? sc_ld64(&range_sum, lane) : 0ull;
     unsigned long long upto = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
+    for (int o = 1; o < cs; o <<= 1) {
       const unsigned long long v = __shfl_up_sync(0xffffffffu, upto, o);
       if (lane >= o) upto += v;
     }
-    const unsigned long long total = __shfl_sync(0xffffffffu, upto, 31);
+    const unsigned long long total = __shfl_sync(0xffffffffu, upto, cs - 1);
     unsigned w[4];
     const unsigned long long seed = seeds[r];
     const unsigned long long ctr = (unsigned long long)gen_index[r];
@@ -650,7 +654,7 @@ sample_cluster_kernel(const float* logits, int V, int ld, const float* temperatu
       const unsigned long long part_sum = lane < WARPS ? wsum[lane] : 0ull;
       unsigned long long run = part_sum;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
+      for (int o = 1; o < WARPS; o <<= 1) {
         const unsigned long long v = __shfl_up_sync(0xffffffffu, run, o);
         if (lane >= o) run += v;
       }

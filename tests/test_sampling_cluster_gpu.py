@@ -31,3 +31,26 @@ def test_clusters_draw_the_tokens_of_one_cta(V, R):
             ops.sample_one_cta(logits, temperature, top_k, top_p, min_p, seeds, gen, one)
             ops.sample(logits, temperature, top_k, top_p, min_p, seeds, gen, many)
             assert one.tolist() == many.tolist()
+
+
+@pytest.mark.parametrize("V,R", [(1500, 2), (5000, 9), (20000, 16), (128256, 2)])
+@pytest.mark.parametrize("like", [1, 63, 65, 130, 511, 513, 1400])
+def test_rows_of_like_values_draw_the_tokens_of_one_cta(V, R, like):
+    """``like`` logits that share 22 bits with the threshold, all in one range or spread over all, equal or not: on both sides
+    of what the ranges' lists hold, of which one alone may run over."""
+    from rllm_b200.kernels import ops
+    g = torch.Generator(device="cuda")
+    g.manual_seed(V + like)
+    for spread in (False, True):
+        for differ in (0, 1):
+            bits = torch.full((like,), 0x40400000, dtype=torch.int32, device="cuda") + differ * torch.randint(0, 1000, (like,), generator=g, device="cuda")
+            logits = torch.randn(R, V, generator=g, device="cuda") - 6
+            at = torch.randperm(V, generator=g, device="cuda")[:like] if spread else (torch.arange(like, device="cuda") + V // 9) % V
+            logits[:, at] = bits.to(torch.int32).view(torch.float32)
+            for k, p in ((max(1, like // 2 + 1), 1.0), (-1, 0.6), (like + 3, 0.9)):
+                args = (torch.ones(R, device="cuda"), torch.full((R,), k, dtype=torch.int32, device="cuda"), torch.full((R,), p, device="cuda"),
+                        torch.zeros(R, device="cuda"), torch.arange(R, device="cuda") * 77, torch.arange(R, device="cuda") + 3)
+                one, many = (torch.full((R,), -1, dtype=torch.int32, device="cuda") for _ in range(2))
+                ops.sample_one_cta(logits, *args, one)
+                ops.sample(logits, *args, many)
+                assert one.tolist() == many.tolist()
