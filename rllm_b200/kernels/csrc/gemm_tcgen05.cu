@@ -178,9 +178,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     // The whole warp walks and one lane issues, with the warp's number and the accumulator's address taken from lane 0:
     // the compiler then knows the instruction's operands to be the same in all lanes, and a product costs the warp half
     // of the 100 cycles that a lane on its own took (tiles of 128 columns, 1,024 x 2,048 x 8,192: 40.5 -> 31.5 us, pairs
-    // 39.1 -> 28.8; of 256 columns unchanged: there a step's 96 KB into and out of shared memory, 80 of a pair's CTA,
-    // set the pace, at 135 to 140 bytes a cycle).  The next stage's barrier is looked at before this stage's products are
-    // issued, so that the answer is there afterwards.
+    // 39.1 -> 28.8; of 256 columns unchanged: a step there brings 48 KB into shared memory and reads them, 40 in a pair's
+    // CTA, 135 to 140 bytes a cycle of both together, whichever of the two sets the pace).  The next stage's barrier is
+    // looked at before this stage's products are issued, so that the answer is there afterwards.
     int s = 0;
     unsigned phase = 0, ti = 0;
     bool ok = true, ready = false;
@@ -499,6 +499,8 @@ static int tg_launch(const void* a, int lda, const void* w, int ldw, int w_rows,
 //   2,047 x 3,072 x 2,048 30.5 / 24.4 / 27.4, 27.9 / 23.7 / 24.4;    700 x 3,072 x 2,048 17.6 / 14.1 / 11.6, 17.3 / 14.7 / 11.8
 //   2,048 x 1,344 x 2,048 17.2 / 13.7 / 17.8, 17.2 / 14.0 / 16.2;    1,024 x 2,048 x 8,192 49 / 40 / 31.5, 42 / 39 / 28.8
 //   6,327 x 3,072 x 2,048 69 / 67 / 76, 61 / 63 / 68
+// (Products of fewer than ops.TCGEN05_MIN_TILES tiles of 128 x 256, as 700 x 3,072 x 2,048 and 1,024 x 2,048 x 8,192, come only
+// from callers that ask for this kernel themselves: linear gives them to the library.)
 // With the gate a tile has half as many output columns.
 // Every column of tiles passes over A once more, from HBM where A is larger than what L2 (126 MB) keeps of it: tiles of 128
 // are left out there unless one or two of them span all columns.  Pairs of 256 / 128 columns, M x N x K (A in MB): 8,192 x 1,344 x

@@ -16,7 +16,9 @@
 // that share a weight panel run side by side and the panel comes from HBM once.
 //
 // What bounds it: 2,048 tokens x top 4 of 32, 2048 -> 1024 -> 2048, is 103 GFLOP and 403 MB of weights, 62 us
-// either way; the two kernels and the sort take 152 us (the mma.sync tiles of moe.cu: 485 us).  200 tokens (800 pairs),
+// either way; the two kernels and the sort take 152 us (the mma.sync tiles of moe.cu: 485 us).  A step of 64 k of a whole tile
+// writes 48 KB into shared memory and its products read 64 KB of it (the pairs for either panel), in 512 cycles of tensor
+// work: some 220 bytes a cycle, where L2 brings 96.  200 tokens (800 pairs),
 // where the weights are the bound: 83 us, 4.9 TB/s, against 141 us; 24 tokens: 76 against 125 us.  The sums' order over
 // k is the tensor core's own in both forms; their results agreed bit for bit wherever they were compared.
 // Every wait on an mbarrier is bounded (bit 16 of the error word), as in gemm_tcgen05.cu.

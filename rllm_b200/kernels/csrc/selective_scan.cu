@@ -124,7 +124,7 @@ causal_conv_run_kernel(const T* x, int stride, const TW* w, const TW* bias, floa
 // CV4_RUN tokens.  Where a run lies in one sequence, which is nearly always, all its inputs are asked for at once.  A
 // channel's four weights come in one load: one value a load, the lanes' 64 bytes apart, the 20 loads of weights and bias
 // were most of the wavefronts of a run of eight tokens.  2,048 x 4,608 (38 MB; 6 us at the copy rate): one channel a
-// thread 33 us, four and eight tokens 28, so 16.6.  The same sums in the same order and the same silu as
+// thread 33 us, four and eight tokens 28, so 16.6 (float32 weights; in a graph 29.0 -> 17.7, bfloat16 weights 24.9 -> 19.0).  The same sums in the same order and the same silu as
 // causal_conv_run_kernel: a decoded token has the same bits whether or not another sequence of the step brings a prompt.
 #define CV4_RUN 16
 __device__ __forceinline__ void cv4_load(const float* p, float (&v)[4]) {
@@ -430,7 +430,8 @@ RLLM_EXPORT int rllm_causal_conv(const void* x, int stride, int dtype, const voi
   const long long total = (long long)T * E;
   // Four channels a thread need work for the GPU and runs within one sequence.  One channel / four, us: 2,048 x 4,608 33 / 16.6,
   // 8,192 x 2,880 101 / 44.5, in portions of 12 tokens 2,040 x 2,880 25 / 22; but 64 x 4,608 6.7 / 6.7, 1,020 x 2,880 in portions
-  // of 12 15.4 / 17.2, 64 x 4,608 in portions of 4 7.2 / 9.3.
+  // of 12 15.4 / 17.2, 64 x 4,608 in portions of 4 7.2 / 9.3.  (Float32 weights.  With bfloat16 weights, in a graph: 2,048 x 4,608
+  // 24.9 / 19.0, 8,192 x 2,880 63 / 55, 8,192 x 4,608 91 / 83.)
   if (any_long && total >= (1ll << 22) && T >= 8ll * num_seqs && taps == 4 && dtype == RLLM_DT_BF16 && E % 4 == 0 && stride % 4 == 0 &&
       (((uintptr_t)x | (uintptr_t)out) & 7) == 0 && (((uintptr_t)w | (uintptr_t)bias) & (w_dtype == RLLM_DT_F32 ? 15 : 7)) == 0 &&
       (T + CV4_RUN - 1) / CV4_RUN <= 65535) {

@@ -434,7 +434,8 @@ def gemm_tcgen05(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, epilogue: 
 
 
 TCGEN05_MIN_TILES = 96    # below this many 128 x 256 output tiles the GPU is not filled: the library's
-                          # small-tile kernels read the weight faster
+                          # small-tile kernels read the weight faster (measured with tiles of 128 x 256 alone; the
+                          # kernel has narrower ones since, and products below the line were not compared again)
 
 
 def tcgen05_takes(x: torch.Tensor, w: torch.Tensor, silu: bool = False) -> bool:

@@ -37,7 +37,7 @@ class SamplingRow:
 class _OptionViews:
     """R rows' options in a pinned buffer and on the device, and the views through which they are written and read: int64
     first (seeds, token indices), then float32 bits (temperature, top_p, min_p) and int32 (top_k), so that one copy takes
-    them.  Kept, since the views of a batch cost the host as much as its launch."""
+    them.  Kept, since the views of a batch cost the host as much as its launch (a batch size's first four calls make them)."""
 
     def __init__(self, pinned: torch.Tensor, copied: torch.cuda.Event, device: torch.Tensor, R: int):
         host = pinned.numpy()
