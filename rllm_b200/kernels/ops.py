@@ -144,6 +144,8 @@ class _Entries:
     first call)."""
 
     def __getattr__(self, symbol: str):
+        if symbol not in _TABLE:
+            raise AttributeError(f"no entry point {symbol}")
         library, signature, what = _TABLE[symbol]
 
         def find() -> int:

@@ -1,5 +1,6 @@
 """The way from Python to the kernels' entry points (native/csrc/launch.cc): every signature against the sources, what an
 argument becomes, what a refusal raises, and the products that are checked, allocated and launched in one go."""
+import copy
 import ctypes
 import glob
 import os
@@ -52,6 +53,10 @@ def test_what_is_refused_before_anything_is_called():
     with pytest.raises(ValueError, match="no signature"):
         ops._launch().entry("pxp", lambda: 0, "odd")
     assert ops.product(x, x) is None and ops.product(x.bfloat16(), x.bfloat16()) is None
+
+
+def test_a_name_that_is_no_entry_point_is_no_attribute():
+    assert not hasattr(ops._entries, "rllm_no_such_kernel") and copy.copy(ops._entries) is not ops._entries
 
 
 def test_what_the_tensor_library_throws_is_an_exception():
